@@ -413,17 +413,18 @@ int quic_graph_destroy(void *graph);
 
 /* ------------------------------------------------------------------------
  * The decode token loop as one persistent kernel (1..quic_persist_max_rows()
- * batch rows, contexts up to 16 x 256 tokens).  Opt-in: on B200 it measures
- * slower than quic_decode_step's kernel chain (587 vs 352 us per token).
+ * batch rows, packed or fp16 weights).  On B200 it is the faster form from two
+ * rows on and for fp16 weights (445 against 667 us per step at 8 rows of 1000
+ * tokens, 348 against 494 us at one fp16 row), and equal at one packed row.
  *
  * Replaces the same reference code as quic_decode_step, for `steps` consecutive
  * greedy tokens in ONE launch: Engine.step + QUICForCausalLM.forward with
  * seq_len == 1 (src/engine.py:78-107, src/model.py:211-224, 272-303).  148
  * resident CTAs walk layers and tokens; a layer phase hands its result to the
- * next through 8-byte {payload, tag} words in `sync`, and the weights stream
- * from a per-CTA copy of the W4 matrices ("W4S", built once by
- * quic_persist_pack from the W4T matrices of quic_model_t) into a
- * shared-memory ring.  Arithmetic and rounding points are those of
+ * next through 16-byte words in `sync` that are empty (zero) until their data is
+ * there, and the weights stream from a copy of the layer matrices in mma
+ * fragment order ("W4S", built once by quic_persist_pack) into a shared-memory
+ * ring.  Arithmetic and rounding points are those of
  * quic_decode_step.  The kernel is launched cooperatively: it needs a GPU with
  * at least 148 SMs on which all its CTAs can be resident, and it occupies the
  * whole GPU until the burst ends (work on other streams waits).
@@ -432,23 +433,25 @@ int quic_graph_destroy(void *graph);
  *    filled by quic_persist_pack (replaces, like quic_w4_prepack, the repack of
  *    src/quant/marlin.py:105-125).
  *  - `sync`: quic_persist_sync_bytes() bytes, 256-byte aligned, zeroed once by
- *    the caller; one area serves every launch on a stream, launches that can
- *    overlap on the GPU need an area each.
+ *    the caller.  Launches of one process on one device follow one another
+ *    whatever their streams are; processes need areas of their own.
  *  - quic_decode_t: `scratch` is not used; `attn_splits` 0 lets the library
  *    choose from `ctx_hint` (an upper bound of pos + steps over the rows);
  *    `logits` only with steps == 1.
  *  - Every wait inside the kernel is bounded.  If one gives up the kernel ends
  *    early, the tokens of that launch are invalid and the status word of `sync`
- *    is non-zero: quic_decode_persist_status() returns and clears it (it
- *    synchronises the stream), quic_decode_persist_run_host() checks it itself
- *    and returns QUIC_E_TIMEOUT.  No reference counterpart (its kernels have no
+ *    is non-zero; later launches on the area return at once until it is taken:
+ *    quic_decode_persist_status() returns it and clears the area (it synchronises
+ *    the stream), quic_decode_persist_run_host() does so itself and returns
+ *    QUIC_E_TIMEOUT.  No reference counterpart (its kernels have no
  *    bounded waits, kernels/cuda/marlin.cu:1467-1476).
  * ---------------------------------------------------------------------- */
 int32_t quic_persist_max_rows(void);
 int64_t quic_persist_stream_bytes(int32_t n_layers);
+int64_t quic_persist_stream_bytes_f16(int32_t n_layers); /* of an un-quantised model */
 int64_t quic_persist_sync_bytes(void);
 /* Attention splits per (row, kv head) for contexts up to `ctx`; more than 16
- * means the context is too long for this kernel (use quic_decode_step). */
+ * means that this kernel is no choice for the batch (use quic_decode_step). */
 int32_t quic_persist_pick_splits(int32_t batch, int32_t ctx);
 int quic_persist_pack(const quic_model_t *m, void *wstream_out, void *stream);
 int quic_decode_persist(const quic_model_t *m, const quic_decode_t *d,

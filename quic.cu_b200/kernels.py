@@ -164,6 +164,7 @@ SIGNATURES = {
     "quic_graph_destroy": (C.c_int, [_P]),
     "quic_persist_max_rows": (_I32, []),
     "quic_persist_stream_bytes": (_I64, [_I32]),
+    "quic_persist_stream_bytes_f16": (_I64, [_I32]),
     "quic_persist_sync_bytes": (_I64, []),
     "quic_persist_pick_splits": (_I32, [_I32, _I32]),
     "quic_persist_pack": (C.c_int, [C.POINTER(Model), _P, _P]),

@@ -29,10 +29,9 @@ from . import kernels as K
 from .checkpoint import LAYER_LINEARS, detect_group_size, packed_prefixes
 
 DTYPE = torch.float16
-# QUIC_PERSIST=1 (or model.use_persist = True) decodes batches of up to quic_persist_max_rows()
-# rows in the persistent kernel: one launch per burst of tokens.  Off by default: measured at
-# 587 us per token against 352 us for the kernel chain (24 layers, one row).
-PERSIST = os.environ.get("QUIC_PERSIST", "0") == "1"
+# Which decode batches run in the persistent kernel (one launch per burst of tokens): None = those it
+# is faster for (_persist_pays), True = all it can take, False = none (the kernel chain).
+PERSIST = {"0": False, "1": True}.get(os.environ.get("QUIC_PERSIST", ""))
 HIDDEN, HEADS, KV_HEADS, HEAD_DIM, INTER, QKV_N = K.HIDDEN, K.HEADS, K.KV_HEADS, K.HEAD_DIM, K.INTER, K.QKV_N
 
 
@@ -67,7 +66,7 @@ class SlotCache:
         self._scratch: dict[tuple, torch.Tensor] = {}
         self._graphs: dict[tuple, int] = {}
         self.max_graphs = 512                      # captured graphs kept; beyond that all are dropped and rebuilt
-        self._plans: dict[tuple, tuple] = {}       # decode(): per (rows, steps) launch plan
+        self._plans: dict[tuple, _DecodePlan] = {}  # decode(): per (rows, steps) launch plan
         self._rows_loaded: dict[int, torch.Tensor] = {}  # row->slot map now on the device, per batch size
         self.host_steps = 0                        # host mirror of step_counter
 
@@ -147,6 +146,27 @@ def _ctx_bucket(n: int, batch: int = 1) -> int:
     while b < n:
         b *= 2
     return b
+
+
+class _DecodePlan:
+    """What decode() keeps between calls for the same rows (see there)."""
+
+    __slots__ = ("bound", "rows", "tok", "out", "host", "host_np", "handle", "persist", "status", "feed", "feed_ptr")
+
+    def __init__(self):
+        self.feed = None
+
+
+def _persist_pays(dense: bool, batch: int, ctx: int) -> bool:
+    """Where the persistent kernel beats the kernel chain, from B200 measurements (us per step,
+    persistent / chain).  One packed row: 342 / 347 while the context is one attention split (768
+    tokens), 413 / 353 beyond.  Two rows: 373 / 462 at 512 tokens, 455 / 465 at 2100, 538 / 689 at
+    7000.  3..16 rows: 402 / 570 (3 x 300), 498 / 618 (4 x 1000), 445 / 667 (8 x 1000), 500 / 704
+    (16 x 300), 660 / 784 (16 x 2000), equal at 3000-4000 tokens.  fp16 weights: 348 / 494 at one
+    row, 420 / 497 at 2100 tokens, 416 / 899 at eight rows."""
+    if batch == 1:
+        return ctx <= (4096 if dense else 768)
+    return ctx <= (8192 if batch == 2 else 4096 if dense else 2048)
 
 
 class QUICForCausalLM:
@@ -327,10 +347,11 @@ class QUICForCausalLM:
 
     # ---- persistent decode kernel ------------------------------------------------------
     def persist_stream(self) -> torch.Tensor:
-        """The per-CTA weight stream of the persistent kernel, packed on first use from the
-        W4T matrices (a second copy of the layer weights, ~10 MB per layer)."""
+        """The weight stream of the persistent kernel, packed on first use from the device
+        matrices (a second copy of the layer weights, 9 MB per layer, 32 MB in fp16)."""
         if self._wstream is None:
-            need = K.lib().quic_persist_stream_bytes(self.n_layers)
+            lib = K.lib()
+            need = (lib.quic_persist_stream_bytes_f16 if self.dense else lib.quic_persist_stream_bytes)(self.n_layers)
             if need <= 0:
                 raise RuntimeError("persistent decode: unsupported layer count")
             t = torch.empty(need, dtype=torch.uint8, device=self.device)
@@ -340,8 +361,10 @@ class QUICForCausalLM:
 
     def persist_ok(self, batch: int, ctx: int) -> bool:
         """Whether ``batch`` rows with contexts up to ``ctx`` tokens run in the persistent kernel."""
+        if self.use_persist is False or (self.use_persist is None and not _persist_pays(self.dense, batch, ctx)):
+            return False
         lib = K.lib()
-        return (self.use_persist and not self.dense and batch <= lib.quic_persist_max_rows() and self.vocab >= 296
+        return (batch <= lib.quic_persist_max_rows() and self.vocab >= 296
                 and lib.quic_persist_stream_bytes(self.n_layers) > 0
                 and lib.quic_persist_pick_splits(batch, ctx) <= 16)
 
@@ -368,7 +391,7 @@ class QUICForCausalLM:
         if longest + steps > cache.s_max or longest + steps > self.max_pos:
             raise RuntimeError("decode: context would exceed the KV slot length")
         ctx = min(_ctx_bucket(longest + steps, len(slots)), cache.s_max)
-        if self.persist_ok(len(slots), ctx):
+        if (logits is None or steps == 1) and self.persist_ok(len(slots), ctx):  # (it keeps one step's logits)
             g, rows = self._decode_struct(cache, len(slots), ctx, logits, persist=True)
         else:
             g, rows = self._graph(cache, len(slots), ctx, steps, logits)
@@ -414,60 +437,58 @@ class QUICForCausalLM:
         row consumes first; ``slots`` must then be consecutive) travels host -> device, the
         captured steps run, the generated ids travel device -> host into a page-locked
         buffer, and the call returns when they have arrived."""
-        n_in = 0
-        if feed is not None:
-            if feed.dtype != torch.int32 or feed.numel() != len(slots) or feed.is_cuda:
-                raise ValueError("decode: feed must be a host int32 tensor with one token per row")
-            n_in = len(slots)
         # A plan keeps everything that stays the same between calls for the same rows while
-        # the context stays inside the captured graph's bound.
+        # the context stays inside the bound the launch was made for.
         key = (tuple(slots), steps)
         plan = cache._plans.get(key)
-        first = cache.host_steps % cache.ring
-        host_len = cache.host_len
-        if (plan is not None and first + steps <= cache.ring
-                and max(host_len[s] for s in slots) + steps <= plan[1]
-                and cache._rows_loaded.get(len(slots)) is plan[2]):
-            g = plan[0]
+        host_len, ring = cache.host_len, cache.ring
+        n_in = 0
+        if feed is not None:
+            n_in = len(slots)
+            if plan is None or plan.feed is not feed:
+                if feed.dtype != torch.int32 or feed.numel() != n_in or feed.is_cuda:
+                    raise ValueError("decode: feed must be a host int32 tensor with one token per row")
+                if any(b - a != 1 for a, b in zip(slots, slots[1:])):
+                    raise ValueError("decode: feed needs consecutive slots")
+        first = cache.host_steps % ring
+        longest = (host_len[slots[0]] if len(slots) == 1 else max(host_len[s] for s in slots)) if plan is not None else 0
+        if plan is not None and longest + steps <= plan.bound and cache._rows_loaded.get(len(slots)) is plan.rows:
             cache.host_steps += steps
             for s in slots:
                 host_len[s] += steps
         else:
-            if n_in and any(b - a != 1 for a, b in zip(slots, slots[1:])):
-                raise ValueError("decode: feed needs consecutive slots")
-            g, first = self._prepare_decode(cache, slots, steps, None)
+            handle, first = self._prepare_decode(cache, slots, steps, None)
             longest = max(host_len[s] for s in slots)  # already advanced by `steps`
-            bound = min(_ctx_bucket(longest, len(slots)), cache.s_max, self.max_pos)
-            host = cache.host_out()
-            plan = (g, bound, cache.rows_tensor(slots), cache.tok.data_ptr() + 4 * slots[0],
-                    cache.out_tokens.data_ptr(), host.data_ptr(), host.numpy())
+            plan = _DecodePlan()
+            plan.bound = min(_ctx_bucket(longest, len(slots)), cache.s_max, self.max_pos)
+            plan.rows = cache.rows_tensor(slots)
+            plan.tok = cache.tok.data_ptr() + 4 * slots[0]
+            plan.out, plan.host, plan.host_np = cache.out_tokens.data_ptr(), cache.host_out().data_ptr(), cache.host_out().numpy()
+            plan.handle, plan.persist = handle, None
+            if isinstance(handle, K.Decode):
+                plan.persist = (C.byref(self._c_model), C.byref(handle), K.ptr(self.persist_stream()),
+                                K.ptr(cache.persist_sync()), steps)
+                plan.status = cache._persist_status.data_ptr()
             if len(cache._plans) > 64:
                 cache._plans.clear()
             cache._plans[key] = plan
-            if first + steps > cache.ring:  # the block of rows wraps around the ring
-                if n_in:
-                    cache.tok[slots[0]: slots[0] + n_in].copy_(feed, non_blocking=True)
-                self._launch(cache, g, steps)
-                idx = (torch.arange(steps, device=self.device) + first) % cache.ring
-                toks = cache.out_tokens.index_select(0, idx).index_select(1, cache.rows_tensor(slots).long())
-                return toks.t().cpu().tolist()
-        n = cache.n_slots
-        offset = 4 * first * n
-        if isinstance(g, K.Decode):
-            sync = cache.persist_sync()
-            rc = K.lib().quic_decode_persist_run_host(
-                C.byref(self._c_model), C.byref(g), K.ptr(self.persist_stream()), K.ptr(sync), steps, K.stream_ptr(),
-                feed.data_ptr() if n_in else None, plan[3], n_in, plan[4] + offset, plan[5] + offset, steps * n,
-                cache._persist_status.data_ptr())
+        plan.feed = feed
+        plan.feed_ptr = feed.data_ptr() if n_in else None
+        # the block of generated rows, or the whole ring where the block wraps around its end
+        n, wraps = cache.n_slots, first + steps > ring
+        offset, count = (0, ring * n) if wraps else (4 * first * n, steps * n)
+        if plan.persist is not None:
+            rc = K.lib().quic_decode_persist_run_host(*plan.persist, K.stream_ptr(), plan.feed_ptr, plan.tok, n_in,
+                                                      plan.out + offset, plan.host + offset, count, plan.status)
         else:
-            rc = K.lib().quic_graph_run_host(g, K.stream_ptr(), feed.data_ptr() if n_in else None, plan[3], n_in,
-                                             plan[4] + offset, plan[5] + offset, steps * n)
+            rc = K.lib().quic_graph_run_host(plan.handle, K.stream_ptr(), plan.feed_ptr, plan.tok, n_in,
+                                             plan.out + offset, plan.host + offset, count)
         if rc != 0:
             K.check(rc, "decode run_host")
-        host_np = plan[6]
         if steps == 1 and len(slots) == 1:
-            return [[int(host_np[first, slots[0]])]]
-        return host_np[first: first + steps][:, slots].T.tolist()
+            return [[int(plan.host_np[first, slots[0]])]]
+        rows = [(first + j) % ring for j in range(steps)] if wraps else slice(first, first + steps)
+        return plan.host_np[rows][:, slots].T.tolist()
 
     # ---- prefill -----------------------------------------------------------------
     @torch.inference_mode()
