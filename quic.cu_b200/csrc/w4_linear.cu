@@ -259,13 +259,20 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
   QUIC_REQUIRE(mchunks <= 65535, QUIC_E_SHAPE, "w4a16_linear: too many rows");
   const size_t smem = (size_t)M * gps * kGroup * 2 + (size_t)nwarp * M * 32 * 4;
   dim3 grid(w->n / 32, splits, mchunks);
+  if (smem > (48 << 10)) {  // (48 KB need no permission; given once per device and size)
+    static size_t allowed[64][2] = {};
+    int dev = 0;
+    QUIC_CUDA(cudaGetDevice(&dev));
+    size_t* have = &allowed[dev & 63][M == 1 ? 0 : 1];
+    if (dev > 63 || smem > *have) {
+      QUIC_CUDA(M == 1 ? cudaFuncSetAttribute(w4_gemv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                       : cudaFuncSetAttribute(w4_gemv_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      *have = smem;
+    }
+  }
   if (M == 1) {
-    QUIC_CUDA(cudaFuncSetAttribute(w4_gemv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
     w4_gemv_kernel<1><<<grid, nwarp * 32, smem, st>>>((const half*)x, *w, (half*)y, part, m, gps);
   } else {
-    QUIC_CUDA(cudaFuncSetAttribute(w4_gemv_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
     w4_gemv_kernel<8><<<grid, nwarp * 32, smem, st>>>((const half*)x, *w, (half*)y, part, m, gps);
   }
   QUIC_CUDA(cudaGetLastError());

@@ -207,6 +207,13 @@ def stream_ptr() -> int:
         return torch.cuda.current_stream().cuda_stream
 
 
+try:
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+except AttributeError:
+    def _raw_stream(device: int) -> int:
+        return torch.cuda.current_stream(device).cuda_stream
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
@@ -240,7 +247,7 @@ class W4Weight:
         self.sc = torch.empty(k // GROUP, n, dtype=torch.float16, device=device)
         self.zp = torch.empty(k // GROUP, n // 2, dtype=torch.uint8, device=device)
         self.bias = bias
-        self._workspace: torch.Tensor | None = None
+        self._launch: tuple | None = None
 
     def put(self, packed: torch.Tensor, scale: torch.Tensor, zero_point: torch.Tensor,
             row_offset: int = 0, row_order: int = ROWS_NATURAL) -> None:
@@ -268,7 +275,7 @@ class W4Weight:
 
     def workspace(self, m: int) -> torch.Tensor:
         """Split-K workspace, shared by every weight on the device (calls on one stream are ordered)."""
-        need = lib().quic_w4a16_workspace_bytes(m, self.size_n, self.size_k)
+        need = _linear_workspace_bytes(m, self.size_n, self.size_k)
         key = self.qw.device.index
         ws = _linear_workspace.get(key)
         if ws is None or ws.numel() * 4 < need:
@@ -293,6 +300,7 @@ class F16Weight:
         self.size_n, self.size_k = n, k
         self.w = torch.empty(n, k, dtype=torch.float16, device=device)
         self.bias = bias
+        self._launch: tuple | None = None
 
     def put(self, weight: torch.Tensor, row_offset: int = 0, row_order: int = ROWS_NATURAL) -> None:
         """Places one checkpoint layer [N_layer, K] at rows [row_offset, row_offset + N_layer)."""
@@ -318,6 +326,22 @@ class F16Weight:
         return self.w.numel() * 2
 
 
+def _launch_ref(w):
+    """``byref`` of the weight's C struct, kept while its tensors stay where they are."""
+    tensors = (w.qw, w.sc, w.zp, w.bias) if isinstance(w, W4Weight) else (w.w, w.bias)
+    where = [None if t is None else t.data_ptr() for t in tensors]
+    kept = w._launch
+    if kept is None or kept[0] != where:
+        struct = w.struct()
+        kept = w._launch = (where, struct, C.byref(struct))
+    return kept[2]
+
+
+@functools.lru_cache(maxsize=4096)
+def _linear_workspace_bytes(m: int, n: int, k: int) -> int:
+    return lib().quic_w4a16_workspace_bytes(m, n, k)
+
+
 _linear_workspace: dict = {}
 MAX_LINEAR_ROWS = 8192  # rows per launch; longer inputs are processed in chunks to bound scratch memory
 
@@ -327,17 +351,22 @@ def w4a16_linear(w, x: torch.Tensor, use_tensor: bool | None = None) -> torch.Te
     F16Weight the dense linear of the un-quantised model (_linear, src/model.py:35-41)."""
     _need_cuda(x)
     _need_half(x)
-    x2 = x.contiguous().reshape(-1, w.size_k)
+    plain = x.dim() == 2 and x.shape[1] == w.size_k
+    x2 = x.contiguous() if plain else x.contiguous().reshape(-1, w.size_k)
     m = x2.shape[0]
-    y = torch.empty(m, w.size_n, dtype=torch.float16, device=x.device)
+    y = x2.new_empty((m, w.size_n))
     if use_tensor is None:
         use_tensor = TENSOR_PATH and m >= TENSOR_MIN_ROWS
-    s = w.struct()
-    for r0 in range(0, m, MAX_LINEAR_ROWS):
-        rows = min(MAX_LINEAR_ROWS, m - r0)
-        check(lib().quic_w4a16_linear(ptr(x2[r0:r0 + rows]), C.byref(s), ptr(y[r0:r0 + rows]), rows,
-                                      int(bool(use_tensor)), ptr(w.workspace(rows)), stream_ptr()), "w4a16_linear")
-    return y.reshape(*x.shape[:-1], w.size_n)
+    ref, run, stream = _launch_ref(w), lib().quic_w4a16_linear, _raw_stream(x2.get_device())
+    xp, yp, done = x2.data_ptr(), y.data_ptr(), 0
+    while done < m:
+        rows = min(MAX_LINEAR_ROWS, m - done)
+        rc = run(xp + 2 * done * w.size_k, ref, yp + 2 * done * w.size_n, rows, 1 if use_tensor else 0,
+                 ptr(w.workspace(rows)), stream)
+        if rc != 0:
+            check(rc, "w4a16_linear")
+        done += rows
+    return y if plain else y.reshape(*x.shape[:-1], w.size_n)
 
 
 # ---------------------------------------------------------------------------------
@@ -543,6 +572,13 @@ def _gemm_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = 
     return y.reshape(*x.shape[:-1], n)
 
 
+@functools.lru_cache(maxsize=4096)
+def _attn_plan(b: int, s: int, splits: int) -> tuple[int, int]:
+    """(splits, scratch bytes) of a decode attention; ``splits`` 0 = the library's choice."""
+    splits = splits if splits > 0 else lib().quic_attn_pick_splits(b, s)
+    return splits, (lib().quic_attn_scratch_bytes(b, splits) if splits > 1 else 0)
+
+
 _attn_scratch: dict = {}
 _lm_scratch: dict = {}
 
@@ -587,7 +623,7 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
                                      pad_lens.shape[0] == b and pad_lens.is_contiguous()):
         raise RuntimeError("flash_attn_decode: pad_lens must be a contiguous CUDA int32 tensor of shape [B]")
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    out = torch.empty(b, nh, 1, HEAD_DIM, dtype=torch.float16, device=q.device)
+    out = q.new_empty((b, nh, 1, HEAD_DIM))
     if s == 0:
         return out.zero_()
     scale = float(softmax_scale) if softmax_scale and softmax_scale > 0 else HEAD_DIM ** -0.5
@@ -596,20 +632,21 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
                                          ptr(pad_lens), None, s, scale, ptr(out), b, stream_ptr()),
               "attn_decode_cta")
         return out
-    asked = splits
-    if splits <= 0:  # the library chooses (the same count, or its streamed kernel, which needs no scratch)
-        splits = lib().quic_attn_pick_splits(b, s)
+    # with splits 0 the library chooses (at most as many as the scratch is sized for, or a kernel without)
+    asked, (splits, need) = splits, _attn_plan(b, s, splits)
+    device = q.get_device()
+    stream = _raw_stream(device)
     scratch = None
-    if splits > 1:
-        need = lib().quic_attn_scratch_bytes(b, splits)
-        key = (q.device.index, torch.cuda.current_stream().cuda_stream)
-        scratch = _attn_scratch.get(key)
+    if need > 0:
+        scratch = _attn_scratch.get((device, stream))
         if scratch is None or scratch.numel() < need:
             scratch = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=q.device)
-            _attn_scratch[key] = scratch
-    check(lib().quic_attn_decode(ptr(q), ptr(k), ptr(v), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
-                                 ptr(pad_lens), None, s, scale, ptr(out), b, splits if asked > 0 else 0, ptr(scratch),
-                                 stream_ptr()), "attn_decode")
+            _attn_scratch[(device, stream)] = scratch
+    rc = lib().quic_attn_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
+                                ptr(pad_lens), None, s, scale, out.data_ptr(), b, splits if asked > 0 else 0,
+                                ptr(scratch), stream)
+    if rc != 0:
+        check(rc, "attn_decode")
     return out
 
 
