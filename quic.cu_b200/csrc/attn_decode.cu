@@ -658,12 +658,12 @@ extern "C" int quic_attn_decode(const void* q, const void* k, const void* v, int
   QUIC_REQUIRE(((uintptr_t)k % 16 == 0) && ((uintptr_t)v % 16 == 0) && stride_b % 8 == 0 &&
                    stride_h % 8 == 0,
                QUIC_E_ARG, "attn_decode: K/V must be 16-byte aligned with strides multiple of 8");
-  // Left to choose (splits <= 0), 21..128 rows of up to 8192 tokens over contiguous
-  // [b][2][s_max][64] planes take the streamed kernel of the decode step (one CTA per (row, KV
-  // head), no scratch), where it was measured ahead of the split kernels (64 x 8192: 49 us against
-  // 57; at 64 x 32768 the split kernel's 167 us stay ahead of 189).
-  if (splits <= 0 && b >= 21 && b <= 128 && s_max <= 8192 && stride_h == (int64_t)s_max * kHeadDim &&
-      stride_b == (int64_t)kKvHeads * s_max * kHeadDim && tc_status_words() != nullptr) {
+  // Left to choose (splits <= 0): the flow kernel, over any planes that a tensor map can describe.  The
+  // split kernels keep caches of up to 256 tokens with more rows than SMs: their tiles are fewer than a
+  // CTA's six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).
+  const int64_t widest = int64_t(1) << 38;
+  if (splits <= 0 && !(s_max <= 256 && b > 148) && stride_b > 0 && stride_h > 0 && stride_b < widest &&
+      stride_h < widest && tc_status_words() != nullptr) {
     AttnArgs a = {};
     a.q = (const half*)q;
     a.k = (const half*)k;
@@ -673,11 +673,10 @@ extern "C" int quic_attn_decode(const void* q, const void* k, const void* v, int
     a.start = start;
     a.end = end;
     a.s_cap = s_max;
-    a.splits = 1;
-    a.chunk = s_max;
+    a.splits = attn_flow_splits(b, s_max);
     a.scale = scale > 0.f ? scale : 0.125f;
     a.out = (half*)out;
-    return launch_attn_stream(a, nullptr, b, b, s_max, tc_status_words(), (cudaStream_t)stream, false);
+    return launch_attn_flow(a, b, tc_status_words(), (cudaStream_t)stream);
   }
   if (splits <= 0) splits = quic_attn_pick_splits(b, s_max);
   QUIC_REQUIRE(splits <= 4096, QUIC_E_SHAPE, "attn_decode: too many splits");

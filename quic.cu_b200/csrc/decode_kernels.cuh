@@ -118,6 +118,9 @@ struct QkvFinish {
   const half* sin_t;
   int32_t max_pos;
 };
+// Stand-alone op: (row, KV head) ranges in up to eight splits, a TMA stage per warp (attn_decode_flow.cu).
+int attn_flow_splits(int b, int s_max);
+int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t stream);
 int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int n_slots, int s_max, int* status,
                        cudaStream_t stream, bool pdl);
 
@@ -200,7 +203,8 @@ cudaError_t launch_swiglu_fused(const half* gu, half* act, int batch, cudaStream
 // prefill pieces, chainable with programmatic dependent launch
 cudaError_t launch_qkv_rope_append(const half* qkv, const int32_t* slots, const int32_t* positions, const half* cos_t,
                                    const half* sin_t, int max_pos, half* q_out, half* kcache, half* vcache, int s_max,
-                                   int n_slots, int rows, cudaStream_t st, bool pdl);
+                                   int n_slots, int rows, cudaStream_t st, bool pdl, const float* part = nullptr,
+                                   int splits = 0, const half* bias = nullptr);
 // tcgen05 + TMA form for prompts of 128 tokens and more (attn_prefill_tc.cu)
 bool attn_prefill_tc_supported(int n_seq, int max_len, int rows, int s_max, int n_slots);
 int attn_prefill_tc_launch(const void* q, const void* kcache, const void* vcache, const int32_t* seq_start,
