@@ -364,12 +364,12 @@ int enqueue_step_rows16(const quic_model_t* m, const quic_decode_t* d, cudaStrea
   la.n_slots = d->n_slots;
   la.ring = d->ring > 0 ? d->ring : 1;
   la.step_counter = d->step_counter;
-  if (B > 4 && lm_head_tc_supported(B, m->vocab)) {
+  if (B > 2 && lm_head_tc_supported(B, m->vocab)) {
     QUIC_CUDA(launch_rmsnorm(xa, nullptr, (const half*)m->final_norm, m->eps, xn, nullptr, B, st));
     la.x_normed = xn;
     return launch_lm_head_tc(la, st);
   }
-  // up to four rows: the GEMV form, final norm fused, one launch
+  // up to two rows (from three the tensor kernel is ahead, 77 -> 50 us): the GEMV form, final norm fused, one launch
   la.ln = (const half*)m->final_norm;
   la.xres_in = xa;
   QUIC_CUDA(launch_lm_head(la, lm_head_grid(m->vocab), st, true));
@@ -694,7 +694,7 @@ extern "C" int32_t quic_decode_launch_count(const quic_model_t* m, const quic_de
     if (ctx > d->s_max) ctx = d->s_max;
     return (attention_streams(d->batch, ctx) ? 7 : 8) * m->n_layers + 3;  // the streamed attention finishes the QKV linear
   }
-  if (d && d->batch >= g_mma_chain_min_batch) return 5 * m->n_layers + ((d->batch > 4 && lm_head_tc_supported(d->batch, m->vocab)) ? 2 : 1);
+  if (d && d->batch >= g_mma_chain_min_batch) return 5 * m->n_layers + ((d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab)) ? 2 : 1);
   return 5 * m->n_layers + 1;
 }
 
@@ -736,7 +736,7 @@ extern "C" int quic_decode_graph_create(const quic_model_t* m, const quic_decode
   const bool dense = m->layers[0].qkv.w16 != nullptr;
   g->tensor_kernels = dense ? d->batch > kF16ChainMaxRows
                             : (d->batch >= g_tensor_min_batch ||
-                               (d->batch >= g_mma_chain_min_batch && d->batch > 4 && lm_head_tc_supported(d->batch, m->vocab)));
+                               (d->batch >= g_mma_chain_min_batch && d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab)));
   *graph_out = g;
   return QUIC_OK;
 }

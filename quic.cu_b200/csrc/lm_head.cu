@@ -332,6 +332,38 @@ extern "C" int quic_lm_head_argmax(const void* x, const void* norm_w, float eps,
   const int grid = lm_head_grid(vocab);
   const int64_t per = ((int64_t)b * grid * 4 + 255) / 256 * 256;
   char* base = static_cast<char*>(scratch);
+  // Two finished rows and more: the tensor kernel, which reads the table once per 128 rows where the
+  // GEMV reads it once per eight and is bound by its fp32 products even then (151936 words, us:
+  // 2 rows 47 -> 50, 3 rows 77 -> 50, 8 rows 126 -> 51, 16 rows 242 -> 50, 128 rows 1836 -> 74; two
+  // rows take it too, so that a row's bits do not depend on how many are beside it).  Its counter
+  // and its rows' maxima (zero between calls) stand in the 256 bytes that start zeroed; more than 31 rows'
+  // maxima lie behind them and are cleared here.
+  if (norm_w == nullptr && b >= 2 && lm_head_tc_supported(2, vocab) && (uintptr_t)x % 16 == 0) {
+    constexpr int kChunk = 128, kHeadRows = 31;
+    for (int r0 = 0; r0 < b; r0 += kChunk) {
+      LmHeadArgs a = {};
+      a.embed = (const half*)embed;
+      a.x_normed = (const half*)x + (size_t)r0 * kHidden;
+      a.batch = b - r0 < kChunk ? b - r0 : kChunk;
+      a.vocab = vocab;
+      a.logits = logits != nullptr ? (half*)logits + (size_t)r0 * vocab : nullptr;
+      a.counter = reinterpret_cast<int32_t*>(base);
+      a.keys = reinterpret_cast<unsigned long long*>(base + 8);
+      a.argmax_out = out != nullptr ? out + r0 : nullptr;
+      a.ring = 1;
+      if (a.batch > kHeadRows)
+        QUIC_CUDA(cudaMemsetAsync(base + 256, 0, (size_t)(a.batch - kHeadRows) * 8, (cudaStream_t)stream));
+      if (a.batch == 1) {  // (the last row of a longer batch)
+        a.best_val = reinterpret_cast<float*>(base + 256);
+        a.best_idx = reinterpret_cast<int32_t*>(base + 256 + per);
+        QUIC_CUDA(launch_lm_head(a, grid, (cudaStream_t)stream, false));
+        continue;
+      }
+      const int rc = launch_lm_head_tc(a, (cudaStream_t)stream);
+      if (rc != QUIC_OK) return rc;
+    }
+    return QUIC_OK;
+  }
   LmHeadArgs a = {};
   a.embed = (const half*)embed;
   a.batch = b;
