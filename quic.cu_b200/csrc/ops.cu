@@ -302,7 +302,8 @@ __global__ void qkv_post_kernel(const half* __restrict__ qkv, const float* __res
 __global__ void __launch_bounds__(256) qkv_rope_rows_kernel(
     const half* __restrict__ qkv, const int32_t* __restrict__ slots, const int32_t* __restrict__ row_pos,
     const half* __restrict__ cos_t, const half* __restrict__ sin_t, int max_pos, half* __restrict__ qbuf,
-    half* __restrict__ kcache, half* __restrict__ vcache, int s_max, int rows, int n_slots) {
+    half* __restrict__ kcache, half* __restrict__ vcache, int s_max, int rows, int n_slots,
+    const float* __restrict__ part, int splits, const half* __restrict__ bias) {
   constexpr int kPerRow = (kHeads + 2 * kKvHeads) * 8;  // 144 threads per row
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
@@ -313,8 +314,39 @@ __global__ void __launch_bounds__(256) qkv_rope_rows_kernel(
   const int pair0 = (piece & 3) * 8;            // their pairs: dims d and d + 32 are stored side by side
   const bool high = piece >= 4;                 // dims 32..63: the second element of the rotated pair
   const int slot = slots[b], p = row_pos[b];
-  const half2* src = reinterpret_cast<const half2*>(qkv + (size_t)b * kQkvN + head * kHeadDim) + pair0;
-  const uint4 in0 = *reinterpret_cast<const uint4*>(src), in1 = *reinterpret_cast<const uint4*>(src + 4);
+  const size_t col = (size_t)head * kHeadDim + 2 * pair0;
+  uint4 in0, in1;
+  if (part != nullptr) {  // the linear's K splits, summed, rounded and biased as its own finish would
+    float v[16] = {};
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      const float4* src = reinterpret_cast<const float4*>(part + ((size_t)s * rows + b) * kQkvN + col);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 f = __ldcg(src + i);
+        v[4 * i] += f.x;
+        v[4 * i + 1] += f.y;
+        v[4 * i + 2] += f.z;
+        v[4 * i + 3] += f.w;
+      }
+    }
+    uint32_t o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      half2 r = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+      if (bias != nullptr) {
+        const float2 f = __half22float2(r), bb = __half22float2(*reinterpret_cast<const half2*>(bias + col + 2 * i));
+        r = __floats2half2_rn(f.x + bb.x, f.y + bb.y);
+      }
+      o[i] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    in0 = make_uint4(o[0], o[1], o[2], o[3]);
+    in1 = make_uint4(o[4], o[5], o[6], o[7]);
+  } else {
+    const half* src = qkv + (size_t)b * kQkvN + col;
+    in0 = *reinterpret_cast<const uint4*>(src);
+    in1 = *reinterpret_cast<const uint4*>(src + 8);
+  }
   const half2 xy[8] = {*reinterpret_cast<const half2*>(&in0.x), *reinterpret_cast<const half2*>(&in0.y),
                        *reinterpret_cast<const half2*>(&in0.z), *reinterpret_cast<const half2*>(&in0.w),
                        *reinterpret_cast<const half2*>(&in1.x), *reinterpret_cast<const half2*>(&in1.y),
@@ -404,10 +436,11 @@ cudaError_t launch_qkv_post(const half* qkv, const int32_t* rows, const int32_t*
 }
 cudaError_t launch_qkv_rope_append(const half* qkv, const int32_t* slots, const int32_t* positions, const half* cos_t,
                                    const half* sin_t, int max_pos, half* q_out, half* kcache, half* vcache, int s_max,
-                                   int n_slots, int rows, cudaStream_t st, bool pdl) {
+                                   int n_slots, int rows, cudaStream_t st, bool pdl, const float* part, int splits,
+                                   const half* bias) {
   const size_t total = (size_t)rows * (kHeads + 2 * kKvHeads) * 8;
   return launch(qkv_rope_rows_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, pdl, qkv, slots, positions,
-                cos_t, sin_t, max_pos, q_out, kcache, vcache, s_max, rows, n_slots);
+                cos_t, sin_t, max_pos, q_out, kcache, vcache, s_max, rows, n_slots, part, splits, bias);
 }
 cudaError_t launch_qkv_post_part(const float* part, int splits, const half* bias, const int32_t* rows,
                                  const int32_t* pos, const half* cos_t, const half* sin_t, int max_pos, half* qbuf,

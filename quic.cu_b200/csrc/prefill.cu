@@ -112,6 +112,17 @@ int linear_rows(const half* x, const quic_w4_t& w, half* y, int rows, void* ws, 
   return QUIC_OK;
 }
 
+// The linear for a consumer that sums K splits itself: with packed weights and rows of one launch
+// *splits > 1 fp32 partials stay in the workspace and y is not written; else y holds the result.
+// (A finish kernel of its own costs a small prefill 2 us, three times a layer: 1 x 87 rows
+// 1120 -> 1055 us.)
+int linear_parts(const half* x, const quic_w4_t& w, half* y, int rows, void* ws, cudaStream_t st, int* splits) {
+  *splits = 0;
+  if (w.w16 == nullptr && rows >= 2 && rows <= kPrefillChunk && w4a16_gemm_tc_workspace(rows, w.n, w.k) > 0)
+    return w4a16_gemm_tc(x, w, nullptr, rows, static_cast<float*>(ws), st, splits);
+  return linear_rows(x, w, y, rows, ws, st);
+}
+
 }  // namespace
 }  // namespace quic
 
@@ -153,20 +164,23 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
   // From here on the kernels are chained with programmatic dependent launch: each one does
   // its set-up (and the GEMMs request their weight tiles) while its predecessor drains.
   QUIC_CUDA(launch_rmsnorm(h, nullptr, (const half*)m->layers[0].ln1, m->eps, xn, nullptr, rows, st));
-  int rc = QUIC_OK;
+  int rc = QUIC_OK, sp = 0;
+  const float* part = static_cast<const float*>(ws) + 4096;  // (behind the workspace's 16 KB head)
   for (int l = 0; l < m->n_layers; ++l) {
     const quic_layer_t& L = m->layers[l];
     half* kc = static_cast<half*>(p->kv) + (size_t)(2 * l) * kv_plane;
     half* vc = kc + kv_plane;
-    if ((rc = linear_rows(xn, L.qkv, qkv, rows, ws, stream)) != QUIC_OK) return rc;
+    if ((rc = linear_parts(xn, L.qkv, qkv, rows, ws, st, &sp)) != QUIC_OK) return rc;
     QUIC_CUDA(launch_qkv_rope_append(qkv, p->row_slot, p->row_pos, (const half*)m->rope_cos, (const half*)m->rope_sin,
-                                     m->max_pos, q, kc, vc, p->s_max, p->n_slots, rows, st, true));
+                                     m->max_pos, q, kc, vc, p->s_max, p->n_slots, rows, st, true, sp > 0 ? part : nullptr, sp,
+                                     (const half*)L.qkv.bias));
     if ((rc = attn_prefill_launch(q, kc, vc, p->seq_start, p->seq_len, p->seq_slot, p->seq_off, p->n_seq, p->max_len,
                                   rows, p->s_max, p->n_slots, 0.125f /* 64^-0.5, src/model.py:129 */, attn, st, true)) != QUIC_OK)
       return rc;
-    if ((rc = linear_rows(attn, L.o, tmp, rows, ws, stream)) != QUIC_OK) return rc;
+    if ((rc = linear_parts(attn, L.o, tmp, rows, ws, st, &sp)) != QUIC_OK) return rc;
     // h += o ; xn = norm(h)
-    QUIC_CUDA(launch_rmsnorm(tmp, h, (const half*)L.ln2, m->eps, xn, h, rows, st));
+    QUIC_CUDA(sp > 0 ? launch_rmsnorm_part(part, sp, h, (const half*)L.ln2, m->eps, xn, h, rows, st)
+                     : launch_rmsnorm(tmp, h, (const half*)L.ln2, m->eps, xn, h, rows, st));
     if (L.gate_up.w16 != nullptr) {  // dense fp16 weights: GEMM, then SwiGLU, a chunk of rows at a time
       for (int r0 = 0; r0 < rows; r0 += kGuChunk) {
         const int mrows = rows - r0 < kGuChunk ? rows - r0 : kGuChunk;
@@ -185,9 +199,10 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
       if ((rc = linear_rows(xn, L.gate_up, gu, rows, ws, stream)) != QUIC_OK) return rc;
       QUIC_CUDA(launch_swiglu_fused(gu, act, rows, st));
     }
-    if ((rc = linear_rows(act, L.down, tmp, rows, ws, stream)) != QUIC_OK) return rc;
+    if ((rc = linear_parts(act, L.down, tmp, rows, ws, st, &sp)) != QUIC_OK) return rc;
     const void* next_ln = (l + 1 < m->n_layers) ? m->layers[l + 1].ln1 : m->final_norm;
-    QUIC_CUDA(launch_rmsnorm(tmp, h, (const half*)next_ln, m->eps, xn, h, rows, st));
+    QUIC_CUDA(sp > 0 ? launch_rmsnorm_part(part, sp, h, (const half*)next_ln, m->eps, xn, h, rows, st)
+                     : launch_rmsnorm(tmp, h, (const half*)next_ln, m->eps, xn, h, rows, st));
   }
   // xn holds the finally normalised rows: lm_head + argmax on the last one of every sequence
   gather_last_kernel<<<p->n_seq, 224, 0, st>>>(xn, p->seq_start, p->seq_len, xlast);
