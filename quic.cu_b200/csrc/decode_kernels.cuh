@@ -220,6 +220,13 @@ cudaError_t launch_rmsnorm(const half* x, const half* residual, const half* w, f
 int w4a16_gemm_tc(const half* x, const quic_w4_t& w, half* y, int m, float* workspace, cudaStream_t st,
                   int* splits_out = nullptr);
 int64_t w4a16_gemm_tc_workspace(int m, int n, int k);
+// many rows: dense fp16 GEMM on SM pairs, and the fp16 copies of packed weights that it reads (gemm_pair.cu)
+bool gemm_pair_supported(int m, int n, int k, bool swiglu);
+int gemm_pair_splits(int m, int n, int k);
+int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, bool swiglu, cudaStream_t st,
+              float* part = nullptr, int* splits = nullptr);
+int splitk_finish(const float* part, const half* bias, half* y, int m, int n, int splits, cudaStream_t st);
+int w4_unpack(const quic_w4_t* const* w, half* const* out, int count, cudaStream_t st);
 int w4a16_gemm_tc_swiglu(const half* x, const quic_w4_t& w, half* act, int m, cudaStream_t st);
 bool lm_head_tc_supported(int batch, int vocab);
 int lm_head_tc_tiles(int vocab);

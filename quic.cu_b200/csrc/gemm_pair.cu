@@ -1,0 +1,425 @@
+// Dense fp16 GEMM for many rows, y[M, N] = x[M, K] . W[N, K]^T, on pairs of SMs
+// (tcgen05.mma.cta_group::2), with bias or SwiGLU in the epilogue, and the unpacking of int4 weights to
+// the fp16 operand it reads.
+//
+// A prefill of a few thousand tokens and more is bound by the tensor cores.  The W4A16 kernel
+// (w4_gemm_tc.cu) unpacks its weight tile again for every 256 rows, in the loop that feeds the MMAs, and
+// reads each operand tile into one SM only: 770-870 TFLOP/s.  At these sizes a layer's weights are
+// cheaper to unpack once per call (15 M weights, 30 MB written) than a hundred times, and two SMs
+// then share one 256 x NT tile: each holds 128 of its token rows and half of its weight rows, so
+// an SM reads 32 KB per 64-wide k block of 512 tensor cycles.
+//
+// One persistent CTA pair per two SMs takes tiles in turn, weight tile fastest (the pairs that run
+// together share token rows, the weights stay in L2).  Warp 0 loads (each CTA its own half of
+// both operands, the bytes counted on the leading CTA's barrier), warp 1 of the leading CTA
+// issues the MMAs, warps 2-17 read the accumulator back (four per lane quarter: with one, the
+// epilogue's 16 us a tile hid 4 us of MMAs); there are two accumulators of 256
+// columns, so the epilogue of a tile runs under the next tile's MMAs.  Token rows are on
+// the M side: a thread of the epilogue owns a row and, with 128 gate and 128 up columns in a tile, both
+// factors of its SwiGLU outputs.  Waits are bounded by the clock: one that runs out sets word 0
+// of the tensor path's error words and the pair leaves with its tensor memory released.
+#include "tc_common.cuh"
+
+namespace quic {
+namespace {
+
+constexpr int kPairStages = 5, kPairEpilogueWarps = 16, kPairThreads = 64 + 32 * kPairEpilogueWarps;
+constexpr uint32_t kPairPitch = 80;                                        // staged row: 32 halves, padded
+constexpr uint32_t kPairStaging = kPairEpilogueWarps * 32 * kPairPitch;
+constexpr uint32_t kPairA = 128 * 128;                                     // 128 token rows x 64 k
+
+template <int NT>
+struct PairSmem {
+  static constexpr uint32_t kB = NT / 2 * 128;  // half of the weight rows x 64 k
+  static constexpr uint32_t kStage = kPairA + kB;
+  static constexpr uint32_t kTotal = kPairStages * kStage + kPairStaging + 1024;
+};
+
+struct PairArgs {
+  const half* bias;  // [N] or nullptr
+  half* y;           // [M, N], or [M, N / 2] with SwiGLU
+  float* part;       // split K: [splits][M][N] fp32 partial sums (then y and bias belong to the consumer)
+  int m_total, n, k;
+  int splits;
+  int* status;
+};
+
+// Waits at most a second or so for the phase with the given parity.
+__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 0;; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(2000u)
+        : "memory");
+    if (done) return true;
+    if ((i & 255u) == 255u) {
+      uint64_t now;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      if (now - t0 > 1000000000ull) return false;
+    }
+  }
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void pair_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Tiled load into this CTA's shared memory whose bytes count on the barrier of the pair's leading CTA
+// (the same address there: bit 24 of a cluster address tells the two apart).
+__device__ __forceinline__ void pair_load(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar & 0xFEFFFFFFu), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void pair_umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier of both CTAs once the MMAs issued so far are complete
+__device__ __forceinline__ void pair_commit(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void arrive_leader(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
+      : "memory");
+}
+
+template <int NT, bool kSwiglu>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const PairArgs a) {
+  using L = PairSmem<NT>;
+  constexpr int kOut = kSwiglu ? NT / 2 : NT;  // output columns of a tile
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bar_full[kPairStages], bar_empty[kPairStages], bar_acc[2], bar_free[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int fail_s;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_rank();
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int ntiles = a.n / NT, flat = ntiles * ((a.m_total + 255) / 256), tiles = flat * a.splits, kblocks = a.k / kBlockK;
+  const int first = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+  if (tid == 0) {
+    tma_prefetch_desc(&tm_x);
+    tma_prefetch_desc(&tm_w);
+    for (int s = 0; s < kPairStages; ++s) {
+      mbar_init(smem_u32(&bar_full[s]), 1);
+      mbar_init(smem_u32(&bar_empty[s]), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&bar_acc[s]), 1);
+      mbar_init(smem_u32(&bar_free[s]), 2 * kPairEpilogueWarps);
+    }
+    fail_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base_s)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  pair_sync();
+  tc_fence_after();
+  const uint32_t tmem_d = tmem_base_s;
+  pdl_launch_dependents();
+  pdl_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0, pass = 0;
+      bool ok = true;
+      for (int t = first; ok && t < tiles; t += pairs) {
+        const int split = t / flat, f = t % flat, nt = f % ntiles, m0 = (f / ntiles) * 256 + (int)rank * 128;
+        const int kb1 = kblocks * (split + 1) / a.splits;
+        const int w0 = kSwiglu ? (int)rank * (a.n / 2) + nt * (NT / 2) : nt * NT + (int)rank * (NT / 2);
+        for (int kb = kblocks * split / a.splits; kb < kb1; ++kb) {
+          if (pass > 0 && !pair_wait(smem_u32(&bar_empty[stage]), (pass - 1) & 1)) {
+            fail_s = 2;
+            ok = false;
+            for (int i = 0; i < 64; ++i) __nanosleep(1000);  // (copies in flight land within microseconds)
+            break;
+          }
+          const uint32_t a_s = base + stage * L::kStage, full = smem_u32(&bar_full[stage]);
+          if (rank == 0) mbar_expect_tx(full, 2 * L::kStage);
+          pair_load(a_s, &tm_x, kb * kBlockK, m0, full);
+          pair_load(a_s + kPairA, &tm_w, kb * kBlockK, w0, full);
+          if (++stage == kPairStages) {
+            stage = 0;
+            ++pass;
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      // fp16 x fp16 -> fp32, both operands K-major, M = 256 over the pair, N = NT
+      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+      int stage = 0, pass = 0, j = 0;
+      bool ok = true;
+      for (int t = first; ok && t < tiles; t += pairs, ++j) {
+        const int buf = j & 1;
+        if (j >= 2 && !pair_wait(smem_u32(&bar_free[buf]), ((j >> 1) - 1) & 1)) {
+          fail_s = 4;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t d = tmem_d + 256u * buf;
+        const int split = t / flat, nkb = kblocks * (split + 1) / a.splits - kblocks * split / a.splits;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!pair_wait(smem_u32(&bar_full[stage]), pass & 1)) {
+            fail_s = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a_s = base + stage * L::kStage, b_s = a_s + kPairA;
+#pragma unroll
+          for (int k = 0; k < kBlockK / 16; ++k)
+            pair_umma(d, umma_desc_sw128(a_s + k * 32), umma_desc_sw128(b_s + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          pair_commit(smem_u32(&bar_empty[stage]));
+          if (++stage == kPairStages) {
+            stage = 0;
+            ++pass;
+          }
+        }
+        if (ok) pair_commit(smem_u32(&bar_acc[buf]));
+      }
+    }
+  } else {
+    const int quarter = warp & 3, group = (warp - 2) >> 2;  // TMEM lanes that this warp may read, 32-column share
+    unsigned char* out_s = smem_raw + (base - smem_u32(smem_raw)) + kPairStages * L::kStage + (warp - 2) * 32 * kPairPitch;
+    int j = 0;
+    const int ld_y = kSwiglu ? a.n / 2 : a.n;
+    for (int t = first; t < tiles; t += pairs, ++j) {
+      const int buf = j & 1;
+      const int split = t / flat, f = t % flat;
+      const int row0 = (f / ntiles) * 256 + (int)rank * 128 + quarter * 32, col0 = (f % ntiles) * kOut;
+      if (!__all_sync(0xffffffffu, pair_wait(smem_u32(&bar_acc[buf]), (j >> 1) & 1))) {
+        fail_s = 3;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t taddr = tmem_d + 256u * buf + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+      for (int c = 32 * group; c < kOut; c += 128) {
+        uint32_t o[16];
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          float v[16];
+          tmem_ld_cols<16>(taddr + c + 16 * hh, v);
+          if (!kSwiglu && a.part != nullptr) {
+            if (row0 + lane < a.m_total) {
+              float4* dst = reinterpret_cast<float4*>(a.part + ((size_t)split * a.m_total + row0 + lane) * a.n + col0 + c + 16 * hh);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+            continue;
+          }
+          if (kSwiglu) {
+            float u[16];
+            tmem_ld_cols<16>(taddr + NT / 2 + c + 16 * hh, u);
+#pragma unroll
+            for (int i = 0; i < 16; ++i)  // the linear's outputs are fp16 tensors: round both factors
+              v[i] = silu_mul(__half2float(__float2half_rn(v[i])), __half2float(__float2half_rn(u[i])));
+          } else if (a.bias != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              const float2 b = __half22float2(*reinterpret_cast<const half2*>(a.bias + col0 + c + 16 * hh + i));
+              v[i] = __half2float(__float2half_rn(v[i])) + b.x;
+              v[i + 1] = __half2float(__float2half_rn(v[i + 1])) + b.y;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            o[8 * hh + i] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+        }
+        if (c + 128 >= kOut) {  // read out: the accumulator may be overwritten
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) arrive_leader(smem_u32(&bar_free[buf]));
+        }
+        if (!kSwiglu && a.part != nullptr) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(out_s + lane * kPairPitch + 16 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // eight rows of 64 contiguous bytes per store
+          const int r = 8 * i + (lane >> 2), piece = lane & 3;
+          if (row0 + r < a.m_total)
+            *reinterpret_cast<uint4*>(a.y + (size_t)(row0 + r) * ld_y + col0 + c + 8 * piece) =
+                *reinterpret_cast<const uint4*>(out_s + r * kPairPitch + 16 * piece);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (tid == 0 && fail_s != 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+  pair_sync();  // nobody leaves while the pair's copies, arrivals or MMAs use its shared memory
+  if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_d) : "memory");
+}
+
+template <int NT, bool kSwiglu>
+int run_pair(const half* x, const half* w, const PairArgs& a, cudaStream_t st) {
+  CUtensorMap tm_x, tm_w;
+  int rc = make_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)a.m_total, (uint64_t)a.k, 128, kBlockK,
+                    CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != QUIC_OK) return rc;
+  rc = make_map(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w, (uint64_t)a.n, (uint64_t)a.k, NT / 2, kBlockK,
+                CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != QUIC_OK) return rc;
+  auto kernel = gemm_pair_kernel<NT, kSwiglu>;
+  static bool allowed[64] = {};
+  int dev = 0;
+  QUIC_CUDA(cudaGetDevice(&dev));
+  if (dev > 63 || !allowed[dev]) {
+    QUIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem<NT>::kTotal));
+    if (dev <= 63) allowed[dev] = true;
+  }
+  const int64_t tiles = (int64_t)(a.n / NT) * ((a.m_total + 255) / 256) * a.splits;
+  const int pairs = tiles < 74 ? (int)tiles : 74;
+  QUIC_CUDA(launch(kernel, dim3(2 * pairs), dim3(kPairThreads), (size_t)PairSmem<NT>::kTotal, st, true, tm_x, tm_w, a));
+  return QUIC_OK;
+}
+
+// The weight tile's width: the widest that divides N (with SwiGLU, 128 gate and 128 up columns).
+int pair_nt(int n, bool swiglu) {
+  if (swiglu) return n % 256 == 0 ? 256 : 0;
+  return n % 256 == 0 ? 256 : n % 224 == 0 ? 224 : n % 192 == 0 ? 192 : 0;
+}
+
+// W fp16 [N][K] from packed [K/8][N] int32 words, for up to four weights in one launch: a thread takes
+// 64 k of one row (reads coalesced over rows), a warp's rows leave through shared memory, 128
+// contiguous bytes each.
+struct UnpackJob {
+  quic_w4_t w;
+  half* out;
+  int first_block;  // blocks of 256 rows x 64 k, rows fastest
+};
+struct UnpackArgs {
+  UnpackJob job[4];
+};
+__global__ void __launch_bounds__(256) w4_unpack_kernel(const __grid_constant__ UnpackArgs a) {
+  __shared__ __align__(16) unsigned char stage_s[8][32 * 144];  // a warp's 32 rows of 128 bytes, padded
+  pdl_launch_dependents();
+  int i = 0;
+  while (i < 3 && (int)blockIdx.x >= a.job[i + 1].first_block) ++i;
+  const UnpackJob& J = a.job[i];
+  const int blk = (int)blockIdx.x - J.first_block, nb = (J.w.n + 255) / 256;
+  const int n = (blk % nb) * 256 + (int)threadIdx.x, k0 = (blk / nb) * 64;
+  const bool live = n < J.w.n;
+  uint32_t word[8];
+  half2 s2, zp;
+  if (live) {
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(J.w.qw) + (size_t)(k0 / 8) * J.w.n + n;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) word[j] = __ldg(q + (size_t)j * J.w.n);
+    const int g = k0 / kGroup;
+    s2 = __half2half2(reinterpret_cast<const half*>(J.w.sc)[(size_t)g * J.w.n + n]);
+    const uint8_t z = reinterpret_cast<const uint8_t*>(J.w.zp)[(size_t)g * (J.w.n >> 1) + (n >> 1)];
+    zp = zp_to_half2((z >> (4 * (n & 1))) & 15);
+  }
+  unsigned char* mine = stage_s[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      half2 d[4];
+      dequant8(word[j], zp, s2, d);  // d[p] = (k = p, k = p + 4)
+      const uint32_t u0 = *reinterpret_cast<uint32_t*>(&d[0]), u1 = *reinterpret_cast<uint32_t*>(&d[1]);
+      const uint32_t u2 = *reinterpret_cast<uint32_t*>(&d[2]), u3 = *reinterpret_cast<uint32_t*>(&d[3]);
+      *reinterpret_cast<uint4*>(mine + lane * 144 + 16 * j) =
+          make_uint4(__byte_perm(u0, u1, 0x5410), __byte_perm(u2, u3, 0x5410), __byte_perm(u0, u1, 0x7632),
+                     __byte_perm(u2, u3, 0x7632));
+    }
+  }
+  __syncwarp();
+  pdl_wait();  // the fp16 copies may still be read by the previous layer's linears
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int r = 4 * j + (lane >> 3), row = n - lane + r;
+    if (row < J.w.n)
+      *reinterpret_cast<uint4*>(J.out + (size_t)row * J.w.k + k0 + 8 * (lane & 7)) =
+          *reinterpret_cast<const uint4*>(mine + r * 144 + 16 * (lane & 7));
+  }
+}
+
+}  // namespace
+
+bool gemm_pair_supported(int m, int n, int k, bool swiglu) {
+  return m >= 1 && m <= (1 << 24) && k >= kBlockK && k % kBlockK == 0 && pair_nt(n, swiglu) != 0;
+}
+
+// K splits: while the tiles leave most pairs idle, at least eight k blocks each (down at 1024 rows is 16
+// tiles of 76 k blocks: 28 us in one piece).
+int gemm_pair_splits(int m, int n, int k) {
+  const int64_t tiles = (int64_t)(n / pair_nt(n, false)) * ((m + 255) / 256);
+  int s = tiles >= 74 ? 1 : (int)(74 / tiles);
+  if (s > k / kBlockK / 8) s = k / kBlockK / 8;
+  return s < 1 ? 1 : s > 16 ? 16 : s;
+}
+
+// `part` (gemm_pair_splits x m x n fp32, may be null): where that is more than one split their partial sums
+// stay there for a consumer, y is not written and *splits says how many.
+int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, bool swiglu, cudaStream_t st,
+              float* part, int* splits) {
+  QUIC_REQUIRE(gemm_pair_supported(m, n, k, swiglu), QUIC_E_SHAPE, "gemm_pair: unsupported shape");
+  QUIC_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 16 == 0), QUIC_E_ARG,
+               "gemm_pair: tensors must be 16-byte aligned");
+  PairArgs a = {bias, y, nullptr, m, n, k, 1, tc_status_words()};
+  if (splits != nullptr) *splits = 0;
+  if (part != nullptr && gemm_pair_splits(m, n, k) > 1) {
+    a.part = part;
+    a.splits = *splits = gemm_pair_splits(m, n, k);
+  }
+  QUIC_REQUIRE(a.status != nullptr, QUIC_E_CUDA, "gemm_pair: no address for the tensor path's error words");
+  if (swiglu) return run_pair<256, true>(x, w, a, st);
+  switch (pair_nt(n, false)) {
+    case 256: return run_pair<256, false>(x, w, a, st);
+    case 224: return run_pair<224, false>(x, w, a, st);
+    default: return run_pair<192, false>(x, w, a, st);
+  }
+}
+
+// Packed weights -> fp16 [N][K] copies in `out[i]`, up to four in one launch; dense ones are passed over.
+int w4_unpack(const quic_w4_t* const* w, half* const* out, int count, cudaStream_t st) {
+  UnpackArgs a = {};
+  int blocks = 0;
+  for (int i = 0; i < 4; ++i) {
+    a.job[i].first_block = blocks;
+    if (i >= count || w[i]->w16 != nullptr) continue;
+    a.job[i].w = *w[i];
+    a.job[i].out = out[i];
+    blocks += ((w[i]->n + 255) / 256) * (w[i]->k / 64);
+  }
+  QUIC_CUDA(launch(w4_unpack_kernel, dim3(blocks), dim3(256), 0, st, true, a));
+  return QUIC_OK;
+}
+
+}  // namespace quic

@@ -8,17 +8,22 @@
 namespace quic {
 namespace {
 
-constexpr int kPrefillChunk = 8192;  // rows per linear call (bounds the split-K workspace)
-constexpr int kGuChunk = 1024;      // rows of gate|up output held at once by the dense fp16 path
+// Rows from which a layer's linears run on SM pairs over fp16 weights (gemm_pair.cu).  Packed weights are
+// unpacked for it once per call and layer, 8 us: 1 x 1024 tokens 2705 -> 2635 us, 2 x 1024 3670 -> 3120,
+// 16 x 2048 42.0 -> 33.1 ms.  Dense weights are read as they are: 1 x 130 tokens 1578 -> 1690 us,
+// 1 x 200 1768 -> 1747, 1 x 500 2426 -> 2041, 2 x 1024 5826 -> 3196.
+constexpr int kPairRows = 1024, kDensePairRows = 192;
+constexpr int64_t kLayerWeights = (int64_t)(kQkvN + kHidden + 2 * kInter) * kHidden + (int64_t)kHidden * kInter;
 
 inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
 struct PrefillArena {
-  int64_t lm, h, xn, tmp, qkv, q, attn, gu, act, xlast, ws, total;
+  int64_t lm, h, xn, tmp, qkv, q, attn, gu, act, xlast, ws, w16, total;
 };
 
 int64_t linear_ws(int rows) {
-  const int m = rows < kPrefillChunk ? rows : kPrefillChunk;
+  if (rows >= kPairRows) return (int64_t)gemm_pair_splits(rows, kHidden, kInter) * rows * kHidden * 4;
+  const int m = rows;
   int64_t w = quic_w4a16_workspace_bytes(m, kQkvN, kHidden);
   const int64_t o = quic_w4a16_workspace_bytes(m, kHidden, kHidden);
   const int64_t g = quic_w4a16_workspace_bytes(m, 2 * kInter, kHidden);
@@ -47,14 +52,16 @@ PrefillArena carve_prefill(int rows, int n_seq, int vocab) {
   a.attn = off;
   off += align256((int64_t)rows * kHidden * 2);
   a.gu = off;
-  // gate|up is materialised by the one-row fallback and, kGuChunk rows at a time, by the dense fp16 path
-  off += align256((int64_t)(rows < kGuChunk ? rows : kGuChunk) * 2 * kInter * 2);
+  // gate|up is materialised by the one-row fallback and by dense weights below kDensePairRows rows
+  off += align256((int64_t)(rows < kPairRows ? rows : 1) * 2 * kInter * 2);
   a.act = off;
   off += align256((int64_t)rows * kInter * 2);
   a.xlast = off;
   off += align256((int64_t)n_seq * kHidden * 2);
   a.ws = off;
   off += align256(linear_ws(rows));
+  a.w16 = off;  // fp16 copies of one layer's packed weights
+  if (rows >= kPairRows) off += kLayerWeights * 2;
   a.total = off;
   return a;
 }
@@ -92,35 +99,22 @@ __global__ void set_slot_state_kernel(const int64_t* __restrict__ first, const i
   pos[slot] = seq_len[i] + (seq_off != nullptr ? seq_off[i] : 0);
 }
 
-// Rows per call of a linear: packed weights beyond kPrefillChunk rows never split K (their CTAs
-// fill the SMs many times over), so they need no workspace and one launch covers all rows --
-// fewer partial waves than a launch per 8192 rows.  Dense weights keep the chunks.
-int linear_chunk(const quic_w4_t& w, int rows) {
-  constexpr int kMaxRowsPerLaunch = 1 << 22;  // grid.z = rows / 256 stays far below 65535
-  if (w.w16 != nullptr || rows <= kPrefillChunk) return kPrefillChunk;
-  return rows < kMaxRowsPerLaunch ? rows : kMaxRowsPerLaunch;
+bool layer_pairs(const quic_layer_t& L, int rows) {
+  const bool dense = L.qkv.w16 != nullptr && L.o.w16 != nullptr && L.gate_up.w16 != nullptr && L.down.w16 != nullptr;
+  return rows >= (dense ? kDensePairRows : kPairRows);
 }
 
-// One W4A16 linear over all rows, in chunks that bound the split-K workspace.
-int linear_rows(const half* x, const quic_w4_t& w, half* y, int rows, void* ws, void* stream) {
-  const int chunk = linear_chunk(w, rows);
-  for (int r0 = 0; r0 < rows; r0 += chunk) {
-    const int m = rows - r0 < chunk ? rows - r0 : chunk;
-    const int rc = quic_w4a16_linear(x + (size_t)r0 * w.k, &w, y + (size_t)r0 * w.n, m, 1, ws, stream);
-    if (rc != QUIC_OK) return rc;
-  }
-  return QUIC_OK;
-}
-
-// The linear for a consumer that sums K splits itself: with packed weights and rows of one launch
+// The linear for a consumer that sums K splits itself: with packed weights
 // *splits > 1 fp32 partials stay in the workspace and y is not written; else y holds the result.
 // (A finish kernel of its own costs a small prefill 2 us, three times a layer: 1 x 87 rows
 // 1120 -> 1055 us.)
-int linear_parts(const half* x, const quic_w4_t& w, half* y, int rows, void* ws, cudaStream_t st, int* splits) {
+int linear_parts(const half* x, const quic_w4_t& w, half* y, int rows, void* ws, cudaStream_t st, int* splits,
+                 bool adds_bias = false) {
   *splits = 0;
-  if (w.w16 == nullptr && rows >= 2 && rows <= kPrefillChunk && w4a16_gemm_tc_workspace(rows, w.n, w.k) > 0)
+  if (w.w16 == nullptr && rows >= 2 && (adds_bias || w.bias == nullptr) &&
+      w4a16_gemm_tc_workspace(rows, w.n, w.k) > 0)
     return w4a16_gemm_tc(x, w, nullptr, rows, static_cast<float*>(ws), st, splits);
-  return linear_rows(x, w, y, rows, ws, st);
+  return quic_w4a16_linear(x, &w, y, rows, 1, ws, st);
 }
 
 }  // namespace
@@ -156,6 +150,9 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
   half* act = reinterpret_cast<half*>(base + ar.act);
   half* xlast = reinterpret_cast<half*>(base + ar.xlast);
   void* ws = base + ar.ws;
+  half* const w16[4] = {reinterpret_cast<half*>(base + ar.w16), reinterpret_cast<half*>(base + ar.w16) + kQkvN * kHidden,
+                        reinterpret_cast<half*>(base + ar.w16) + (kQkvN + kHidden) * kHidden,
+                        reinterpret_cast<half*>(base + ar.w16) + (kQkvN + kHidden + 2 * kInter) * kHidden};
   const size_t slot_stride = (size_t)kKvHeads * p->s_max * kHeadDim;
   const size_t kv_plane = (size_t)p->n_slots * slot_stride;
 
@@ -170,7 +167,33 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
     const quic_layer_t& L = m->layers[l];
     half* kc = static_cast<half*>(p->kv) + (size_t)(2 * l) * kv_plane;
     half* vc = kc + kv_plane;
-    if ((rc = linear_parts(xn, L.qkv, qkv, rows, ws, st, &sp)) != QUIC_OK) return rc;
+    if (layer_pairs(L, rows)) {
+      const quic_w4_t* const w[4] = {&L.qkv, &L.o, &L.gate_up, &L.down};
+      const half* f[4];
+      int packed = 0;
+      for (int i = 0; i < 4; ++i) {
+        f[i] = w[i]->w16 != nullptr ? (const half*)w[i]->w16 : w16[i];
+        packed += w[i]->w16 == nullptr;
+      }
+      if (packed > 0 && (rc = w4_unpack(w, w16, 4, st)) != QUIC_OK) return rc;
+      if ((rc = gemm_pair(xn, f[0], (const half*)L.qkv.bias, qkv, rows, kQkvN, kHidden, false, st)) != QUIC_OK) return rc;
+      QUIC_CUDA(launch_qkv_rope_append(qkv, p->row_slot, p->row_pos, (const half*)m->rope_cos, (const half*)m->rope_sin,
+                                       m->max_pos, q, kc, vc, p->s_max, p->n_slots, rows, st, true));
+      if ((rc = attn_prefill_launch(q, kc, vc, p->seq_start, p->seq_len, p->seq_slot, p->seq_off, p->n_seq, p->max_len,
+                                    rows, p->s_max, p->n_slots, 0.125f, attn, st, true)) != QUIC_OK)
+        return rc;
+      if ((rc = gemm_pair(attn, f[1], (const half*)L.o.bias, tmp, rows, kHidden, kHidden, false, st)) != QUIC_OK) return rc;
+      QUIC_CUDA(launch_rmsnorm(tmp, h, (const half*)L.ln2, m->eps, xn, h, rows, st));
+      if ((rc = gemm_pair(xn, f[2], nullptr, act, rows, 2 * kInter, kHidden, true, st)) != QUIC_OK) return rc;
+      if ((rc = gemm_pair(act, f[3], (const half*)L.down.bias, tmp, rows, kHidden, kInter, false, st,
+                          L.down.bias == nullptr ? static_cast<float*>(ws) : nullptr, &sp)) != QUIC_OK)
+        return rc;
+      const void* next_ln = (l + 1 < m->n_layers) ? m->layers[l + 1].ln1 : m->final_norm;
+      QUIC_CUDA(sp > 0 ? launch_rmsnorm_part(static_cast<const float*>(ws), sp, h, (const half*)next_ln, m->eps, xn, h, rows, st)
+                       : launch_rmsnorm(tmp, h, (const half*)next_ln, m->eps, xn, h, rows, st));
+      continue;
+    }
+    if ((rc = linear_parts(xn, L.qkv, qkv, rows, ws, st, &sp, true)) != QUIC_OK) return rc;
     QUIC_CUDA(launch_qkv_rope_append(qkv, p->row_slot, p->row_pos, (const half*)m->rope_cos, (const half*)m->rope_sin,
                                      m->max_pos, q, kc, vc, p->s_max, p->n_slots, rows, st, true, sp > 0 ? part : nullptr, sp,
                                      (const half*)L.qkv.bias));
@@ -181,22 +204,11 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
     // h += o ; xn = norm(h)
     QUIC_CUDA(sp > 0 ? launch_rmsnorm_part(part, sp, h, (const half*)L.ln2, m->eps, xn, h, rows, st)
                      : launch_rmsnorm(tmp, h, (const half*)L.ln2, m->eps, xn, h, rows, st));
-    if (L.gate_up.w16 != nullptr) {  // dense fp16 weights: GEMM, then SwiGLU, a chunk of rows at a time
-      for (int r0 = 0; r0 < rows; r0 += kGuChunk) {
-        const int mrows = rows - r0 < kGuChunk ? rows - r0 : kGuChunk;
-        if ((rc = linear_rows(xn + (size_t)r0 * kHidden, L.gate_up, gu, mrows, ws, stream)) != QUIC_OK) return rc;
-        QUIC_CUDA(launch_swiglu_fused(gu, act + (size_t)r0 * kInter, mrows, st));
-      }
-    } else if (rows >= 2) {  // gate|up GEMM with SwiGLU in its epilogue: the [rows, 9728] intermediate never exists
-      const int chunk = linear_chunk(L.gate_up, rows);
-      for (int r0 = 0; r0 < rows; r0 += chunk) {
-        const int mrows = rows - r0 < chunk ? rows - r0 : chunk;
-        if ((rc = w4a16_gemm_tc_swiglu(xn + (size_t)r0 * kHidden, L.gate_up, act + (size_t)r0 * kInter, mrows, st)) !=
-            QUIC_OK)
-          return rc;
-      }
+    if (L.gate_up.w16 == nullptr && rows >= 2) {
+      // gate|up GEMM with SwiGLU in its epilogue: the [rows, 9728] intermediate never exists
+      if ((rc = w4a16_gemm_tc_swiglu(xn, L.gate_up, act, rows, st)) != QUIC_OK) return rc;
     } else {
-      if ((rc = linear_rows(xn, L.gate_up, gu, rows, ws, stream)) != QUIC_OK) return rc;
+      if ((rc = quic_w4a16_linear(xn, &L.gate_up, gu, rows, 1, ws, stream)) != QUIC_OK) return rc;
       QUIC_CUDA(launch_swiglu_fused(gu, act, rows, st));
     }
     if ((rc = linear_parts(act, L.down, tmp, rows, ws, st, &sp)) != QUIC_OK) return rc;

@@ -540,10 +540,16 @@ int w4a16_gemm_tc(const half* x, const quic_w4_t& w, half* y, int m, float* work
   }
   if (rc != QUIC_OK) return rc;
   if (splits > 1 && y != nullptr) {
-    const size_t total = (size_t)m * w.n;
-    QUIC_CUDA(launch(tc_splitk_finish_kernel, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, st, true,
-                     (const float*)a.part, (const half*)w.bias, y, m, w.n, splits));
+    return splitk_finish(a.part, (const half*)w.bias, y, m, w.n, splits, st);
   }
+  return QUIC_OK;
+}
+
+// y[m, n] = fp16(sum of the K splits' fp32 partials) (+ bias)
+int splitk_finish(const float* part, const half* bias, half* y, int m, int n, int splits, cudaStream_t st) {
+  const size_t total = (size_t)m * n;
+  QUIC_CUDA(launch(tc_splitk_finish_kernel, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, st, true, part, bias,
+                   y, m, n, splits));
   return QUIC_OK;
 }
 

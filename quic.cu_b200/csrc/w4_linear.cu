@@ -200,14 +200,28 @@ extern "C" int quic_w4_dequant(const quic_w4_t* w, void* out, void* stream) {
 // Rows from which the tcgen05 GEMM beats the dequant GEMV (measured per layer shape: 5-9 us
 // against 10-19 us at 4 rows; the GEMV runs 2..8 rows on one 8-row instantiation).
 static constexpr int kTensorMinRows = 2;
+// The SM pair GEMM: dense weights from 128 rows (9728 x 896 at 130 rows 14.1 -> 11.3 us, at 8192 369 -> 117);
+// packed ones, which it unpacks first, where the products outweigh that (us: 9728 x 896 at 1024 rows
+// 33.6 -> 25.3, 896 x 4864 at 1024 23.3 -> 26.7 and at 1500 33.8 -> 27.8, 896 x 896 at 4096 12.5 -> 13.6 and at
+// 8192 21.6 -> 19.6).
+static constexpr int kDensePairMinRows = 128;
+static bool packed_pairs(int64_t m, int64_t n, int64_t k) {
+  return m * n * k >= 6000000000ll && k % kGroup == 0 && gemm_pair_supported((int)m, (int)n, (int)k, false);
+}
 
 static int64_t packed_workspace_bytes(int32_t m, int32_t n, int32_t k);
+static int64_t pair_part_bytes(int32_t m, int32_t n, int32_t k) {
+  if (!gemm_pair_supported(m, n, k, false)) return 0;
+  const int splits = gemm_pair_splits(m, n, k);
+  return splits > 1 ? (int64_t)splits * m * n * 4 : 0;
+}
 
 extern "C" int64_t quic_w4a16_workspace_bytes(int32_t m, int32_t n, int32_t k) {
   if (m <= 0 || n <= 0 || k <= 0) return 0;
   // the same block serves a packed or a dense weight of this shape
   const int64_t packed = packed_workspace_bytes(m, n, k), dense = gemm_f16_tc_workspace(m, n, k);
-  return packed > dense ? packed : dense;
+  const int64_t pair = m >= kDensePairMinRows ? pair_part_bytes(m, n, k) : 0, most = packed > dense ? packed : dense;
+  return most > pair ? most : pair;
 }
 
 static int64_t packed_workspace_bytes(int32_t m, int32_t n, int32_t k) {
@@ -216,10 +230,20 @@ static int64_t packed_workspace_bytes(int32_t m, int32_t n, int32_t k) {
   if (m >= kTensorMinRows && n % 128 == 0 && k % 64 == 0) {
     const int64_t tc = 16384 + w4a16_gemm_tc_workspace(m, n, k);
     const int64_t gv = m > 8 ? 16384 + (int64_t)2 * m * n * 4 : 16384 + (int64_t)gemv_splits(n, k) * m * n * 4;
-    return tc > gv ? tc : gv;  // the caller may force either path
+    const int64_t pair = packed_pairs(m, n, k) ? 16384 + (int64_t)n * k * 2 + pair_part_bytes(m, n, k) : 0;  // fp16 copy, splits
+    const int64_t most = tc > gv ? tc : gv;  // the caller may force either path
+    return most > pair ? most : pair;
   }
   if (m > 8) return 16384 + (int64_t)2 * m * n * 4;  // row-chunked GEMV splits only to fit shared memory
   return 16384 + (int64_t)gemv_splits(n, k) * m * n * 4;
+}
+
+// The SM pair GEMM, its K splits (if any) summed by a kernel of their own.
+static int pair_linear(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, float* part,
+                       cudaStream_t st) {
+  int splits = 0;
+  const int rc = gemm_pair(x, w, bias, y, m, n, k, false, st, part, &splits);
+  return rc != QUIC_OK || splits == 0 ? rc : splitk_finish(part, bias, y, m, n, splits, st);
 }
 
 extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int32_t m,
@@ -228,6 +252,9 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
   if (w->w16 != nullptr) {  // dense fp16 weight [N, K]: a row or two on the GEMV, more on the tcgen05 GEMM
     QUIC_REQUIRE(w->n > 0 && w->k > 0 && w->k % 8 == 0 && m >= 0, QUIC_E_SHAPE, "linear: bad dense shape");
     if (m == 0) return QUIC_OK;
+    if (m >= kDensePairMinRows && use_tensor && gemm_pair_supported(m, w->n, w->k, false))
+      return pair_linear((const half*)x, (const half*)w->w16, (const half*)w->bias, (half*)y, m, w->n, w->k,
+                         (float*)workspace, (cudaStream_t)stream);
     if (m >= 2 && use_tensor && gemm_f16_tc_supported(m, w->n, w->k))
       return gemm_f16_tc((const half*)x, (const half*)w->w16, (const half*)w->bias, (half*)y, m, w->n, w->k,
                          (float*)workspace, (cudaStream_t)stream, true);
@@ -239,6 +266,14 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
   QUIC_REQUIRE(m >= 0, QUIC_E_SHAPE, "w4a16_linear: negative M");
   if (m == 0) return QUIC_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (use_tensor && packed_pairs(m, w->n, w->k)) {
+    QUIC_REQUIRE(workspace != nullptr, QUIC_E_ARG, "w4a16_linear: tensor path needs a workspace");
+    half* const w16 = reinterpret_cast<half*>(static_cast<char*>(workspace) + 16384);
+    const int rc = w4_unpack(&w, &w16, 1, st);
+    if (rc != QUIC_OK) return rc;
+    return pair_linear((const half*)x, w16, (const half*)w->bias, (half*)y, m, w->n, w->k,
+                       reinterpret_cast<float*>(w16 + (size_t)w->n * w->k), st);
+  }
   if (use_tensor && m >= kTensorMinRows && w->n % 128 == 0 && w->k % 64 == 0) {
     QUIC_REQUIRE(workspace != nullptr, QUIC_E_ARG, "w4a16_linear: tensor path needs a workspace");
     return w4a16_gemm_tc((const half*)x, *w, (half*)y, m, (float*)workspace, st, nullptr);

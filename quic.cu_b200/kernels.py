@@ -274,9 +274,10 @@ class W4Weight:
         return out
 
     def workspace(self, m: int) -> torch.Tensor:
-        """Split-K workspace, shared by every weight on the device (calls on one stream are ordered)."""
+        """Workspace of a call, shared by every weight on the stream (whose calls are ordered)."""
         need = _linear_workspace_bytes(m, self.size_n, self.size_k)
-        key = self.qw.device.index
+        device = self.qw.get_device()
+        key = (device, _raw_stream(device))
         ws = _linear_workspace.get(key)
         if ws is None or ws.numel() * 4 < need:
             ws = torch.zeros((max(need, 1 << 22) + 3) // 4, dtype=torch.float32, device=self.qw.device)

@@ -1,0 +1,54 @@
+"""Linears of many rows (the SM pair GEMM) against fp32 products: tile edges, every tile width, K splits
+with and without room for them, bias; and a prefill that takes it against the same prompts in calls that do not."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from quic_cu_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 256, 64), (129, 896, 896), (255, 1152, 896), (257, 192, 4864), (300, 9728, 128),
+                                   (385, 896, 4864), (5000, 1152, 128)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_dense_linear(m, n, k, bias):
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    b = torch.randn(n, device="cuda", generator=gen).half() if bias else None
+    w = kernels.F16Weight(n, k, torch.device("cuda"), bias=b)
+    w.w.copy_(torch.randn(n, k, device="cuda", generator=gen) * 0.05)
+    x = torch.randn(m, k, device="cuda", generator=gen).half()
+    want = (x.float() @ w.w.float().T).half().float() + (0 if b is None else b.float())
+    y = kernels.w4a16_linear(w, x)
+    assert (y.float() - want).norm() <= 1e-3 * want.norm()
+
+
+@pytest.mark.parametrize("m,n,k", [(689, 9728, 896), (1377, 896, 4864), (1500, 896, 4864), (5900, 1152, 896)])
+def test_packed_linear_equals_the_same_rows_in_smaller_calls(m, n, k):
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    w = kernels.W4Weight(n, k, torch.device("cuda"))
+    w.qw.random_(-2 ** 31, 2 ** 31 - 1, generator=gen)
+    w.zp.random_(0, 255, generator=gen)
+    w.sc.copy_(torch.rand(w.sc.shape, device="cuda", generator=gen) * 0.02)
+    x = torch.randn(m, k, device="cuda", generator=gen).half()
+    want = torch.cat([kernels.w4a16_linear(w, x[i:i + 500]) for i in range(0, m, 500)]).float()
+    y = kernels.w4a16_linear(w, x)
+    assert (y.float() - want).norm() <= 1e-3 * want.norm()
+
+
+@pytest.mark.parametrize("lens", [[1024], [600, 423, 2], [700, 700, 650]], ids=str)
+def test_prefill_equals_one_prompt_at_a_time(tiny_model, lens):
+    net = tiny_model[0]
+    gen = torch.Generator().manual_seed(sum(lens))
+    prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
+    whole, parts = (net.new_cache(n_slots=4, s_max=1100) for _ in range(2))
+    _, logits = net.prefill(whole, list(range(len(lens))), prompts)
+    for i, p in enumerate(prompts):
+        half = len(p) // 2
+        if half > 1:  # in two calls of fewer rows
+            net.prefill(parts, [i], [p[:half]])
+        _, one = net.prefill(parts, [i], [p[half:]] if half > 1 else [p], offsets=[half] if half > 1 else None)
+        assert (logits[i].float() - one[0].float()).norm() <= 1e-2 * one[0].float().norm()
+    assert (whole.kv.float() - parts.kv.float()).norm() <= 5e-3 * parts.kv.float().norm()
