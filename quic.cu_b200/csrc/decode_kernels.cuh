@@ -225,6 +225,17 @@ bool gemm_pair_supported(int m, int n, int k, bool swiglu);
 int gemm_pair_splits(int m, int n, int k);
 int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, bool swiglu, cudaStream_t st,
               float* part = nullptr, int* splits = nullptr);
+struct PairRope {
+  const int32_t* slots;      // [rows]
+  const int32_t* positions;  // [rows]
+  const half* cos_t;
+  const half* sin_t;
+  half* q;                   // [heads][rows][64]
+  half* kcache;
+  half* vcache;
+  int32_t max_pos, s_max, n_slots;
+};
+int gemm_pair_qkv(const half* x, const half* w, const half* bias, int m, const PairRope& rope, cudaStream_t st);
 int splitk_finish(const float* part, const half* bias, half* y, int m, int n, int splits, cudaStream_t st);
 int w4_unpack(const quic_w4_t* const* w, half* const* out, int count, cudaStream_t st);
 int w4a16_gemm_tc_swiglu(const half* x, const quic_w4_t& w, half* act, int m, cudaStream_t st);

@@ -42,6 +42,7 @@ struct PairArgs {
   int m_total, n, k;
   int splits;
   int* status;
+  PairRope rope;
 };
 
 // Waits at most a second or so for the phase with the given parity.
@@ -90,6 +91,43 @@ __device__ __forceinline__ void pair_umma(uint32_t tmem_d, uint64_t adesc, uint6
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Sixteen finished qkv outputs of a token, columns col .. col + 15 (eight stored pairs: dims d and d + 32 side by
+// side), rotated by its position (queries and keys) and written to their heads: sixteen bytes of either half.
+// Same arithmetic as qkv_rope_rows_kernel, whose 150 MB at 32768 tokens (50 us a layer) this saves.
+__device__ __forceinline__ void rope_store(const PairRope& r, const float (&v)[16], int col, int tok, int pos, int slot, int rows) {
+  const int head = col >> 6, d0 = (col & 63) >> 1;
+  __align__(16) half lo[8], hi[8];
+  if (head < kHeads + kKvHeads) {
+    const int pp = pos < r.max_pos ? (pos < 0 ? 0 : pos) : r.max_pos - 1;
+    const uint4 c4 = *reinterpret_cast<const uint4*>(r.cos_t + (size_t)pp * 32 + d0);
+    const uint4 s4 = *reinterpret_cast<const uint4*>(r.sin_t + (size_t)pp * 32 + d0);
+    const half* ch = reinterpret_cast<const half*>(&c4);
+    const half* sh = reinterpret_cast<const half*>(&s4);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float x = __half2float(__float2half_rn(v[2 * i])), y = __half2float(__float2half_rn(v[2 * i + 1]));
+      const float c = __half2float(ch[i]), sn = __half2float(sh[i]);
+      lo[i] = __float2half_rn(x * c - y * sn);
+      hi[i] = __float2half_rn(x * sn + y * c);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      lo[i] = __float2half_rn(v[2 * i]);
+      hi[i] = __float2half_rn(v[2 * i + 1]);
+    }
+  }
+  half* dst;
+  if (head < kHeads) {
+    dst = r.q + ((size_t)head * rows + tok) * kHeadDim;
+  } else {
+    if (pos >= r.s_max || pos < 0 || slot < 0 || slot >= r.n_slots) return;  // nothing is appended for such a row
+    half* plane = head < kHeads + kKvHeads ? r.kcache : r.vcache;
+    dst = plane + (((size_t)slot * kKvHeads + ((head - kHeads) & 1)) * r.s_max + pos) * kHeadDim;
+  }
+  *reinterpret_cast<uint4*>(dst + d0) = *reinterpret_cast<const uint4*>(lo);
+  *reinterpret_cast<uint4*>(dst + 32 + d0) = *reinterpret_cast<const uint4*>(hi);
+}
 // arrives on the barrier of both CTAs once the MMAs issued so far are complete
 __device__ __forceinline__ void pair_commit(uint32_t bar) {
   asm volatile(
@@ -104,7 +142,7 @@ __device__ __forceinline__ void arrive_leader(uint32_t bar) {
       : "memory");
 }
 
-template <int NT, bool kSwiglu>
+template <int NT, bool kSwiglu, bool kRope>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const PairArgs a) {
   using L = PairSmem<NT>;
@@ -215,6 +253,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       const int buf = j & 1;
       const int split = t / flat, f = t % flat;
       const int row0 = (f / ntiles) * 256 + (int)rank * 128 + quarter * 32, col0 = (f % ntiles) * kOut;
+      // RoPE form: the lane's token (rows past the end: none)
+      const int tok = row0 + lane;
+      const bool live = kRope && tok < a.m_total;
+      const int pos = live ? a.rope.positions[tok] : 0, slot = live ? a.rope.slots[tok] : -1;
       if (!__all_sync(0xffffffffu, pair_wait(smem_u32(&bar_acc[buf]), (j >> 1) & 1))) {
         fail_s = 3;
         break;
@@ -250,10 +292,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
               v[i + 1] = __half2float(__float2half_rn(v[i + 1])) + b.y;
             }
           }
+          if constexpr (kRope) {
+            if (live) rope_store(a.rope, v, col0 + c + 16 * hh, tok, pos, slot, a.m_total);
+          } else {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-            o[8 * hh + i] = *reinterpret_cast<const uint32_t*>(&h);
+            for (int i = 0; i < 8; ++i) {
+              const half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+              o[8 * hh + i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
           }
         }
         if (c + 128 >= kOut) {  // read out: the accumulator may be overwritten
@@ -261,19 +307,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           __syncwarp();
           if (lane == 0) arrive_leader(smem_u32(&bar_free[buf]));
         }
-        if (!kSwiglu && a.part != nullptr) continue;
+        if constexpr (!kRope) {
+          if (!kSwiglu && a.part != nullptr) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(out_s + lane * kPairPitch + 16 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-        __syncwarp();
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(out_s + lane * kPairPitch + 16 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+          __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {  // eight rows of 64 contiguous bytes per store
-          const int r = 8 * i + (lane >> 2), piece = lane & 3;
-          if (row0 + r < a.m_total)
-            *reinterpret_cast<uint4*>(a.y + (size_t)(row0 + r) * ld_y + col0 + c + 8 * piece) =
-                *reinterpret_cast<const uint4*>(out_s + r * kPairPitch + 16 * piece);
+          for (int i = 0; i < 4; ++i) {  // eight rows of 64 contiguous bytes per store
+            const int r = 8 * i + (lane >> 2), piece = lane & 3;
+            if (row0 + r < a.m_total)
+              *reinterpret_cast<uint4*>(a.y + (size_t)(row0 + r) * ld_y + col0 + c + 8 * piece) =
+                  *reinterpret_cast<const uint4*>(out_s + r * kPairPitch + 16 * piece);
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
     }
   }
@@ -285,7 +333,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_d) : "memory");
 }
 
-template <int NT, bool kSwiglu>
+template <int NT, bool kSwiglu, bool kRope = false>
 int run_pair(const half* x, const half* w, const PairArgs& a, cudaStream_t st) {
   CUtensorMap tm_x, tm_w;
   int rc = make_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)a.m_total, (uint64_t)a.k, 128, kBlockK,
@@ -294,7 +342,7 @@ int run_pair(const half* x, const half* w, const PairArgs& a, cudaStream_t st) {
   rc = make_map(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w, (uint64_t)a.n, (uint64_t)a.k, NT / 2, kBlockK,
                 CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != QUIC_OK) return rc;
-  auto kernel = gemm_pair_kernel<NT, kSwiglu>;
+  auto kernel = gemm_pair_kernel<NT, kSwiglu, kRope>;
   static bool allowed[64] = {};
   int dev = 0;
   QUIC_CUDA(cudaGetDevice(&dev));
@@ -392,7 +440,7 @@ int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, in
   QUIC_REQUIRE(gemm_pair_supported(m, n, k, swiglu), QUIC_E_SHAPE, "gemm_pair: unsupported shape");
   QUIC_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 16 == 0), QUIC_E_ARG,
                "gemm_pair: tensors must be 16-byte aligned");
-  PairArgs a = {bias, y, nullptr, m, n, k, 1, tc_status_words()};
+  PairArgs a = {bias, y, nullptr, m, n, k, 1, tc_status_words(), {}};
   if (splits != nullptr) *splits = 0;
   if (part != nullptr && gemm_pair_splits(m, n, k) > 1) {
     a.part = part;
@@ -405,6 +453,15 @@ int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, in
     case 224: return run_pair<224, false>(x, w, a, st);
     default: return run_pair<192, false>(x, w, a, st);
   }
+}
+
+// The fused qkv linear with RoPE and the KV append in its epilogue: y never exists.
+int gemm_pair_qkv(const half* x, const half* w, const half* bias, int m, const PairRope& rope, cudaStream_t st) {
+  static_assert(kQkvN % 192 == 0 && 192 % kHeadDim == 0, "whole heads in a tile");
+  QUIC_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0), QUIC_E_ARG, "gemm_pair: tensors must be 16-byte aligned");
+  PairArgs a = {bias, nullptr, nullptr, m, kQkvN, kHidden, 1, tc_status_words(), rope};
+  QUIC_REQUIRE(a.status != nullptr, QUIC_E_CUDA, "gemm_pair: no address for the tensor path's error words");
+  return run_pair<192, false, true>(x, w, a, st);
 }
 
 // Packed weights -> fp16 [N][K] copies in `out[i]`, up to four in one launch; dense ones are passed over.

@@ -176,9 +176,9 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
         packed += w[i]->w16 == nullptr;
       }
       if (packed > 0 && (rc = w4_unpack(w, w16, 4, st)) != QUIC_OK) return rc;
-      if ((rc = gemm_pair(xn, f[0], (const half*)L.qkv.bias, qkv, rows, kQkvN, kHidden, false, st)) != QUIC_OK) return rc;
-      QUIC_CUDA(launch_qkv_rope_append(qkv, p->row_slot, p->row_pos, (const half*)m->rope_cos, (const half*)m->rope_sin,
-                                       m->max_pos, q, kc, vc, p->s_max, p->n_slots, rows, st, true));
+      const PairRope rope = {p->row_slot, p->row_pos, (const half*)m->rope_cos, (const half*)m->rope_sin, q, kc, vc,
+                             m->max_pos, p->s_max, p->n_slots};
+      if ((rc = gemm_pair_qkv(xn, f[0], (const half*)L.qkv.bias, rows, rope, st)) != QUIC_OK) return rc;
       if ((rc = attn_prefill_launch(q, kc, vc, p->seq_start, p->seq_len, p->seq_slot, p->seq_off, p->n_seq, p->max_len,
                                     rows, p->s_max, p->n_slots, 0.125f, attn, st, true)) != QUIC_OK)
         return rc;
