@@ -15,9 +15,8 @@
 // Same mathematics as fad_decode_kernel + fad_combine_kernel of the reference
 // (kernels/cuda/flash_attn_decode.cu:12,104): fp32 softmax over the tokens [start_b, end_b) of
 // each row, rows without tokens give zeros (:118-121).
-#include "attn_warp.cuh"
+#include "attn_flow_tile.cuh"
 #include "decode_kernels.cuh"
-#include "tc_common.cuh"
 
 namespace quic {
 namespace {
@@ -28,23 +27,6 @@ constexpr uint32_t kFlowTile = kWarpChunk * kHeadDim * 2;  // 8 KB: 64 tokens x 
 constexpr uint32_t kFlowStage = 2 * kFlowTile;             // K tile, V tile
 constexpr int kFlowSmem = kFlowWarps * kFlowStage + 1024;
 
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(a)
-               : "memory");
-}
-__device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], uint32_t a) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(a)
-               : "memory");
-}
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
-  uint32_t d;
-  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
-  return d;
-}
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -77,7 +59,7 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
   __shared__ float part_s[kGroupHeads * 66];  // this split's sums, {max, sum} behind each head's
   __shared__ int fail_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3, mi = lane >> 3, mr = lane & 7;
+  const int g = lane >> 2, t = lane & 3;
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t k_s = base + warp * kFlowStage, v_s = k_s + kFlowTile, bar = smem_u32(&bar_full[warp]);
@@ -113,7 +95,7 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
     qb[ks][0] = g < kGroupHeads ? q[0] : 0u;
     qb[ks][1] = g < kGroupHeads ? q[4] : 0u;
   }
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[4][4] = {};
+  FlowState st;
   uint32_t parity = 0;
   for (int i = i0 + warp; i < i1; i += kFlowWarps) {
     if (!__all_sync(0xffffffffu, mbar_wait(bar, parity))) {
@@ -122,107 +104,17 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
       break;
     }
     parity ^= 1u;
-    uint32_t K[4][4][4], V[4][4][4];
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt) ldsm4(K[mt][ks], k_s + sw128_offset(16 * mt + 8 * (mi & 1) + mr, 2 * ks + (mi >> 1)));
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int dt = 0; dt < 4; ++dt)
-        ldsm4_trans(V[dt][ks], v_s + sw128_offset(16 * ks + 8 * (mi >> 1) + mr, 2 * dt + (mi & 1)));
-    float sc[4][4] = {};
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-        mma16816(sc[mt], K[mt][ks][0], K[mt][ks][1], K[mt][ks][2], K[mt][ks][3], qb[ks][0], qb[ks][1]);
+    uint32_t V[4][4][4];
+    float sc[4][4];
+    flow_scores(k_s, v_s, qb, lane, V, sc);
     // the stage is in registers: refill it (the reads come before the copy, another proxy)
     fence_proxy_async();
     __syncwarp();
     if (i + kFlowWarps < i1) request(i + kFlowWarps);
-    const int t0 = (tile0 + i) * kWarpChunk;
-    const bool edge = t0 < t_begin || t0 + kWarpChunk > t_end;
-    if (edge) {  // values outside the row's tokens may be anything, 0 x NaN included
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int tok = t0 + 16 * ks + 8 * hh + 2 * t;
-          const uint32_t keep_v = (tok >= t_begin && tok < t_end ? 0xffffu : 0u) |
-                                  (tok + 1 >= t_begin && tok + 1 < t_end ? 0xffff0000u : 0u);
-#pragma unroll
-          for (int dt = 0; dt < 4; ++dt) {
-            V[dt][ks][2 * hh] &= keep_v;
-            V[dt][ks][2 * hh + 1] &= keep_v;
-          }
-        }
-    }
-    float mx[2] = {m[0], m[1]};
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float s = sc[mt][e] * a.scale;
-        if (edge) {
-          const int tok = t0 + 16 * mt + g + 8 * (e >> 1);
-          s = tok >= t_begin && tok < t_end ? s : -INFINITY;
-        }
-        sc[mt][e] = s;
-        mx[e & 1] = fmaxf(mx[e & 1], s);
-      }
-#pragma unroll
-    for (int x = 4; x < 32; x <<= 1) {
-      mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], x));
-      mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], x));
-    }
-    float keep[2], ref[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      ref[e] = mx[e] == -INFINITY ? 0.f : mx[e];
-      keep[e] = __expf(m[e] - ref[e]);  // (0 before the first token)
-      m[e] = mx[e];
-      l[e] *= keep[e];
-    }
-    uint32_t pb[4][2];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const half2 ph = __floats2half2_rn(__expf(sc[mt][2 * hh] - ref[0]), __expf(sc[mt][2 * hh + 1] - ref[1]));
-        l[0] += __low2float(ph);
-        l[1] += __high2float(ph);
-        pb[mt][hh] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&ph));
-      }
-#pragma unroll
-    for (int dt = 0; dt < 4; ++dt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) o[dt][e] *= keep[e & 1];
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-      for (int dt = 0; dt < 4; ++dt)
-        mma16816(o[dt], V[dt][ks][0], V[dt][ks][1], V[dt][ks][2], V[dt][ks][3], pb[ks][0], pb[ks][1]);
+    flow_attend(st, V, sc, (tile0 + i) * kWarpChunk, t_begin, t_end, a.scale, lane);
   }
-  // ---- the warps meet in shared memory; a lane's heads are 2t, 2t + 1, its dims g + 8 .. ----
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-#pragma unroll
-    for (int x = 4; x < 32; x <<= 1) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
-    const int hd = 2 * t + e;
-    if (hd < kGroupHeads) {
-#pragma unroll
-      for (int dt = 0; dt < 4; ++dt) {
-        o_s[warp][hd][16 * dt + g] = o[dt][e];
-        o_s[warp][hd][16 * dt + 8 + g] = o[dt][2 + e];
-      }
-      if (g == 0) {
-        m_s[warp][hd] = m[e];
-        l_s[warp][hd] = l[e];
-      }
-    }
-  }
+  // ---- the warps meet in shared memory ----
+  flow_store(st, m_s[warp], l_s[warp], o_s[warp], lane);
   __syncthreads();
   if (fail_s != 0 && tid == 0)  // a bounded wait gave up: say so (the row's output is then invalid)
     atomicCAS(status, 0, (7 << 16) | 0x4000 | ((int)blockIdx.z & 0x3fff));

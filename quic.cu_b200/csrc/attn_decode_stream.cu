@@ -1,7 +1,7 @@
 // GQA decode attention for many rows (the tensor-core step beyond 20 rows): ONE CTA per
 // (row, KV head) streams that head's cached keys and values through a ring of shared-memory
 // stages filled by TMA (64-token tiles, 128-byte swizzle), six warps take the tiles in turn
-// -- the 64-token tile arithmetic of attn_warp.cuh on mma.sync, each warp keeping a running
+// -- the 64-token tile arithmetic of attn_flow_tile.cuh on mma.sync, each warp keeping a running
 // softmax over its tiles -- and meet once in shared memory.  No partial results in global
 // memory, no counters, no second pass, and nothing is read beyond a row's own length.
 //
@@ -32,9 +32,8 @@
 // Same mathematics as fad_decode_kernel + fad_combine_kernel of the reference
 // (kernels/cuda/flash_attn_decode.cu:12,104): fp32 softmax over the tokens [start_b, end_b) of
 // each row, rows without tokens give zeros (:118-121).
-#include "attn_warp.cuh"
+#include "attn_flow_tile.cuh"
 #include "decode_kernels.cuh"
-#include "tc_common.cuh"
 
 namespace quic {
 namespace {
@@ -55,31 +54,6 @@ constexpr size_t kStreamSmem = (size_t)kStreamStages * kStageBytes + 1024;
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-  return v;
-}
-
-// The fragments of warp_tile_request, from a swizzled tile pair in shared memory (conflict-free:
-// a quarter warp reads eight different 16-byte chunks of the 128-byte bank cycle).
-__device__ __forceinline__ void warp_tile_from_smem(WarpTile& t, uint32_t k_s, uint32_t v_s, int g, int c) {
-#pragma unroll
-  for (int nb = 0; nb < 8; ++nb) {
-    const int row = 8 * nb + g;
-    t.kr[nb][0] = lds128(k_s + sw128_offset(row, 2 * c));
-    t.kr[nb][1] = lds128(k_s + sw128_offset(row, 2 * c + 1));
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int row = 16 * j + 2 * c + (r & 1) + 8 * (r >> 1);
-      t.vr[j][r] = lds128(v_s + sw128_offset(row, g));
-    }
-  }
-}
-
 __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                               const AttnArgs a, const QkvFinish fin, int n_slots, int s_max, int* status,
@@ -87,8 +61,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kStreamStages];   // a stage's two tiles landed
   __shared__ __align__(8) uint64_t bar_empty[kStreamStages];  // its consumer warp holds them in registers
-  __shared__ float m_s[kStreamWarps][kGroupHeads];
-  __shared__ float l_s[kStreamWarps][kGroupHeads];
+  __shared__ float m_s[kStreamWarps][8], l_s[kStreamWarps][8];
   __shared__ __align__(16) float o_s[kStreamWarps][kGroupHeads][kHeadDim];
   __shared__ int fail_s, pre_s, epoch_s;
   __shared__ __align__(16) half q_s[kGroupHeads][kHeadDim];  // finished q heads (fin.part set)
@@ -148,9 +121,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
   const int n_tiles = t_end > t_begin ? (t_end + kWarpChunk - 1) / kWarpChunk - tile0 : 0;
   const int row0 = (slot * kKvHeads + kvh) * s_max;  // first cache row of this (slot, KV head)
 
-  float m = -INFINITY, l = 0.f, o[8][4];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  FlowState st;
 
   const bool finish = fin.part != nullptr || fin.qkv != nullptr;
   if (finish && warp < kStreamWarps) {
@@ -250,19 +221,13 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     }
   } else if (n_tiles > 0) {
     // ---------------- compute warps: tile i belongs to warp i % kStreamWarps ----------------
-    uint32_t qa0[4], qa2[4];
-    if (finish) {
+    uint32_t qb[4][2];  // Q^T fragments: column g = head (column 7 is zero)
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        qa0[ks] = qa2[ks] = 0u;
-        if (g < kGroupHeads) {
-          const uint2 u = *reinterpret_cast<const uint2*>(&q_s[g][16 * c + 4 * ks]);
-          qa0[ks] = u.x;
-          qa2[ks] = u.y;
-        }
-      }
-    } else {
-      warp_q_fragments(qa0, qa2, a.q + ((size_t)b * kHeads + kvh * kGroupHeads) * kHeadDim, g, c);
+    for (int ks = 0; ks < 4; ++ks) {
+      const half* q = finish ? &q_s[g < kGroupHeads ? g : 0][0]
+                             : a.q + ((size_t)b * kHeads + kvh * kGroupHeads + (g < kGroupHeads ? g : 0)) * kHeadDim;
+      qb[ks][0] = g < kGroupHeads ? *reinterpret_cast<const uint32_t*>(q + 16 * ks + 2 * c) : 0u;
+      qb[ks][1] = g < kGroupHeads ? *reinterpret_cast<const uint32_t*>(q + 16 * ks + 2 * c + 8) : 0u;
     }
     for (int i = warp; i < n_tiles; i += kStreamWarps) {
       const int s = i % kStreamStages;
@@ -286,39 +251,16 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
         }
         __syncwarp();
       }
-      WarpTile tile;
-      warp_tile_from_smem(tile, base + s * kStageBytes, base + s * kStageBytes + kTileBytes, g, c);
+      uint32_t V[4][4][4];
+      float sc[4][4];
+      flow_scores(base + s * kStageBytes, base + s * kStageBytes + kTileBytes, qb, lane, V, sc);
+      fence_proxy_async();  // the reads come before the copy that refills the stage, another proxy
       __syncwarp();
       if (lane == 0) mbar_arrive_local(smem_u32(&bar_empty[s]));  // the stage may be refilled
-      float m1, l1, o1[8][4];
-      warp_tile_attend(tile, qa0, qa2, t0, max(t_begin, t0), min(t_end, t0 + kWarpChunk), a.scale, c, m1, l1, o1);
-      // running softmax over this warp's tiles (m, l are equal in the four lanes of a head)
-      const float mx = fmaxf(m, m1);
-      if (mx != -INFINITY) {
-        const float e0 = (m == -INFINITY) ? 0.f : __expf(m - mx);
-        const float e1 = (m1 == -INFINITY) ? 0.f : __expf(m1 - mx);
-        l = e0 * l + e1 * l1;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          o[j][0] = e0 * o[j][0] + e1 * o1[j][0];
-          o[j][1] = e0 * o[j][1] + e1 * o1[j][1];
-        }
-        m = mx;
-      }
+      flow_attend(st, V, sc, t0, t_begin, t_end, a.scale, lane);
     }
   }
-  if (warp < kStreamWarps && g < kGroupHeads) {
-    // C columns 2c, 2c+1 of mma j are dims 16c + j and 16c + 8 + j of head g
-    float4* op = reinterpret_cast<float4*>(&o_s[warp][g][16 * c]);
-    op[0] = make_float4(o[0][0], o[1][0], o[2][0], o[3][0]);
-    op[1] = make_float4(o[4][0], o[5][0], o[6][0], o[7][0]);
-    op[2] = make_float4(o[0][1], o[1][1], o[2][1], o[3][1]);
-    op[3] = make_float4(o[4][1], o[5][1], o[6][1], o[7][1]);
-    if (c == 0) {
-      m_s[warp][g] = m;
-      l_s[warp][g] = l;
-    }
-  }
+  if (warp < kStreamWarps) flow_store(st, m_s[warp], l_s[warp], o_s[warp], lane);
   __syncthreads();
   if (fail_s != 0) {  // a bounded wait gave up: say so, leave the row's output as it is
     if (tid == 0) atomicCAS(status, 0, ((4 + fail_s) << 16) | 0x4000 | ((int)blockIdx.y & 0x3fff));
