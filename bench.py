@@ -254,8 +254,7 @@ def run_gpu(args) -> None:
            "note": "per 256-token step: 256 public decode calls, each with a 4-byte token id H2D from "
                    "pinned memory and a 4-byte sampled id D2H"}
 
-    # ---- rooflines.  By time the step is its 120 layer kernels (87 %), by bytes the lm_head
-    # (58 %): `roofline` names the group that dominates by time, `roofline_kernels` lists every
+    # ---- rooflines.  By time the step is its layers (87 %), by bytes the lm_head (58 %): `roofline` names the group that dominates by time, `roofline_kernels` lists every
     # kernel type, `roofline_step` is the whole token.
     peak, peak_kind = peaks()
     prof = profile_shares()
@@ -280,29 +279,38 @@ def run_gpu(args) -> None:
     layer_bytes = step_bytes - lm_bytes                     # W4 weights of 24 layers + K/V read and written
     per_layer = {"qkv_kernel<1>": 536256 + 2304 + 1792 + 512, "attn_decode_cta_kernel<true>": 512 * (mean_ctx + 1),
                  "oproj_kernel<1>": 417088, "gateup_kernel<1>": 4528384 + 1792, "down_kernel<1>": 2264192}
+    # one packed row up to 768 tokens: the persistent kernel, one launch per burst of BURST tokens
+    persist = bool(net.persist_ok(1, PROMPT_LEN + GEN_TOKENS))
     kernels = []
-    for name, share in prof["layer_kernel_share"].items():
+    for name, share in {} if persist else prof["layer_kernel_share"].items():
         us = layers_us / net.n_layers * share
         kernels.append({"kernel": name, "launches_per_token": net.n_layers, "algorithmic_bytes": per_layer[name],
                         "us_per_launch": us, "achieved": per_layer[name] / us / 1e3, "unit": "GB/s",
                         "frac": per_layer[name] / us / 1e3 / peak, "share_of_step": us * net.n_layers / us_per_token,
                         "timing": "(token time - live lm_head time) / layers x the kernel's share of the layer "
                                   "kernels' time in the committed ncu launch list"})
-    kernels.append({"kernel": "lm_head_kernel<1>", "launches_per_token": 1, "algorithmic_bytes": lm_bytes,
+    if persist:
+        kernels.append({"kernel": "decode_persist_kernel<1>", "launches_per_token": 1 / BURST,
+                        "algorithmic_bytes": step_bytes, "us_per_token": us_per_token, "achieved": step_gbs,
+                        "unit": "GB/s", "frac": step_gbs / peak, "share_of_step": 1.0,
+                        "timing": "the timed region itself: every burst is one launch of this kernel"})
+    kernels.append({"kernel": "lm_head_kernel<1>" + (" (stand-alone: a phase of the persistent kernel here)" if persist
+                                                     else ""), "launches_per_token": 0 if persist else 1, "algorithmic_bytes": lm_bytes,
                     "us_per_launch": lm_us, "achieved": lm_bytes / lm_us / 1e3, "unit": "GB/s",
                     "frac": lm_bytes / lm_us / 1e3 / peak, "share_of_step": lm_us / us_per_token,
                     "traffic": prof["dram_traffic_bytes_per_launch"]["lm_head_kernel<1>"],
                     "traffic_source": "ncu capture summarised under profiles/ (not measured by this run)",
                     "timing": f"{reps} back-to-back launches between CUDA events on the launching stream; the "
                               "272 MB table exceeds L2"})
-    roofline = {"bound": "hbm", "kernel": "the 120 layer kernels of a token (qkv, attention, o_proj, gate_up, down "
-                                          "x 24: dominant by time)",
+    roofline = {"bound": "hbm", "kernel": ("the layer phases of the persistent kernel" if persist else
+                                            "the 120 layer kernels of a token") + " (qkv, attention, o_proj, gate_up, "
+                                           "down x 24: dominant by time)",
                 "achieved": layer_bytes / layers_us / 1e3, "peak": peak, "unit": "GB/s",
                 "frac": layer_bytes / layers_us / 1e3 / peak, "peak_kind": f"of {peak_kind}",
                 "share_of_step": layers_us / us_per_token, "us_per_token": layers_us,
                 "algorithmic_bytes": layer_bytes, "traffic": None,
                 "timing": "token time (CUDA events over the timed region) minus the lm_head kernel's live time"}
-    roofline_step = {"bound": "hbm", "scope": "whole decode step (121 kernels)", "achieved": step_gbs,
+    roofline_step = {"bound": "hbm", "scope": "whole decode step" + ("" if persist else " (121 kernels)"), "achieved": step_gbs,
                      "peak": peak, "unit": "GB/s", "frac": step_gbs / peak, "us_per_token": us_per_token,
                      "algorithmic_bytes": step_bytes}
 
@@ -332,7 +340,8 @@ def run_gpu(args) -> None:
         "warmup": max(args.warmup, 3), "ms_per_step": elapsed_ms / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "int4 weights x fp16 activations, fp32 accumulate",
         "data": "synthetic", "config": CONFIG, "parallelism": f"{world} independent replica(s), no collective",
-        "clocks": clocks, "e2e": e2e, "gpu_launches": world * args.steps * GEN_TOKENS * net.launches_per_step(cache, 1, PROMPT_LEN + GEN_TOKENS),
+        "clocks": clocks, "e2e": e2e, "gpu_launches": world * args.steps * (GEN_TOKENS // BURST if persist else GEN_TOKENS * net.launches_per_step(
+            cache, 1, PROMPT_LEN + GEN_TOKENS)),
         "roofline": roofline, "roofline_kernels": kernels, "roofline_step": roofline_step, "batch64": batch64,
         "serving": serving,
     }
