@@ -9,10 +9,10 @@ namespace quic {
 namespace {
 
 // Rows from which a layer's linears run on SM pairs over fp16 weights (gemm_pair.cu).  Packed weights are
-// unpacked for it once per call and layer, 8 us: 1 x 1024 tokens 2705 -> 2635 us, 2 x 1024 3670 -> 3120,
-// 16 x 2048 42.0 -> 33.1 ms.  Dense weights are read as they are: 1 x 130 tokens 1578 -> 1690 us,
+// unpacked for it once per call and layer, 8 us: 1 x 600 tokens 1848 -> 2196 us, 1 x 768 2190 -> 2179,
+// 1 x 1000 2728 -> 2515, 16 x 2048 42.0 -> 33.1 ms.  Dense weights are read as they are: 1 x 130 tokens 1578 -> 1690 us,
 // 1 x 200 1768 -> 1747, 1 x 500 2426 -> 2041, 2 x 1024 5826 -> 3196.
-constexpr int kPairRows = 1024, kDensePairRows = 192;
+constexpr int kPairRows = 768, kDensePairRows = 192;
 constexpr int64_t kLayerWeights = (int64_t)(kQkvN + kHidden + 2 * kInter) * kHidden + (int64_t)kHidden * kInter;
 
 inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }

@@ -38,7 +38,7 @@ def test_packed_linear_equals_the_same_rows_in_smaller_calls(m, n, k):
     assert (y.float() - want).norm() <= 1e-3 * want.norm()
 
 
-@pytest.mark.parametrize("lens", [[1024], [600, 423, 2], [700, 700, 650]], ids=str)
+@pytest.mark.parametrize("lens", [[768], [500, 266, 2], [700, 700, 650]], ids=str)
 def test_prefill_equals_one_prompt_at_a_time(tiny_model, lens):
     net = tiny_model[0]
     gen = torch.Generator().manual_seed(sum(lens))
