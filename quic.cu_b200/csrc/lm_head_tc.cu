@@ -17,7 +17,6 @@
 namespace quic {
 namespace {
 
-constexpr int kLmStages = 3;  // 3 x 24 KB at 64 rows: three CTAs share an SM, so loads, MMAs and epilogues of different tiles overlap
 constexpr int kLmThreads = 128 + 32;  // 4 epilogue warps (thread 0 issues MMAs) + 1 TMA warp
 
 template <int MT>
@@ -25,13 +24,18 @@ struct LmSmem {
   static constexpr uint32_t kA = kTileN * 128;
   static constexpr uint32_t kB = ((uint32_t)MT * 128u + 1023u) & ~1023u;
   static constexpr uint32_t kStage = kA + kB;
-  static constexpr uint32_t kTotal = kLmStages * kStage + 1024;
+  // Several CTAs share an SM, so loads, MMAs and epilogues of different tiles overlap: two stages and one CTA
+  // more beat three (us, 3 -> 2 stages: 50.8 -> 50.4 at 16 rows, 54.9 -> 52.8 at 32, 73.2 -> 67.1 at 128) but at
+  // 64 rows (57.0 -> 57.3).
+  static constexpr int kStages = MT == 64 ? 3 : 2;
+  static constexpr uint32_t kTotal = kStages * kStage + 1024;
 };
 
 template <int MT>
 __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_constant__ CUtensorMap tm_e,
                                                                 const __grid_constant__ CUtensorMap tm_x,
                                                                 const LmHeadArgs a, int* status) {
+  constexpr int kLmStages = LmSmem<MT>::kStages;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kLmStages];
   __shared__ __align__(8) uint64_t bar_empty[kLmStages];
