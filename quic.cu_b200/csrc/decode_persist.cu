@@ -43,7 +43,8 @@
 // Words: eight fp16 values (or four fp32) in one 128-bit store; the all-zero word means "not there yet".
 // Each exchange buffer exists three times (layer number mod 3): a word is emptied one layer before
 // it is written again, by its writer, when everybody who read its last contents has been heard from
-// (transitively), and every launch leaves all of them empty.
+// (transitively), and every launch leaves all of them empty.  A lm_head candidate carries the number of
+// its token's last layer instead; those words are emptied when a launch starts.
 //
 // Waits: every poll and every mbarrier wait is bounded; on a timeout the CTA records a code in
 // the status word, the others see it within a few hundred probes, all wait for their own copies in
@@ -98,6 +99,11 @@ constexpr int kMaxParts = 30;                 // rows x splits
 // phase ids of a wait (status word, tags)
 constexpr int kPhX = 0, kPhQkv = 1, kPhAtt = 2, kPhXb = 3, kPhAct = 4, kPhCand = 6;
 constexpr uint32_t kPollLimit = 1u << 20;
+// Layers are numbered through the life of an exchange area (header word 0).  A launch starts below kNumbers and
+// counts at most 4096 x 64 on from there, so that within a launch no number overflows (0xFFFFFFFF and 0 would be the
+// same copy) and none is zero, the tag of an area that has just been cleared.
+constexpr uint32_t kNumbers = 3u << 28;
+static_assert(kNumbers % 3u == 0u && (uint64_t)kNumbers + 4096u * kMaxLayers + 2u < (uint64_t(1) << 32), "numbers of a launch");
 
 // Exchange buffers, each three times: the copy of layer number n is n % 3.
 struct SyncLayout {
@@ -1643,6 +1649,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
       tk = tk < 0 ? 0 : (tk >= a.vocab ? a.vocab - 1 : tk);
     }
     if (cta == 0 && tid < a.n_feed) a.feed_dst[tid] = a.feed[tid];
+    // the candidate words keep their last contents and tag, and the tags come round again with the layer numbers
+    empty_word(a.sync + sync_layout().cand + ((size_t)tid * kCtas + cta) * 16);
     state[tid] = p;
     state[16 + tid] = slot;
     state[32 + tid] = tk;
@@ -1660,7 +1668,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
     const uint32_t limit = ld_relaxed_u32(hdr + 2);
     sa.poll_limit = limit != 0u ? limit : kPollLimit;
     sa.withhold_layer = (int)ld_relaxed_u32(hdr + 3) - 1;
-    sa.no0 = ld_relaxed_u32(hdr);
+    sa.no0 = ld_relaxed_u32(hdr) % kNumbers;
     sa.step0 = a.step_counter != nullptr ? __ldcg(a.step_counter) : 0;
     sa.q0 = q0;
     sa.row_magic = (65536u + (uint32_t)a.batch - 1u) / (uint32_t)a.batch;

@@ -103,7 +103,7 @@ class SlotCache:
         return t
 
     def persist_sync(self) -> torch.Tensor:
-        """Exchange area of the persistent decode kernel (zeroed once; its tags only grow)."""
+        """Exchange area of the persistent decode kernel (zeroed once)."""
         t = self.__dict__.get("_persist_sync")
         if t is None:
             t = torch.zeros(K.lib().quic_persist_sync_bytes(), dtype=torch.uint8, device=self.device)

@@ -189,3 +189,32 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_launch_works(persist_net)
     cache.host_len[0] -= 1
     more = net.decode(cache, [0], 3)[0]
     assert more == net.decode(want_cache, [0], 3)[0]
+
+
+@pytest.mark.parametrize("rows", [1, 3])
+def test_layer_numbers_may_run_over(persist_net, rows):
+    """Header word 0 counts layers over the life of an exchange area.  A burst that starts a few layers below the
+    end of 32 bits, or of the range the numbers are kept in, gives the tokens of one that starts at zero, and so
+    does a start number that was used before: the candidates of the burst that had it are still in the area."""
+    net = persist_net
+    gen = torch.Generator().manual_seed(rows)
+    prompts = [torch.randint(0, 2048, (20 + 9 * i,), generator=gen) for i in range(rows)]
+    others = [torch.randint(0, 2048, (31,), generator=gen) for _ in range(rows)]
+    slots = list(range(rows))
+
+    def burst(cache, tokens, number=None):
+        net.prefill(cache, slots, tokens)
+        if number is not None:
+            cache.persist_sync()[:4].view(torch.int32)[0] = number - (1 << 32) if number >= 1 << 31 else number
+        got = net.decode(cache, slots, 16)
+        logits = torch.empty(rows, 2048, dtype=torch.float16, device="cuda")
+        net.decode_async(cache, slots, 1, logits=logits)
+        assert net.persist_status(cache) == 0
+        return got, logits
+
+    fresh = [burst(net.new_cache(n_slots=4, s_max=256), p) for p in (prompts, others)]
+    cache = net.new_cache(n_slots=4, s_max=256)
+    for number in (0, (1 << 32) - 13, (1 << 32) - 1, (3 << 28) - 13, (3 << 28) - 1, 0):
+        for want, p in zip(fresh, (prompts, others)):
+            got = burst(cache, p, number)
+            assert got[0] == want[0] and torch.equal(got[1], want[1]), number
