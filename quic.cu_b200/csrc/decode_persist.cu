@@ -1567,7 +1567,8 @@ __device__ __forceinline__ void token_begin() {
     if (th.tid == 0) {
       AttnRole& r = sa.role;
       r.pos = state[r.row];
-      const int hi = r.t_lo + a.chunk_tokens;
+      // the last split takes the rest: every position belongs to a split, whatever the context hint said
+      const int hi = r.split + 1 < a.splits ? r.t_lo + a.chunk_tokens : a.s_max;
       r.t_end = r.slot < 0 ? r.t_lo : (r.pos + 1 < hi ? r.pos + 1 : hi);
       if (r.t_end < r.t_lo) r.t_end = r.t_lo;
     }
@@ -2016,8 +2017,7 @@ int launch_persist(const quic_model_t* m, const quic_decode_t* d, const void* ws
   pa.sync = static_cast<unsigned char*>(sync);
   pa.steps = steps;
   pa.splits = splits;
-  // every position of a row belongs to a split, whatever the context hint said
-  pa.chunk_tokens = splits == 1 ? (d->s_max + 63) / 64 * 64 : ((ctx + splits - 1) / splits + 63) / 64 * 64;
+  pa.chunk_tokens = ((ctx + splits - 1) / splits + 63) / 64 * 64;
   pa.na = 2 * d->batch * splits;
   pa.ng = kCtas - pa.na;
   const int room = kCtas - kResCtas - pa.na;  // CTAs that can take QKV tiles

@@ -218,3 +218,35 @@ def test_layer_numbers_may_run_over(persist_net, rows):
         for want, p in zip(fresh, (prompts, others)):
             got = burst(cache, p, number)
             assert got[0] == want[0] and torch.equal(got[1], want[1]), number
+
+
+@pytest.mark.parametrize("lens,hint", [([1500], 900), ([1700, 40], 800), ([300, 1900, 5], 1000), ([2000] * 4, 1500), ([1100], 1)])
+def test_a_context_hint_below_the_position_loses_no_token(persist_net, lens, hint):
+    """The last of several attention splits takes whatever the hint left out: logits and the appended keys and
+    values of a step whose hint is too small against the kernel chain with the right one."""
+    import ctypes as C
+
+    from quic_cu_b200 import kernels as K
+
+    net, rows = persist_net, len(lens)
+    gen = torch.Generator().manual_seed(sum(lens))
+    prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
+    cache = net.new_cache(n_slots=4, s_max=2048)
+    slots = list(range(rows))
+    net.prefill(cache, slots, prompts)
+    start = [t.clone() for t in (cache.kv, cache.tok, cache.pos)]
+    logits = [torch.empty(rows, 2048, dtype=torch.float16, device="cuda") for _ in range(2)]
+
+    d, row_map = net._decode_struct(cache, rows, hint, logits[0], persist=True)
+    row_map.copy_(cache.rows_tensor(slots))
+    K.check(K.lib().quic_decode_persist(C.byref(net._c_model), C.byref(d), K.ptr(net.persist_stream()),
+                                        K.ptr(cache.persist_sync()), 1, K.stream_ptr()), "decode_persist")
+    assert net.persist_status(cache) == 0
+    kv = cache.kv.clone()
+    for t, s in zip((cache.kv, cache.tok, cache.pos), start):
+        t.copy_(s)
+    net.use_persist = False
+    net.decode_async(cache, slots, 1, logits=logits[1])
+    ok, err = _close(logits[0], logits[1])
+    assert ok, err
+    assert (kv.float() - cache.kv.float()).abs().max() <= 5e-2
