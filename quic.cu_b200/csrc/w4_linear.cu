@@ -225,17 +225,19 @@ extern "C" int64_t quic_w4a16_workspace_bytes(int32_t m, int32_t n, int32_t k) {
 }
 
 static int64_t packed_workspace_bytes(int32_t m, int32_t n, int32_t k) {
-  // 16 KB reserved head, then split-K partials: of the tensor path from 2 rows (it stops
-  // splitting once the output tiles fill the SMs, so large m needs none), of the GEMV below.
+  // 16 KB reserved head, then the most that a path may put behind it (the caller may force any of them): split-K
+  // partials of the GEMV, whose row chunks split only to fit shared memory; of the tensor path, which stops
+  // splitting once the output tiles fill the SMs; or the pair GEMM's fp16 copy of the weight and its partials.
+  int64_t most = m > 8 ? (int64_t)2 * m * n * 4 : (int64_t)gemv_splits(n, k) * m * n * 4;
   if (m >= kTensorMinRows && n % 128 == 0 && k % 64 == 0) {
-    const int64_t tc = 16384 + w4a16_gemm_tc_workspace(m, n, k);
-    const int64_t gv = m > 8 ? 16384 + (int64_t)2 * m * n * 4 : 16384 + (int64_t)gemv_splits(n, k) * m * n * 4;
-    const int64_t pair = packed_pairs(m, n, k) ? 16384 + (int64_t)n * k * 2 + pair_part_bytes(m, n, k) : 0;  // fp16 copy, splits
-    const int64_t most = tc > gv ? tc : gv;  // the caller may force either path
-    return most > pair ? most : pair;
+    const int64_t tc = w4a16_gemm_tc_workspace(m, n, k);
+    most = most > tc ? most : tc;
   }
-  if (m > 8) return 16384 + (int64_t)2 * m * n * 4;  // row-chunked GEMV splits only to fit shared memory
-  return 16384 + (int64_t)gemv_splits(n, k) * m * n * 4;
+  if (packed_pairs(m, n, k)) {  // (N a multiple of 192 or 224 is enough for it)
+    const int64_t pair = (int64_t)n * k * 2 + pair_part_bytes(m, n, k);
+    most = most > pair ? most : pair;
+  }
+  return 16384 + most;
 }
 
 // The SM pair GEMM, its K splits (if any) summed by a kernel of their own.

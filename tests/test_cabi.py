@@ -47,6 +47,16 @@ def test_host_only_queries():
     assert 1 <= lib.quic_decode_pick_splits(64, 8192) <= 64
 
 
+def test_linear_workspace_holds_the_weight_copy_and_the_splits():
+    """Packed linears of many rows unpack their weight into the workspace (N x K fp16) and put the partial sums of
+    74 // tiles K splits (tiles of 256 rows) behind it, also where N is no multiple of 128."""
+    for m, n, k, width in ((7000, 192, 4864, 192), (8192, 448, 4864, 224), (3000, 448, 4864, 224), (1500, 896, 4864, 224)):
+        tiles = n // width * -(-m // 256)
+        splits = max(1, 74 // tiles)
+        need = 16384 + n * k * 2 + (splits * m * n * 4 if splits > 1 else 0)
+        assert K.lib().quic_w4a16_workspace_bytes(m, n, k) >= need, (m, n, k)
+
+
 def test_struct_sizes_match_the_header():
     assert ctypes.sizeof(K.W4) == 48  # four pointers, two ints, the dense-weight pointer
     assert ctypes.sizeof(K.Layer) == 4 * 48 + 16

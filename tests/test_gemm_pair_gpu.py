@@ -3,6 +3,8 @@ with and without room for them, bias; and a prefill that takes it against the sa
 
 from __future__ import annotations
 
+import ctypes as C
+
 import pytest
 import torch
 
@@ -36,6 +38,26 @@ def test_packed_linear_equals_the_same_rows_in_smaller_calls(m, n, k):
     want = torch.cat([kernels.w4a16_linear(w, x[i:i + 500]) for i in range(0, m, 500)]).float()
     y = kernels.w4a16_linear(w, x)
     assert (y.float() - want).norm() <= 1e-3 * want.norm()
+
+
+@pytest.mark.parametrize("m,n,k", [(7000, 192, 4864), (3000, 448, 4864)])
+def test_packed_linear_stays_inside_its_workspace(m, n, k):
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    w = kernels.W4Weight(n, k, torch.device("cuda"))
+    w.qw.random_(-2 ** 31, 2 ** 31 - 1, generator=gen)
+    w.zp.random_(0, 255, generator=gen)
+    w.sc.copy_(torch.rand(w.sc.shape, device="cuda", generator=gen) * 0.02)
+    x = torch.randn(m, k, device="cuda", generator=gen).half()
+    size = kernels.lib().quic_w4a16_workspace_bytes(m, n, k)
+    arena = torch.full((size + (32 << 20),), 0x5a, dtype=torch.uint8, device="cuda")
+    arena[:size] = 0
+    y = torch.empty(m, n, dtype=torch.float16, device="cuda")
+    s = w.struct()
+    kernels.check(kernels.lib().quic_w4a16_linear(x.data_ptr(), C.byref(s), y.data_ptr(), m, 1, arena.data_ptr(),
+                                                  kernels.stream_ptr()), "w4a16_linear")
+    want = x.float() @ w.dequant().float().T
+    assert (y.float() - want).norm() <= 1e-3 * want.norm()
+    assert bool((arena[size:] == 0x5a).all())
 
 
 @pytest.mark.parametrize("lens", [[768], [500, 266, 2], [700, 700, 650]], ids=str)
