@@ -102,7 +102,10 @@ int quic_w4_dequant(const quic_w4_t *w, void *out_f16, void *stream);
  * Replaces marlin.forward (kernels/cuda/marlin.cu:4769 marlin_gemm, reached
  * through src/quant/marlin.py:190 marlin_linear).  One row runs the dequant
  * GEMV; two rows and more run the tcgen05 GEMM when `use_tensor` is non-zero
- * (N and K multiples of 128) and the GEMV in row chunks otherwise.  `workspace` (>= quic_w4a16_workspace_bytes)
+ * (N and K multiples of 128) and the GEMV in row chunks otherwise; with enough
+ * rows the tensor path is an SM pair GEMM (N a multiple of 192, 224 or 256).
+ * The tensor path wants x, w and y 16-byte aligned; a dense weight takes any y
+ * and any bias, at less speed.  `workspace` (>= quic_w4a16_workspace_bytes)
  * holds split-K partials; its first 16 KB (arrival counters of the tensor
  * path) must be zero before the first call and are left zero. */
 int quic_w4a16_linear(const void *x_f16, const quic_w4_t *w, void *y_f16,

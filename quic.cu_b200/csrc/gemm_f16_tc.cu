@@ -245,7 +245,7 @@ int gemm_f16_tc(const half* x, const half* w, const half* bias, half* y, int m, 
   QUIC_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0), QUIC_E_ARG,
                "gemm_f16: x and w must be 16-byte aligned");
   const int mt = dense_mt(m);
-  int splits = ws != nullptr ? dense_splits(m, n, k, mt) : 1;
+  int splits = ws != nullptr && (uintptr_t)y % 8 == 0 ? dense_splits(m, n, k, mt) : 1;  // (the sum of the splits stores 8 bytes)
   const int nkb = k / kBlockK;
   DenseArgs a = {};
   a.bias = bias;

@@ -438,8 +438,8 @@ int gemm_pair_splits(int m, int n, int k) {
 int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, bool swiglu, cudaStream_t st,
               float* part, int* splits) {
   QUIC_REQUIRE(gemm_pair_supported(m, n, k, swiglu), QUIC_E_SHAPE, "gemm_pair: unsupported shape");
-  QUIC_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 16 == 0), QUIC_E_ARG,
-               "gemm_pair: tensors must be 16-byte aligned");
+  QUIC_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)part) % 16 == 0 && (uintptr_t)bias % 4 == 0, QUIC_E_ARG,
+               "gemm_pair: tensors must be 16-byte aligned, the bias 4-byte");
   PairArgs a = {bias, y, nullptr, m, n, k, 1, tc_status_words(), {}};
   if (splits != nullptr) *splits = 0;
   if (part != nullptr && gemm_pair_splits(m, n, k) > 1) {
@@ -458,7 +458,8 @@ int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, in
 // The fused qkv linear with RoPE and the KV append in its epilogue: y never exists.
 int gemm_pair_qkv(const half* x, const half* w, const half* bias, int m, const PairRope& rope, cudaStream_t st) {
   static_assert(kQkvN % 192 == 0 && 192 % kHeadDim == 0, "whole heads in a tile");
-  QUIC_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0), QUIC_E_ARG, "gemm_pair: tensors must be 16-byte aligned");
+  QUIC_REQUIRE(((uintptr_t)x | (uintptr_t)w) % 16 == 0 && (uintptr_t)bias % 4 == 0, QUIC_E_ARG,
+               "gemm_pair: tensors must be 16-byte aligned, the bias 4-byte");
   PairArgs a = {bias, nullptr, nullptr, m, kQkvN, kHidden, 1, tc_status_words(), rope};
   QUIC_REQUIRE(a.status != nullptr, QUIC_E_CUDA, "gemm_pair: no address for the tensor path's error words");
   return run_pair<192, false, true>(x, w, a, st);

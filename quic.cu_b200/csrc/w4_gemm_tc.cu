@@ -521,6 +521,8 @@ int w4a16_gemm_tc(const half* x, const quic_w4_t& w, half* y, int m, float* work
   tc_plan(m, w.n, w.k, &mt, &splits, &per, &mtl);
   QUIC_REQUIRE((splits == 1 && y != nullptr) || workspace != nullptr, QUIC_E_ARG,
                "w4a16_linear: split-K needs a workspace");
+  QUIC_REQUIRE((uintptr_t)y % (splits == 1 ? 16 : 8) == 0 && (splits == 1 || y == nullptr || (uintptr_t)w.bias % 4 == 0), QUIC_E_ARG,
+               "w4a16_linear: y must be 16-byte aligned on the tensor path (8 with split K, and the bias 4)");
   if (splits_out != nullptr) *splits_out = splits;
   GemmArgs a = {};
   a.w = w;

@@ -240,6 +240,12 @@ static int64_t packed_workspace_bytes(int32_t m, int32_t n, int32_t k) {
   return 16384 + most;
 }
 
+// The pair GEMM stores 16 bytes of y and reads two bias values at a time; where a tensor does not allow it the general
+// path takes the call.
+static bool pair_aligned(const void* x, const quic_w4_t* w, const void* y, const void* workspace) {
+  return ((uintptr_t)x | (uintptr_t)w->w16 | (uintptr_t)y | (uintptr_t)workspace) % 16 == 0 && (uintptr_t)w->bias % 4 == 0;
+}
+
 // The SM pair GEMM, its K splits (if any) summed by a kernel of their own.
 static int pair_linear(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, float* part,
                        cudaStream_t st) {
@@ -254,7 +260,7 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
   if (w->w16 != nullptr) {  // dense fp16 weight [N, K]: a row or two on the GEMV, more on the tcgen05 GEMM
     QUIC_REQUIRE(w->n > 0 && w->k > 0 && w->k % 8 == 0 && m >= 0, QUIC_E_SHAPE, "linear: bad dense shape");
     if (m == 0) return QUIC_OK;
-    if (m >= kDensePairMinRows && use_tensor && gemm_pair_supported(m, w->n, w->k, false))
+    if (m >= kDensePairMinRows && use_tensor && gemm_pair_supported(m, w->n, w->k, false) && pair_aligned(x, w, y, workspace))
       return pair_linear((const half*)x, (const half*)w->w16, (const half*)w->bias, (half*)y, m, w->n, w->k,
                          (float*)workspace, (cudaStream_t)stream);
     if (m >= 2 && use_tensor && gemm_f16_tc_supported(m, w->n, w->k))
@@ -268,7 +274,7 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
   QUIC_REQUIRE(m >= 0, QUIC_E_SHAPE, "w4a16_linear: negative M");
   if (m == 0) return QUIC_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (use_tensor && packed_pairs(m, w->n, w->k)) {
+  if (use_tensor && packed_pairs(m, w->n, w->k) && pair_aligned(x, w, y, workspace)) {
     QUIC_REQUIRE(workspace != nullptr, QUIC_E_ARG, "w4a16_linear: tensor path needs a workspace");
     half* const w16 = reinterpret_cast<half*>(static_cast<char*>(workspace) + 16384);
     const int rc = w4_unpack(&w, &w16, 1, st);

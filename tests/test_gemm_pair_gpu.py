@@ -60,6 +60,26 @@ def test_packed_linear_stays_inside_its_workspace(m, n, k):
     assert bool((arena[size:] == 0x5a).all())
 
 
+@pytest.mark.parametrize("n", [896, 192])
+@pytest.mark.parametrize("y_off,bias_off,room", [(1, 0, False), (4, 0, True), (1, 0, True), (0, 1, False), (0, 1, True), (3, 3, True)])
+def test_dense_linear_takes_any_output_and_bias_address(n, y_off, bias_off, room):
+    m, k = 130, 896
+    gen = torch.Generator(device="cuda").manual_seed(n + y_off)
+    bias = torch.randn(n + 8, device="cuda", generator=gen).half()[bias_off:bias_off + n]
+    w = kernels.F16Weight(n, k, torch.device("cuda"), bias=bias)
+    w.w.copy_(torch.randn(n, k, device="cuda", generator=gen) * 0.05)
+    x = torch.randn(m, k, device="cuda", generator=gen).half()
+    out = torch.zeros(m * n + 8, dtype=torch.float16, device="cuda")
+    ws = torch.zeros(kernels.lib().quic_w4a16_workspace_bytes(m, n, k) + 16, dtype=torch.uint8, device="cuda") if room else None
+    s = w.struct()
+    kernels.check(kernels.lib().quic_w4a16_linear(x.data_ptr(), C.byref(s), out.data_ptr() + 2 * y_off, m, 1, kernels.ptr(ws),
+                                                  kernels.stream_ptr()), "linear")
+    want = (x.float() @ w.w.float().T).half().float() + bias.float()
+    y = out[y_off:y_off + m * n].view(m, n).float()
+    assert (y - want).norm() <= 1e-3 * want.norm()
+    assert not out[:y_off].any() and not out[y_off + m * n:].any()
+
+
 @pytest.mark.parametrize("lens", [[768], [500, 266, 2], [700, 700, 650]], ids=str)
 def test_prefill_equals_one_prompt_at_a_time(tiny_model, lens):
     net = tiny_model[0]
