@@ -74,12 +74,17 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void pair_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Tiled load into this CTA's shared memory whose bytes count on the barrier of the pair's leading CTA
-// (the same address there: bit 24 of a cluster address tells the two apart).
+// the same shared-memory address in the pair's leading CTA
+__device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
+  uint32_t ra;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(addr));
+  return ra;
+}
+// Tiled load into this CTA's shared memory whose bytes count on a barrier of the pair, given by its cluster address.
 __device__ __forceinline__ void pair_load(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar & 0xFEFFFFFFu), "r"(c0), "r"(c1)
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
 __device__ __forceinline__ void pair_umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -136,10 +141,7 @@ __device__ __forceinline__ void pair_commit(uint32_t bar) {
       : "memory");
 }
 __device__ __forceinline__ void arrive_leader(uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
-      : "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_leader(bar)) : "memory");
 }
 
 template <int NT, bool kSwiglu, bool kRope>
@@ -198,10 +200,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             for (int i = 0; i < 64; ++i) __nanosleep(1000);  // (copies in flight land within microseconds)
             break;
           }
-          const uint32_t a_s = base + stage * L::kStage, full = smem_u32(&bar_full[stage]);
+          const uint32_t a_s = base + stage * L::kStage, full = smem_u32(&bar_full[stage]), lead = in_leader(full);
           if (rank == 0) mbar_expect_tx(full, 2 * L::kStage);
-          pair_load(a_s, &tm_x, kb * kBlockK, m0, full);
-          pair_load(a_s + kPairA, &tm_w, kb * kBlockK, w0, full);
+          pair_load(a_s, &tm_x, kb * kBlockK, m0, lead);
+          pair_load(a_s + kPairA, &tm_w, kb * kBlockK, w0, lead);
           if (++stage == kPairStages) {
             stage = 0;
             ++pass;
