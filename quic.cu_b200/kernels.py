@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes as C
 import functools
 import os
+import threading
 from types import SimpleNamespace
 
 import torch
@@ -214,6 +215,24 @@ except AttributeError:
         return torch.cuda.current_stream(device).cuda_stream
 
 
+class _Scratch(threading.local):
+    def __init__(self):
+        self.blocks: dict = {}
+
+
+_scratch = _Scratch()
+
+
+def _thread_scratch(kind: str, device: int, stream: int, need: int, least: int) -> torch.Tensor:
+    """Scratch memory (zeroed once) of an operator on a stream.  Calls on a stream are ordered, but one call is
+    several launches, and those of two threads may interleave: each thread has its own, until it ends."""
+    key = (kind, device, stream)
+    t = _scratch.blocks.get(key)
+    if t is None or t.numel() < need:
+        t = _scratch.blocks[key] = torch.zeros(max(need, least), dtype=torch.uint8, device=torch.device("cuda", device))
+    return t
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
@@ -274,15 +293,10 @@ class W4Weight:
         return out
 
     def workspace(self, m: int) -> torch.Tensor:
-        """Workspace of a call, shared by every weight on the stream (whose calls are ordered)."""
-        need = _linear_workspace_bytes(m, self.size_n, self.size_k)
+        """Workspace of a call, shared by every weight that the thread uses on the stream."""
         device = self.qw.get_device()
-        key = (device, _raw_stream(device))
-        ws = _linear_workspace.get(key)
-        if ws is None or ws.numel() * 4 < need:
-            ws = torch.zeros((max(need, 1 << 22) + 3) // 4, dtype=torch.float32, device=self.qw.device)
-            _linear_workspace[key] = ws
-        return ws
+        return _thread_scratch("linear", device, _raw_stream(device), _linear_workspace_bytes(m, self.size_n, self.size_k),
+                               1 << 22)
 
     @property
     def weight_bytes(self) -> int:
@@ -343,7 +357,6 @@ def _linear_workspace_bytes(m: int, n: int, k: int) -> int:
     return lib().quic_w4a16_workspace_bytes(m, n, k)
 
 
-_linear_workspace: dict = {}
 MAX_LINEAR_ROWS = 8192  # rows per launch; longer inputs are processed in chunks to bound scratch memory
 
 
@@ -580,10 +593,6 @@ def _attn_plan(b: int, s: int, splits: int) -> tuple[int, int]:
     return splits, (lib().quic_attn_scratch_bytes(b, splits) if splits > 1 else 0)
 
 
-_attn_scratch: dict = {}
-_lm_scratch: dict = {}
-
-
 def lm_head_argmax(x: torch.Tensor, embed: torch.Tensor, norm_weight: torch.Tensor | None = None,
                    eps: float = 1e-6, want_logits: bool = False):
     """Final norm (optional) + tied lm_head + greedy argmax in one kernel.
@@ -593,11 +602,7 @@ def lm_head_argmax(x: torch.Tensor, embed: torch.Tensor, norm_weight: torch.Tens
     x = x.contiguous().view(-1, HIDDEN)
     b, vocab = x.shape[0], embed.shape[0]
     need = lib().quic_lm_head_scratch_bytes(b, vocab)
-    key = (x.device.index, torch.cuda.current_stream().cuda_stream)
-    scratch = _lm_scratch.get(key)
-    if scratch is None or scratch.numel() < need:
-        scratch = torch.zeros(max(need, 1 << 16), dtype=torch.uint8, device=x.device)
-        _lm_scratch[key] = scratch
+    scratch = _thread_scratch("lm_head", x.get_device(), stream_ptr(), need, 1 << 16)
     out = torch.empty(b, dtype=torch.int64, device=x.device)
     logits = torch.empty(b, vocab, dtype=torch.float16, device=x.device) if want_logits else None
     check(lib().quic_lm_head_argmax(ptr(x), ptr(norm_weight), float(eps), ptr(embed), vocab, b,
@@ -637,12 +642,7 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     asked, (splits, need) = splits, _attn_plan(b, s, splits)
     device = q.get_device()
     stream = _raw_stream(device)
-    scratch = None
-    if need > 0:
-        scratch = _attn_scratch.get((device, stream))
-        if scratch is None or scratch.numel() < need:
-            scratch = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=q.device)
-            _attn_scratch[(device, stream)] = scratch
+    scratch = _thread_scratch("attention", device, stream, need, 1 << 20) if need > 0 else None
     rc = lib().quic_attn_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
                                 ptr(pad_lens), None, s, scale, out.data_ptr(), b, splits if asked > 0 else 0,
                                 ptr(scratch), stream)

@@ -1,0 +1,65 @@
+"""Stand-alone operators called from several threads on one stream: a call that is several launches keeps its
+scratch memory to itself."""
+
+from __future__ import annotations
+
+import threading
+
+import pytest
+import torch
+
+from quic_cu_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def _linear(seed):
+    """A packed linear whose K is split: partial sums and their sum are two launches."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    w = kernels.W4Weight(896, 4864, torch.device("cuda"))
+    w.qw.random_(-2 ** 31, 2 ** 31 - 1, generator=gen)
+    w.zp.random_(0, 255, generator=gen)
+    w.sc.copy_(torch.rand(w.sc.shape, device="cuda", generator=gen) * 0.02)
+    x = torch.randn(100 + seed, 4864, device="cuda", generator=gen).half()
+    return lambda: kernels.w4a16_linear(w, x)
+
+
+def _pair_linear(seed):
+    """Rows enough for the pair GEMM, which unpacks the weight into its scratch first."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    w = kernels.W4Weight(9728, 896, torch.device("cuda"))
+    w.qw.random_(-2 ** 31, 2 ** 31 - 1, generator=gen)
+    w.zp.random_(0, 255, generator=gen)
+    w.sc.copy_(torch.rand(w.sc.shape, device="cuda", generator=gen) * 0.02)
+    x = torch.randn(700 + seed, 896, device="cuda", generator=gen).half()
+    return lambda: kernels.w4a16_linear(w, x)
+
+
+def _head(seed):
+    """More rows than the candidates of one launch: two launches and a clear between them."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(200 + seed, 896, device="cuda", generator=gen).half()
+    table = torch.randn(2048, 896, device="cuda", generator=gen).half()
+    return lambda: kernels.lm_head_argmax(x, table)[0]
+
+
+@pytest.mark.parametrize("make", [_linear, _pair_linear, _head])
+def test_two_threads_on_one_stream(make):
+    calls = [make(seed) for seed in range(3)]
+    want = [call() for call in calls]
+    got = [[] for _ in calls]
+    start = threading.Barrier(len(calls))
+
+    def work(i):
+        start.wait()
+        for _ in range(300):
+            got[i].append(calls[i]())
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for w, outs in zip(want, got):
+        assert len(outs) == 300 and all(torch.equal(o, w) for o in outs)
