@@ -173,17 +173,11 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
 
 // (head dim, token, KV head, row) over planes with any strides; tokens past the end read as zero
 int make_kv_map(CUtensorMap* map, const void* p, int64_t stride_b, int64_t stride_h, int b, int s) {
-  EncodeTiledFn fn = encode_tiled();
-  QUIC_REQUIRE(fn != nullptr, QUIC_E_CUDA, "attn_decode: cuTensorMapEncodeTiled is not available");
   const cuuint64_t dims[4] = {(cuuint64_t)kHeadDim, (cuuint64_t)s, (cuuint64_t)kKvHeads, (cuuint64_t)b};
   const cuuint64_t strides[3] = {kHeadDim * 2, (cuuint64_t)stride_h * 2, (cuuint64_t)stride_b * 2};
   const cuuint32_t box[4] = {kHeadDim, kWarpChunk, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(p), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  QUIC_REQUIRE(r == CUDA_SUCCESS, QUIC_E_CUDA, "attn_decode: cuTensorMapEncodeTiled failed");
-  return QUIC_OK;
+  return make_tiled_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, p, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
 }  // namespace

@@ -178,20 +178,36 @@ inline EncodeTiledFn encode_tiled() {
   return fn;
 }
 
+// Tiled map of a tensor of `rank` dimensions, innermost first; elements past the end read as zero.  A thread that has
+// made no runtime call yet has no current context, and this may be its first: it is then given the device's.
+inline int make_tiled_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* ptr, const cuuint64_t* dims,
+                          const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle,
+                          CUtensorMapL2promotion promotion) {
+  EncodeTiledFn fn = encode_tiled();
+  QUIC_REQUIRE(fn != nullptr, QUIC_E_CUDA, "tensor map: cuTensorMapEncodeTiled is not available");
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  auto encode = [&] {
+    return fn(map, type, (cuuint32_t)rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+              promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r != CUDA_SUCCESS) {
+    int dev = 0;
+    QUIC_CUDA(cudaGetDevice(&dev));
+    QUIC_CUDA(cudaSetDevice(dev));
+    r = encode();
+  }
+  QUIC_REQUIRE(r == CUDA_SUCCESS, QUIC_E_CUDA, "tensor map: cuTensorMapEncodeTiled failed");
+  return QUIC_OK;
+}
+
 // 2-D row-major tensor [rows, cols] of `elem_bytes` elements, box [box_rows, box_cols].
 inline int make_map(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, const void* ptr, uint64_t rows,
-             uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle) {
-  EncodeTiledFn fn = encode_tiled();
-  QUIC_REQUIRE(fn != nullptr, QUIC_E_CUDA, "w4a16_linear: cuTensorMapEncodeTiled is not available");
+                    uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle) {
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * (uint64_t)elem_bytes};
   const cuuint32_t box[2] = {box_cols, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(map, type, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  QUIC_REQUIRE(r == CUDA_SUCCESS, QUIC_E_CUDA, "w4a16_linear: cuTensorMapEncodeTiled failed");
-  return QUIC_OK;
+  return make_tiled_map(map, type, 2, ptr, dims, strides, box, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
 

@@ -63,3 +63,27 @@ def test_two_threads_on_one_stream(make):
     torch.cuda.synchronize()
     for w, outs in zip(want, got):
         assert len(outs) == 300 and all(torch.equal(o, w) for o in outs)
+
+
+def _dense_linear(seed):
+    w = kernels.F16Weight(896, 896, torch.device("cuda"))
+    w.w.normal_(generator=torch.Generator(device="cuda").manual_seed(seed))
+    x = torch.randn(200, 896, device="cuda").half()
+    return lambda: kernels.w4a16_linear(w, x)
+
+
+def _attention(seed):
+    q, k, v = (torch.randn(2, h, n, 64, device="cuda").half() for h, n in ((14, 1), (2, 700), (2, 700)))
+    return lambda: kernels.flash_attn_decode().forward(q, k, v)
+
+
+@pytest.mark.parametrize("make", [_dense_linear, _attention])
+def test_a_thread_may_start_with_a_kernel_of_the_library(make):
+    """The call is the thread's first use of CUDA: no context is current in it yet."""
+    call = make(1)
+    want, got = call(), []
+    torch.cuda.synchronize()
+    thread = threading.Thread(target=lambda: got.append(call()))
+    thread.start()
+    thread.join()
+    assert len(got) == 1 and torch.equal(got[0], want)
