@@ -449,6 +449,9 @@ int quic_graph_destroy(void *graph);
  *    bounded waits, kernels/cuda/marlin.cu:1467-1476).
  * ---------------------------------------------------------------------- */
 int32_t quic_persist_max_rows(void);
+/* 1 if the current device can hold the kernel (148 SMs, cooperative launch),
+ * else 0: quic_decode_step then serves every batch. */
+int32_t quic_persist_device_ok(void);
 int64_t quic_persist_stream_bytes(int32_t n_layers);
 int64_t quic_persist_stream_bytes_f16(int32_t n_layers); /* of an un-quantised model */
 int64_t quic_persist_sync_bytes(void);

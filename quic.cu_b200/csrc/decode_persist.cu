@@ -1835,15 +1835,24 @@ struct LaunchOrder {
 };
 LaunchOrder g_order[64];
 
+// Whether all CTAs can be resident on the device at once (MIG and MPS limits show in its count of SMs).
+bool device_holds_kernel(int dev) {
+  int sms = 0, coop = 0, smem = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return sms >= kCtas && coop != 0 && smem >= kSmemMax;
+}
+
 template <int MR, bool F16>
 int launch_token_kernel(const PersistArgs& pa, int dev, cudaStream_t st) {
   static bool configured[64] = {};
   constexpr int smem = SL<MR, F16>::total;
   if (!configured[dev]) {
-    int sms = 0, coop = 0;
-    QUIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    QUIC_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    QUIC_REQUIRE(sms >= kCtas && coop != 0, QUIC_E_SHAPE,
+    QUIC_REQUIRE(device_holds_kernel(dev), QUIC_E_SHAPE,
                  "decode_persist: needs 148 SMs and cooperative launch (every CTA must be resident)");
     QUIC_CUDA(cudaFuncSetAttribute(token_kernel<MR, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int per_sm = 0;
@@ -1890,6 +1899,15 @@ inline bool dense_model(const quic_model_t* m) { return m->layers[0].qkv.w16 != 
 using namespace quic;
 
 extern "C" int32_t quic_persist_max_rows(void) { return kMaxRows; }
+
+extern "C" int32_t quic_persist_device_ok(void) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return device_holds_kernel(dev) ? 1 : 0;
+}
 
 extern "C" int64_t quic_persist_stream_bytes(int32_t n_layers) { return stream_bytes<false>(n_layers); }
 extern "C" int64_t quic_persist_stream_bytes_f16(int32_t n_layers) { return stream_bytes<true>(n_layers); }

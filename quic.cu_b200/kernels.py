@@ -164,6 +164,7 @@ SIGNATURES = {
     "quic_graph_run_host": (C.c_int, [_P, _P, _P, _P, C.c_int32, _P, _P, C.c_int32]),
     "quic_graph_destroy": (C.c_int, [_P]),
     "quic_persist_max_rows": (_I32, []),
+    "quic_persist_device_ok": (_I32, []),
     "quic_persist_stream_bytes": (_I64, [_I32]),
     "quic_persist_stream_bytes_f16": (_I64, [_I32]),
     "quic_persist_sync_bytes": (_I64, []),

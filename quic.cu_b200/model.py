@@ -199,6 +199,7 @@ class QUICForCausalLM:
         self.use_persist = PERSIST
         self.dense = False  # True: un-quantised fp16 weights (F16Weight), the dense kernels
         self._wstream: torch.Tensor | None = None
+        self._persist_device: bool | None = None  # whether the device can hold the persistent kernel
 
     # ---- weights -------------------------------------------------------------
     def load_state(self, weights: dict) -> None:
@@ -364,7 +365,9 @@ class QUICForCausalLM:
         if self.use_persist is False or (self.use_persist is None and not _persist_pays(self.dense, batch, ctx)):
             return False
         lib = K.lib()
-        return (batch <= lib.quic_persist_max_rows() and self.vocab >= 296
+        if self._persist_device is None:  # (a MIG slice or an MPS limit may leave too few SMs: the kernel chain)
+            self._persist_device = bool(lib.quic_persist_device_ok())
+        return (self._persist_device and batch <= lib.quic_persist_max_rows() and self.vocab >= 296
                 and lib.quic_persist_stream_bytes(self.n_layers) > 0
                 and lib.quic_persist_pick_splits(batch, ctx) <= 16)
 

@@ -1,0 +1,26 @@
+"""Which decode batches take the persistent kernel: the device has to hold it (no GPU needed here)."""
+
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+
+from quic_cu_b200 import kernels, model
+from quic_cu_b200.checkpoint import qwen_config_dict
+
+
+@pytest.mark.parametrize("asked", [None, True])
+@pytest.mark.parametrize("dense", [False, True])
+def test_a_device_with_fewer_sms_keeps_the_kernel_chain(monkeypatch, asked, dense):
+    real = kernels.lib()
+    fits = [1]
+    fake = SimpleNamespace(quic_persist_device_ok=lambda: fits[0], quic_persist_max_rows=real.quic_persist_max_rows,
+                           quic_persist_stream_bytes=real.quic_persist_stream_bytes,
+                           quic_persist_pick_splits=real.quic_persist_pick_splits)
+    monkeypatch.setattr(kernels, "lib", lambda: fake)
+    batches = [(rows, ctx) for rows in (2, 5, 16) for ctx in (128, 1024)]
+    for fits[0], want in ((1, True), (0, False)):
+        net = model.QUICForCausalLM(qwen_config_dict(24, 151936), device="cpu")
+        net.use_persist, net.dense = asked, dense
+        assert [net.persist_ok(*b) for b in batches] == [want] * len(batches)
