@@ -159,13 +159,20 @@ class _DecodePlan:
 
 def _persist_pays(dense: bool, batch: int, ctx: int) -> bool:
     """Where the persistent kernel beats the kernel chain, from B200 measurements (us per step,
-    persistent / chain).  One packed row: 342 / 347 while the context is one attention split (768
-    tokens), 413 / 353 beyond.  Two rows: 373 / 462 at 512 tokens, 455 / 465 at 2100, 538 / 689 at
-    7000.  3..16 rows: 402 / 570 (3 x 300), 498 / 618 (4 x 1000), 445 / 667 (8 x 1000), 500 / 704
-    (16 x 300), 660 / 784 (16 x 2000), equal at 3000-4000 tokens.  fp16 weights: 348 / 494 at one
-    row, 420 / 497 at 2100 tokens, 416 / 899 at eight rows."""
+    persistent / chain).  One packed row: up to 512 tokens the chain's attention is one CTA without a
+    merge and ahead, 329 / 325 at 16 tokens, 332 / 323 at 230, 340 / 339 at 440, 350 / 333 at 500 (behind
+    at 48 only, 325 / 328); from there to 768, one split of the persistent kernel, 345 / 353 at 520, 354 / 354 at 600,
+    349 / 359 at 680, 360 / 358 at 745; beyond, 412 / 350 at 900.  Two rows: 352 / 430 at 16 tokens,
+    373 / 462 at 512, 455 / 465 at 2100, 538 / 689 at 7000.  3..16 rows: 402 / 570 (3 x 300), 498 / 618
+    (4 x 1000), 445 / 667 (8 x 1000), 473 / 685 (16 x 16), 500 / 704 (16 x 300), 660 / 784 (16 x 2000), equal at
+    3000-4000 tokens.  fp16 weights: 347 / 473 at one row of 16 tokens, 348 / 494 at 512, 420 / 497 at 2100,
+    416 / 899 at eight rows.
+
+    A burst holds every SM, so a prefill beside it (Engine with ``overlap_prefill``) runs before or after it;
+    the queue is still served sooner than with the chain (ms, persistent / chain, both with overlap:
+    2 slots 499 / 555, 8 slots 368 / 469, 8 slots with prompts of 400..2000 tokens 474 / 480, 16 slots 273 / 364)."""
     if batch == 1:
-        return ctx <= (4096 if dense else 768)
+        return ctx <= 4096 if dense else 512 < ctx <= 768
     return ctx <= (8192 if batch == 2 else 4096 if dense else 2048)
 
 

@@ -1,4 +1,4 @@
-"""Which decode batches take the persistent kernel: the device has to hold it (no GPU needed here)."""
+"""Which decode batches take the persistent kernel (no GPU needed here)."""
 
 from __future__ import annotations
 
@@ -24,3 +24,11 @@ def test_a_device_with_fewer_sms_keeps_the_kernel_chain(monkeypatch, asked, dens
         net = model.QUICForCausalLM(qwen_config_dict(24, 151936), device="cpu")
         net.use_persist, net.dense = asked, dense
         assert [net.persist_ok(*b) for b in batches] == [want] * len(batches)
+
+
+def test_one_packed_row_takes_it_where_it_was_measured_ahead():
+    """Context bounds as decode() rounds them up: the chain serves 1..512 tokens and more than 768."""
+    takes = {ctx for ctx in range(128, 4097, 128) if model._persist_pays(False, 1, ctx)}
+    assert takes == {640, 768}
+    assert all(model._persist_pays(True, 1, ctx) for ctx in (128, 512, 4096))
+    assert all(model._persist_pays(dense, rows, 512) for dense in (False, True) for rows in (2, 3, 16))
