@@ -660,9 +660,10 @@ extern "C" int quic_attn_decode(const void* q, const void* k, const void* v, int
                QUIC_E_ARG, "attn_decode: K/V must be 16-byte aligned with strides multiple of 8");
   // Left to choose (splits <= 0): the flow kernel, over any planes that a tensor map can describe.  The
   // split kernels keep caches of up to 256 tokens with more rows than SMs: their tiles are fewer than a
-  // CTA's six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).
+  // CTA's six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).  It reads q two values at a
+  // time; the split kernel for long caches of few rows reads one.
   const int64_t widest = int64_t(1) << 38;
-  if (splits <= 0 && !(s_max <= 256 && b > 148) && stride_b > 0 && stride_h > 0 && stride_b < widest &&
+  if (splits <= 0 && !(s_max <= 256 && b > 148) && (uintptr_t)q % 4 == 0 && stride_b > 0 && stride_h > 0 && stride_b < widest &&
       stride_h < widest && tc_status_words() != nullptr) {
     AttnArgs a = {};
     a.q = (const half*)q;
@@ -696,6 +697,7 @@ extern "C" int quic_attn_decode(const void* q, const void* k, const void* v, int
   a.out = (half*)out;
   a.use_mma = ((int64_t)b * s_max >= 8192) ? 1 : 0;  // enough work for the throughput variant
   a.small = (!a.use_mma && (int64_t)splits * kWarpChunk >= s_max) ? 1 : 0;
+  QUIC_REQUIRE((uintptr_t)q % 8 == 0 || (!a.use_mma && !a.small), QUIC_E_ARG, "attn_decode: q must be 8-byte aligned");
   if (splits > 1) attn_carve_scratch(scratch, b, splits, &a);
   QUIC_CUDA(launch_attn(a, b, (cudaStream_t)stream, false));
   return QUIC_OK;

@@ -42,3 +42,30 @@ def test_attention_over_row_ranges(rows, tokens):
     want = torch.einsum("bht,bhtd->bhd", prob, vf)
     assert torch.isfinite(out).all()
     assert (out.float() - want).norm() <= 2e-3 * want.norm()
+
+
+@pytest.mark.parametrize("rows,tokens,offset", [(1, 4096, 1), (3, 2500, 1), (2, 3000, 3), (1, 700, 2), (20, 900, 2), (1, 4096, 2)])
+def test_queries_at_any_address_that_was_taken(rows, tokens, offset):
+    """q starts `offset` values into its allocation; keys and values outside the rows' tokens are NaN."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + tokens)
+    buf = torch.randn(rows * HEADS * HD + 8, device="cuda", generator=gen).half()
+    q = buf[offset:offset + rows * HEADS * HD].view(rows, HEADS, 1, HD)
+    k, v = (torch.randn(rows, KV, tokens, HD, device="cuda", generator=gen).half() for _ in range(2))
+    pads = torch.tensor([(37 * i + 5) % (tokens // 2) for i in range(rows)], dtype=torch.int32, device="cuda")
+    dead = torch.arange(tokens, device="cuda") < pads[:, None]
+    if offset % 2 == 0:  # (the scalar kernel multiplies what it masks)
+        for t in (k, v):
+            t.masked_fill_(dead[:, None, :, None], float("nan"))
+    got = kernels.flash_attn_decode().forward(q, k, v, 0.125, pads)
+    kf, vf = (t.float().masked_fill(dead[:, None, :, None], 0).repeat_interleave(HEADS // KV, 1) for t in (k, v))
+    score = torch.einsum("bhod,bhtd->bhot", q.float(), kf) * 0.125
+    want = torch.softmax(score.masked_fill(dead[:, None, None], float("-inf")), -1) @ vf
+    assert (got.float() - want).norm() <= 2e-3 * want.norm()
+
+
+@pytest.mark.parametrize("rows,tokens", [(1, 100), (16, 1024)])
+def test_queries_at_an_odd_address_are_refused_where_they_are_read_in_pairs(rows, tokens):
+    buf = torch.zeros(rows * HEADS * HD + 8, device="cuda").half()
+    k = torch.zeros(rows, KV, tokens, HD, device="cuda").half()
+    with pytest.raises(RuntimeError, match="aligned"):
+        kernels.flash_attn_decode().forward(buf[1:1 + rows * HEADS * HD].view(rows, HEADS, 1, HD), k, k)
