@@ -21,6 +21,7 @@ import ctypes as C
 import json
 import numbers
 import os
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -206,6 +207,7 @@ class QUICForCausalLM:
         self.use_persist = PERSIST
         self.dense = False  # True: un-quantised fp16 weights (F16Weight), the dense kernels
         self._wstream: torch.Tensor | None = None
+        self._wstream_lock = threading.Lock()
         self._persist_device: bool | None = None  # whether the device can hold the persistent kernel
 
     # ---- weights -------------------------------------------------------------
@@ -356,15 +358,20 @@ class QUICForCausalLM:
     # ---- persistent decode kernel ------------------------------------------------------
     def persist_stream(self) -> torch.Tensor:
         """The weight stream of the persistent kernel, packed on first use from the device
-        matrices (a second copy of the layer weights, 9 MB per layer, 32 MB in fp16)."""
+        matrices (a second copy of the layer weights, 9 MB per layer, 32 MB in fp16).  Complete when the call
+        returns: launches on any stream and of any thread read it."""
         if self._wstream is None:
-            lib = K.lib()
-            need = (lib.quic_persist_stream_bytes_f16 if self.dense else lib.quic_persist_stream_bytes)(self.n_layers)
-            if need <= 0:
-                raise RuntimeError("persistent decode: unsupported layer count")
-            t = torch.empty(need, dtype=torch.uint8, device=self.device)
-            K.check(K.lib().quic_persist_pack(C.byref(self._c_model), K.ptr(t), K.stream_ptr()), "persist_pack")
-            self._wstream = t
+            with self._wstream_lock:
+                if self._wstream is None:
+                    lib = K.lib()
+                    size = lib.quic_persist_stream_bytes_f16 if self.dense else lib.quic_persist_stream_bytes
+                    need = size(self.n_layers)
+                    if need <= 0:
+                        raise RuntimeError("persistent decode: unsupported layer count")
+                    t = torch.empty(need, dtype=torch.uint8, device=self.device)
+                    K.check(lib.quic_persist_pack(C.byref(self._c_model), K.ptr(t), K.stream_ptr()), "persist_pack")
+                    torch.cuda.current_stream().synchronize()
+                    self._wstream = t
         return self._wstream
 
     def persist_ok(self, batch: int, ctx: int) -> bool:

@@ -250,3 +250,30 @@ def test_a_context_hint_below_the_position_loses_no_token(persist_net, lens, hin
     ok, err = _close(logits[0], logits[1])
     assert ok, err
     assert (kv.float() - cache.kv.float()).abs().max() <= 5e-2
+
+
+def test_the_weight_stream_is_complete_when_it_is_handed_out(persist_net):
+    """It is packed on the stream of the first caller, behind whatever that stream still has to do; callers on other
+    streams and of other threads read the same copy."""
+    import threading
+
+    net = persist_net
+    want = net.persist_stream()
+    kept, net._wstream = want.clone(), None
+    torch.cuda.synchronize()
+    got = []
+
+    def first_use():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda._sleep(20_000_000)
+            t = net.persist_stream()
+            got.append((t.data_ptr(), torch.cuda.current_stream().query()))
+
+    threads = [threading.Thread(target=first_use) for _ in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    # the last caller's own sleep may still run, the packing may not
+    assert len({p for p, _ in got}) == 1 and any(done for _, done in got)
+    assert torch.equal(net.persist_stream(), kept)
