@@ -24,9 +24,11 @@ struct LmSmem {
   static constexpr uint32_t kA = kTileN * 128;
   static constexpr uint32_t kB = ((uint32_t)MT * 128u + 1023u) & ~1023u;
   static constexpr uint32_t kStage = kA + kB;
-  // Several CTAs share an SM, so loads, MMAs and epilogues of different tiles overlap: two stages and one CTA
-  // more beat three (us, 3 -> 2 stages: 50.8 -> 50.4 at 16 rows, 54.9 -> 52.8 at 32, 73.2 -> 67.1 at 128) but at
-  // 64 rows (57.0 -> 57.3).
+  // Several CTAs share an SM, so loads, MMAs and epilogues of different tiles overlap: two stages and one CTA more
+  // beat three, alone and inside the steps that use them, but for 33..64 rows (us, two / three stages, alone: 3 rows
+  // 49.9 / 51.8, 32 rows 52.3 / 54.8, 48 rows 59.5 / 57.3, 64 rows 57.8 / 57.2, 128 rows 69 / 75; steps of 300 tokens:
+  // 3 rows 569 / 602, 8 rows 626 / 660, 16 rows 701.9 / 704.1, 32 rows 691.4 / 692.4, 48 rows 768.5 / 766.1, 64 rows
+  // 774.4 / 774.8; runs of one form differ by 0.3).
   static constexpr int kStages = MT == 64 ? 3 : 2;
   static constexpr uint32_t kTotal = kStages * kStage + 1024;
 };
