@@ -1497,7 +1497,7 @@ __device__ __forceinline__ bool phase_lm_head(uint32_t last_no) {
     }
     if (lane == 0) {
       const uint32_t idx = ~(uint32_t)key;
-      s_tok[m] = idx < (uint32_t)a.vocab ? (int)idx : a.vocab - 1;
+      s_tok[m] = idx < (uint32_t)a.vocab ? (int)idx : 0;  // (no logit above -inf: token 0, as the chain)
     }
   }
   return !cbar_or(bad);

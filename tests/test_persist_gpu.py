@@ -277,3 +277,26 @@ def test_the_weight_stream_is_complete_when_it_is_handed_out(persist_net):
     # the last caller's own sleep may still run, the packing may not
     assert len({p for p, _ in got}) == 1 and any(done for _, done in got)
     assert torch.equal(net.persist_stream(), kept)
+
+
+@pytest.mark.parametrize("bits", [0x7E00, 0xFFFF], ids=hex)
+def test_a_row_of_nan_ends_like_the_chain_and_leaves_the_others_alone(persist_net, bits):
+    """A row whose input is NaN has no logit to choose from: token 0 in either form; no wait runs out over it
+    (0xFFFF pairs are what an empty exchange word decodes to), and the row beside it is untouched."""
+    net = persist_net
+    gen = torch.Generator().manual_seed(5)
+    prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in (12, 40)]
+    kept, got = net.embed[77].clone(), []
+    try:
+        for persist in (True, False):
+            net.use_persist = persist
+            cache = net.new_cache(n_slots=2, s_max=128)
+            net.prefill(cache, [0, 1], prompts)
+            cache.tok[0] = 77
+            net.embed[77].view(torch.int16).fill_(bits - 0x10000 if bits >= 0x8000 else bits)
+            got.append(net.decode(cache, [0, 1], 1))
+            net.embed[77] = kept
+            assert not persist or net.persist_status(cache) == 0
+    finally:
+        net.embed[77] = kept
+    assert got[0] == got[1] and got[0][0] == [0]
