@@ -226,11 +226,15 @@ _scratch = _Scratch()
 
 def _thread_scratch(kind: str, device: int, stream: int, need: int, least: int) -> torch.Tensor:
     """Scratch memory (zeroed once) of an operator on a stream.  Calls on a stream are ordered, but one call is
-    several launches, and those of two threads may interleave: each thread has its own, until it ends."""
+    several launches, and those of two threads may interleave: each thread has its own, until it ends.  A block
+    made during a graph capture is the graph's, cleared by it, and no other call's."""
     key = (kind, device, stream)
     t = _scratch.blocks.get(key)
     if t is None or t.numel() < need:
-        t = _scratch.blocks[key] = torch.zeros(max(need, least), dtype=torch.uint8, device=torch.device("cuda", device))
+        where = torch.device("cuda", device)
+        if torch.cuda.is_current_stream_capturing():
+            return torch.zeros(need, dtype=torch.uint8, device=where)
+        t = _scratch.blocks[key] = torch.zeros(max(need, least), dtype=torch.uint8, device=where)
     return t
 
 

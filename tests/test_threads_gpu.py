@@ -1,5 +1,5 @@
-"""Stand-alone operators called from several threads on one stream: a call that is several launches keeps its
-scratch memory to itself."""
+"""Stand-alone operators called from several threads on one stream, or captured into graphs: a call that is several
+launches keeps its scratch memory to itself."""
 
 from __future__ import annotations
 
@@ -87,3 +87,27 @@ def test_a_thread_may_start_with_a_kernel_of_the_library(make):
     thread.start()
     thread.join()
     assert len(got) == 1 and torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("make", [_linear, _pair_linear, _head])
+def test_a_captured_call_has_scratch_of_its_own(make):
+    """Two graphs, the second replayed alone and then both: what one clears or leaves behind is not the other's."""
+    calls = [make(seed) for seed in (1, 2)]
+    want = [call() for call in calls]
+    torch.cuda.synchronize()
+    kept = set(kernels._scratch.blocks)
+    graphs, outs = [], []
+    for call in calls:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(call())
+        graphs.append(g)
+    assert set(kernels._scratch.blocks) == kept
+    for order in ((1,), (0, 1), (1, 0, 1)):
+        for o in outs:
+            o.zero_()
+        for i in order:
+            graphs[i].replay()
+        torch.cuda.synchronize()
+        for i in set(order):
+            assert torch.equal(outs[i], want[i])
