@@ -279,7 +279,7 @@ def run_gpu(args) -> None:
     layer_bytes = step_bytes - lm_bytes                     # W4 weights of 24 layers + K/V read and written
     per_layer = {"qkv_kernel<1>": 536256 + 2304 + 1792 + 512, "attn_decode_cta_kernel<true>": 512 * (mean_ctx + 1),
                  "oproj_kernel<1>": 417088, "gateup_kernel<1>": 4528384 + 1792, "down_kernel<1>": 2264192}
-    # one packed row up to 768 tokens: the persistent kernel, one launch per burst of BURST tokens
+    # one packed row of 513..768 tokens: the persistent kernel, one launch per burst of BURST tokens
     persist = bool(net.persist_ok(1, PROMPT_LEN + GEN_TOKENS))
     kernels = []
     for name, share in {} if persist else prof["layer_kernel_share"].items():
@@ -290,7 +290,7 @@ def run_gpu(args) -> None:
                         "timing": "(token time - live lm_head time) / layers x the kernel's share of the layer "
                                   "kernels' time in the committed ncu launch list"})
     if persist:
-        kernels.append({"kernel": "decode_persist_kernel<1>", "launches_per_token": 1 / BURST,
+        kernels.append({"kernel": "token_kernel<1, 0>", "launches_per_token": 1 / BURST,
                         "algorithmic_bytes": step_bytes, "us_per_token": us_per_token, "achieved": step_gbs,
                         "unit": "GB/s", "frac": step_gbs / peak, "share_of_step": 1.0,
                         "timing": "the timed region itself: every burst is one launch of this kernel"})
@@ -309,7 +309,9 @@ def run_gpu(args) -> None:
                 "frac": layer_bytes / layers_us / 1e3 / peak, "peak_kind": f"of {peak_kind}",
                 "share_of_step": layers_us / us_per_token, "us_per_token": layers_us,
                 "algorithmic_bytes": layer_bytes, "traffic": None,
-                "timing": "token time (CUDA events over the timed region) minus the lm_head kernel's live time"}
+                "timing": "token time (CUDA events over the timed region) minus the lm_head kernel's live time" +
+                          (" measured alone (here the lm_head is a phase of the token's kernel, so this is an estimate "
+                           "of the other phases)" if persist else "")}
     roofline_step = {"bound": "hbm", "scope": "whole decode step" + ("" if persist else " (121 kernels)"), "achieved": step_gbs,
                      "peak": peak, "unit": "GB/s", "frac": step_gbs / peak, "us_per_token": us_per_token,
                      "algorithmic_bytes": step_bytes}
@@ -615,8 +617,8 @@ def _time_decode(net, device, rows: int, ctx: int = PROMPT_LEN, steps: int = 64,
 
 
 def measure_rows_sweep(net, device) -> dict:
-    """Decode step time against the number of rows: one row on the GEMV chain, two on its
-    two-row form, 3..16 on the mma.sync chain, more on the tcgen05 step."""
+    """Decode step time against the number of rows: up to 16 rows in the persistent kernel (one packed
+    row of up to 512 tokens on the GEMV chain), more on the tcgen05 step."""
     out = {}
     for rows in (1, 2, 3, 4, 8, 16, 32):
         us = _time_decode(net, device, rows)
@@ -661,21 +663,28 @@ def measure_prefill(net, device) -> dict:
             K.lib().quic_set_prefill_tensor_attention(mode)
             for _ in range(3):
                 K.attn_prefill(q, kc, vc, starts, lens, slots, n, 0.125)
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                for _ in range(10):
+                    K.attn_prefill(q, kc, vc, starts, lens, slots, n, 0.125)
+            graph.replay()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            for _ in range(10):
-                K.attn_prefill(q, kc, vc, starts, lens, slots, n, 0.125)
+            graph.replay()
             e1.record()
             torch.cuda.synchronize()
             us = e0.elapsed_time(e1) * 100
+            del graph
             kernels.append({"sequences": seqs, "tokens": n, "kernel": name, "us": us, "tflops": flops / us / 1e6})
         K.lib().quic_set_prefill_tensor_attention(1)
     return {"ttft_ms": ttft_ms, "prompts": n_seq, "prompt_tokens": n, "attention": kernels,
-            "note": "W4A16 linears on the tcgen05 GEMM at M = 32768, attention on tcgen05; causal flops counted"}
+            "note": "linears at M = 32768 as fp16 GEMMs on SM pairs (packed weights unpacked once a layer), attention on "
+                    "tcgen05; attention timed as a CUDA graph of launches, causal flops counted"}
 
 
 def measure_dense(device) -> dict:
-    """The un-quantised fp16 model through the same step: one-row decode (GEMV chain over
+    """The un-quantised fp16 model through the same step: one-row decode (persistent kernel over
     988 MB of weights per token) and 64 rows (tcgen05 fp16 GEMM)."""
     from quic_cu_b200 import model as qmodel
     from quic_cu_b200.checkpoint import qwen_config_dict, synthetic_dense_checkpoint
