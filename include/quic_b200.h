@@ -106,8 +106,8 @@ int quic_w4_dequant(const quic_w4_t *w, void *out_f16, void *stream);
  * rows the tensor path is an SM pair GEMM (N a multiple of 192, 224 or 256).
  * The tensor path wants x, w and y 16-byte aligned; a dense weight takes any y
  * and any bias, at less speed.  `workspace` (>= quic_w4a16_workspace_bytes)
- * holds split-K partials; its first 16 KB (arrival counters of the tensor
- * path) must be zero before the first call and are left zero. */
+ * holds split-K partials; its first 16 KB are reserved.  It need not be
+ * initialised and one call's contents mean nothing to the next. */
 int quic_w4a16_linear(const void *x_f16, const quic_w4_t *w, void *y_f16,
                       int32_t m, int32_t use_tensor, void *workspace,
                       void *stream);
@@ -245,9 +245,10 @@ int64_t quic_lm_head_scratch_bytes(int32_t b, int32_t vocab);
  * (flash_attn_decode.cu:118-121).  `scratch` holds the split partials and the
  * arrival counters: quic_attn_scratch_bytes(b, splits) bytes, whose first
  * b*2*4 bytes (the counters) must be zero before the first call; the kernel
- * leaves them zero.  `splits` 0 lets the library choose: its streaming kernel,
- * which uses no scratch, or quic_attn_pick_splits(b, s_max) splits (size the
- * scratch for that count). */
+ * leaves them zero.  `splits` 0 lets the library choose: where
+ * quic_attn_decode_streams(b, s_max) is 1 its streaming kernel, which uses no
+ * scratch (q 4-byte aligned), else quic_attn_pick_splits(b, s_max) splits (size
+ * the scratch for that count; without scratch there is one). */
 int quic_attn_decode(const void *q_f16, const void *k_f16, const void *v_f16,
                      int64_t stride_b, int64_t stride_h, const int32_t *start,
                      const int32_t *end, int32_t s_max, float scale,
@@ -285,6 +286,7 @@ int quic_attn_decode_cta(const void *q_f16, const void *k_f16, const void *v_f16
                          void *out_f16, int32_t b, void *stream);
 int32_t quic_attn_decode_cta_max_tokens(void);
 int32_t quic_attn_pick_splits(int32_t b, int32_t s_max);
+int32_t quic_attn_decode_streams(int32_t b, int32_t s_max);
 int64_t quic_attn_scratch_bytes(int32_t b, int32_t splits);
 
 /* ------------------------------------------------------------------------

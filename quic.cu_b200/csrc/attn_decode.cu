@@ -628,6 +628,10 @@ extern "C" int32_t quic_attn_pick_splits(int32_t b, int32_t s_max) {
   return s;
 }
 
+// The split kernels keep caches of up to 256 tokens with more rows than SMs: their tiles are fewer than a flow CTA's
+// six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).
+extern "C" int32_t quic_attn_decode_streams(int32_t b, int32_t s_max) { return s_max <= 256 && b > 148 ? 0 : 1; }
+
 extern "C" int64_t quic_attn_scratch_bytes(int32_t b, int32_t splits) {
   if (b < 1 || splits < 1) return 0;
   int64_t counters = counter_bytes(b);
@@ -658,12 +662,10 @@ extern "C" int quic_attn_decode(const void* q, const void* k, const void* v, int
   QUIC_REQUIRE(((uintptr_t)k % 16 == 0) && ((uintptr_t)v % 16 == 0) && stride_b % 8 == 0 &&
                    stride_h % 8 == 0,
                QUIC_E_ARG, "attn_decode: K/V must be 16-byte aligned with strides multiple of 8");
-  // Left to choose (splits <= 0): the flow kernel, over any planes that a tensor map can describe.  The
-  // split kernels keep caches of up to 256 tokens with more rows than SMs: their tiles are fewer than a
-  // CTA's six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).  It reads q two values at a
-  // time; the split kernel for long caches of few rows reads one.
+  // Left to choose (splits <= 0): the flow kernel where it is the faster one, over any planes that a tensor map can
+  // describe.  It reads q two values at a time; the split kernel for long caches of few rows reads one.
   const int64_t widest = int64_t(1) << 38;
-  if (splits <= 0 && !(s_max <= 256 && b > 148) && (uintptr_t)q % 4 == 0 && stride_b > 0 && stride_h > 0 && stride_b < widest &&
+  if (splits <= 0 && quic_attn_decode_streams(b, s_max) && (uintptr_t)q % 4 == 0 && stride_b > 0 && stride_h > 0 && stride_b < widest &&
       stride_h < widest && tc_status_words() != nullptr) {
     AttnArgs a = {};
     a.q = (const half*)q;
@@ -679,7 +681,7 @@ extern "C" int quic_attn_decode(const void* q, const void* k, const void* v, int
     a.out = (half*)out;
     return launch_attn_flow(a, b, tc_status_words(), (cudaStream_t)stream);
   }
-  if (splits <= 0) splits = quic_attn_pick_splits(b, s_max);
+  if (splits <= 0) splits = scratch != nullptr ? quic_attn_pick_splits(b, s_max) : 1;
   QUIC_REQUIRE(splits <= 4096, QUIC_E_SHAPE, "attn_decode: too many splits");
   QUIC_REQUIRE(splits == 1 || scratch != nullptr, QUIC_E_ARG, "attn_decode: scratch required");
   AttnArgs a = {};

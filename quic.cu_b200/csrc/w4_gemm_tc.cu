@@ -26,7 +26,7 @@
 namespace quic {
 namespace {
 
-constexpr int kCounterInts = 4096;  // arrival counters at the head of the split-K workspace
+constexpr int kHeadInts = 4096;  // reserved at the head of the split-K workspace
 
 // Error words of the tensor path: [0] the GEMM, [1] the tensor lm_head.  0 = ok; otherwise
 // (code << 16) | block of the first bounded wait that gave up.
@@ -41,7 +41,6 @@ struct GemmArgs {
   quic_w4_t w;
   half* y;         // [m_total, N]    (splits == 1)
   float* part;     // [splits, m_total, N] fp32 (splits > 1)
-  int* counters;   // one per (n tile, m tile), zero on entry, left zero
   int m_total;
   int kblocks_per_split;
   int mtl;     // batch-row tiles per CTA (2 from 129 rows up)
@@ -527,8 +526,7 @@ int w4a16_gemm_tc(const half* x, const quic_w4_t& w, half* y, int m, float* work
   GemmArgs a = {};
   a.w = w;
   a.y = y;
-  a.counters = reinterpret_cast<int*>(workspace);
-  a.part = workspace + kCounterInts;
+  a.part = workspace + kHeadInts;
   QUIC_REQUIRE((m + mt - 1) / mt <= 65535, QUIC_E_LIMIT, "w4a16_linear: too many rows on the tensor path");
   a.m_total = m;
   a.kblocks_per_split = per;

@@ -286,7 +286,7 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
     QUIC_REQUIRE(workspace != nullptr, QUIC_E_ARG, "w4a16_linear: tensor path needs a workspace");
     return w4a16_gemm_tc((const half*)x, *w, (half*)y, m, (float*)workspace, st, nullptr);
   }
-  // the first 16 KB of the workspace belong to the tensor path's arrival counters
+  // (the first 16 KB of the workspace are reserved)
   float* part = workspace != nullptr ? static_cast<float*>(workspace) + 4096 : nullptr;
   const int ng = w->k / kGroup;
   int splits = (workspace != nullptr && m <= 8) ? gemv_splits(w->n, w->k) : 1;

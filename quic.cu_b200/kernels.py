@@ -149,6 +149,7 @@ SIGNATURES = {
     "quic_attn_decode_cta": (C.c_int, [_P, _P, _P, _I64, _I64, _P, _P, _I32, _F, _P, _I32, _P]),
     "quic_attn_decode_cta_max_tokens": (_I32, []),
     "quic_attn_pick_splits": (_I32, [_I32, _I32]),
+    "quic_attn_decode_streams": (_I32, [_I32, _I32]),
     "quic_attn_scratch_bytes": (_I64, [_I32, _I32]),
     "quic_set_tensor_min_batch": (None, [_I32]),
     "quic_set_prefill_tensor_attention": (None, [C.c_int]),
@@ -224,16 +225,19 @@ class _Scratch(threading.local):
 _scratch = _Scratch()
 
 
-def _thread_scratch(kind: str, device: int, stream: int, need: int, least: int) -> torch.Tensor:
-    """Scratch memory (zeroed once) of an operator on a stream.  Calls on a stream are ordered, but one call is
-    several launches, and those of two threads may interleave: each thread has its own, until it ends.  A block
-    made during a graph capture is the graph's, cleared by it, and no other call's."""
+def _thread_scratch(kind: str, device: int, stream: int, need: int, least: int, head: int) -> torch.Tensor:
+    """Scratch memory of an operator on a stream; its first ``head`` bytes start zeroed and are left so.  Calls on a
+    stream are ordered, but one call is several launches, and those of two threads may interleave: each thread
+    has its own, until it ends.  A block made during a graph capture is the graph's and no other call's."""
     key = (kind, device, stream)
     t = _scratch.blocks.get(key)
     if t is None or t.numel() < need:
         where = torch.device("cuda", device)
         if torch.cuda.is_current_stream_capturing():
-            return torch.zeros(need, dtype=torch.uint8, device=where)
+            t = torch.empty(need, dtype=torch.uint8, device=where)
+            if head:
+                t[:head].zero_()
+            return t
         t = _scratch.blocks[key] = torch.zeros(max(need, least), dtype=torch.uint8, device=where)
     return t
 
@@ -301,7 +305,7 @@ class W4Weight:
         """Workspace of a call, shared by every weight that the thread uses on the stream."""
         device = self.qw.get_device()
         return _thread_scratch("linear", device, _raw_stream(device), _linear_workspace_bytes(m, self.size_n, self.size_k),
-                               1 << 22)
+                               1 << 22, 0)
 
     @property
     def weight_bytes(self) -> int:
@@ -592,9 +596,13 @@ def _gemm_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = 
 
 
 @functools.lru_cache(maxsize=4096)
-def _attn_plan(b: int, s: int, splits: int) -> tuple[int, int]:
-    """(splits, scratch bytes) of a decode attention; ``splits`` 0 = the library's choice."""
-    splits = splits if splits > 0 else lib().quic_attn_pick_splits(b, s)
+def _attn_plan(b: int, s: int, splits: int, paired: bool) -> tuple[int, int]:
+    """(splits to ask for, scratch bytes) of a decode attention; ``splits`` 0 = the library's choice, whose
+    streaming kernel needs no scratch but queries that can be read in pairs."""
+    if splits <= 0:
+        if paired and lib().quic_attn_decode_streams(b, s):
+            return 0, 0
+        splits = lib().quic_attn_pick_splits(b, s)
     return splits, (lib().quic_attn_scratch_bytes(b, splits) if splits > 1 else 0)
 
 
@@ -607,7 +615,7 @@ def lm_head_argmax(x: torch.Tensor, embed: torch.Tensor, norm_weight: torch.Tens
     x = x.contiguous().view(-1, HIDDEN)
     b, vocab = x.shape[0], embed.shape[0]
     need = lib().quic_lm_head_scratch_bytes(b, vocab)
-    scratch = _thread_scratch("lm_head", x.get_device(), stream_ptr(), need, 1 << 16)
+    scratch = _thread_scratch("lm_head", x.get_device(), stream_ptr(), need, 1 << 16, 256)
     out = torch.empty(b, dtype=torch.int64, device=x.device)
     logits = torch.empty(b, vocab, dtype=torch.float16, device=x.device) if want_logits else None
     check(lib().quic_lm_head_argmax(ptr(x), ptr(norm_weight), float(eps), ptr(embed), vocab, b,
@@ -643,14 +651,13 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
                                          ptr(pad_lens), None, s, scale, ptr(out), b, stream_ptr()),
               "attn_decode_cta")
         return out
-    # with splits 0 the library chooses (at most as many as the scratch is sized for, or a kernel without)
-    asked, (splits, need) = splits, _attn_plan(b, s, splits)
+    q_ptr = q.data_ptr()
+    splits, need = _attn_plan(b, s, splits, q_ptr % 4 == 0)
     device = q.get_device()
     stream = _raw_stream(device)
-    scratch = _thread_scratch("attention", device, stream, need, 1 << 20) if need > 0 else None
-    rc = lib().quic_attn_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
-                                ptr(pad_lens), None, s, scale, out.data_ptr(), b, splits if asked > 0 else 0,
-                                ptr(scratch), stream)
+    scratch = _thread_scratch("attention", device, stream, need, 1 << 20, max(8 * b, 1 << 16)) if need > 0 else None
+    rc = lib().quic_attn_decode(q_ptr, k.data_ptr(), v.data_ptr(), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
+                                ptr(pad_lens), None, s, scale, out.data_ptr(), b, splits, ptr(scratch), stream)
     if rc != 0:
         check(rc, "attn_decode")
     return out

@@ -43,7 +43,14 @@ def _head(seed):
     return lambda: kernels.lm_head_argmax(x, table)[0]
 
 
-@pytest.mark.parametrize("make", [_linear, _pair_linear, _head])
+def _split_attention(seed):
+    """Split partials merged by the CTA that arrives last at a counter."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(4, h, n, 64, device="cuda", generator=gen).half() for h, n in ((14, 1), (2, 2500), (2, 2500)))
+    return lambda: kernels.flash_attn_decode().forward(q, k, v, splits=9)
+
+
+@pytest.mark.parametrize("make", [_linear, _pair_linear, _head, _split_attention])
 def test_two_threads_on_one_stream(make):
     calls = [make(seed) for seed in range(3)]
     want = [call() for call in calls]
@@ -89,7 +96,7 @@ def test_a_thread_may_start_with_a_kernel_of_the_library(make):
     assert len(got) == 1 and torch.equal(got[0], want)
 
 
-@pytest.mark.parametrize("make", [_linear, _pair_linear, _head])
+@pytest.mark.parametrize("make", [_linear, _pair_linear, _head, _split_attention])
 def test_a_captured_call_has_scratch_of_its_own(make):
     """Two graphs, the second replayed alone and then both: what one clears or leaves behind is not the other's."""
     calls = [make(seed) for seed in (1, 2)]
