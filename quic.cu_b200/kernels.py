@@ -225,14 +225,13 @@ class _Scratch(threading.local):
 _scratch = _Scratch()
 
 
-def _thread_scratch(kind: str, device: int, stream: int, need: int, least: int, head: int) -> torch.Tensor:
-    """Scratch memory of an operator on a stream; its first ``head`` bytes start zeroed and are left so.  Calls on a
+def _thread_scratch(key: tuple[str, int, int], need: int, least: int, head: int) -> torch.Tensor:
+    """Scratch memory of (operator, device, stream); its first ``head`` bytes start zeroed and are left so.  Calls on a
     stream are ordered, but one call is several launches, and those of two threads may interleave: each thread
     has its own, until it ends.  A block made during a graph capture is the graph's and no other call's."""
-    key = (kind, device, stream)
     t = _scratch.blocks.get(key)
     if t is None or t.numel() < need:
-        where = torch.device("cuda", device)
+        where = torch.device("cuda", key[1])
         if torch.cuda.is_current_stream_capturing():
             t = torch.empty(need, dtype=torch.uint8, device=where)
             if head:
@@ -301,11 +300,13 @@ class W4Weight:
         check(lib().quic_w4_dequant(C.byref(s), ptr(out), stream_ptr()), "w4_dequant")
         return out
 
-    def workspace(self, m: int) -> torch.Tensor:
-        """Workspace of a call, shared by every weight that the thread uses on the stream."""
+    def workspace(self, m: int, stream: int | None = None) -> torch.Tensor:
+        """Workspace of a call, shared by every weight that the thread uses on the stream (None: the current one)."""
+        need = _linear_workspace_bytes(m, self.size_n, self.size_k)
         device = self.qw.get_device()
-        return _thread_scratch("linear", device, _raw_stream(device), _linear_workspace_bytes(m, self.size_n, self.size_k),
-                               1 << 22, 0)
+        key = ("linear", device, _raw_stream(device) if stream is None else stream)
+        ws = _scratch.blocks.get(key)
+        return ws if ws is not None and ws.numel() >= need else _thread_scratch(key, need, 1 << 22, 0)
 
     @property
     def weight_bytes(self) -> int:
@@ -342,7 +343,7 @@ class F16Weight:
     def dequant(self) -> torch.Tensor:
         return self.w
 
-    def workspace(self, m: int):
+    def workspace(self, m: int, stream: int | None = None):
         return None
 
     @property
@@ -385,7 +386,7 @@ def w4a16_linear(w, x: torch.Tensor, use_tensor: bool | None = None) -> torch.Te
     while done < m:
         rows = min(MAX_LINEAR_ROWS, m - done)
         rc = run(xp + 2 * done * w.size_k, ref, yp + 2 * done * w.size_n, rows, 1 if use_tensor else 0,
-                 ptr(w.workspace(rows)), stream)
+                 ptr(w.workspace(rows, stream)), stream)
         if rc != 0:
             check(rc, "w4a16_linear")
         done += rows
@@ -615,7 +616,7 @@ def lm_head_argmax(x: torch.Tensor, embed: torch.Tensor, norm_weight: torch.Tens
     x = x.contiguous().view(-1, HIDDEN)
     b, vocab = x.shape[0], embed.shape[0]
     need = lib().quic_lm_head_scratch_bytes(b, vocab)
-    scratch = _thread_scratch("lm_head", x.get_device(), stream_ptr(), need, 1 << 16, 256)
+    scratch = _thread_scratch(("lm_head", x.get_device(), stream_ptr()), need, 1 << 16, 256)
     out = torch.empty(b, dtype=torch.int64, device=x.device)
     logits = torch.empty(b, vocab, dtype=torch.float16, device=x.device) if want_logits else None
     check(lib().quic_lm_head_argmax(ptr(x), ptr(norm_weight), float(eps), ptr(embed), vocab, b,
@@ -655,7 +656,7 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     splits, need = _attn_plan(b, s, splits, q_ptr % 4 == 0)
     device = q.get_device()
     stream = _raw_stream(device)
-    scratch = _thread_scratch("attention", device, stream, need, 1 << 20, max(8 * b, 1 << 16)) if need > 0 else None
+    scratch = _thread_scratch(("attention", device, stream), need, 1 << 20, max(8 * b, 1 << 16)) if need > 0 else None
     rc = lib().quic_attn_decode(q_ptr, k.data_ptr(), v.data_ptr(), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
                                 ptr(pad_lens), None, s, scale, out.data_ptr(), b, splits, ptr(scratch), stream)
     if rc != 0:
