@@ -223,6 +223,8 @@ int64_t w4a16_gemm_tc_workspace(int m, int n, int k);
 // many rows: dense fp16 GEMM on SM pairs, and the fp16 copies of packed weights that it reads (gemm_pair.cu)
 bool gemm_pair_supported(int m, int n, int k, bool swiglu);
 int gemm_pair_splits(int m, int n, int k);
+double gemm_pair_us(int m, int n, int k);
+double w4a16_gemm_tc_us(int m, int n, int k);
 int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, bool swiglu, cudaStream_t st,
               float* part = nullptr, int* splits = nullptr);
 struct PairRope {

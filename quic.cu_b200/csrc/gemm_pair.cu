@@ -435,6 +435,15 @@ int gemm_pair_splits(int m, int n, int k) {
   return s < 1 ? 1 : s > 16 ? 16 : s;
 }
 
+// About how long a packed linear takes here, in us: the fp16 copy of the weight, full waves of tiles over 74 pairs, the
+// output's stores, and the sum of K splits (constants from the four layer shapes at 400..8192 rows, mean error 7 %).
+double gemm_pair_us(int m, int n, int k) {
+  const int nt = pair_nt(n, false), splits = gemm_pair_splits(m, n, k);
+  const int64_t tiles = (int64_t)(n / nt) * ((m + 255) / 256) * splits;
+  const double out_mb = 2e-6 * m * n, wave = 0.3 + 1.4e-3 * nt * (k / kBlockK) / splits;
+  return 6.0 + 0.4e-6 * n * k + (double)((tiles + 73) / 74) * wave + 0.1 * out_mb + (splits > 1 ? 2.5 + 0.8 * splits * out_mb : 0.0);
+}
+
 // `part` (gemm_pair_splits x m x n fp32, may be null): where that is more than one split their partial sums
 // stay there for a consumer, y is not written and *splits says how many.
 int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, bool swiglu, cudaStream_t st,

@@ -500,6 +500,15 @@ static void tc_plan(int m, int n, int k, int* mt_out, int* splits_out, int* per_
   if (mtl_out != nullptr) *mtl_out = mtl;
 }
 
+// About how long it takes for many rows, in us: waves of CTAs with an SM each, or of two to an SM (run()).
+double w4a16_gemm_tc_us(int m, int n, int k) {
+  int mt, splits, per, mtl;
+  tc_plan(m, n, k, &mt, &splits, &per, &mtl);
+  const int ctas = (n / kTileN) * (((m + mt - 1) / mt + mtl - 1) / mtl);
+  const double wave = 2.3 + 0.008 * k, alone = (ctas + 147) / 148 * wave, shared = (ctas + 295) / 296 * 1.8 * wave;
+  return 2.0 + (mtl == 1 ? 0.75 * alone : alone < shared ? alone : shared);
+}
+
 int64_t w4a16_gemm_tc_workspace(int m, int n, int k) {
   int mt, splits, per;
   tc_plan(m, n, k, &mt, &splits, &per);

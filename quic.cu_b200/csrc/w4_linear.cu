@@ -201,12 +201,14 @@ extern "C" int quic_w4_dequant(const quic_w4_t* w, void* out, void* stream) {
 // against 10-19 us at 4 rows; the GEMV runs 2..8 rows on one 8-row instantiation).
 static constexpr int kTensorMinRows = 2;
 // The SM pair GEMM: dense weights from 128 rows (9728 x 896 at 130 rows 14.1 -> 11.3 us, at 8192 369 -> 117);
-// packed ones, which it unpacks first, where the products outweigh that (us: 9728 x 896 at 1024 rows
-// 33.6 -> 25.3, 896 x 4864 at 1024 23.3 -> 26.7 and at 1500 33.8 -> 27.8, 896 x 896 at 4096 12.5 -> 13.6 and at
-// 8192 21.6 -> 19.6).
+// packed ones, which it unpacks first, where the products outweigh that and its waves of tiles come out ahead
+// of the W4A16 GEMM's (us, W4A16 / pair: 9728 x 896 at 689 rows 20.0 / 20.6, at 1024 31.8 / 25.1, at 8192 161 / 116;
+// 896 x 4864 at 1024 22.5 / 26.3, at 2860 43.1 / 32.9, at 5000 43.7 / 56.4, at 5813 79.9 / 56.7; 1152 x 896 at 5813
+// 20.1 / 18.5, at 8192 19.9 / 23.3; 896 x 896 at 4096 11.7 / 13.6, at 8192 20.2 / 19.1).
 static constexpr int kDensePairMinRows = 128;
-static bool packed_pairs(int64_t m, int64_t n, int64_t k) {
-  return m * n * k >= 6000000000ll && k % kGroup == 0 && gemm_pair_supported((int)m, (int)n, (int)k, false);
+static bool packed_pairs(int m, int n, int k) {
+  if ((int64_t)m * n * k < 6000000000ll || k % kGroup != 0 || !gemm_pair_supported(m, n, k, false)) return false;
+  return n % 128 != 0 || gemm_pair_us(m, n, k) < w4a16_gemm_tc_us(m, n, k);  // (else the GEMV would take it)
 }
 
 static int64_t packed_workspace_bytes(int32_t m, int32_t n, int32_t k);

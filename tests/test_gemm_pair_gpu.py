@@ -40,6 +40,13 @@ def test_packed_linear_equals_the_same_rows_in_smaller_calls(m, n, k):
     assert (y.float() - want).norm() <= 1e-3 * want.norm()
 
 
+# either side of the lines where a packed linear's waves of tiles make one GEMM or the other the faster
+@pytest.mark.parametrize("m,n,k", [(768, 9728, 896), (769, 9728, 896), (4864, 896, 4864), (4865, 896, 4864), (5377, 896, 4864),
+                                   (6144, 1152, 896), (6145, 1152, 896)])
+def test_packed_linear_around_the_lines_of_the_rule(m, n, k):
+    test_packed_linear_equals_the_same_rows_in_smaller_calls(m, n, k)
+
+
 @pytest.mark.parametrize("m,n,k", [(7000, 192, 4864), (3000, 448, 4864)])
 def test_packed_linear_stays_inside_its_workspace(m, n, k):
     gen = torch.Generator(device="cuda").manual_seed(m + n)

@@ -31,7 +31,7 @@ def _pair_linear(seed):
     w.qw.random_(-2 ** 31, 2 ** 31 - 1, generator=gen)
     w.zp.random_(0, 255, generator=gen)
     w.sc.copy_(torch.rand(w.sc.shape, device="cuda", generator=gen) * 0.02)
-    x = torch.randn(700 + seed, 896, device="cuda", generator=gen).half()
+    x = torch.randn(800 + seed, 896, device="cuda", generator=gen).half()
     return lambda: kernels.w4a16_linear(w, x)
 
 
