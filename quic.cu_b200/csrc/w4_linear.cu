@@ -200,12 +200,18 @@ extern "C" int quic_w4_dequant(const quic_w4_t* w, void* out, void* stream) {
 // Rows from which the tcgen05 GEMM beats the dequant GEMV (measured per layer shape: 5-9 us
 // against 10-19 us at 4 rows; the GEMV runs 2..8 rows on one 8-row instantiation).
 static constexpr int kTensorMinRows = 2;
-// The SM pair GEMM: dense weights from 128 rows (9728 x 896 at 130 rows 14.1 -> 11.3 us, at 8192 369 -> 117);
+// The SM pair GEMM: dense weights from 129 rows (9728 x 896 at 130 rows 14.1 -> 11.3 us, at 8192 369 -> 117; 128 rows are
+// one tile of gemm_f16_tc, and a prefill of them takes 1546 us with it, 1601 with pairs) unless it
+// would split K more than four ways, whose parts cost more than they save (us, gemm_f16_tc / pair, 896 x 4864 with a
+// workspace: 128 rows 11.7 / 16.0, 640 rows, six ways, 17.0 / 19.9, 800 rows, four ways, 23.5 / 21.4);
 // packed ones, which it unpacks first, where the products outweigh that and its waves of tiles come out ahead
 // of the W4A16 GEMM's (us, W4A16 / pair: 9728 x 896 at 689 rows 20.0 / 20.6, at 1024 31.8 / 25.1, at 8192 161 / 116;
 // 896 x 4864 at 1024 22.5 / 26.3, at 2860 43.1 / 32.9, at 5000 43.7 / 56.4, at 5813 79.9 / 56.7; 1152 x 896 at 5813
 // 20.1 / 18.5, at 8192 19.9 / 23.3; 896 x 896 at 4096 11.7 / 13.6, at 8192 20.2 / 19.1).
-static constexpr int kDensePairMinRows = 128;
+static constexpr int kDensePairMinRows = 129;
+static bool dense_pairs(int m, int n, int k, bool parts) {
+  return m >= kDensePairMinRows && gemm_pair_supported(m, n, k, false) && (!parts || gemm_pair_splits(m, n, k) <= 4);
+}
 static bool packed_pairs(int m, int n, int k) {
   if ((int64_t)m * n * k < 6000000000ll || k % kGroup != 0 || !gemm_pair_supported(m, n, k, false)) return false;
   return n % 128 != 0 || gemm_pair_us(m, n, k) < w4a16_gemm_tc_us(m, n, k);  // (else the GEMV would take it)
@@ -262,7 +268,7 @@ extern "C" int quic_w4a16_linear(const void* x, const quic_w4_t* w, void* y, int
   if (w->w16 != nullptr) {  // dense fp16 weight [N, K]: a row or two on the GEMV, more on the tcgen05 GEMM
     QUIC_REQUIRE(w->n > 0 && w->k > 0 && w->k % 8 == 0 && m >= 0, QUIC_E_SHAPE, "linear: bad dense shape");
     if (m == 0) return QUIC_OK;
-    if (m >= kDensePairMinRows && use_tensor && gemm_pair_supported(m, w->n, w->k, false) && pair_aligned(x, w, y, workspace))
+    if (use_tensor && dense_pairs(m, w->n, w->k, workspace != nullptr) && pair_aligned(x, w, y, workspace))
       return pair_linear((const half*)x, (const half*)w->w16, (const half*)w->bias, (half*)y, m, w->n, w->k,
                          (float*)workspace, (cudaStream_t)stream);
     if (m >= 2 && use_tensor && gemm_f16_tc_supported(m, w->n, w->k))

@@ -67,6 +67,21 @@ def test_packed_linear_stays_inside_its_workspace(m, n, k):
     assert bool((arena[size:] == 0x5a).all())
 
 
+# the last row count that the pair GEMM would split six ways, and the first at four
+@pytest.mark.parametrize("m", [128, 129, 768, 769])
+def test_dense_linear_of_long_k_with_a_workspace(m):
+    n, k = 896, 4864
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    w = kernels.F16Weight(n, k, torch.device("cuda"))
+    w.w.copy_(torch.randn(n, k, device="cuda", generator=gen) * 0.05)
+    x = torch.randn(m, k, device="cuda", generator=gen).half()
+    y, ws = torch.empty(m, n, device="cuda").half(), torch.empty(kernels.lib().quic_w4a16_workspace_bytes(m, n, k), dtype=torch.uint8, device="cuda")
+    s = w.struct()
+    kernels.check(kernels.lib().quic_w4a16_linear(x.data_ptr(), C.byref(s), y.data_ptr(), m, 1, ws.data_ptr(), kernels.stream_ptr()), "linear")
+    want = x.float() @ w.w.float().T
+    assert (y.float() - want).norm() <= 1e-3 * want.norm()
+
+
 @pytest.mark.parametrize("n", [896, 192])
 @pytest.mark.parametrize("y_off,bias_off,room", [(1, 0, False), (4, 0, True), (1, 0, True), (0, 1, False), (0, 1, True), (3, 3, True)])
 def test_dense_linear_takes_any_output_and_bias_address(n, y_off, bias_off, room):
