@@ -152,10 +152,7 @@ def _ctx_bucket(n: int, batch: int = 1) -> int:
 class _DecodePlan:
     """What decode() keeps between calls for the same rows (see there)."""
 
-    __slots__ = ("bound", "rows", "tok", "out", "host", "host_np", "handle", "persist", "status", "feed", "feed_ptr")
-
-    def __init__(self):
-        self.feed = None
+    __slots__ = ("bound", "rows", "tok", "out", "host", "host_np", "handle", "persist", "status")
 
 
 def _persist_pays(dense: bool, batch: int, ctx: int) -> bool:
@@ -462,11 +459,11 @@ class QUICForCausalLM:
         n_in = 0
         if feed is not None:
             n_in = len(slots)
-            if plan is None or plan.feed is not feed:
-                if feed.dtype != torch.int32 or feed.numel() != n_in or feed.is_cuda:
-                    raise ValueError("decode: feed must be a host int32 tensor with one token per row")
-                if any(b - a != 1 for a, b in zip(slots, slots[1:])):
-                    raise ValueError("decode: feed needs consecutive slots")
+            if (feed.dtype is not torch.int32 or feed.numel() != n_in or feed.is_cuda
+                    or (n_in > 1 and not feed.is_contiguous())):
+                raise ValueError("decode: feed must be a contiguous host int32 tensor with one token per row")
+            if n_in > 1 and any(b - a != 1 for a, b in zip(slots, slots[1:])):
+                raise ValueError("decode: feed needs consecutive slots")
         first = cache.host_steps % ring
         longest = (host_len[slots[0]] if len(slots) == 1 else max(host_len[s] for s in slots)) if plan is not None else 0
         if plan is not None and longest + steps <= plan.bound and cache._rows_loaded.get(len(slots)) is plan.rows:
@@ -489,16 +486,15 @@ class QUICForCausalLM:
             if len(cache._plans) > 64:
                 cache._plans.clear()
             cache._plans[key] = plan
-        plan.feed = feed
-        plan.feed_ptr = feed.data_ptr() if n_in else None
+        feed_ptr = feed.data_ptr() if n_in else None
         # the block of generated rows, or the whole ring where the block wraps around its end
         n, wraps = cache.n_slots, first + steps > ring
         offset, count = (0, ring * n) if wraps else (4 * first * n, steps * n)
         if plan.persist is not None:
-            rc = K.lib().quic_decode_persist_run_host(*plan.persist, K.stream_ptr(), plan.feed_ptr, plan.tok, n_in,
+            rc = K.lib().quic_decode_persist_run_host(*plan.persist, K.stream_ptr(), feed_ptr, plan.tok, n_in,
                                                       plan.out + offset, plan.host + offset, count, plan.status)
         else:
-            rc = K.lib().quic_graph_run_host(plan.handle, K.stream_ptr(), plan.feed_ptr, plan.tok, n_in,
+            rc = K.lib().quic_graph_run_host(plan.handle, K.stream_ptr(), feed_ptr, plan.tok, n_in,
                                              plan.out + offset, plan.host + offset, count)
         if rc != 0:
             K.check(rc, "decode run_host")

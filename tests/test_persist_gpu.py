@@ -148,6 +148,23 @@ def test_host_fed_single_steps_agree_with_a_burst(persist_net):
     assert fed == burst
 
 
+def test_a_feed_is_checked_at_every_call(persist_net):
+    """The same tensor object may have another size or layout at the next call, or other slots."""
+    net = persist_net
+    cache = net.new_cache(n_slots=2, s_max=256)
+    net.prefill(cache, [0, 1], [torch.tensor([5, 6, 7]), torch.tensor([8, 9])])
+    feed = torch.tensor([3, 4], dtype=torch.int32).pin_memory()
+    net.decode(cache, [0, 1], 1, feed=feed)
+    for spoil in (lambda: feed.resize_(1), lambda: feed.set_(torch.zeros(4, dtype=torch.int32)[::2]),
+                  lambda: feed.resize_(0)):
+        spoil()
+        with pytest.raises(ValueError, match="feed"):
+            net.decode(cache, [0, 1], 1, feed=feed)
+    net.decode(cache, [1, 0], 1)
+    with pytest.raises(ValueError, match="consecutive"):
+        net.decode(cache, [1, 0], 1, feed=torch.tensor([3, 4], dtype=torch.int32).pin_memory())
+
+
 def test_a_wait_that_runs_out_is_reported_and_the_next_launch_works(persist_net):
     """Bounded waits: with the probe limit lowered to 4096 and CTA 0 withholding its o_proj
     result of layer 0 (both through the header words of the exchange area), the polls that
