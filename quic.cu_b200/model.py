@@ -18,6 +18,7 @@ tokenizer_path) -> (QUICForCausalLM, tokenizer)`` (src/model.py:306) and
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import json
 import numbers
 import os
@@ -174,6 +175,9 @@ def _persist_pays(dense: bool, batch: int, ctx: int) -> bool:
     return ctx <= (8192 if batch == 2 else 4096 if dense else 2048)
 
 
+_serials = itertools.count()
+
+
 class QUICForCausalLM:
     """The model: W4A16 (or, for an un-quantised checkpoint, dense fp16) weights in device
     layout + the C structs the kernels read."""
@@ -202,6 +206,7 @@ class QUICForCausalLM:
         self.default_slots = 8
         self.default_context = 4096
         self.use_persist = PERSIST
+        self._serial = next(_serials)  # graphs and launch plans of a cache belong to the model that made them
         self.dense = False  # True: un-quantised fp16 weights (F16Weight), the dense kernels
         self._wstream: torch.Tensor | None = None
         self._wstream_lock = threading.Lock()
@@ -331,7 +336,7 @@ class QUICForCausalLM:
         return d, rows
 
     def _graph(self, cache: SlotCache, batch: int, ctx: int, steps: int, logits: torch.Tensor | None):
-        key = (batch, ctx, steps, K.ptr(logits))
+        key = (self._serial, batch, ctx, steps, K.ptr(logits))
         g = cache._graphs.get(key)
         if g is None and len(cache._graphs) >= cache.max_graphs:
             # a long-lived engine with ragged batches meets ever new (rows, context bound, steps):
@@ -453,7 +458,7 @@ class QUICForCausalLM:
         buffer, and the call returns when they have arrived."""
         # A plan keeps everything that stays the same between calls for the same rows while
         # the context stays inside the bound the launch was made for.
-        key = (tuple(slots), steps)
+        key = (self._serial, self.use_persist, tuple(slots), steps)
         plan = cache._plans.get(key)
         host_len, ring = cache.host_len, cache.ring
         n_in = 0

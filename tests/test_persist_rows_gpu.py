@@ -18,6 +18,37 @@ def dense_model():
     return qmodel.from_state_dict(synthetic_dense_checkpoint(n_layers=2, vocab=2048, seed=4), config)
 
 
+@pytest.mark.parametrize("persist", [True, False])
+@pytest.mark.parametrize("rows", [1, 4])
+def test_two_models_on_one_cache(tiny_model, dense_model, persist, rows):
+    """Launch plans and graphs that a cache keeps are those of the model that made them, and of its choice of kernel."""
+    nets = (tiny_model[0], dense_model)
+    old = [net.use_persist for net in nets]
+    gen = torch.Generator().manual_seed(rows)
+    prompts = [torch.randint(0, 2048, (20 + i,), generator=gen) for i in range(rows)]
+    slots = list(range(rows))
+
+    def answer(net, cache):
+        net.prefill(cache, slots, prompts)
+        return net.decode(cache, slots, 8)
+
+    try:
+        for net in nets:
+            net.use_persist = persist
+        want = [answer(net, net.new_cache(n_slots=4, s_max=128)) for net in nets]
+        cache = nets[0].new_cache(n_slots=4, s_max=128)
+        for _ in range(2):
+            assert [answer(net, cache) for net in nets] == want
+        kinds = {type(p.handle) for p in cache._plans.values()}
+        for net in nets:
+            net.use_persist = not persist
+            answer(net, cache)
+        assert len({type(p.handle) for p in cache._plans.values()}) == 2 and len(kinds) == 1
+    finally:
+        for net, flag in zip(nets, old):
+            net.use_persist = flag
+
+
 # tokens cached before the step: the step's own token opens or closes a 32-token half tile (31, 32, 63),
 # falls to the first warp's second half tile (448), lies beyond what stays in shared memory (1000 at 16
 # rows, one split) or in a later split (800 at one row, 1700 at two)
