@@ -419,7 +419,8 @@ int quic_graph_destroy(void *graph);
  * The decode token loop as one persistent kernel (1..quic_persist_max_rows()
  * batch rows, packed or fp16 weights).  On B200 it is the faster form from two
  * rows on and for fp16 weights (445 against 667 us per step at 8 rows of 1000
- * tokens, 348 against 494 us at one fp16 row), and equal at one packed row.
+ * tokens, 348 against 494 us at one fp16 row); one packed row gains from 513 to
+ * 768 tokens only (345 against 353 us at 520, 350 against 333 at 500).
  *
  * Replaces the same reference code as quic_decode_step, for `steps` consecutive
  * greedy tokens in ONE launch: Engine.step + QUICForCausalLM.forward with

@@ -629,7 +629,8 @@ extern "C" int32_t quic_attn_pick_splits(int32_t b, int32_t s_max) {
 }
 
 // The split kernels keep caches of up to 256 tokens with more rows than SMs: their tiles are fewer than a flow CTA's
-// six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).
+// six warps there (256 x 192: 9.0 us against 10.4; 150 x 700: 24 against 13.6).  (Caches of one tile would be up to a
+// microsecond faster there too, 1 x 64 2.8 against 3.6, but the split kernels multiply the values that they mask.)
 extern "C" int32_t quic_attn_decode_streams(int32_t b, int32_t s_max) { return s_max <= 256 && b > 148 ? 0 : 1; }
 
 extern "C" int64_t quic_attn_scratch_bytes(int32_t b, int32_t splits) {

@@ -21,8 +21,8 @@
 // The stages of a tile wait for one another; what hides that is the four CTAs of an SM (128 TMEM
 // columns and 49 KB each) or, for a grid that is too small for it, scores that run a tile ahead (256 columns).
 // The form before it had eight warps that shared rows, transposed V and kept O in registers, two
-// CTAs an SM, us: 1 x 512 14.7 -> 12.6, 8 x 517 33 -> 25,
-// 16 x 2048 360 -> 239 (510 TFLOP/s of causal flops).
+// CTAs an SM, us (launches of a graph): 1 x 512 14.7 -> 11.7, 8 x 517 33 -> 24,
+// 16 x 2048 360 -> 231 (521 TFLOP/s of causal flops; 244 after seconds of it, under the power limit).
 //
 // Roles: warps 0-3 softmax and epilogue, warp 4 TMA producer (two stages of K and V), warp 5 MMA issuer.
 // Every wait is bounded; a wait that runs out sets word 0 of the tensor path's error words
@@ -361,8 +361,8 @@ int attn_prefill_tc_launch(const void* q, const void* kcache, const void* vcache
   a.n_slots = n_slots;
   a.scale_log2 = (scale > 0.f ? scale : 0.125f) * 1.4426950408889634f;
   // Up to four CTAs an SM in all: too few to hide a tile's latency, so its scores run a tile ahead, in twice
-  // the tensor memory (plain / ahead, us: 1 x 2048 44.3 / 32.1, 4 x 1000 30.0 / 27.1, 8 x 517 22.8 / 22.8,
-  // 16 x 2048 225 / 250).
+  // the tensor memory (plain / ahead, us: 1 x 512 15.0 / 11.7, 1 x 2048 46.5 / 34.8, 4 x 1000 28.8 / 28.2,
+  // 8 x 517 22.0 / 23.6, 16 x 2048 231 / 273).
   const dim3 grid(kHeads, n_seq, (max_len + kQRows - 1) / kQRows);
   const bool ahead = (int64_t)grid.x * grid.y * grid.z <= 4 * 148;
   auto kernel = ahead ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>;

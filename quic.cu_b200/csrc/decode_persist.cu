@@ -16,9 +16,10 @@
 // mma fragments in registers, cached keys and values as fragments) is in place before the word
 // arrives.  Measured per layer at one row: ~1 us from a publication to the last reader's arithmetic,
 // five times, and 0.3 to 1.8 us of arithmetic and reductions per phase (the attention of one KV head
-// on one SM is the longest).  Per step, persistent / kernel chain: 342 / 347 us at one row of 512
-// tokens, 373 / 462 at two, 408 / 653 at five of 700, 445 / 667 at eight of 1000, 500 / 704 at 16 of
-// 300; fp16 weights 348 / 494 at one row, 416 / 899 at eight.
+// on one SM is the longest).  Per step, persistent / kernel chain: 345 / 353 us at one row of 520
+// tokens (350 / 333 at 500, where the chain needs no merge: it serves one packed row up to 512), 373 / 462 at
+// two, 408 / 653 at five of 700, 445 / 667 at eight of 1000, 500 / 704 at 16 of 300; fp16 weights 348 / 494 at
+// one row, 416 / 899 at eight.
 //
 // Roles (a CTA can have several; `na` = attention CTAs, the last ones of the grid):
 //   residual   CTAs 0..55    16 output columns of o_proj AND of down; the residual stream of those

@@ -15,16 +15,18 @@ What differs is where the state lives.  The reference keeps one left-padded batc
 cache length only grows and rebuilds it with torch.cat on every admission
 (src/engine.py:225-277).  Here every request owns a KV slot that stores real tokens only;
 admission prefills into a free slot, release frees it, and an iteration is a burst of
-``decode_burst`` greedy steps that run on the device from one CUDA graph launch, with one
+``decode_burst`` greedy steps that run on the device from one launch, with one
 device->host copy of the burst's tokens.  Tokens produced by a row after it finished are
 discarded exactly as the reference discards them (src/engine.py:180-182).
 
 With ``overlap_prefill`` (default) a request admitted while other rows are running is
 prefilled on a second CUDA stream during those rows' next decode burst and joins the batch at
 the following iteration: slots are disjoint, so the two never touch the same cache rows, and
-the side stream is synchronised before any decode launch that includes the new rows.  The
-outputs are the same (every request is an independent greedy decode); only the iteration at
-which a request starts to decode moves by one.
+the side stream is synchronised before any decode launch that includes the new rows.  (A burst of
+the persistent decode kernel, up to 16 rows, holds every SM: such a prefill runs before or after
+it on the device, and only their host work overlaps.)  The outputs are the same (every request
+is an independent greedy decode); only the iteration at which a request starts to decode moves
+by one.
 
 ``model_module.load(**options)`` must return ``(model, tokenizer)``; the model is driven
 through three calls: ``new_cache(n_slots, s_max)``, ``prefill(cache, slots, prompts)`` and

@@ -11,8 +11,9 @@ tokenizer_path) -> (QUICForCausalLM, tokenizer)`` (src/model.py:306) and
   benchmarks/collect.py:61-92);
 * a prefill returns logits of the last position only unless ``prefill_all_logits`` is set;
 * decode (``seq_len == 1``) is ONE fused call: embedding, 24 layers, final norm, lm_head and
-  argmax run as a chain of kernels with state on the device.  ``decode`` runs several
-  consecutive greedy steps from a captured CUDA graph without a host round trip.
+  argmax run as one persistent kernel or a chain of kernels (``_persist_pays``) with state on
+  the device.  ``decode`` runs several consecutive greedy steps, in one launch of that kernel or
+  from a captured CUDA graph of the chain, without a host round trip.
 """
 
 from __future__ import annotations
@@ -360,7 +361,7 @@ class QUICForCausalLM:
     # ---- persistent decode kernel ------------------------------------------------------
     def persist_stream(self) -> torch.Tensor:
         """The weight stream of the persistent kernel, packed on first use from the device
-        matrices (a second copy of the layer weights, 9 MB per layer, 32 MB in fp16).  Complete when the call
+        matrices (a second copy of the layer weights, 8.7 MB per layer, 31 MB in fp16).  Complete when the call
         returns: launches on any stream and of any thread read it."""
         if self._wstream is None:
             with self._wstream_lock:
