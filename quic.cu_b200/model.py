@@ -154,7 +154,11 @@ def _ctx_bucket(n: int, batch: int = 1) -> int:
 class _DecodePlan:
     """What decode() keeps between calls for the same rows (see there)."""
 
-    __slots__ = ("bound", "rows", "tok", "out", "host", "host_np", "handle", "persist", "status")
+    __slots__ = ("bound", "rows", "tok", "out", "host", "host_np", "handle", "persist", "status", "scattered")
+
+
+def _scattered(slots) -> bool:
+    return any(b - a != 1 for a, b in zip(slots, slots[1:]))
 
 
 def _persist_pays(dense: bool, batch: int, ctx: int) -> bool:
@@ -468,7 +472,7 @@ class QUICForCausalLM:
             if (feed.dtype is not torch.int32 or feed.numel() != n_in or feed.is_cuda
                     or (n_in > 1 and not feed.is_contiguous())):
                 raise ValueError("decode: feed must be a contiguous host int32 tensor with one token per row")
-            if n_in > 1 and any(b - a != 1 for a, b in zip(slots, slots[1:])):
+            if plan.scattered if plan is not None else _scattered(slots):
                 raise ValueError("decode: feed needs consecutive slots")
         first = cache.host_steps % ring
         longest = (host_len[slots[0]] if len(slots) == 1 else max(host_len[s] for s in slots)) if plan is not None else 0
@@ -484,7 +488,7 @@ class QUICForCausalLM:
             plan.rows = cache.rows_tensor(slots)
             plan.tok = cache.tok.data_ptr() + 4 * slots[0]
             plan.out, plan.host, plan.host_np = cache.out_tokens.data_ptr(), cache.host_out().data_ptr(), cache.host_out().numpy()
-            plan.handle, plan.persist = handle, None
+            plan.handle, plan.persist, plan.scattered = handle, None, _scattered(slots)
             if isinstance(handle, K.Decode):
                 plan.persist = (C.byref(self._c_model), C.byref(handle), K.ptr(self.persist_stream()),
                                 K.ptr(cache.persist_sync()), steps)
