@@ -1,4 +1,4 @@
-"""The persistent decode kernel (one launch per burst of tokens, 1..4 rows) against the CPU
+"""The persistent decode kernel (one launch per burst of tokens, 1..4 rows here) against the CPU
 oracle and against the kernel chain it replaces, through the C ABI."""
 
 import pytest
@@ -103,12 +103,16 @@ def test_bursts_match_the_kernel_chain_and_the_oracle(persist_net, tiny_model, r
     assert a.argmax(-1).tolist() == b.argmax(-1).tolist() or err < 2e-2
 
 
-@pytest.mark.parametrize("prompt_len", [383, 384, 1100, 3900])
+@pytest.mark.parametrize("prompt_len", [383, 384, 766, 1100, 2110, 2814, 3900])
 def test_split_boundaries_and_long_contexts(persist_net, tiny_model, prompt_len):
-    """Contexts around a split boundary (splits of 192 tokens below 512: the row being decoded
-    is the last of a split at 383 and the first of the next at 384) and up to the kernel's
-    longest context, sixteen splits of 256 tokens merged by the o_proj CTAs in rounds of four:
-    logits against the oracle's teacher-forced pass."""
+    """One split (383, 384: the token closes or opens a half tile), the change from one split to two
+    within the five steps (766: the bound goes from 768 to 896), two splits of 576 tokens (1100) and, at the bound
+    of 4096, six of 704: the tokens being decoded cross from the third into the fourth (2110) and from
+    the fourth into the fifth (2814), or end in the sixth (3900).  Merged by the o_proj CTAs; logits against the
+    oracle's teacher-forced pass."""
+    from quic_cu_b200 import kernels as K
+
+    assert [K.lib().quic_persist_pick_splits(1, n) for n in (768, 896, 1152, 4096)] == [1, 2, 2, 6]
     from oracle.quic_ref import RefModel
 
     net = persist_net
