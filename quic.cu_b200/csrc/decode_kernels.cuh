@@ -187,6 +187,47 @@ int64_t gemm_f16_tc_workspace(int m, int n, int k);
 int gemm_f16_tc(const half* x, const half* w, const half* bias, half* y, int m, int n, int k, float* ws,
                 cudaStream_t st, bool pdl);
 
+// The linears of a layer for a few rows, each one launch with what stands around it (rows_chain.cu).
+constexpr int kRowsSsq = 14;  // partial sums of squares of a row of the residual stream: [rows][kRowsSsq] fp32
+struct RowsArgs {
+  quic_w4_t w;
+  int32_t rows;
+  half* y;              // qkv: the queries; o_proj, down: the residual stream [rows][896]; gate|up: the activation [rows][4864]
+  // norm of the input rows (qkv, gate|up): weights, the sums that its writer left and how many a row has
+  const half* ln;
+  const float* ssq_in;
+  int32_t n_ssq;
+  float eps;
+  // o_proj, down: what is added, and the sums for the next norm
+  const half* res;
+  float* ssq_out;
+  // qkv: slot of a row; its position is row_pos[row], or without row_pos that of its slot
+  const int32_t* slots;
+  const int32_t* row_pos;
+  const int32_t* pos;
+  const half* cos_t;
+  const half* sin_t;
+  half* kcache;         // [n_slots][2][s_max][64]
+  half* vcache;
+  int32_t max_pos, s_max, n_slots;
+  int32_t head_major;   // queries as [14][rows][64] instead of [rows][14][64]
+  // weights (packed words, scales, zero points) of the next linear, brought into L2 meanwhile
+  const void* next_w[3];
+  int64_t next_bytes[3];
+  // filled in by the launcher
+  const half* x;
+  int32_t* status;
+  uint32_t spin_limit;
+  int32_t skip_stage;
+};
+void rows_next(RowsArgs* a, const quic_w4_t* w);  // nullptr: none
+int rows_qkv(const half* x, const RowsArgs& a, cudaStream_t st);
+int rows_out(const half* x, const RowsArgs& a, cudaStream_t st);
+int rows_swiglu(const half* x, const RowsArgs& a, cudaStream_t st);
+int rows_down(const half* x, const RowsArgs& a, cudaStream_t st);
+cudaError_t launch_embed_ssq(const half* embed, const int32_t* slots, const int32_t* tok, int vocab, half* x, float* ssq, int rows,
+                             cudaStream_t st, bool pdl);
+
 // pieces of the batched (batch > 8) decode step
 cudaError_t launch_embed_rows(const half* embed, const int32_t* rows, const int32_t* tok, int vocab, half* x,
                               int batch, cudaStream_t st, bool pdl);
@@ -248,6 +289,7 @@ int launch_lm_head_tc(const LmHeadArgs& a, cudaStream_t st);
 // an asynchronous copy to page-locked memory, and the value seen by that copy (taken, i.e.
 // exchanged with zero, when it is not 0).
 int* tc_status_words();
+void tc_test_hook(uint32_t* spin_limit, int32_t* skip_kblock);  // what quic_w4a16_tensor_test_hook last set
 int tc_status_poll_async(cudaStream_t st);
 int tc_status_polled(cudaStream_t st);
 

@@ -131,8 +131,16 @@ int g_mma_chain_min_batch = 3;
 int enqueue_step_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head);
 int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head);
 
+int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head);
+
+// Rows that the chain of rows_chain.cu serves (from g_tensor_min_batch, un-quantised from kF16ChainMaxRows + 1 rows):
+// one tile of 128 on the M side of its MMAs.
+constexpr int kRowsChainMaxRows = 128;
+
 int enqueue_step(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
+  if (B <= kRowsChainMaxRows && B > (m->layers[0].qkv.w16 != nullptr ? kF16ChainMaxRows : g_tensor_min_batch - 1))
+    return enqueue_step_rows(m, d, st, chain_head);
   if (m->layers[0].qkv.w16 != nullptr)  // dense fp16 weights
     return B <= kF16ChainMaxRows ? enqueue_step_f16(m, d, st, chain_head) : enqueue_step_batched_f16(m, d, st, chain_head);
   if (B >= g_tensor_min_batch) return enqueue_step_batched(m, d, st, chain_head);
@@ -518,6 +526,78 @@ int enqueue_attention(const quic_decode_t* d, const Arena& ar, int splits, int c
   return QUIC_OK;
 }
 
+LmHeadArgs lm_head_args(const quic_model_t* m, const quic_decode_t* d, const Arena& ar);
+
+// 17..128 rows, un-quantised from 3: five launches a layer (rows_chain.cu).
+int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
+  const int B = d->batch;
+  const int splits = pick_splits(d);
+  const Arena ar = carve(B, m->vocab, splits);
+  char* base = static_cast<char*>(d->scratch);
+  half* h = reinterpret_cast<half*>(base + ar.xres);  // residual stream
+  half* qbuf = reinterpret_cast<half*>(base + ar.qbuf);
+  half* attn_out = reinterpret_cast<half*>(base + ar.attn_out);
+  half* xn = reinterpret_cast<half*>(base + ar.xn);
+  half* act = reinterpret_cast<half*>(base + ar.act16);
+  float* ssq = reinterpret_cast<float*>(base + ar.act);  // [B][kRowsSsq], of h after the attention, after the layer
+  float* const ssq_mid = ssq;
+  float* const ssq_end = ssq + (size_t)B * kRowsSsq;
+  const size_t kv_plane = (size_t)d->n_slots * kKvHeads * d->s_max * kHeadDim;
+  int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
+  if (ctx > d->s_max) ctx = d->s_max;
+  RowsArgs a = {};
+  a.rows = B;
+  a.eps = m->eps;
+  a.slots = d->rows;
+  a.pos = d->pos;
+  a.cos_t = (const half*)m->rope_cos;
+  a.sin_t = (const half*)m->rope_sin;
+  a.max_pos = m->max_pos;
+  a.s_max = d->s_max;
+  a.n_slots = d->n_slots;
+  a.res = h;
+
+  // (the head of a sequence starts only after everything enqueued before it has completed)
+  QUIC_CUDA(launch_embed_ssq((const half*)m->embed, d->rows, d->tok, m->vocab, h, ssq_end, B, st, !chain_head));
+  int rc;
+  for (int l = 0; l < m->n_layers; ++l) {
+    const quic_layer_t& L = m->layers[l];
+    a.kcache = static_cast<half*>(d->kv) + (size_t)(2 * l) * kv_plane;
+    a.vcache = a.kcache + kv_plane;
+    a.w = L.qkv;
+    a.y = qbuf;
+    a.ln = (const half*)L.ln1;
+    a.ssq_in = ssq_end;
+    a.n_ssq = l == 0 ? 1 : kRowsSsq;
+    rows_next(&a, &L.o);  // a launch brings the next linear's weights into L2
+    if ((rc = rows_qkv(h, a, st)) != QUIC_OK) return rc;
+    if ((rc = enqueue_attention(d, ar, splits, ctx, qbuf, a.kcache, a.vcache, attn_out, st)) != QUIC_OK) return rc;
+    a.w = L.o;
+    a.y = h;
+    a.ssq_out = ssq_mid;
+    rows_next(&a, &L.gate_up);
+    if ((rc = rows_out(attn_out, a, st)) != QUIC_OK) return rc;
+    a.w = L.gate_up;
+    a.y = act;
+    a.ln = (const half*)L.ln2;
+    a.ssq_in = ssq_mid;
+    a.n_ssq = kRowsSsq;
+    rows_next(&a, &L.down);
+    if ((rc = rows_swiglu(h, a, st)) != QUIC_OK) return rc;
+    a.w = L.down;
+    a.y = h;
+    a.ssq_out = ssq_end;
+    rows_next(&a, l + 1 < m->n_layers ? &m->layers[l + 1].qkv : nullptr);
+    if ((rc = rows_down(act, a, st)) != QUIC_OK) return rc;
+  }
+  QUIC_CUDA(launch_rmsnorm(h, nullptr, (const half*)m->final_norm, m->eps, xn, nullptr, B, st));
+  LmHeadArgs la = lm_head_args(m, d, ar);
+  la.x_normed = xn;
+  if (lm_head_tc_supported(B, m->vocab)) return launch_lm_head_tc(la, st);
+  QUIC_CUDA(launch_lm_head(la, lm_head_grid(m->vocab), st, false));
+  return QUIC_OK;
+}
+
 LmHeadArgs lm_head_args(const quic_model_t* m, const quic_decode_t* d, const Arena& ar) {
   char* base = static_cast<char*>(d->scratch);
   LmHeadArgs la = {};
@@ -681,6 +761,9 @@ extern "C" int64_t quic_decode_scratch_bytes(int32_t batch, int32_t vocab, int32
 
 extern "C" int32_t quic_decode_launch_count(const quic_model_t* m, const quic_decode_t* d) {
   if (!m) return 0;
+  if (d && m->layers && d->batch <= kRowsChainMaxRows &&
+      d->batch > (m->layers[0].qkv.w16 != nullptr ? kF16ChainMaxRows : g_tensor_min_batch - 1))
+    return 5 * m->n_layers + 3;
   if (m->layers && m->layers[0].qkv.w16 != nullptr) {
     if (d && d->batch > kF16ChainMaxRows) {
       int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;

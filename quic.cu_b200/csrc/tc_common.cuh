@@ -17,20 +17,28 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
-// Bounded wait for the phase with the given parity; false on timeout (after `limit` probes).
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Bounded wait for the phase with the given parity; false on timeout (after `limit` probes).  The first probe stands
+// outside the loop: a phase that is complete already then costs ~100 clocks instead of ~200.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = kSpinLimit) {
-  for (uint32_t i = 0; i < limit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
+  bool done = mbar_try(bar, parity);
+  if (!done)
+    for (uint32_t i = 1; i < limit; ++i)
+      if (mbar_try(bar, parity)) {
+        done = true;
+        break;
+      }
+  return done;
 }
 // The same wait for roles that are many warps wide and not on the critical path of the MMA
 // issue: sleeps between probes so the probes do not crowd the issuing thread's instructions
@@ -86,6 +94,35 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float (&v)[N]) {
   for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// N blocks of 16 lanes x 8 fp32 columns: a thread has columns 2 (t % 4) and + 1 of lanes t / 4 (v[.][0], v[.][1]) and t / 4 + 8
+template <int N>
+__device__ __forceinline__ void tmem_ld_16x8(uint32_t taddr, float (&v)[N][4]) {
+  uint32_t r[4 * N];
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[4 * q]), "=r"(r[4 * q + 1]), "=r"(r[4 * q + 2]), "=r"(r[4 * q + 3])
+                 : "r"(taddr + 8u * q));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4 * N; ++i) v[i / 4][i % 4] = __uint_as_float(r[i]);
+}
+// a block here and one there, one wait
+__device__ __forceinline__ void tmem_ld_16x8_two(uint32_t ta, uint32_t tb, float (&a)[4], float (&b)[4]) {
+  uint32_t r[8];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[4 * q]), "=r"(r[4 * q + 1]), "=r"(r[4 * q + 2]), "=r"(r[4 * q + 3])
+                 : "r"(q == 0 ? ta : tb));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    a[i] = __uint_as_float(r[i]);
+    b[i] = __uint_as_float(r[4 + i]);
+  }
+}
+
 // 32 consecutive fp32 columns of this thread's TMEM lane: two loads in flight, one wait
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
@@ -113,9 +150,17 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
   d |= (uint64_t)2 << 61;                    // SWIZZLE_128B
   return d;
 }
-// kind::f16, fp16 x fp16 -> fp32, both operands K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t umma_idesc_f16(int n) {
-  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
+// kind::f16, fp16 x fp16 -> fp32, both operands K-major, M = m, N = n.
+__device__ __forceinline__ uint32_t umma_idesc_f16(int m, int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+__device__ __forceinline__ uint32_t umma_idesc_f16(int n) { return umma_idesc_f16(kTileN, n); }
+// One lane of a converged warp.  An MMA issued under it, with descriptors that are advanced by adds, takes 25-50 clocks of
+// the issuing warp (M = 64, N = 16 .. M = 128, N = 64); under `lane == 0`, 69.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
@@ -157,7 +202,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
 
 // ---- host side ----------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

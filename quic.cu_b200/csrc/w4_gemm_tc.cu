@@ -616,6 +616,11 @@ int* tc_status_words() {
   return g_status_host.words[dev];
 }
 
+void tc_test_hook(uint32_t* spin_limit, int32_t* skip_kblock) {
+  *spin_limit = g_spin_limit;
+  *skip_kblock = g_skip_kblock;
+}
+
 // Enqueues a copy of the error words to page-locked host memory on `st`; tc_status_polled()
 // reads them once the stream has been synchronised.  Costs no synchronisation of its own.
 int tc_status_poll_async(cudaStream_t st) {

@@ -1,0 +1,75 @@
+"""The decode step of 17..128 rows (un-quantised from 3): one launch per linear with norm, RoPE + KV
+append, residual or SwiGLU inside, `down` over clusters of eight CTAs."""
+
+import pytest
+import torch
+from torch.linalg import vector_norm as norm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def nets(tiny_model):
+    from quic_cu_b200 import model as qmodel
+    from quic_cu_b200.checkpoint import qwen_config_dict, synthetic_dense_checkpoint
+
+    config = qwen_config_dict(2, 2048)
+    config.pop("quantization_config", None)
+    # packed weights of the spread of the un-quantised ones: with the checkpoint's own, gates of 30 and more turn a
+    # rounding of theirs into thirty
+    _, _, state, packed_config = tiny_model
+    state = {k: v * 0.25 if k.endswith("weight_scale") else v for k, v in state.items()}
+    return {"w4": qmodel.from_state_dict(state, packed_config),
+            "fp16": qmodel.from_state_dict(synthetic_dense_checkpoint(n_layers=2, vocab=2048, seed=99), config)}
+
+
+@pytest.mark.parametrize("weights,rows", [("w4", n) for n in (17, 63, 64, 65, 127, 128)] + [("fp16", n) for n in (3, 16, 64, 65, 128)])
+def test_appended_keys_and_values_match_a_prefill_of_the_same_tokens(nets, weights, rows):
+    """Edges of the row tiles (64, 128) and of what the path takes.  A step appends K and V of the token it feeds
+    in every layer; a prefill of prompt + token, other kernels, has to leave the same there.  On the way to K and V of
+    the second layer lie 17 roundings to fp16 (two norms and the third, four linears with their sums, bias, rotation,
+    probabilities, activation), each 2^-11 / sqrt(3) in the root mean square, on either side; the worst of up to
+    512 (row, plane) pairs is allowed twice their root of 34."""
+    from quic_cu_b200 import kernels as K
+
+    net = nets[weights]
+    gen = torch.Generator().manual_seed(rows)
+    lens = torch.randint(8, 90, (rows,), generator=gen).tolist()
+    lens[0] = 300  # (more rows in the prefills than any of the forms under test takes)
+    prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
+    slots = torch.randperm(rows + 2, generator=gen)[:rows].tolist()  # rows need not sit in slot order, nor fill the cache
+    cache, other = (net.new_cache(n_slots=rows + 2, s_max=320) for _ in range(2))
+    first, _ = net.prefill(cache, slots, prompts)
+    idle = [s for s in range(rows + 2) if s not in slots]
+    before = cache.kv[:, :, idle].clone()
+    net.decode(cache, slots, 1)
+    net.prefill(other, slots, [torch.cat([p, first[i:i + 1].cpu()]) for i, p in enumerate(prompts)])
+    at = torch.tensor(lens, device="cuda")
+    got, want = (c.kv[:, :, slots].float().gather(4, at.view(1, 1, rows, 1, 1, 1).expand(2, 2, rows, 2, 1, 64)) for c in (cache, other))
+    worst = (norm(got - want, dim=(3, 4, 5)) / norm(want, dim=(3, 4, 5))).max().item()
+    assert worst < 2 * (34 / 3) ** 0.5 * 2 ** -11, worst
+    assert torch.equal(cache.kv[:, :, idle], before)
+    assert K.lib().quic_w4a16_tensor_status() == 0
+
+
+def test_rows_of_very_small_and_large_norm(nets):
+    """The rows' factors are a power of two, applied before the product, and a rest of 1 to 2, after it: rows far from 1 in
+    size must come out as a norm in 32 bits gives them."""
+    net = nets["w4"]
+    embed = net.embed.clone()
+    try:
+        scale = torch.tensor([2.0 ** -14, 2.0 ** -7, 1.0, 37.0, 1500.0], device="cuda", dtype=torch.float32)
+        net.embed[:40] = (embed[:40].float().sign() * scale.repeat(8).view(40, 1) *
+                          (0.5 + torch.rand(40, 896, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)))).half()
+        ids = torch.arange(40).view(40, 1)
+        cache, other = (net.new_cache(n_slots=40, s_max=64) for _ in range(2))
+        for c in (cache, other):
+            net.prefill(c, list(range(40)), [torch.tensor([5])] * 40)
+        cache.tok.copy_(ids.view(-1))
+        net.decode(cache, list(range(40)), 1)
+        net.prefill(other, list(range(40)), list(ids), offsets=[1] * 40)
+        got, want = cache.kv[0, :, :, :, 1].float(), other.kv[0, :, :, :, 1].float()
+        worst = (norm(got - want, dim=(2, 3)) / norm(want, dim=(2, 3))).max().item()
+        assert worst < 2 * 3 ** 0.5 * 2 ** -12, worst  # three roundings on either side
+    finally:
+        net.embed.copy_(embed)
