@@ -59,7 +59,10 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
                               const AttnArgs a, const QkvFinish fin, int n_slots, int s_max, int* status,
                               int force_reload, int skip_tile0, uint32_t spin_limit) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[kStreamStages];   // a stage's two tiles landed
+  // A stage's two tiles landed: by the requests made before the dependency wait, by all others.  (One barrier for both
+  // would not do where early requests are repeated: a wait for its second phase returns at once while the first runs, and
+  // one for the first never does once both are complete.)
+  __shared__ __align__(8) uint64_t bar_early[kStreamStages], bar_full[kStreamStages];
   __shared__ __align__(8) uint64_t bar_empty[kStreamStages];  // its consumer warp holds them in registers
   __shared__ float m_s[kStreamWarps][8], l_s[kStreamWarps][8];
   __shared__ __align__(16) float o_s[kStreamWarps][kGroupHeads][kHeadDim];
@@ -75,6 +78,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
     for (int s = 0; s < kStreamStages; ++s) {
+      mbar_init(smem_u32(&bar_early[s]), 1);
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
@@ -92,7 +96,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     const int pre = min(p0 > 0 ? p0 / kWarpChunk : 0, kStreamStages);
     const int row0p = (slot0 * kKvHeads + kvh) * s_max;
     for (int i = skip_tile0 ? 1 : 0; i < pre; ++i) {  // (test hook: the wait for tile 0 runs out)
-      const uint32_t full = smem_u32(&bar_full[i]), dst = base + i * kStageBytes;
+      const uint32_t full = smem_u32(&bar_early[i]), dst = base + i * kStageBytes;
       mbar_expect_tx(full, kStageBytes);
       tma_load_2d(dst, &tm_k, 0, row0p + i * kWarpChunk, full);
       tma_load_2d(dst + kTileBytes, &tm_v, 0, row0p + i * kWarpChunk, full);
@@ -122,6 +126,8 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
   const int row0 = (slot * kKvHeads + kvh) * s_max;  // first cache row of this (slot, KV head)
 
   FlowState st;
+  // the use of bar_full that tile i of stage s is: the first tile of a stage may have come on the other barrier
+  auto full_phase = [&](int i, int s) { return i / kStreamStages - (!stale && s < pre ? 1 : 0); };
 
   const bool finish = fin.part != nullptr || fin.qkv != nullptr;
   if (finish && warp < kStreamWarps) {
@@ -184,11 +190,11 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
   if (warp == kStreamWarps) {
     // ---------------- producer: one thread keeps the ring full ----------------
     if (lane == 0) {
-      int repeated = 0, issued = pre;  // early copies fetched again; tiles requested so far
-      if (stale) {  // wait for the early copies to land, then fetch the same tiles again
-        for (int i = 0; i < pre; ++i, ++repeated) {
+      int issued = pre;  // tiles requested so far
+      if (stale) {       // wait for the early copies to land, then fetch the same tiles again
+        for (int i = 0; i < pre; ++i) {
           const uint32_t full = smem_u32(&bar_full[i]), dst = base + i * kStageBytes;
-          if (!mbar_wait(full, 0, spin_limit)) {
+          if (!mbar_wait(smem_u32(&bar_early[i]), 0, spin_limit)) {
             fail_s = 1;
             break;
           }
@@ -215,8 +221,8 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
       // In the normal course the consumers needed these phases anyway.
       for (int i = issued > kStreamStages ? issued - kStreamStages : 0; i < issued; ++i) {
         const int s = i % kStreamStages;
-        const int phase = i / kStreamStages + ((i < pre ? i < repeated : (stale && s < pre)) ? 1 : 0);
-        if (!mbar_wait(smem_u32(&bar_full[s]), phase & 1, spin_limit)) fail_s = 1;
+        const bool early = i < pre && !stale;
+        if (!mbar_wait(smem_u32(early ? &bar_early[s] : &bar_full[s]), early ? 0 : full_phase(i, s) & 1, spin_limit)) fail_s = 1;
       }
     }
   } else if (n_tiles > 0) {
@@ -231,9 +237,8 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     }
     for (int i = warp; i < n_tiles; i += kStreamWarps) {
       const int s = i % kStreamStages;
-      // (a stage whose early copy was repeated is one phase ahead for the rest of the kernel)
-      const int shift = (stale && s < pre) ? 1 : 0;
-      bool ok = mbar_wait(smem_u32(&bar_full[s]), ((i / kStreamStages) + shift) & 1, spin_limit);
+      const bool early = i < pre && !stale;
+      bool ok = mbar_wait(smem_u32(early ? &bar_early[s] : &bar_full[s]), early ? 0 : full_phase(i, s) & 1, spin_limit);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) fail_s = 2;

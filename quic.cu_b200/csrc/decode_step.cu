@@ -556,7 +556,6 @@ int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_
   a.s_max = d->s_max;
   a.n_slots = d->n_slots;
   a.res = h;
-
   // (the head of a sequence starts only after everything enqueued before it has completed)
   QUIC_CUDA(launch_embed_ssq((const half*)m->embed, d->rows, d->tok, m->vocab, h, ssq_end, B, st, !chain_head));
   int rc;
