@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
     }
   } else if (warp == kSoftmaxWarps + 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
+      const uint64_t q0 = umma_desc_sw128(base + kSmemQ), k0 = umma_desc_sw128(base + kSmemK), v0 = umma_desc_sw128(base + kSmemV);
       const uint32_t idesc = umma_idesc_f16(kKeys);         // M = 128, N = 64
       const uint32_t idesc_v = idesc | (1u << 16);           // B transposed: N (the head dims) contiguous
       auto scores = [&](int i) {
@@ -187,8 +188,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          umma_f16(tmem_s + kColS1 * st, umma_desc_sw128(base + kSmemQ + k * 32),
-                   umma_desc_sw128(base + kSmemK + st * kTileBytes + k * 32), idesc, k > 0 ? 1u : 0u);
+          umma_f16(tmem_s + kColS1 * st, q0 + 2 * k, k0 + (uint64_t)(st * (kTileBytes / 16)) + 2 * k, idesc, k > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_s[st]));
         return true;
       };
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 4; ++k)  // sixteen tokens a step: two groups of eight rows of the V tile, eight columns of P
-          umma_f16_ts(tmem_o, tmem_p + 8u * k, umma_desc_sw128(base + kSmemV + st * kTileBytes + k * 2048), idesc_v,
+          umma_f16_ts(tmem_o, tmem_p + 8u * k, v0 + (uint64_t)(st * (kTileBytes / 16)) + k * (2048 / 16), idesc_v,
                       (i > 0 || k > 0) ? 1u : 0u);
         umma_commit(smem_u32(&bar_empty[st]));
         if (!kAhead && i + 1 < n_tiles)  // P(i) shares S's columns: its product has to be complete

@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
         tma_load_2d(b_s, &tm_x, (kb0 + it) * kBlockK, m0, full);
       }
     }
-  } else if (tid == 0) {
+  } else if (warp == 0 && elect_one()) {
+    const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + L::kA);
     for (int it = 0; it < nkb; ++it) {
       const int stage = it % kDenseStages;
       if (!mbar_wait(smem_u32(&bar_full[stage]), (it / kDenseStages) & 1)) {
@@ -118,11 +119,9 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
         break;
       }
       tc_fence_after();
-      const uint32_t a_s = base + stage * L::kStage, b_s = a_s + L::kA;
+      const uint64_t at = (uint64_t)(stage * (L::kStage / 16));
 #pragma unroll
-      for (int k = 0; k < kBlockK / 16; ++k)
-        umma_f16(tmem_d, umma_desc_sw128(a_s + k * 32), umma_desc_sw128(b_s + k * 32), idesc,
-                 (it > 0 || k > 0) ? 1u : 0u);
+      for (int k = 0; k < kBlockK / 16; ++k) umma_f16(tmem_d, a0 + at + 2 * k, b0 + at + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
       if (it + kDenseStages < nkb) umma_commit(smem_u32(&bar_empty[stage]));
       if (it == nkb - 1) umma_commit(smem_u32(&bar_done));
     }

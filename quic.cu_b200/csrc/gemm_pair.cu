@@ -212,7 +212,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
+      const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + kPairA);
       // fp16 x fp16 -> fp32, both operands K-major, M = 256 over the pair, N = NT
       constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       int stage = 0, pass = 0, j = 0;
@@ -233,10 +234,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             break;
           }
           tc_fence_after();
-          const uint32_t a_s = base + stage * L::kStage, b_s = a_s + kPairA;
+          const uint64_t at = (uint64_t)(stage * (L::kStage / 16));
 #pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k)
-            pair_umma(d, umma_desc_sw128(a_s + k * 32), umma_desc_sw128(b_s + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < kBlockK / 16; ++k) pair_umma(d, a0 + at + 2 * k, b0 + at + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           pair_commit(smem_u32(&bar_empty[stage]));
           if (++stage == kPairStages) {
             stage = 0;

@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
         tma_load_2d(b_s, &tm_x, kb * kBlockK, 0, full);
       }
     }
-  } else if (tid == 0) {
+  } else if (warp == 0 && elect_one()) {
+    const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + L::kA);
     for (int it = 0; it < nkb; ++it) {
       const int stage = it % kLmStages;
       if (!mbar_wait(smem_u32(&bar_full[stage]), (it / kLmStages) & 1)) {
@@ -108,11 +109,9 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
         break;
       }
       tc_fence_after();
-      const uint32_t a_s = base + stage * L::kStage, b_s = a_s + L::kA;
+      const uint64_t at = (uint64_t)(stage * (L::kStage / 16));
 #pragma unroll
-      for (int k = 0; k < kBlockK / 16; ++k)
-        umma_f16(tmem_d, umma_desc_sw128(a_s + k * 32), umma_desc_sw128(b_s + k * 32), idesc,
-                 (it > 0 || k > 0) ? 1u : 0u);
+      for (int k = 0; k < kBlockK / 16; ++k) umma_f16(tmem_d, a0 + at + 2 * k, b0 + at + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
       umma_commit(smem_u32(&bar_empty[stage]));
       if (it == nkb - 1) umma_commit(smem_u32(&bar_done));
     }

@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
     }
   } else if (warp == kConsumers / 32 + 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
+      const uint64_t b0 = umma_desc_sw128(base + kRawBytes), a0 = umma_desc_sw128(base + kRawBytes + L::kB);
       // One wait per k block (operand A written by the consumer warps and operand B landed by
       // TMA arrive on the same barrier) and a commit only where somebody waits for it: each
       // of these costs the issuing thread a round trip, and at these sizes the loop is bound
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
           break;
         }
         if (it == 0) tc_fence_after();
-        const uint32_t b_s = base + stage * L::kStage + kRawBytes, a_s = b_s + L::kB;
+        const uint64_t at = (uint64_t)(stage * (L::kStage / 16));
 #pragma unroll
         for (int i = 0; i < MTL; ++i) {
           if (i > 0 && m0 + i * MT >= a.m_total) break;  // tile of rows beyond the end
@@ -229,8 +230,8 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
           for (int sub = 0; sub < kSub; ++sub)
 #pragma unroll
             for (int k = 0; k < kBlockK / 16; ++k)
-              umma_f16(tmem_d + (uint32_t)(i * MT), umma_desc_sw128(a_s + sub * L::kASub + k * 32),
-                       umma_desc_sw128(b_s + (i * kSub + sub) * L::kBTile + k * 32), idesc,
+              umma_f16(tmem_d + (uint32_t)(i * MT), a0 + at + sub * (L::kASub / 16) + 2 * k,
+                       b0 + at + (i * kSub + sub) * (L::kBTile / 16) + 2 * k, idesc,
                        (it > 0 || sub > 0 || k > 0) ? 1u : 0u);
         }
         if (it + kStages < nkb) umma_commit(smem_u32(&bar_empty[stage]));
