@@ -13,12 +13,16 @@ namespace {
 // 1 x 1000 2728 -> 2515, 16 x 2048 42.0 -> 33.1 ms.  Dense weights are read as they are: 1 x 130 tokens 1578 -> 1690 us,
 // 1 x 200 1768 -> 1747, 1 x 500 2426 -> 2041, 2 x 1024 5826 -> 3196.
 constexpr int kPairRows = 768, kDensePairRows = 192;
+// Rows up to which a layer runs on the chain of rows_chain.cu: one tile of 128 rows of packed weights (us, GEMMs / chain: 2 rows
+// 816 / 772, 40 948 / 802, 87 1146 / 958, 128 1168 / 1041, 129 1402 / 1419, 256 1432 / 1573), which it unpacks again for every
+// tile; un-quantised ones it reads again (40 1142 / 739, 128 1550 / 1047, 256 1687 / 1461, 300 1927 / 1728, 384 1903 / 1902).
+constexpr int kRowsChain = 128, kDenseRowsChain = 320;
 constexpr int64_t kLayerWeights = (int64_t)(kQkvN + kHidden + 2 * kInter) * kHidden + (int64_t)kHidden * kInter;
 
 inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
 struct PrefillArena {
-  int64_t lm, h, xn, tmp, qkv, q, attn, gu, act, xlast, ws, w16, total;
+  int64_t lm, h, xn, tmp, qkv, q, attn, gu, act, xlast, ssq, ws, w16, total;
 };
 
 int64_t linear_ws(int rows) {
@@ -58,6 +62,8 @@ PrefillArena carve_prefill(int rows, int n_seq, int vocab) {
   off += align256((int64_t)rows * kInter * 2);
   a.xlast = off;
   off += align256((int64_t)n_seq * kHidden * 2);
+  a.ssq = off;  // sums of squares of the residual stream's rows, twice (rows chain)
+  off += align256((int64_t)2 * rows * kRowsSsq * 4);
   a.ws = off;
   off += align256(linear_ws(rows));
   a.w16 = off;  // fp16 copies of one layer's packed weights
@@ -117,6 +123,81 @@ int linear_parts(const half* x, const quic_w4_t& w, half* y, int rows, void* ws,
   return quic_w4a16_linear(x, &w, y, rows, 1, ws, st);
 }
 
+// xn holds the finally normalised rows: lm_head + argmax on the last one of every sequence
+int prefill_finish(const quic_model_t* m, const quic_prefill_t* p, const PrefillArena& ar, cudaStream_t st) {
+  char* base = static_cast<char*>(p->scratch);
+  const half* xn = reinterpret_cast<const half*>(base + ar.xn);
+  half* xlast = reinterpret_cast<half*>(base + ar.xlast);
+  gather_last_kernel<<<p->n_seq, 224, 0, st>>>(xn, p->seq_start, p->seq_len, xlast);
+  QUIC_CUDA(cudaGetLastError());
+  const int rc = quic_lm_head_argmax(xlast, nullptr, m->eps, m->embed, m->vocab, p->n_seq, p->logits, p->first_tokens, base + ar.lm, st);
+  if (rc != QUIC_OK) return rc;
+  set_slot_state_kernel<<<(p->n_seq + 127) / 128, 128, 0, st>>>(p->first_tokens, p->seq_len, p->seq_slot, p->seq_off,
+                                                               p->n_seq, p->n_slots, p->tok, p->pos);
+  QUIC_CUDA(cudaGetLastError());
+  return QUIC_OK;
+}
+
+// Few rows: five launches a layer (rows_chain.cu and the attention).
+int prefill_rows(const quic_model_t* m, const quic_prefill_t* p, const PrefillArena& ar, cudaStream_t st) {
+  char* base = static_cast<char*>(p->scratch);
+  half* h = reinterpret_cast<half*>(base + ar.h);
+  half* q = reinterpret_cast<half*>(base + ar.q);
+  half* attn = reinterpret_cast<half*>(base + ar.attn);
+  half* act = reinterpret_cast<half*>(base + ar.act);
+  float* const ssq_mid = reinterpret_cast<float*>(base + ar.ssq);
+  float* const ssq_end = ssq_mid + (size_t)p->rows * kRowsSsq;
+  const size_t kv_plane = (size_t)p->n_slots * kKvHeads * p->s_max * kHeadDim;
+  RowsArgs a = {};
+  a.rows = p->rows;
+  a.eps = m->eps;
+  a.slots = p->row_slot;
+  a.row_pos = p->row_pos;
+  a.cos_t = (const half*)m->rope_cos;
+  a.sin_t = (const half*)m->rope_sin;
+  a.max_pos = m->max_pos;
+  a.s_max = p->s_max;
+  a.n_slots = p->n_slots;
+  a.head_major = 1;
+  a.res = h;
+  QUIC_CUDA(launch_embed_ssq((const half*)m->embed, nullptr, p->ids, m->vocab, h, ssq_end, p->rows, st, false));
+  int rc;
+  for (int l = 0; l < m->n_layers; ++l) {
+    const quic_layer_t& L = m->layers[l];
+    a.kcache = static_cast<half*>(p->kv) + (size_t)(2 * l) * kv_plane;
+    a.vcache = a.kcache + kv_plane;
+    a.w = L.qkv;
+    a.y = q;
+    a.ln = (const half*)L.ln1;
+    a.ssq_in = ssq_end;
+    a.n_ssq = l == 0 ? 1 : kRowsSsq;
+    rows_next(&a, &L.o);
+    if ((rc = rows_qkv(h, a, st)) != QUIC_OK) return rc;
+    if ((rc = attn_prefill_launch(q, a.kcache, a.vcache, p->seq_start, p->seq_len, p->seq_slot, p->seq_off, p->n_seq, p->max_len, p->rows,
+                                  p->s_max, p->n_slots, 0.125f /* 64^-0.5, src/model.py:129 */, attn, st, true)) != QUIC_OK)
+      return rc;
+    a.w = L.o;
+    a.y = h;
+    a.ssq_out = ssq_mid;
+    rows_next(&a, &L.gate_up);
+    if ((rc = rows_out(attn, a, st)) != QUIC_OK) return rc;
+    a.w = L.gate_up;
+    a.y = act;
+    a.ln = (const half*)L.ln2;
+    a.ssq_in = ssq_mid;
+    a.n_ssq = kRowsSsq;
+    rows_next(&a, &L.down);
+    if ((rc = rows_swiglu(h, a, st)) != QUIC_OK) return rc;
+    a.w = L.down;
+    a.y = h;
+    a.ssq_out = ssq_end;
+    rows_next(&a, l + 1 < m->n_layers ? &m->layers[l + 1].qkv : nullptr);
+    if ((rc = rows_down(act, a, st)) != QUIC_OK) return rc;
+  }
+  QUIC_CUDA(launch_rmsnorm(h, nullptr, (const half*)m->final_norm, m->eps, reinterpret_cast<half*>(base + ar.xn), nullptr, p->rows, st));
+  return QUIC_OK;
+}
+
 }  // namespace
 }  // namespace quic
 
@@ -148,7 +229,6 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
   half* attn = reinterpret_cast<half*>(base + ar.attn);
   half* gu = reinterpret_cast<half*>(base + ar.gu);
   half* act = reinterpret_cast<half*>(base + ar.act);
-  half* xlast = reinterpret_cast<half*>(base + ar.xlast);
   void* ws = base + ar.ws;
   half* const w16[4] = {reinterpret_cast<half*>(base + ar.w16), reinterpret_cast<half*>(base + ar.w16) + kQkvN * kHidden,
                         reinterpret_cast<half*>(base + ar.w16) + (kQkvN + kHidden) * kHidden,
@@ -156,12 +236,16 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
   const size_t slot_stride = (size_t)kKvHeads * p->s_max * kHeadDim;
   const size_t kv_plane = (size_t)p->n_slots * slot_stride;
 
+  int rc = QUIC_OK, sp = 0;
+  if (rows >= 2 && rows <= (m->layers[0].qkv.w16 != nullptr ? kDenseRowsChain : kRowsChain)) {
+    if ((rc = prefill_rows(m, p, ar, st)) != QUIC_OK) return rc;
+    return prefill_finish(m, p, ar, st);
+  }
   embed_tokens_kernel<<<rows, 224, 0, st>>>((const half*)m->embed, p->ids, m->vocab, h);
   QUIC_CUDA(cudaGetLastError());
   // From here on the kernels are chained with programmatic dependent launch: each one does
   // its set-up (and the GEMMs request their weight tiles) while its predecessor drains.
   QUIC_CUDA(launch_rmsnorm(h, nullptr, (const half*)m->layers[0].ln1, m->eps, xn, nullptr, rows, st));
-  int rc = QUIC_OK, sp = 0;
   const float* part = static_cast<const float*>(ws) + 4096;  // (behind the workspace's 16 KB head)
   for (int l = 0; l < m->n_layers; ++l) {
     const quic_layer_t& L = m->layers[l];
@@ -216,14 +300,5 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
     QUIC_CUDA(sp > 0 ? launch_rmsnorm_part(part, sp, h, (const half*)next_ln, m->eps, xn, h, rows, st)
                      : launch_rmsnorm(tmp, h, (const half*)next_ln, m->eps, xn, h, rows, st));
   }
-  // xn holds the finally normalised rows: lm_head + argmax on the last one of every sequence
-  gather_last_kernel<<<p->n_seq, 224, 0, st>>>(xn, p->seq_start, p->seq_len, xlast);
-  QUIC_CUDA(cudaGetLastError());
-  if ((rc = quic_lm_head_argmax(xlast, nullptr, m->eps, m->embed, m->vocab, p->n_seq, p->logits, p->first_tokens,
-                                base + ar.lm, stream)) != QUIC_OK)
-    return rc;
-  set_slot_state_kernel<<<(p->n_seq + 127) / 128, 128, 0, st>>>(p->first_tokens, p->seq_len, p->seq_slot, p->seq_off,
-                                                               p->n_seq, p->n_slots, p->tok, p->pos);
-  QUIC_CUDA(cudaGetLastError());
-  return QUIC_OK;
+  return prefill_finish(m, p, ar, st);
 }

@@ -73,3 +73,25 @@ def test_rows_of_very_small_and_large_norm(nets):
         assert worst < 2 * 3 ** 0.5 * 2 ** -12, worst  # three roundings on either side
     finally:
         net.embed.copy_(embed)
+
+
+@pytest.mark.parametrize("weights,lens", [("w4", [2]), ("w4", [64]), ("w4", [40, 25]), ("w4", [128]), ("w4", [1] * 20), ("fp16", [3]),
+                                          ("fp16", [65]), ("fp16", [129]), ("fp16", [200, 120])])
+def test_a_short_prefill_matches_the_operators_one_by_one(nets, weights, lens):
+    """Edges of the row tiles and of what the chain takes of prompts (128 rows, un-quantised 320): keys, values and the last
+    rows' logits against the per-operator prefill.  Roundings as above, three more for a logit."""
+    net = nets[weights]
+    gen = torch.Generator().manual_seed(sum(lens))
+    prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
+    slots = torch.randperm(len(lens) + 1, generator=gen)[:len(lens)].tolist()
+    cache, other = (net.new_cache(n_slots=len(lens) + 1, s_max=256) for _ in range(2))
+    first, logits = net.prefill(cache, slots, prompts)
+    _, want = net.prefill(other, slots, prompts, all_logits=True)
+    last = torch.tensor(lens).cumsum(0) - 1
+    worst = (norm(logits.float() - want.view(-1, 2048)[last].float(), dim=1) / norm(want.view(-1, 2048)[last].float(), dim=1)).max().item()
+    assert worst < 2 * (40 / 3) ** 0.5 * 2 ** -11, worst
+    for slot, n in zip(slots, lens):
+        got, ref = cache.kv[:, :, slot, :, :n].float(), other.kv[:, :, slot, :, :n].float()
+        worst = (norm(got - ref, dim=(2, 4)) / norm(ref, dim=(2, 4))).max().item()
+        assert worst < 2 * (34 / 3) ** 0.5 * 2 ** -11, worst
+    assert cache.pos[slots].tolist() == lens and cache.tok[slots].tolist() == first.tolist()
