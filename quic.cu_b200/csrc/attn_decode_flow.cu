@@ -70,6 +70,9 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncthreads();
+  pdl_launch_dependents();
+  pdl_wait();  // the set-up runs under the kernel in front
   int t_begin = a.start != nullptr ? a.start[b] : 0, t_end = a.end != nullptr ? a.end[b] : a.s_cap;
   if (t_end > a.s_cap) t_end = a.s_cap;
   if (t_begin < 0) t_begin = 0;
@@ -77,7 +80,6 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
   const int tile0 = t_begin / kWarpChunk;
   const int tiles = t_end > t_begin ? (t_end + kWarpChunk - 1) / kWarpChunk - tile0 : 0;
   const int i0 = (int)((int64_t)tiles * split / a.splits), i1 = (int)((int64_t)tiles * (split + 1) / a.splits);
-  __syncthreads();
 
   auto request = [&](int i) {
     if (lane == 0) {
@@ -203,25 +205,21 @@ int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t str
   if (rc != QUIC_OK) return rc;
   rc = make_kv_map(&tm_v, a.v, a.stride_b, a.stride_h, batch, a.s_cap);
   if (rc != QUIC_OK) return rc;
-  static bool allowed[64] = {};
-  int dev = 0;
-  QUIC_CUDA(cudaGetDevice(&dev));
-  if (dev > 63 || !allowed[dev]) {
-    QUIC_CUDA(cudaFuncSetAttribute(attn_decode_flow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlowSmem));
-    if (dev <= 63) allowed[dev] = true;
-  }
+  QUIC_CUDA(allow_smem<attn_decode_flow_kernel>(kFlowSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.splits, kKvHeads, batch);
   cfg.blockDim = dim3(kFlowWarps * 32);
   cfg.dynamicSmemBytes = kFlowSmem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)a.splits;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
   QUIC_CUDA(cudaLaunchKernelEx(&cfg, attn_decode_flow_kernel, tm_k, tm_v, a, status));
   return QUIC_OK;
 }

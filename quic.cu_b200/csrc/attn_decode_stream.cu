@@ -321,12 +321,7 @@ int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int 
   rc = make_map(&tm_v, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.v, rows, kHeadDim, kWarpChunk, kHeadDim,
                 CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != QUIC_OK) return rc;
-  static bool attr_set = false;
-  if (!attr_set) {
-    QUIC_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kStreamSmem));
-    attr_set = true;
-  }
+  QUIC_CUDA(allow_smem<attn_decode_stream_kernel>(kStreamSmem));
   QUIC_CUDA(launch(attn_decode_stream_kernel, dim3(kKvHeads, batch), dim3((kStreamWarps + 1) * 32), kStreamSmem, stream,
                    pdl, tm_k, tm_v, a, fin, n_slots, s_max, status, g_stream_hook == 1 ? 1 : 0, g_stream_hook == 2 ? 1 : 0,
                    g_stream_hook == 2 ? 20000u : kSpinLimit));

@@ -366,7 +366,7 @@ int attn_prefill_tc_launch(const void* q, const void* kcache, const void* vcache
   const dim3 grid(kHeads, n_seq, (max_len + kQRows - 1) / kQRows);
   const bool ahead = (int64_t)grid.x * grid.y * grid.z <= 4 * 148;
   auto kernel = ahead ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>;
-  QUIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal));
+  QUIC_CUDA(ahead ? allow_smem<attn_prefill_tc_kernel<true>>(kSmemTotal) : allow_smem<attn_prefill_tc_kernel<false>>(kSmemTotal));
   QUIC_CUDA(launch(kernel, grid, dim3(kAttThreads), kSmemTotal, stream, pdl, tm_q, tm_k, tm_v, a, status));
   return QUIC_OK;
 }

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/quic_b200.h"
 
 namespace quic {
@@ -58,6 +60,18 @@ __device__ __forceinline__ void pdl_wait() {
 // Process-wide switch (quic_set_pdl): when 0 every kernel is launched with plain
 // stream ordering.  For A/B timing and debugging only.
 bool pdl_enabled();
+
+// Lets a kernel use this much dynamic shared memory, once per device (asked at every launch it costs the host 0.4 us).
+template <auto* Kernel>
+inline cudaError_t allow_smem(size_t bytes) {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev < 64 && (done.load(std::memory_order_relaxed) >> dev & 1))) return e;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && dev < 64) done.fetch_or(uint64_t(1) << dev, std::memory_order_relaxed);
+  return e;
+}
 
 // Launch helper: `pdl` chains the kernel to the previous launch on the stream.
 template <typename... KArgs, typename... Args>

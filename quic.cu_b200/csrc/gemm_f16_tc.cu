@@ -216,7 +216,7 @@ int run(const half* x, const half* w, const DenseArgs& a, int splits, cudaStream
   int* status = tc_status_words();
   QUIC_REQUIRE(status != nullptr, QUIC_E_CUDA, "gemm_f16: no address for the tensor path's error words");
   const size_t smem = DenseSmem<MT>::kTotal;
-  QUIC_CUDA(cudaFuncSetAttribute(gemm_f16_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QUIC_CUDA(allow_smem<gemm_f16_tc_kernel<MT>>(smem));
   dim3 grid(a.n / kTileN, (a.m_total + MT - 1) / MT, splits);
   QUIC_CUDA(launch(gemm_f16_tc_kernel<MT>, grid, dim3(kDenseThreads), smem, st, pdl, tm_w, tm_x, a, status));
   return QUIC_OK;

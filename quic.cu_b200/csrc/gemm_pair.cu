@@ -345,13 +345,7 @@ int run_pair(const half* x, const half* w, const PairArgs& a, cudaStream_t st) {
                 CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != QUIC_OK) return rc;
   auto kernel = gemm_pair_kernel<NT, kSwiglu, kRope>;
-  static bool allowed[64] = {};
-  int dev = 0;
-  QUIC_CUDA(cudaGetDevice(&dev));
-  if (dev > 63 || !allowed[dev]) {
-    QUIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairSmem<NT>::kTotal));
-    if (dev <= 63) allowed[dev] = true;
-  }
+  QUIC_CUDA((allow_smem<gemm_pair_kernel<NT, kSwiglu, kRope>>(PairSmem<NT>::kTotal)));
   const int64_t tiles = (int64_t)(a.n / NT) * ((a.m_total + 255) / 256) * a.splits;
   const int pairs = tiles < 74 ? (int)tiles : 74;
   QUIC_CUDA(launch(kernel, dim3(2 * pairs), dim3(kPairThreads), (size_t)PairSmem<NT>::kTotal, st, true, tm_x, tm_w, a));

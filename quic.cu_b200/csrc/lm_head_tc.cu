@@ -215,7 +215,7 @@ int run(const LmHeadArgs& a, cudaStream_t st) {
   QUIC_REQUIRE(status != nullptr, QUIC_E_CUDA, "lm_head: no address for the tensor path's error words");
   status += 1;
   const size_t smem = LmSmem<MT>::kTotal;
-  QUIC_CUDA(cudaFuncSetAttribute(lm_head_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QUIC_CUDA(allow_smem<lm_head_tc_kernel<MT>>(smem));
   QUIC_CUDA(launch(lm_head_tc_kernel<MT>, dim3(a.vocab / kTileN), dim3(kLmThreads), smem, st, true, tm_e, tm_x, a,
                    status));
   return QUIC_OK;

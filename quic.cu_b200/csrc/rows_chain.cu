@@ -30,8 +30,6 @@
 //
 // Every mbarrier wait is bounded: on a timeout the CTA records a code, takes part in the cluster's barriers, waits for
 // its own copies in flight, frees its tensor memory and returns.
-#include <atomic>
-
 #include "tc_common.cuh"
 
 namespace quic {
@@ -621,13 +619,7 @@ int launch_rows(const half* x, const RowsArgs& a, cudaStream_t st, bool pdl) {
                   CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != QUIC_OK) return rc;
   }
-  int dev = 0;
-  QUIC_CUDA(cudaGetDevice(&dev));
-  static std::atomic<uint64_t> ready{0};  // devices on which the kernel may use this much shared memory
-  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1)) {
-    QUIC_CUDA(cudaFuncSetAttribute(rows_linear_kernel<MODE, M, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
-    if (dev < 64) ready.fetch_or(uint64_t(1) << dev, std::memory_order_relaxed);
-  }
+  QUIC_CUDA((allow_smem<rows_linear_kernel<MODE, M, DENSE>>(C::smem)));
   const int mtiles = (a.rows + M - 1) / M;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = C::split ? dim3(C::cluster, kHidden / kTileCols, mtiles)

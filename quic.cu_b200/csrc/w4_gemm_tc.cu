@@ -448,8 +448,7 @@ int run_variant(const half* x, GemmArgs a, int splits, cudaStream_t st) {
   const int mtiles = (a.m_total + MT - 1) / MT;
   const size_t smem = (size_t)kDeep * L::kStage + 1024;
   dim3 grid(a.w.n / kTileN, splits, (mtiles + MTL - 1) / MTL);
-  QUIC_CUDA(cudaFuncSetAttribute(w4a16_gemm_tc_kernel<MT, kDeep, MTL, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  QUIC_CUDA((allow_smem<w4a16_gemm_tc_kernel<MT, kDeep, MTL, KS>>(smem)));
   QUIC_CUDA(launch(w4a16_gemm_tc_kernel<MT, kDeep, MTL, KS>, grid, dim3(kGemmThreads), smem, st, true, tm_w, tm_x, a));
   return QUIC_OK;
 }

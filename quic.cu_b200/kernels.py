@@ -241,6 +241,9 @@ def _thread_scratch(key: tuple[str, int, int], need: int, least: int, head: int)
     return t
 
 
+_HALF = torch.float16
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
@@ -373,24 +376,26 @@ MAX_LINEAR_ROWS = 8192  # rows per launch; longer inputs are processed in chunks
 def w4a16_linear(w, x: torch.Tensor, use_tensor: bool | None = None) -> torch.Tensor:
     """y = x · dequant(W)^T + bias.  Replaces marlin_linear (src/quant/marlin.py:190); with an
     F16Weight the dense linear of the un-quantised model (_linear, src/model.py:35-41)."""
-    _need_cuda(x)
-    _need_half(x)
-    plain = x.dim() == 2 and x.shape[1] == w.size_k
-    x2 = x.contiguous() if plain else x.contiguous().reshape(-1, w.size_k)
-    m = x2.shape[0]
-    y = x2.new_empty((m, w.size_n))
+    if not x.is_cuda or x.dtype is not _HALF:
+        _need_cuda(x)
+        _need_half(x)
+    k, n, shape = w.size_k, w.size_n, x.shape
+    plain = len(shape) == 2 and shape[1] == k
+    x2 = x.contiguous() if plain else x.contiguous().reshape(-1, k)
+    m = shape[0] if plain else x2.shape[0]
+    y = x2.new_empty(m, n)
     if use_tensor is None:
         use_tensor = TENSOR_PATH and m >= TENSOR_MIN_ROWS
-    ref, run, stream = _launch_ref(w), lib().quic_w4a16_linear, _raw_stream(x2.get_device())
+    tensor, ref, run, stream = 1 if use_tensor else 0, _launch_ref(w), lib().quic_w4a16_linear, _raw_stream(x2.get_device())
     xp, yp, done = x2.data_ptr(), y.data_ptr(), 0
     while done < m:
         rows = min(MAX_LINEAR_ROWS, m - done)
-        rc = run(xp + 2 * done * w.size_k, ref, yp + 2 * done * w.size_n, rows, 1 if use_tensor else 0,
-                 ptr(w.workspace(rows, stream)), stream)
+        ws = w.workspace(rows, stream)
+        rc = run(xp + 2 * done * k, ref, yp + 2 * done * n, rows, tensor, None if ws is None else ws.data_ptr(), stream)
         if rc != 0:
             check(rc, "w4a16_linear")
         done += rows
-    return y if plain else y.reshape(*x.shape[:-1], w.size_n)
+    return y if plain else y.reshape(*shape[:-1], n)
 
 
 # ---------------------------------------------------------------------------------
@@ -629,21 +634,24 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
                                splits: int = 0, cta_merge: bool = False) -> torch.Tensor:
     """flash_attn_decode.forward(Q fp16 [B,nh,1,64], K, V fp16 [B,n_kv,S,64], softmax_scale,
     pad_lens int32 [B] or None) -> fp16 [B,nh,1,64] (flash_attn_decode.cu:133-198)."""
-    _need_cuda(q, k, v, pad_lens)
-    _need_half(q, k, v)
-    if q.dim() != 4 or q.shape[2] != 1 or q.shape[3] != HEAD_DIM:
+    if not (q.is_cuda and k.is_cuda and v.is_cuda and q.dtype is _HALF and k.dtype is _HALF and v.dtype is _HALF and
+            (pad_lens is None or pad_lens.is_cuda)):
+        _need_cuda(q, k, v, pad_lens)
+        _need_half(q, k, v)
+    qs, ks = q.shape, k.shape
+    if len(qs) != 4 or qs[2] != 1 or qs[3] != HEAD_DIM:
         raise RuntimeError("flash_attn_decode: Q must be [B, nh, 1, 64]")
-    b, nh = q.shape[0], q.shape[1]
-    if nh != HEADS or k.shape[1] != KV_HEADS:
+    b, nh = qs[0], qs[1]
+    if nh != HEADS or ks[1] != KV_HEADS:
         raise RuntimeError("flash_attn_decode: built for 14 query heads / 2 KV heads")
-    if k.shape[0] != b or v.shape != k.shape or k.shape[3] != HEAD_DIM:
+    if ks[0] != b or v.shape != ks or ks[3] != HEAD_DIM:
         raise RuntimeError("flash_attn_decode: K/V shape mismatch")
-    s = k.shape[2]
+    s = ks[2]
     if pad_lens is not None and not (pad_lens.dtype == torch.int32 and pad_lens.dim() == 1 and
                                      pad_lens.shape[0] == b and pad_lens.is_contiguous()):
         raise RuntimeError("flash_attn_decode: pad_lens must be a contiguous CUDA int32 tensor of shape [B]")
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    out = q.new_empty((b, nh, 1, HEAD_DIM))
+    out = q.new_empty(b, nh, 1, HEAD_DIM)
     if s == 0:
         return out.zero_()
     scale = float(softmax_scale) if softmax_scale and softmax_scale > 0 else HEAD_DIM ** -0.5
@@ -658,7 +666,8 @@ def _flash_attn_decode_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     stream = _raw_stream(device)
     scratch = _thread_scratch(("attention", device, stream), need, 1 << 20, max(8 * b, 1 << 16)) if need > 0 else None
     rc = lib().quic_attn_decode(q_ptr, k.data_ptr(), v.data_ptr(), KV_HEADS * s * HEAD_DIM, s * HEAD_DIM,
-                                ptr(pad_lens), None, s, scale, out.data_ptr(), b, splits, ptr(scratch), stream)
+                                None if pad_lens is None else pad_lens.data_ptr(), None, s, scale, out.data_ptr(), b, splits,
+                                None if scratch is None else scratch.data_ptr(), stream)
     if rc != 0:
         check(rc, "attn_decode")
     return out
