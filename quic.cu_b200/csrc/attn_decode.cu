@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kWarps * 32) attn_decode_kernel(const AttnArgs
       }
     }
   }
-  if (a.splits == 1 || a.consumer_merge) return;
+  if (a.splits == 1) return;
 
   merge_splits_last_cta(a, b, kvh, split, &last_flag);
 }
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(32) attn_decode_warp_kernel(const AttnArgs a) 
       }
     }
   }
-  if (a.splits == 1 || a.consumer_merge) return;
+  if (a.splits == 1) return;
   if (a.splits <= 32) {
     merge_splits_warp(a, b, kvh);
   } else {
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attn_decode_mma_kernel(const A
       }
     }
   }
-  if (a.splits == 1 || a.consumer_merge) return;
+  if (a.splits == 1) return;
   merge_splits_last_cta(a, b, kvh, split, &last_flag);
 }
 

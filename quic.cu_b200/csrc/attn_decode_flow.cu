@@ -73,7 +73,11 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
   __syncthreads();
   pdl_launch_dependents();
   pdl_wait();  // the set-up runs under the kernel in front
-  int t_begin = a.start != nullptr ? a.start[b] : 0, t_end = a.end != nullptr ? a.end[b] : a.s_cap;
+  int t_begin = a.start != nullptr ? a.start[b] : 0, t_end = a.end != nullptr ? a.end[b] : a.s_cap, plane = b;
+  if (a.pos != nullptr) {  // a decode step: the row's slot, up to the token that it has just appended
+    plane = a.rows[b];
+    t_end = __ldcg(a.pos + plane) + 1;
+  }
   if (t_end > a.s_cap) t_end = a.s_cap;
   if (t_begin < 0) t_begin = 0;
   // this split's tiles: an equal share of the tiles that hold the row's tokens
@@ -84,8 +88,8 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
   auto request = [&](int i) {
     if (lane == 0) {
       mbar_expect_tx(bar, kFlowStage);
-      tma_load_4d(k_s, &tm_k, (tile0 + i) * kWarpChunk, kvh, b, bar);
-      tma_load_4d(v_s, &tm_v, (tile0 + i) * kWarpChunk, kvh, b, bar);
+      tma_load_4d(k_s, &tm_k, (tile0 + i) * kWarpChunk, kvh, plane, bar);
+      tma_load_4d(v_s, &tm_v, (tile0 + i) * kWarpChunk, kvh, plane, bar);
     }
   };
   if (i0 + warp < i1) request(i0 + warp);
@@ -198,12 +202,13 @@ int attn_flow_splits(int b, int s_max) {
   return s < 3 ? 1 : s > 8 ? 8 : s;
 }
 
-int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t stream) {
+int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t stream, int n_slots) {
   QUIC_REQUIRE(status != nullptr, QUIC_E_ARG, "attn_decode: no status word");
   CUtensorMap tm_k, tm_v;
-  int rc = make_kv_map(&tm_k, a.k, a.stride_b, a.stride_h, batch, a.s_cap);
+  const int planes = n_slots > 0 ? n_slots : batch;
+  int rc = make_kv_map(&tm_k, a.k, a.stride_b, a.stride_h, planes, a.s_cap);
   if (rc != QUIC_OK) return rc;
-  rc = make_kv_map(&tm_v, a.v, a.stride_b, a.stride_h, batch, a.s_cap);
+  rc = make_kv_map(&tm_v, a.v, a.stride_b, a.stride_h, planes, a.s_cap);
   if (rc != QUIC_OK) return rc;
   QUIC_CUDA(allow_smem<attn_decode_flow_kernel>(kFlowSmem));
   cudaLaunchConfig_t cfg = {};
@@ -221,7 +226,7 @@ int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t str
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   // Only where two CTAs share an SM anyway: the CTAs of the next call find room beside those of this one, and where each
   // was to have an SM to itself some then share one (16 x 8192 16.4 -> 14.9 us a call, 9 x 8252 11.2 -> 11.8).
-  cfg.numAttrs = pdl_enabled() && kKvHeads * batch * a.splits > 148 ? 2 : 1;
+  cfg.numAttrs = pdl_enabled() && (n_slots > 0 || kKvHeads * batch * a.splits > 148) ? 2 : 1;
   QUIC_CUDA(cudaLaunchKernelEx(&cfg, attn_decode_flow_kernel, tm_k, tm_v, a, status));
   return QUIC_OK;
 }

@@ -11,13 +11,6 @@ __host__ __device__ __forceinline__ int down_group_begin(int ks) {
   return ks <= 3 ? ks * 8 : 24 + (ks - 3) * 7;
 }
 constexpr int kMaxM = 8;  // batch rows per CTA pass
-// The o_proj kernel merges the attention splits itself: this many per pass of loads, up to
-// kMaxConsumerSplitsTotal in all.  kWarpMaxSplits: the single-warp attention kernel covers a
-// context of up to this many 64-token tiles (2048 tokens).
-constexpr int kMaxConsumerSplits = 16;
-constexpr int kMaxConsumerSplitsTotal = 64;
-constexpr int kWarpMaxSplits = 32;
-
 struct RowState {
   const int32_t* rows;  // [batch] slot per row
   const int32_t* tok;   // [n_slots]
@@ -47,12 +40,7 @@ struct QkvArgs {
 
 struct OProjArgs {
   quic_w4_t w;
-  // splits > 0: merge the attention kernel's split partials here
-  int32_t splits;
-  const float* o_part;  // [batch][14][splits][64]
-  const float* m_part;  // [batch][14][splits]
-  const float* l_part;
-  const half* attn;     // [batch][896] (splits == 0)
+  const half* attn;     // [batch][896]
   const half* xres_in;  // [batch][896]
   half* xres_out;
   int32_t batch;
@@ -87,7 +75,6 @@ struct AttnArgs {
   int32_t s_cap;  // token range covered by the grid
   int32_t chunk;  // tokens per split
   int32_t splits;
-  int32_t consumer_merge;  // 1: write partials only, the o_proj kernel merges
   int32_t small;           // 1: latency variant (one warp per 64 tokens)
   int32_t prefetch;        // latency variant inside the decode chain: cache tile requested before the wait
   const int32_t* epoch;    // step counter that guards the early request (advanced once per decode step)
@@ -120,7 +107,8 @@ struct QkvFinish {
 };
 // Stand-alone op: (row, KV head) ranges in up to eight splits, a TMA stage per warp (attn_decode_flow.cu).
 int attn_flow_splits(int b, int s_max);
-int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t stream);
+// n_slots > 0: a launch of a decode step, the rows' slots and positions in a.rows and a.pos.
+int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t stream, int n_slots = 0);
 int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int n_slots, int s_max, int* status,
                        cudaStream_t stream, bool pdl);
 

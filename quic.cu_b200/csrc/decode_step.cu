@@ -12,8 +12,6 @@
 #include "decode_kernels.cuh"
 
 namespace quic {
-void attn_carve_scratch(void* scratch, int b, int splits, AttnArgs* a);
-
 namespace {
 
 inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
@@ -137,6 +135,42 @@ int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_
 // one tile of 128 on the M side of its MMAs.
 constexpr int kRowsChainMaxRows = 128;
 
+// Which attention kernel a step takes.
+//   cta     CTAs of 512 tokens, their tiles requested before the dependency wait, clusters beyond: up to 20 rows while the CTAs have
+//           an SM each (us per step, cta / flow: 1 x 2100 362 / 395, 5 x 3000 609 / 681, 16 x 1500 718 / 773).
+//   stream  one CTA per (row, KV head) with a deep ring (17 rows of 200..1500 tokens: 791 cta, 865 streamed; 24: 963, 872).
+//   flow    every row cut into up to eight equal ranges, a cluster each: where the others leave SMs idle or a row is one
+//           CTA's walk.  Instead of cta: 16 x 3000 857 -> 814, 20 x 3500 1048 -> 841; instead of stream, from three ranges and 1536 tokens:
+//           24 x 2000 871 -> 812, 24 x 5000 1234 -> 1005, 37 x 3000 1010 -> 974 (24 x 900 would be 709 -> 734); and
+//           instead of splits merged in global memory, beyond 4096 tokens: 1 x 4200 462 -> 424, 5 x 7000 1140 -> 742, 15 x 8000 1624 -> 1008.
+enum AttnForm { kAttnCta, kAttnStream, kAttnFlow };
+constexpr int kCtaAttnMaxRows = 20, kStreamAnyCtxRows = 48, kFlowMinCtx = 1536;
+AttnForm attention_form(int batch, int ctx) {
+  const int parts = attn_cta_splits(ctx);
+  if (batch <= kCtaAttnMaxRows)
+    return parts <= kAttnCtaMaxSplits && (kKvHeads * batch * parts <= 148 || attn_flow_splits(batch, ctx) < 3) ? kAttnCta : kAttnFlow;
+  return batch < kStreamAnyCtxRows && ctx > kFlowMinCtx && attn_flow_splits(batch, ctx) >= 3 ? kAttnFlow : kAttnStream;
+}
+
+// a: queries, cache, rows, positions, scale, output.  `fuse` (form stream only): the kernel finishes the QKV linear itself.
+int launch_attention(AttnArgs a, const quic_decode_t* d, int ctx, cudaStream_t st, const QkvFinish* fuse = nullptr) {
+  const AttnForm form = attention_form(d->batch, ctx);
+  a.prefetch = d->step_counter != nullptr ? 1 : 0;
+  if (form == kAttnCta) {
+    a.splits = attn_cta_splits(ctx);
+    a.chunk = 512;
+    QUIC_CUDA(launch_attn_cta(a, d->batch, st, true));
+    return QUIC_OK;
+  }
+  if (form == kAttnStream) {
+    a.splits = 1;
+    a.chunk = ctx;
+    return launch_attn_stream(a, fuse, d->batch, d->n_slots, d->s_max, tc_status_words(), st, true);
+  }
+  a.splits = attn_flow_splits(d->batch, ctx);
+  return launch_attn_flow(a, d->batch, tc_status_words(), st, d->n_slots);
+}
+
 int enqueue_step(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
   if (B <= kRowsChainMaxRows && B > (m->layers[0].qkv.w16 != nullptr ? kF16ChainMaxRows : g_tensor_min_batch - 1))
@@ -203,42 +237,15 @@ int enqueue_step(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st,
     aa.rows = d->rows;
     aa.pos = d->pos;
     aa.s_cap = ctx;
-    aa.splits = splits;
-    aa.chunk = (ctx + splits - 1) / splits;
     aa.scale = 0.125f;  // 64^-0.5, src/model.py:129
     aa.out = attn_out;
-    // 64-token single-warp CTAs (latency variant) up to 2048 tokens, merged by the o_proj kernel
-    aa.small = (splits <= kWarpMaxSplits && (int64_t)splits * 64 >= ctx) ? 1 : 0;
-    aa.use_mma = 1;  // beyond 2048 tokens: the mma.sync throughput kernel
-    const bool consumer_merge = splits > 1 && splits <= kMaxConsumerSplitsTotal;
-    aa.consumer_merge = consumer_merge ? 1 : 0;
     aa.epoch = d->step_counter;
-    aa.prefetch = (aa.small && d->step_counter != nullptr) ? 1 : 0;
-    // Up to 4096 tokens: CTAs of 512 tokens (eight warps merged in shared memory, every cache tile
-    // requested before the wait), beyond 512 tokens a cluster merged in distributed shared memory;
-    // the o_proj kernel reads the finished heads.  Measured 318 / 347 / 352 us per token at 200 /
-    // 512..576 / 1500 tokens against 347 / 350 / 375 with one-warp CTAs merged by the o_proj kernel.
-    const int cta_splits = attn_cta_splits(ctx);
-    const bool cta_attn = cta_splits <= kAttnCtaMaxSplits;
-    if (cta_attn) {
-      aa.splits = cta_splits;
-      aa.chunk = 512;
-      aa.small = 0;
-      aa.consumer_merge = 0;
-      aa.prefetch = d->step_counter != nullptr ? 1 : 0;
-      QUIC_CUDA(launch_attn_cta(aa, B, st, true));
-    } else {
-      if (splits > 1) attn_carve_scratch(base + ar.attn, B, splits, &aa);
-      QUIC_CUDA(launch_attn(aa, B, st, true));
-    }
+    const int rc = launch_attention(aa, d, ctx, st);
+    if (rc != QUIC_OK) return rc;
 
     OProjArgs oa = {};
     oa.w = L.o;
     oa.attn = attn_out;
-    oa.splits = (!cta_attn && consumer_merge) ? splits : 0;
-    oa.o_part = aa.o_part;
-    oa.m_part = aa.m_part;
-    oa.l_part = aa.l_part;
     oa.xres_in = xres[0];
     oa.xres_out = xres[1];
     oa.batch = B;
@@ -332,25 +339,11 @@ int enqueue_step_rows16(const quic_model_t* m, const quic_decode_t* d, cudaStrea
     aa.rows = d->rows;
     aa.pos = d->pos;
     aa.s_cap = ctx;
-    aa.splits = splits;
-    aa.chunk = (ctx + splits - 1) / splits;
     aa.scale = 0.125f;
     aa.out = attn_out;
-    aa.small = (splits <= 32 && (int64_t)splits * 64 >= ctx) ? 1 : 0;
-    aa.use_mma = 1;
-    aa.consumer_merge = 0;  // the splits are merged by the last CTA to arrive
     aa.epoch = d->step_counter;
-    aa.prefetch = (aa.small && d->step_counter != nullptr) ? 1 : 0;
-    if (attn_cta_splits(ctx) <= kAttnCtaMaxSplits) {
-      // up to 4096 tokens: CTAs of 512 tokens, merged through (distributed) shared memory
-      aa.splits = attn_cta_splits(ctx);
-      aa.chunk = 512;
-      aa.prefetch = d->step_counter != nullptr ? 1 : 0;
-      QUIC_CUDA(launch_attn_cta(aa, B, st, true));
-    } else {
-      if (splits > 1) attn_carve_scratch(base + ar.attn, B, splits, &aa);
-      QUIC_CUDA(launch_attn(aa, B, st, true));
-    }
+    const int rc = launch_attention(aa, d, ctx, st);
+    if (rc != QUIC_OK) return rc;
     QUIC_CUDA(launch_oproj_mma(L.o, attn_out, xa, xb, ssq_b, B, st));
     QUIC_CUDA(launch_gateup_mma(L.gate_up, (const half*)L.ln2, xb, ssq_b, act, B, m->eps, st));
     QUIC_CUDA(launch_down_mma(L.down, act, xb, xa, ssq_a, partial, down_counters, B, st));
@@ -387,23 +380,9 @@ int enqueue_step_rows16(const quic_model_t* m, const quic_decode_t* d, cudaStrea
 // Batch > 16: every linear is the tcgen05 GEMM; norms, RoPE/KV append and SwiGLU are
 // separate small kernels (at these sizes each kernel does microseconds of real work, so
 // the launch chain is no longer what bounds the step).
-// Up to 20 rows the cluster kernel, whose tiles are requested before the dependency wait (17 rows of
-// 200..1500 tokens: 791 us per step against 865 streamed; 24 rows: 963 against 872).
-constexpr int kCtaAttnMaxRows = 20;
-// One CTA per (row, KV head) is a serial walk over the row: with few rows and very long rows the
-// split kernel, which spreads a row over many CTAs, wins (us per step, streamed / split: 24 rows of
-// 4000..8000 tokens 1430 / 1555, of 8000..16000 2157 / 1822; 64 rows of 16000..32000 4079 / 4598).
-constexpr int kStreamMaxCtx = 8192;
-constexpr int kStreamAnyCtxRows = 48;
-
 // `fuse`: the attention kernel finishes the QKV linear itself (only where attention_streams()).
-int enqueue_attention(const quic_decode_t* d, const Arena& ar, int splits, int ctx, half* qbuf, half* kc, half* vc,
-                      half* attn_out, cudaStream_t st, const QkvFinish* fuse = nullptr);
-
-// More than kCtaAttnMaxRows rows of moderate length: the streamed attention kernel.
-bool attention_streams(int batch, int ctx) {
-  return batch > kCtaAttnMaxRows && (ctx <= kStreamMaxCtx || batch >= kStreamAnyCtxRows);
-}
+int enqueue_attention(const quic_decode_t* d, int ctx, half* qbuf, half* kc, half* vc, half* attn_out, cudaStream_t st,
+                      const QkvFinish* fuse = nullptr);
 
 int enqueue_step_batched(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
@@ -434,16 +413,16 @@ int enqueue_step_batched(const quic_model_t* m, const quic_decode_t* d, cudaStre
     const float* part = ws + 4096;
     int rc = w4a16_gemm_tc(xn, L.qkv, nullptr, B, ws, st, &sp);
     if (rc != QUIC_OK) return rc;
-    if (attention_streams(B, ctx)) {
+    if (attention_form(B, ctx) == kAttnStream) {
       // the attention CTAs sum the partial sums, rotate and append themselves: one launch less
       // (64 rows of 512 tokens: 934 -> 883 us per step, same bits)
       QkvFinish fin = {part, sp, (const half*)L.qkv.bias, nullptr, (const half*)m->rope_cos, (const half*)m->rope_sin,
                        m->max_pos};
-      rc = enqueue_attention(d, ar, splits, ctx, qbuf, kc, vc, attn_out, st, &fin);
+      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st, &fin);
     } else {
       QUIC_CUDA(launch_qkv_post_part(part, sp, (const half*)L.qkv.bias, d->rows, d->pos, (const half*)m->rope_cos,
                                      (const half*)m->rope_sin, m->max_pos, qbuf, kc, vc, d->s_max, d->n_slots, B, st));
-      rc = enqueue_attention(d, ar, splits, ctx, qbuf, kc, vc, attn_out, st);
+      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st);
     }
     if (rc != QUIC_OK) return rc;
     rc = w4a16_gemm_tc(attn_out, L.o, nullptr, B, ws, st, &sp);
@@ -480,50 +459,22 @@ int enqueue_step_batched(const quic_model_t* m, const quic_decode_t* d, cudaStre
   return QUIC_OK;
 }
 
-// Attention of a decode step with finished fp16 output: the scratch-free CTA form up to 4096
-// tokens and 32 rows, the split form merged by the last CTA to arrive beyond.
-int enqueue_attention(const quic_decode_t* d, const Arena& ar, int splits, int ctx, half* qbuf, half* kc, half* vc,
-                      half* attn_out, cudaStream_t st, const QkvFinish* fuse) {
-  const int B = d->batch;
-  char* base = static_cast<char*>(d->scratch);
-  const size_t slot_stride = (size_t)kKvHeads * d->s_max * kHeadDim;
+// Attention of a decode step with finished fp16 output.
+int enqueue_attention(const quic_decode_t* d, int ctx, half* qbuf, half* kc, half* vc, half* attn_out, cudaStream_t st,
+                      const QkvFinish* fuse) {
   AttnArgs aa = {};
   aa.q = qbuf;
   aa.k = kc;
   aa.v = vc;
-  aa.stride_b = (int64_t)slot_stride;
+  aa.stride_b = (int64_t)kKvHeads * d->s_max * kHeadDim;
   aa.stride_h = (int64_t)d->s_max * kHeadDim;
   aa.rows = d->rows;
   aa.pos = d->pos;
   aa.s_cap = ctx;
   aa.scale = 0.125f;  // 64^-0.5, src/model.py:129
   aa.out = attn_out;
-  aa.use_mma = 1;
-  aa.consumer_merge = 0;
   aa.epoch = d->step_counter;
-  // few rows: CTAs of 512 tokens, clusters beyond, no scratch
-  if (attn_cta_splits(ctx) <= kAttnCtaMaxSplits && B <= kCtaAttnMaxRows) {
-    aa.splits = attn_cta_splits(ctx);
-    aa.chunk = 512;
-    aa.prefetch = d->step_counter != nullptr ? 1 : 0;
-    QUIC_CUDA(launch_attn_cta(aa, B, st, true));
-    return QUIC_OK;
-  }
-  if (attention_streams(B, ctx)) {
-    // more rows: one CTA per (row, KV head) streams the row's cache through a TMA ring
-    // (64 rows of 200..1500 tokens: 1266 -> 1015 us per step; of 512: 1050 -> 924; of 2000..4000: 1622 -> 1307)
-    aa.splits = 1;
-    aa.chunk = ctx;
-    aa.prefetch = d->step_counter != nullptr ? 1 : 0;
-    return launch_attn_stream(aa, fuse, B, d->n_slots, d->s_max, tc_status_words(), st, true);
-  }
-  aa.splits = splits;
-  aa.chunk = (ctx + splits - 1) / splits;
-  aa.small = (splits <= 32 && (int64_t)splits * 64 >= ctx) ? 1 : 0;
-  aa.prefetch = (aa.small && d->step_counter != nullptr) ? 1 : 0;
-  if (splits > 1) attn_carve_scratch(base + ar.attn, B, splits, &aa);
-  QUIC_CUDA(launch_attn(aa, B, st, true));
-  return QUIC_OK;
+  return launch_attention(aa, d, ctx, st, fuse);
 }
 
 LmHeadArgs lm_head_args(const quic_model_t* m, const quic_decode_t* d, const Arena& ar);
@@ -570,7 +521,7 @@ int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_
     a.n_ssq = l == 0 ? 1 : kRowsSsq;
     rows_next(&a, &L.o);  // a launch brings the next linear's weights into L2
     if ((rc = rows_qkv(h, a, st)) != QUIC_OK) return rc;
-    if ((rc = enqueue_attention(d, ar, splits, ctx, qbuf, a.kcache, a.vcache, attn_out, st)) != QUIC_OK) return rc;
+    if ((rc = enqueue_attention(d, ctx, qbuf, a.kcache, a.vcache, attn_out, st)) != QUIC_OK) return rc;
     a.w = L.o;
     a.y = h;
     a.ssq_out = ssq_mid;
@@ -646,7 +597,7 @@ int enqueue_step_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t
     QUIC_CUDA(launch_qkv_f16(L.qkv, (const half*)L.ln1, (const half*)m->embed, xa, xa, rs, m->eps, l == 0, m->vocab,
                              (const half*)m->rope_cos, (const half*)m->rope_sin, m->max_pos, qbuf, kc, vc, d->s_max,
                              d->n_slots, st, !(chain_head && l == 0)));
-    int rc = enqueue_attention(d, ar, splits, ctx, qbuf, kc, vc, attn_out, st);
+    int rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st);
     if (rc != QUIC_OK) return rc;
     QUIC_CUDA(launch_residual_f16(L.o, attn_out, xa, xb, B, st));
     QUIC_CUDA(launch_gateup_f16(L.gate_up, (const half*)L.ln2, xb, act, B, m->eps, st));
@@ -685,13 +636,13 @@ int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cuda
     half* vc = kc + kv_plane;
     int rc = gemm_f16_tc(xn, (const half*)L.qkv.w16, (const half*)L.qkv.bias, qkv, B, kQkvN, kHidden, ws, st, true);
     if (rc != QUIC_OK) return rc;
-    if (attention_streams(B, ctx)) {  // the attention CTAs rotate and append themselves
+    if (attention_form(B, ctx) == kAttnStream) {  // the attention CTAs rotate and append themselves
       QkvFinish fin = {nullptr, 0, nullptr, qkv, (const half*)m->rope_cos, (const half*)m->rope_sin, m->max_pos};
-      rc = enqueue_attention(d, ar, splits, ctx, qbuf, kc, vc, attn_out, st, &fin);
+      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st, &fin);
     } else {
       QUIC_CUDA(launch_qkv_post(qkv, d->rows, d->pos, (const half*)m->rope_cos, (const half*)m->rope_sin, m->max_pos,
                                 qbuf, kc, vc, d->s_max, d->n_slots, B, st));
-      rc = enqueue_attention(d, ar, splits, ctx, qbuf, kc, vc, attn_out, st);
+      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st);
     }
     if (rc != QUIC_OK) return rc;
     rc = gemm_f16_tc(attn_out, (const half*)L.o.w16, nullptr, qkv, B, kHidden, kHidden, ws, st, true);
@@ -734,23 +685,11 @@ extern "C" void quic_set_mma_chain_min_batch(int32_t batch) {
 extern "C" int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx) {
   if (batch < 1) batch = 1;
   if (ctx < 1) ctx = 1;
-  // Throughput regime (tensor-core step): 4-warp CTAs that cover 128 tokens per pass; one
-  // pass per CTA while that still leaves at most two waves of four CTAs per SM.
-  if (batch >= g_tensor_min_batch) {
-    if (ctx <= 2048) return (ctx + 63) / 64;  // single-warp CTAs, every cache tile in flight at once
-    const int by_len = (ctx + 127) / 128;
-    int s = 1184 / (batch * kKvHeads);
-    if (s > by_len) s = by_len;
-    if (s > 64) s = 64;
-    return s < 1 ? 1 : s;
-  }
-  // Up to 2048 tokens at small batch: one warp per 64 tokens, merged by the o_proj kernel.
-  const int small = (ctx + 63) / 64;
-  if (small <= kWarpMaxSplits) return small;
-  // Longer: 4-warp CTAs of the throughput kernel over 128 tokens and more each, and no more
-  // splits than the o_proj kernel merges itself.
-  const int by_len = (ctx + 127) / 128;
-  return by_len < kMaxConsumerSplitsTotal ? by_len : kMaxConsumerSplitsTotal;
+  // (no step's attention merges splits in global memory any more; the number only sizes the scratch, and callers pass it on)
+  if (ctx <= 2048) return (ctx + 63) / 64;
+  const int by_len = (ctx + 127) / 128, most = batch >= g_tensor_min_batch ? 1184 / (batch * kKvHeads) : 64;
+  const int s = by_len < most ? by_len : most;
+  return s < 1 ? 1 : s > 64 ? 64 : s;
 }
 
 extern "C" int64_t quic_decode_scratch_bytes(int32_t batch, int32_t vocab, int32_t attn_splits) {
@@ -767,14 +706,14 @@ extern "C" int32_t quic_decode_launch_count(const quic_model_t* m, const quic_de
     if (d && d->batch > kF16ChainMaxRows) {
       int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
       if (ctx > d->s_max) ctx = d->s_max;
-      return (attention_streams(d->batch, ctx) ? 8 : 9) * m->n_layers + 3;
+      return (attention_form(d->batch, ctx) == kAttnStream ? 8 : 9) * m->n_layers + 3;
     }
     return 5 * m->n_layers + 1;
   }
   if (d && d->batch >= g_tensor_min_batch) {
     int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
     if (ctx > d->s_max) ctx = d->s_max;
-    return (attention_streams(d->batch, ctx) ? 7 : 8) * m->n_layers + 3;  // the streamed attention finishes the QKV linear
+    return (attention_form(d->batch, ctx) == kAttnStream ? 7 : 8) * m->n_layers + 3;  // the streamed attention finishes the QKV linear
   }
   if (d && d->batch >= g_mma_chain_min_batch) return 5 * m->n_layers + ((d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab)) ? 2 : 1);
   return 5 * m->n_layers + 1;

@@ -69,3 +69,28 @@ def test_queries_at_an_odd_address_are_refused_where_they_are_read_in_pairs(rows
     k = torch.zeros(rows, KV, tokens, HD, device="cuda").half()
     with pytest.raises(RuntimeError, match="aligned"):
         kernels.flash_attn_decode().forward(buf[1:1 + rows * HEADS * HD].view(rows, HEADS, 1, HD), k, k)
+
+
+@pytest.mark.parametrize("rows,longest", [(1, 4200), (2, 4161), (3, 4500), (9, 4097), (16, 3300), (17, 4200), (20, 3500), (21, 1990), (40, 2100)])
+def test_decode_steps_over_long_rows_match_a_prefill_of_the_same_tokens(tiny_model, rows, longest):
+    """The streaming attention inside a decode step (rows beyond 4096 tokens, more CTAs of 512 tokens than SMs, 21 rows and
+    more from three ranges on): what the step appends in the second layer went through its attention.  A prefill of
+    prompt + token leaves the same there, up to the roundings to fp16 (34 of 2^-11 / sqrt(3), see test_rows_chain_gpu.py)."""
+    from quic_cu_b200 import model as qmodel
+
+    _, _, state, config = tiny_model
+    state = {k: v * 0.25 if k.endswith("weight_scale") else v for k, v in state.items()}
+    net = qmodel.from_state_dict(state, config)
+    gen = torch.Generator().manual_seed(rows)
+    lens = torch.randint(1, longest, (rows,), generator=gen).tolist()
+    lens[0] = longest
+    prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
+    slots = torch.randperm(rows, generator=gen).tolist()
+    cache, other = (net.new_cache(n_slots=rows, s_max=4608) for _ in range(2))
+    first, _ = net.prefill(cache, slots, prompts)
+    net.decode(cache, slots, 1)
+    net.prefill(other, slots, [torch.cat([p, first[i:i + 1].cpu()]) for i, p in enumerate(prompts)])
+    for i, (slot, n) in enumerate(zip(slots, lens)):
+        got, want = cache.kv[1, :, slot, :, n].float(), other.kv[1, :, slot, :, n].float()
+        worst = ((got - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)).max().item()
+        assert worst < 2 * (34 / 3) ** 0.5 * 2 ** -11, (i, n, worst)
