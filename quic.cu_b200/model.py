@@ -166,18 +166,23 @@ def _persist_pays(dense: bool, batch: int, ctx: int) -> bool:
     persistent / chain).  One packed row: up to 512 tokens the chain's attention is one CTA without a
     merge and ahead, 329 / 325 at 16 tokens, 332 / 323 at 230, 340 / 339 at 440, 350 / 333 at 500 (behind
     at 48 only, 325 / 328); from there to 768, one split of the persistent kernel, 345 / 353 at 520, 354 / 354 at 600,
-    349 / 359 at 680, 360 / 358 at 745; beyond, 412 / 350 at 900.  Two rows: 352 / 430 at 16 tokens,
-    373 / 462 at 512, 455 / 465 at 2100, 538 / 689 at 7000.  3..16 rows: 402 / 570 (3 x 300), 498 / 618
-    (4 x 1000), 445 / 667 (8 x 1000), 473 / 685 (16 x 16), 500 / 704 (16 x 300), 660 / 784 (16 x 2000), equal at
-    3000-4000 tokens.  fp16 weights: 347 / 473 at one row of 16 tokens, 348 / 494 at 512, 420 / 497 at 2100,
-    416 / 899 at eight rows.
+    349 / 359 at 680, 360 / 358 at 745; beyond, 412 / 350 at 900.  Two rows: 352 / 430 at 16 tokens, 453 / 471 at 2100,
+    503 / 461 at 3900, beyond 4096 (where the chain's attention reads its cache by TMA) 502 / 521 at 5000, 542 / 564 at
+    7900.  3..16 rows: 508 / 600 (3 x 2500), 573 / 584 (3 x 3900), 584 / 613 (5 x 2500), 626 / 607 (5 x 3500),
+    646 / 641 (8 x 2500), 730 / 754 (12 x 2500), 764 / 778 (16 x 2500).  fp16 weights: 347 / 473 at one row of 16 tokens,
+    452 / 592 at 4500; 559 / 738 at two of 7900; 580 / 623 (3 x 3900), 639 / 626 (5 x 3900), 533 / 623 (8 x 1500),
+    632 / 625 (8 x 2500), 589 / 630 (16 x 1000), 646 / 641 (16 x 1500), 952 / 831 (16 x 3900).
 
     A burst holds every SM, so a prefill beside it (Engine with ``overlap_prefill``) runs before or after it;
     the queue is still served sooner than with the chain (ms, persistent / chain, both with overlap:
     2 slots 499 / 555, 8 slots 368 / 469, 8 slots with prompts of 400..2000 tokens 474 / 480, 16 slots 273 / 364)."""
     if batch == 1:
-        return ctx <= 4096 if dense else 512 < ctx <= 768
-    return ctx <= (8192 if batch == 2 else 4096 if dense else 2048)
+        return ctx <= 8192 if dense else 512 < ctx <= 768
+    if batch == 2:
+        return ctx <= 8192 and (dense or not 2560 < ctx <= 4096)
+    if dense:
+        return ctx <= 4096 and batch * ctx <= 18000
+    return ctx <= (3584 if batch == 3 else 2560)
 
 
 _serials = itertools.count()
