@@ -666,7 +666,7 @@ int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cuda
 struct Graph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  bool tensor_kernels = false;  // the step holds tcgen05 kernels, whose bounded waits report through error words
+  bool tensor_kernels = false;  // the step holds kernels whose bounded waits report through error words
 };
 
 }  // namespace
@@ -755,9 +755,12 @@ extern "C" int quic_decode_graph_create(const quic_model_t* m, const quic_decode
     return rc;
   }
   const bool dense = m->layers[0].qkv.w16 != nullptr;
-  g->tensor_kernels = dense ? d->batch > kF16ChainMaxRows
-                            : (d->batch >= g_tensor_min_batch ||
-                               (d->batch >= g_mma_chain_min_batch && d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab)));
+  int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
+  if (ctx > d->s_max) ctx = d->s_max;
+  g->tensor_kernels = attention_form(d->batch, ctx) != kAttnCta ||
+                      (dense ? d->batch > kF16ChainMaxRows
+                             : (d->batch >= g_tensor_min_batch ||
+                                (d->batch >= g_mma_chain_min_batch && d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab))));
   *graph_out = g;
   return QUIC_OK;
 }
@@ -783,8 +786,8 @@ extern "C" int quic_graph_run_host(void* graph, void* stream, const int32_t* hos
   QUIC_CUDA(cudaGraphLaunch(g->exec, st));
   if (n_out > 0)
     QUIC_CUDA(cudaMemcpyAsync(host_out, dev_out, sizeof(int32_t) * n_out, cudaMemcpyDeviceToHost, st));
-  // the error words of the tensor-core kernels ride along with the tokens (the GEMV and mma.sync
-  // chains hold no kernel that waits on a barrier: nothing to ask for)
+  // the error words of the kernels that wait on barriers ride along with the tokens (the GEMV and mma.sync
+  // chains hold none up to 4096 tokens: nothing to ask for)
   if (g->tensor_kernels) {
     const int rc = tc_status_poll_async(st);
     if (rc != QUIC_OK) return rc;
