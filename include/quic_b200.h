@@ -377,9 +377,11 @@ typedef struct {
 int64_t quic_prefill_scratch_bytes(int32_t rows, int32_t n_seq, int32_t vocab);
 int quic_prefill(const quic_model_t *m, const quic_prefill_t *p, void *stream);
 
-/* Which of the three forms of the decode step a batch takes.  Batches of at
- * least quic_set_tensor_min_batch rows (default 16, range 2..17) run every
- * linear on the tcgen05 GEMM and the tensor lm_head; below that, batches of at
+/* Which form of the decode step a batch takes.  Batches of at least
+ * quic_set_tensor_min_batch rows (default 16, range 2..17) run every linear on
+ * tcgen05 and the tensor lm_head: up to 128 rows five launches a layer with the
+ * norms, RoPE, residuals and SwiGLU inside them, beyond that a GEMM a linear.
+ * Below that, batches of at
  * least quic_set_mma_chain_min_batch rows (default 3, range 2..17) run the
  * five-kernel layer chain with the rows on the M side of mma.sync, whose cost
  * hardly grows with the row count; smaller batches (one row, and two by
@@ -388,7 +390,7 @@ int quic_prefill(const quic_model_t *m, const quic_prefill_t *p, void *stream);
  * (Marlin picks its tile shapes per call, kernels/cuda/marlin.cu:3795-3805). */
 void quic_set_tensor_min_batch(int32_t batch);
 void quic_set_mma_chain_min_batch(int32_t batch);
-/* Attention split count the decode step uses for `batch` rows whose contexts are
+/* Split count that sizes the decode step's scratch for `batch` rows whose contexts are
  * at most `ctx` tokens (pass the result as attn_splits and to the scratch size). */
 int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx);
 int64_t quic_decode_scratch_bytes(int32_t batch, int32_t vocab, int32_t attn_splits);

@@ -62,8 +62,8 @@ PrefillArena carve_prefill(int rows, int n_seq, int vocab) {
   off += align256((int64_t)rows * kInter * 2);
   a.xlast = off;
   off += align256((int64_t)n_seq * kHidden * 2);
-  a.ssq = off;  // sums of squares of the residual stream's rows, twice (rows chain)
-  off += align256((int64_t)2 * rows * kRowsSsq * 4);
+  a.ssq = a.qkv;  // sums of squares of the residual stream's rows, twice: on the rows chain, which leaves no qkv there
+  static_assert(2 * kRowsSsq * 4 <= kQkvN * 2, "the sums fit in the place of the qkv rows");
   a.ws = off;
   off += align256(linear_ws(rows));
   a.w16 = off;  // fp16 copies of one layer's packed weights
