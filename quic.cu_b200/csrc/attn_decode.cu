@@ -5,17 +5,17 @@
 // (kernels/cuda/flash_attn_decode.cu:12,104).  Same mathematics — fp32 online
 // softmax over the tokens [start_b, end_b) of each row, rows without tokens
 // give zeros (:118-121) — with three kernels for three regimes:
-//   * attn_decode_warp_kernel (latency: the decode chain up to 2048 tokens, small problems):
+//   * attn_decode_warp_kernel (latency: small problems):
 //     ONE WARP per 64 tokens of a (row, kv head), both products on mma.sync.m16n8k16, no
-//     shared memory; inside the chain its cache tile is requested before the dependency wait;
+//     shared memory;
 //   * attn_decode_mma_kernel (throughput): 4 or 8 warps per CTA walking 32-token tiles with an
 //     online softmax, the same mma.sync fragment mappings (attn_warp.cuh), warps merged
 //     through shared memory;
 //   * attn_decode_kernel (scalar, kept for small stand-alone problems): one token per lane
 //     for q.k, all 7 query heads of the group at once.
-// Splits go through global fp32 partials; they are merged by the consumer (the o_proj kernel
-// of the small-batch chain) or by the CTA that arrives last at a per-(row, kv head) counter,
-// which re-arms the counter, so no second kernel and no spin-wait is needed.
+// Splits go through global fp32 partials; they are merged by the CTA that arrives last at a
+// per-(row, kv head) counter, which re-arms the counter, so no second kernel and no spin-wait
+// is needed.
 #include "decode_kernels.cuh"
 #include "attn_warp.cuh"
 
@@ -304,55 +304,28 @@ __global__ void __launch_bounds__(kWarps * 32) attn_decode_kernel(const AttnArgs
 
 
 // ---------------------------------------------------------------------------
-// Latency variant for short contexts at small batch (one decode step of a few
-// rows): ONE WARP owns 64 tokens of one (row, kv head); the arithmetic is in
+// Latency variant for short contexts at small batch: ONE WARP owns 64 tokens of one (row, kv head); the arithmetic is in
 // attn_warp.cuh.
-//
-// Inside the decode chain (a.prefetch) the cache tile is requested BEFORE the
-// dependency wait, so it is in registers when the query arrives.  That is sound
-// for every row except the one the preceding qkv kernel appends in this very
-// step, which the lanes that hold it fetch again after the wait.  Rows appended
-// by earlier steps are complete as soon as the step counter (advanced by the
-// last CTA of the lm_head kernel) shows the current step; the counter is read
-// with acquire semantics before the tile is requested and again after the wait,
-// and if the two differ the whole tile is fetched again.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(32) attn_decode_warp_kernel(const AttnArgs a) {
   __shared__ int last_flag;
   const int lane = threadIdx.x;
   const int g = lane >> 2, c = lane & 3;  // fragment row (head) and column pair
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
-  int slot = b;
-  if (a.pos != nullptr) slot = a.rows[b];  // the row -> slot map is not written inside the chain
-  const half* kbase = a.k + (size_t)slot * a.stride_b + (size_t)kvh * a.stride_h;
-  const half* vbase = a.v + (size_t)slot * a.stride_b + (size_t)kvh * a.stride_h;
+  const half* kbase = a.k + (size_t)b * a.stride_b + (size_t)kvh * a.stride_h;
+  const half* vbase = a.v + (size_t)b * a.stride_b + (size_t)kvh * a.stride_h;
   const int last_tok = a.s_cap - 1;
   const int t0 = split * kWarpChunk;
   pdl_trigger_early();
-
-  WarpTile tile;
-  int epoch0 = 0;
-  const bool prefetch = a.prefetch != 0 && a.epoch != nullptr;
-  if (prefetch) {
-    epoch0 = ld_acquire_s32(a.epoch);
-    warp_tile_request(tile, kbase, vbase, t0, last_tok, g, c);
-  }
   pdl_wait();
 
+  WarpTile tile;
   int t_begin = 0, t_end = a.s_cap;
-  int fresh = -1;  // row appended by the preceding kernel of the chain
-  bool refetch = !prefetch;
-  if (a.pos != nullptr) {
-    t_end = __ldcg(a.pos + slot) + 1;
-    fresh = t_end - 1;
-    if (prefetch) refetch = __ldcg(a.epoch) != epoch0;
-  } else {
-    if (a.start != nullptr) t_begin = a.start[b];
-    if (a.end != nullptr) t_end = a.end[b];
-  }
+  if (a.start != nullptr) t_begin = a.start[b];
+  if (a.end != nullptr) t_end = a.end[b];
   uint32_t qa0[4], qa2[4];
   warp_q_fragments(qa0, qa2, a.q + ((size_t)b * kHeads + kvh * kGroupHeads) * kHeadDim, g, c);
-  warp_tile_refetch(tile, kbase, vbase, t0, last_tok, g, c, refetch, fresh);
+  warp_tile_request(tile, kbase, vbase, t0, last_tok, g, c);
   if (t_end > a.s_cap) t_end = a.s_cap;
   if (t_begin < 0) t_begin = 0;
   const int c_begin = max(t_begin, t0);

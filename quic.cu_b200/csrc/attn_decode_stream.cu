@@ -22,7 +22,7 @@
 // kernel appends is never requested early.
 //
 // With `fin.part` (or `fin.qkv`, a finished fp16 output) set the CTA first finishes the fused QKV linear for its row and KV head, which a
-// separate kernel (qkv_post_kernel) would otherwise do between the GEMM and the attention: the
+// separate kernel would otherwise do between the GEMM and the attention: the
 // compute warps sum the split-K partial sums of their seven q heads, their k head and their v head,
 // add the bias with the GEMM epilogue's roundings, rotate q and k (rope.forward of the reference,
 // kernels/cuda/rope.cu), keep q in shared memory for the fragments, append k and v to the cache for

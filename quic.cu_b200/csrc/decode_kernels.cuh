@@ -220,14 +220,8 @@ cudaError_t launch_embed_ssq(const half* embed, const int32_t* slots, const int3
 cudaError_t launch_embed_rows(const half* embed, const int32_t* rows, const int32_t* tok, int vocab, half* x,
                               int batch, cudaStream_t st, bool pdl);
 // Fused consumers of split-K partial sums [splits][batch][N] (fp32).
-cudaError_t launch_qkv_post_part(const float* part, int splits, const half* bias, const int32_t* rows,
-                                 const int32_t* pos, const half* cos_t, const half* sin_t, int max_pos, half* qbuf,
-                                 half* kcache, half* vcache, int s_max, int n_slots, int batch, cudaStream_t st);
 cudaError_t launch_rmsnorm_part(const float* part, int splits, const half* residual, const half* w, float eps,
                                 half* y, half* sum_out, int rows, cudaStream_t st);
-cudaError_t launch_qkv_post(const half* qkv, const int32_t* rows, const int32_t* pos, const half* cos_t,
-                            const half* sin_t, int max_pos, half* qbuf, half* kcache, half* vcache, int s_max,
-                            int n_slots, int batch, cudaStream_t st);
 cudaError_t launch_swiglu_fused(const half* gu, half* act, int batch, cudaStream_t st);
 // prefill pieces, chainable with programmatic dependent launch
 cudaError_t launch_qkv_rope_append(const half* qkv, const int32_t* slots, const int32_t* positions, const half* cos_t,

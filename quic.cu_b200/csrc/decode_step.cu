@@ -377,7 +377,7 @@ int enqueue_step_rows16(const quic_model_t* m, const quic_decode_t* d, cudaStrea
   return QUIC_OK;
 }
 
-// Batch > 16: every linear is the tcgen05 GEMM; norms, RoPE/KV append and SwiGLU are
+// More than kRowsChainMaxRows rows: every linear is the tcgen05 GEMM, norms are
 // separate small kernels (at these sizes each kernel does microseconds of real work, so
 // the launch chain is no longer what bounds the step).
 // `fuse`: the attention kernel finishes the QKV linear itself (only where attention_streams()).
@@ -413,17 +413,11 @@ int enqueue_step_batched(const quic_model_t* m, const quic_decode_t* d, cudaStre
     const float* part = ws + 4096;
     int rc = w4a16_gemm_tc(xn, L.qkv, nullptr, B, ws, st, &sp);
     if (rc != QUIC_OK) return rc;
-    if (attention_form(B, ctx) == kAttnStream) {
-      // the attention CTAs sum the partial sums, rotate and append themselves: one launch less
-      // (64 rows of 512 tokens: 934 -> 883 us per step, same bits)
-      QkvFinish fin = {part, sp, (const half*)L.qkv.bias, nullptr, (const half*)m->rope_cos, (const half*)m->rope_sin,
-                       m->max_pos};
-      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st, &fin);
-    } else {
-      QUIC_CUDA(launch_qkv_post_part(part, sp, (const half*)L.qkv.bias, d->rows, d->pos, (const half*)m->rope_cos,
-                                     (const half*)m->rope_sin, m->max_pos, qbuf, kc, vc, d->s_max, d->n_slots, B, st));
-      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st);
-    }
+    // the attention CTAs sum the partial sums, rotate and append themselves: one launch less
+    // (64 rows of 512 tokens: 934 -> 883 us per step, same bits)
+    QkvFinish fin = {part, sp, (const half*)L.qkv.bias, nullptr, (const half*)m->rope_cos, (const half*)m->rope_sin,
+                     m->max_pos};
+    rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st, &fin);
     if (rc != QUIC_OK) return rc;
     rc = w4a16_gemm_tc(attn_out, L.o, nullptr, B, ws, st, &sp);
     if (rc != QUIC_OK) return rc;
@@ -636,14 +630,9 @@ int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cuda
     half* vc = kc + kv_plane;
     int rc = gemm_f16_tc(xn, (const half*)L.qkv.w16, (const half*)L.qkv.bias, qkv, B, kQkvN, kHidden, ws, st, true);
     if (rc != QUIC_OK) return rc;
-    if (attention_form(B, ctx) == kAttnStream) {  // the attention CTAs rotate and append themselves
-      QkvFinish fin = {nullptr, 0, nullptr, qkv, (const half*)m->rope_cos, (const half*)m->rope_sin, m->max_pos};
-      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st, &fin);
-    } else {
-      QUIC_CUDA(launch_qkv_post(qkv, d->rows, d->pos, (const half*)m->rope_cos, (const half*)m->rope_sin, m->max_pos,
-                                qbuf, kc, vc, d->s_max, d->n_slots, B, st));
-      rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st);
-    }
+    // the attention CTAs rotate and append themselves
+    QkvFinish fin = {nullptr, 0, nullptr, qkv, (const half*)m->rope_cos, (const half*)m->rope_sin, m->max_pos};
+    rc = enqueue_attention(d, ctx, qbuf, kc, vc, attn_out, st, &fin);
     if (rc != QUIC_OK) return rc;
     rc = gemm_f16_tc(attn_out, (const half*)L.o.w16, nullptr, qkv, B, kHidden, kHidden, ws, st, true);
     if (rc != QUIC_OK) return rc;
@@ -703,18 +692,10 @@ extern "C" int32_t quic_decode_launch_count(const quic_model_t* m, const quic_de
       d->batch > (m->layers[0].qkv.w16 != nullptr ? kF16ChainMaxRows : g_tensor_min_batch - 1))
     return 5 * m->n_layers + 3;
   if (m->layers && m->layers[0].qkv.w16 != nullptr) {
-    if (d && d->batch > kF16ChainMaxRows) {
-      int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
-      if (ctx > d->s_max) ctx = d->s_max;
-      return (attention_form(d->batch, ctx) == kAttnStream ? 8 : 9) * m->n_layers + 3;
-    }
+    if (d && d->batch > kF16ChainMaxRows) return 8 * m->n_layers + 3;
     return 5 * m->n_layers + 1;
   }
-  if (d && d->batch >= g_tensor_min_batch) {
-    int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
-    if (ctx > d->s_max) ctx = d->s_max;
-    return (attention_form(d->batch, ctx) == kAttnStream ? 7 : 8) * m->n_layers + 3;  // the streamed attention finishes the QKV linear
-  }
+  if (d && d->batch >= g_tensor_min_batch) return 7 * m->n_layers + 3;  // the streamed attention finishes the QKV linear
   if (d && d->batch >= g_mma_chain_min_batch) return 5 * m->n_layers + ((d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab)) ? 2 : 1);
   return 5 * m->n_layers + 1;
 }

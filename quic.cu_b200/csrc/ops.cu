@@ -239,65 +239,9 @@ __global__ void embed_rows_kernel(const half* __restrict__ embed, const int32_t*
   for (int i = threadIdx.x; i < kHidden / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// RoPE + q buffer + KV append from the fused QKV output (columns in rope-pair order,
-// bias already added).  One thread per (row, column pair).
-__global__ void qkv_post_kernel(const half* __restrict__ qkv, const float* __restrict__ part, int splits,
-                                const half* __restrict__ bias, const int32_t* __restrict__ rows,
-                                const int32_t* __restrict__ pos, const half* __restrict__ cos_t,
-                                const half* __restrict__ sin_t, int max_pos, half* __restrict__ qbuf,
-                                half* __restrict__ kcache, half* __restrict__ vcache, int s_max, int batch,
-                                const int32_t* __restrict__ row_pos, int q_head_major, int n_slots) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait();
-  if (idx >= batch * (kQkvN / 2)) return;
-  const int b = idx / (kQkvN / 2), c2 = idx % (kQkvN / 2);
-  const int head = c2 >> 5, pair = c2 & 31;  // stored columns (2*pair, 2*pair+1) = dims (pair, pair+32)
-  const int slot = rows[b];
-  const bool slot_ok = slot >= 0 && slot < n_slots;  // a row with a slot outside the cache appends nothing
-  // decode: the row's position is its slot's; prefill: every row (token) brings its own
-  const int p = row_pos != nullptr ? row_pos[b] : (slot_ok ? pos[slot] : 0);
-  float2 v;
-  if (part != nullptr) {  // fp16(sum of the split-K partials) + bias, as the GEMM epilogue would do
-    float2 p[16];
-#pragma unroll
-    for (int s = 0; s < 16; ++s)
-      p[s] = s < splits ? __ldcg(reinterpret_cast<const float2*>(part + ((size_t)s * batch + b) * kQkvN + 2 * c2))
-                        : make_float2(0.f, 0.f);
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int s = 0; s < 16; ++s) {
-      acc.x += p[s].x;
-      acc.y += p[s].y;
-    }
-    const float2 bb = __half22float2(*reinterpret_cast<const half2*>(bias + 2 * c2));
-    v.x = __half2float(__float2half_rn(__half2float(__float2half_rn(acc.x)) + bb.x));
-    v.y = __half2float(__float2half_rn(__half2float(__float2half_rn(acc.y)) + bb.y));
-  } else {
-    v = __half22float2(*reinterpret_cast<const half2*>(qkv + (size_t)b * kQkvN + 2 * c2));
-  }
-  float lo = v.x, hi = v.y;
-  if (head < kHeads + kKvHeads) {
-    const int pp = p < max_pos ? (p < 0 ? 0 : p) : max_pos - 1;
-    const float c = __half2float(cos_t[(size_t)pp * 32 + pair]), s = __half2float(sin_t[(size_t)pp * 32 + pair]);
-    lo = v.x * c - v.y * s;
-    hi = v.x * s + v.y * c;
-  }
-  half* dst;
-  if (head < kHeads) {
-    dst = q_head_major ? qbuf + ((size_t)head * batch + b) * kHeadDim : qbuf + ((size_t)b * kHeads + head) * kHeadDim;
-  } else {
-    if (p >= s_max || p < 0 || !slot_ok) return;
-    const int kvh = (head - kHeads) & 1;
-    half* base = (head < kHeads + kKvHeads) ? kcache : vcache;
-    dst = base + (((size_t)slot * kKvHeads + kvh) * s_max + p) * kHeadDim;
-  }
-  dst[pair] = __float2half_rn(lo);
-  dst[pair + 32] = __float2half_rn(hi);
-}
-
-// The same for many rows (prefill: every row brings its own slot and position, q is written
-// head-major): one thread per (row, head, 8 of the 64 dims), which reads the 8 stored pairs
+// RoPE + q buffer + KV append from the fused QKV output (columns in rope-pair order, bias
+// already added) of a prefill: every row brings its own slot and position, q is written
+// head-major.  One thread per (row, head, 8 of the 64 dims), which reads the 8 stored pairs
 // its dims come from (32 bytes) with their cos / sin (16 bytes each) and writes 16 bytes.
 __global__ void __launch_bounds__(256) qkv_rope_rows_kernel(
     const half* __restrict__ qkv, const int32_t* __restrict__ slots, const int32_t* __restrict__ row_pos,
@@ -426,14 +370,6 @@ cudaError_t launch_embed_rows(const half* embed, const int32_t* rows, const int3
                               int batch, cudaStream_t st, bool pdl) {
   return launch(embed_rows_kernel, dim3(batch), dim3(224), 0, st, pdl, embed, rows, tok, vocab, x, batch);
 }
-cudaError_t launch_qkv_post(const half* qkv, const int32_t* rows, const int32_t* pos, const half* cos_t,
-                            const half* sin_t, int max_pos, half* qbuf, half* kcache, half* vcache, int s_max,
-                            int n_slots, int batch, cudaStream_t st) {
-  const int total = batch * (kQkvN / 2);
-  return launch(qkv_post_kernel, dim3((total + 255) / 256), dim3(256), 0, st, true, qkv, (const float*)nullptr, 0,
-                (const half*)nullptr, rows, pos, cos_t, sin_t, max_pos, qbuf, kcache, vcache, s_max, batch,
-                (const int32_t*)nullptr, 0, n_slots);
-}
 cudaError_t launch_qkv_rope_append(const half* qkv, const int32_t* slots, const int32_t* positions, const half* cos_t,
                                    const half* sin_t, int max_pos, half* q_out, half* kcache, half* vcache, int s_max,
                                    int n_slots, int rows, cudaStream_t st, bool pdl, const float* part, int splits,
@@ -441,14 +377,6 @@ cudaError_t launch_qkv_rope_append(const half* qkv, const int32_t* slots, const 
   const size_t total = (size_t)rows * (kHeads + 2 * kKvHeads) * 8;
   return launch(qkv_rope_rows_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, pdl, qkv, slots, positions,
                 cos_t, sin_t, max_pos, q_out, kcache, vcache, s_max, rows, n_slots, part, splits, bias);
-}
-cudaError_t launch_qkv_post_part(const float* part, int splits, const half* bias, const int32_t* rows,
-                                 const int32_t* pos, const half* cos_t, const half* sin_t, int max_pos, half* qbuf,
-                                 half* kcache, half* vcache, int s_max, int n_slots, int batch, cudaStream_t st) {
-  const int total = batch * (kQkvN / 2);
-  return launch(qkv_post_kernel, dim3((total + 255) / 256), dim3(256), 0, st, true, (const half*)nullptr, part,
-                splits, bias, rows, pos, cos_t, sin_t, max_pos, qbuf, kcache, vcache, s_max, batch,
-                (const int32_t*)nullptr, 0, n_slots);
 }
 cudaError_t launch_rmsnorm_part(const float* part, int splits, const half* residual, const half* w, float eps,
                                 half* y, half* sum_out, int rows, cudaStream_t st) {
