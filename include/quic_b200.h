@@ -120,18 +120,18 @@ int64_t quic_w4a16_workspace_bytes(int32_t m, int32_t n, int32_t k);
  * set.  No reference counterpart (Marlin's lock spins are unbounded,
  * kernels/cuda/marlin.cu:1467-1476). */
 int quic_w4a16_tensor_status(void);
-/* Test hook for those bounded waits: the GEMM launches that follow probe at
- * most `spin_limit` times per wait (0: the default, 1 << 22) and never request
+/* Test hook for those bounded waits: the GEMM launches that follow wait
+ * `wait_limit_us` microseconds at most (0: the default, two seconds) and never request
  * the packed weight tile of k block `skip_kblock` (128 k each; -1: none), so
  * the waits for it run out, every role of the CTA leaves its loop, the status
  * word is set and the kernel returns with its tensor memory released.  Call
  * with (0, -1) to restore normal operation. */
-void quic_w4a16_tensor_test_hook(uint32_t spin_limit, int32_t skip_kblock);
+void quic_w4a16_tensor_test_hook(uint32_t wait_limit_us, int32_t skip_kblock);
 
 /* Test hook for the streamed decode attention (more than 20 rows), for the launches and graph
  * captures that follow.  1: repeat the tile requests made before the dependency wait, as the
  * kernel does when the step counter moved between request and wait.  2: never request the
- * first tile of a row and probe 20000 times at most, so that the bounded waits run out, the
+ * first tile of a row and wait 20 ms at most, so that the bounded waits run out, the
  * kernel sets the error word read by quic_w4a16_tensor_status (code 5 or 6 in bits 16..,
  * bit 14 set) and returns.  0 restores the normal behaviour.  No reference counterpart. */
 void quic_attn_stream_test_hook(int32_t mode);

@@ -57,7 +57,7 @@ __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
 __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     attn_decode_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                               const AttnArgs a, const QkvFinish fin, int n_slots, int s_max, int* status,
-                              int force_reload, int skip_tile0, uint32_t spin_limit) {
+                              int force_reload, int skip_tile0, uint32_t wait_limit_us) {
   extern __shared__ unsigned char smem_raw[];
   // A stage's two tiles landed: by the requests made before the dependency wait, by all others.  (One barrier for both
   // would not do where early requests are repeated: a wait for its second phase returns at once while the first runs, and
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
       if (stale) {       // wait for the early copies to land, then fetch the same tiles again
         for (int i = 0; i < pre; ++i) {
           const uint32_t full = smem_u32(&bar_full[i]), dst = base + i * kStageBytes;
-          if (!mbar_wait(smem_u32(&bar_early[i]), 0, spin_limit)) {
+          if (!mbar_wait(smem_u32(&bar_early[i]), 0, wait_limit_us)) {
             fail_s = 1;
             break;
           }
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
       }
       for (int i = pre; i < n_tiles && fail_s == 0; ++i, ++issued) {
         const int s = i % kStreamStages;
-        if (i >= kStreamStages && !mbar_wait(smem_u32(&bar_empty[s]), ((i / kStreamStages) - 1) & 1, spin_limit)) {
+        if (i >= kStreamStages && !mbar_wait(smem_u32(&bar_empty[s]), ((i / kStreamStages) - 1) & 1, wait_limit_us)) {
           fail_s = 1;
           break;
         }
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
       for (int i = issued > kStreamStages ? issued - kStreamStages : 0; i < issued; ++i) {
         const int s = i % kStreamStages;
         const bool early = i < pre && !stale;
-        if (!mbar_wait(smem_u32(early ? &bar_early[s] : &bar_full[s]), early ? 0 : full_phase(i, s) & 1, spin_limit)) fail_s = 1;
+        if (!mbar_wait(smem_u32(early ? &bar_early[s] : &bar_full[s]), early ? 0 : full_phase(i, s) & 1, wait_limit_us)) fail_s = 1;
       }
     }
   } else if (n_tiles > 0) {
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
     for (int i = warp; i < n_tiles; i += kStreamWarps) {
       const int s = i % kStreamStages;
       const bool early = i < pre && !stale;
-      bool ok = mbar_wait(smem_u32(early ? &bar_early[s] : &bar_full[s]), early ? 0 : full_phase(i, s) & 1, spin_limit);
+      bool ok = mbar_wait(smem_u32(early ? &bar_early[s] : &bar_full[s]), early ? 0 : full_phase(i, s) & 1, wait_limit_us);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) fail_s = 2;
@@ -324,7 +324,7 @@ int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int 
   QUIC_CUDA(allow_smem<attn_decode_stream_kernel>(kStreamSmem));
   QUIC_CUDA(launch(attn_decode_stream_kernel, dim3(kKvHeads, batch), dim3((kStreamWarps + 1) * 32), kStreamSmem, stream,
                    pdl, tm_k, tm_v, a, fin, n_slots, s_max, status, g_stream_hook == 1 ? 1 : 0, g_stream_hook == 2 ? 1 : 0,
-                   g_stream_hook == 2 ? 20000u : kSpinLimit));
+                   g_stream_hook == 2 ? 20000u : kWaitLimitUs));
   return QUIC_OK;
 }
 
@@ -333,6 +333,6 @@ int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int 
 // Test hook for the launches (and graph captures) that follow.  1: the kernel treats its early tile
 // requests as made too early and repeats them, as it does when the step counter moved between the
 // request and the dependency wait.  2: the first tile of every row is never requested and the
-// waits probe 20000 times at most, so the wait for that tile runs out, the other roles' waits
+// waits last 20 ms at most, so the wait for that tile runs out, the other roles' waits
 // follow, the CTA sets the error word (code 5 or 6, bit 14) and returns; nothing faults.  0: normal.
 extern "C" void quic_attn_stream_test_hook(int32_t mode) { quic::g_stream_hook = (mode == 1 || mode == 2) ? mode : 0; }

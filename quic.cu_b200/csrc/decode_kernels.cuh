@@ -205,7 +205,7 @@ struct RowsArgs {
   // filled in by the launcher
   const half* x;
   int32_t* status;
-  uint32_t spin_limit;
+  uint32_t wait_limit_us;
   int32_t skip_stage;
 };
 void rows_next(RowsArgs* a, const quic_w4_t* w);  // nullptr: none
@@ -271,7 +271,7 @@ int launch_lm_head_tc(const LmHeadArgs& a, cudaStream_t st);
 // an asynchronous copy to page-locked memory, and the value seen by that copy (taken, i.e.
 // exchanged with zero, when it is not 0).
 int* tc_status_words();
-void tc_test_hook(uint32_t* spin_limit, int32_t* skip_kblock);  // what quic_w4a16_tensor_test_hook last set
+void tc_test_hook(uint32_t* wait_limit_us, int32_t* skip_kblock);  // what quic_w4a16_tensor_test_hook last set
 int tc_status_poll_async(cudaStream_t st);
 int tc_status_polled(cudaStream_t st);
 

@@ -282,7 +282,7 @@ __device__ __forceinline__ u64 global_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) { return mbar_wait(bar, parity, 1u); }
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) { return mbar_try(bar, parity); }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       pdl_wait();
       int issued = 0;
       for (int s = 0, pass = 0; !C::norm && issued < n_st; ++issued) {
-        if (pass > 0 && !mbar_wait(smem_u32(&bar_empty[s]), (pass - 1) & 1, a.spin_limit)) {
+        if (pass > 0 && !mbar_wait(smem_u32(&bar_empty[s]), (pass - 1) & 1, a.wait_limit_us)) {
           fail_s = 2;
           break;
         }
@@ -242,8 +242,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       // no copy may be on its way into this CTA's shared memory when it ends, whatever became of the other roles
       for (int i = issued > kS ? issued - kS : 0; i < issued; ++i)
-        if (!mbar_wait(smem_u32(&bar_x[i % kS]), (i / kS) & 1, a.spin_limit)) fail_s = 2;
-      if (DENSE && !mbar_wait(smem_u32(&bar_w[0]), 0, a.spin_limit)) fail_s = 1;
+        if (!mbar_wait(smem_u32(&bar_x[i % kS]), (i / kS) & 1, a.wait_limit_us)) fail_s = 2;
+      if (DENSE && !mbar_wait(smem_u32(&bar_w[0]), 0, a.wait_limit_us)) fail_s = 1;
     }
   } else if (warp == kWarpsC + 1) {
     // ---------------- MMA issuer ----------------
@@ -253,8 +253,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool ok = true;
       for (int it = 0, s = 0, pass = 0, r = 0; it < n_st; ++it) {
         const int need = DENSE ? 1 : (2 * (it + 1) * ncols + kConsumers - 1) / kConsumers;  // rounds of weights up to this stage
-        for (; r < need && ok; ++r) ok = mbar_wait(smem_u32(&bar_w[r]), 0, a.spin_limit);
-        ok = ok && mbar_wait(smem_u32(C::norm ? &bar_ready[s] : &bar_x[s]), pass & 1, a.spin_limit);
+        for (; r < need && ok; ++r) ok = mbar_wait(smem_u32(&bar_w[r]), 0, a.wait_limit_us);
+        ok = ok && mbar_wait(smem_u32(C::norm ? &bar_ready[s] : &bar_x[s]), pass & 1, a.wait_limit_us);
         if (!ok) break;
         if (it == 0) tc_fence_after();
         const uint64_t x = x0 + (uint64_t)(s * (C::x_stage / 16)), w = w0 + (uint64_t)(it * (C::w_stage / 16));
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int it = 0; it < C::n_stages; ++it) {
         const int s = it % kS;
         const uint4 w = ln_s[k_stage(it) * 16 + piece];
-        if (it >= kS && !mbar_wait(smem_u32(&bar_empty[s]), (it / kS - 1) & 1, a.spin_limit)) {
+        if (it >= kS && !mbar_wait(smem_u32(&bar_empty[s]), (it / kS - 1) & 1, a.wait_limit_us)) {
           fail_s = 1;
           break;
         }
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   bool ok = true;
   if (warp < kWarpsC) {
-    ok = mbar_wait(smem_u32(&bar_done), 0, a.spin_limit);
+    ok = mbar_wait(smem_u32(&bar_done), 0, a.wait_limit_us);
     ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
     tc_fence_after();
     if (!ok) fail_s = 3;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       bulk_to_peer(peer_addr(base + C::off_red + rank * kPart, tid), base + C::off_ring + tid * kPart, kPart,
                    peer_addr(smem_u32(&bar_red), tid));
     if (warp < kWarpsC) {
-      if (!mbar_wait(smem_u32(&bar_red), 0, a.spin_limit)) {
+      if (!mbar_wait(smem_u32(&bar_red), 0, a.wait_limit_us)) {
         ok = false;
         fail_s = 4;
       }
@@ -652,7 +652,7 @@ int run_rows(const half* x, RowsArgs a, cudaStream_t st, bool pdl) {
   a.x = x;
   a.status = tc_status_words();
   QUIC_REQUIRE(a.status != nullptr, QUIC_E_CUDA, "rows_linear: no error word");
-  tc_test_hook(&a.spin_limit, &a.skip_stage);
+  tc_test_hook(&a.wait_limit_us, &a.skip_stage);
   const bool dense = a.w.w16 != nullptr;
   if (a.rows <= 64) return dense ? launch_rows<MODE, 64, true>(x, a, st, pdl) : launch_rows<MODE, 64, false>(x, a, st, pdl);
   return dense ? launch_rows<MODE, 128, true>(x, a, st, pdl) : launch_rows<MODE, 128, false>(x, a, st, pdl);

@@ -1,4 +1,4 @@
-// Shared pieces of the tcgen05 kernels: mbarrier waits with an iteration limit, UMMA
+// Shared pieces of the tcgen05 kernels: mbarrier waits with a time limit, UMMA
 // descriptors (K-major, 128-byte swizzle), TMA 2-D loads and tensor-map creation.
 #pragma once
 #include <cuda.h>
@@ -9,7 +9,7 @@ namespace quic {
 
 constexpr int kTileN = 128;   // rows of the weight-side tile (UMMA M)
 constexpr int kBlockK = 64;   // k per swizzle atom: 64 fp16 = one 128-byte swizzle row (a GEMM stage holds two)
-constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr uint32_t kWaitLimitUs = 2000000;  // a bounded wait gives up after two seconds
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -28,36 +28,37 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-// Bounded wait for the phase with the given parity; false on timeout (after `limit` probes).  The first probe stands
-// outside the loop: a phase that is complete already then costs ~100 clocks instead of ~200.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = kSpinLimit) {
+// Time in units of 1.024 us.
+__device__ __forceinline__ uint32_t clock_us() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return (uint32_t)(t >> 10);
+}
+// Bounded wait for the phase with the given parity; false after `limit_us`.  A probe sleeps until the phase is complete
+// or 4 us are over, so the clock is read only by a wait that is late already.  (A limit in probes, 2^22, was 16.6 s.)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit_us = kWaitLimitUs) {
   bool done = mbar_try(bar, parity);
-  if (!done)
-    for (uint32_t i = 1; i < limit; ++i)
-      if (mbar_try(bar, parity)) {
-        done = true;
-        break;
-      }
+  if (!done) {
+    const uint32_t t0 = clock_us();
+    do done = mbar_try(bar, parity);
+    while (!done && clock_us() - t0 < limit_us);
+  }
   return done;
 }
 // The same wait for roles that are many warps wide and not on the critical path of the MMA
 // issue: sleeps between probes so the probes do not crowd the issuing thread's instructions
 // out of the shared-memory pipeline.
 __device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, uint32_t sleep_ns,
-                                                  uint32_t limit = kSpinLimit) {
-  for (uint32_t i = 0; i < limit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    __nanosleep(sleep_ns);
+                                                  uint32_t limit_us = kWaitLimitUs) {
+  bool done = mbar_try(bar, parity);
+  if (!done) {
+    const uint32_t t0 = clock_us();
+    do {
+      __nanosleep(sleep_ns);
+      done = mbar_try(bar, parity);
+    } while (!done && clock_us() - t0 < limit_us);
   }
-  return false;
+  return done;
 }
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -32,9 +32,9 @@ constexpr int kHeadInts = 4096;  // reserved at the head of the split-K workspac
 // (code << 16) | block of the first bounded wait that gave up.
 __device__ int g_tc_status[2];
 
-// What a test may change for the launches that follow (quic_w4a16_tensor_test_hook): the probe
-// limit of the bounded waits and one k block whose packed weight tile the producer never requests.
-uint32_t g_spin_limit = kSpinLimit;
+// What a test may change for the launches that follow (quic_w4a16_tensor_test_hook): the limit
+// of the bounded waits and one k block whose packed weight tile the producer never requests.
+uint32_t g_wait_limit_us = kWaitLimitUs;
 int g_skip_kblock = -1;
 
 struct GemmArgs {
@@ -44,7 +44,7 @@ struct GemmArgs {
   int m_total;
   int kblocks_per_split;
   int mtl;     // batch-row tiles per CTA (2 from 129 rows up)
-  uint32_t spin_limit;  // probes of a bounded wait
+  uint32_t wait_limit_us;  // of a bounded wait
   int skip_kblock;      // test hook: the weight tile of this k block is never requested (-1: none)
   // SwiGLU fused into the epilogue of the gate|up linear: the CTA's 128 weight rows are 64
   // gate rows and the 64 up rows of the same columns (two 64-row TMA boxes per stage), and y
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
       }
       // (ring position and phase are carried along: the depth is a run-time value)
       for (int it = first, stage = 0, pass = 1; it < nkb; ++it) {
-        if (!mbar_wait(smem_u32(&bar_empty[stage]), (pass - 1) & 1, a.spin_limit)) {
+        if (!mbar_wait(smem_u32(&bar_empty[stage]), (pass - 1) & 1, a.wait_limit_us)) {
           fail_s = 2;
           break;
         }
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
       // of these costs the issuing thread a round trip, and at these sizes the loop is bound
       // by that, not by the tensor pipe.
       for (int it = 0, stage = 0, pass = 0; it < nkb; ++it) {
-        if (!mbar_wait(smem_u32(&bar_aready[stage]), pass & 1, a.spin_limit)) {
+        if (!mbar_wait(smem_u32(&bar_aready[stage]), pass & 1, a.wait_limit_us)) {
           fail_s = 3;
           break;
         }
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
     for (int it = 0, stage = 0, pass = 0; it < nkb; ++it) {
       // "full" of this phase also means the MMAs of the stage's previous use are complete
       // (the TMA warp refilled it only after "empty"), so the A tile may be overwritten.
-      if (!mbar_wait(smem_u32(&bar_full[stage]), pass & 1, a.spin_limit)) {
+      if (!mbar_wait(smem_u32(&bar_full[stage]), pass & 1, a.wait_limit_us)) {
         fail_s = 1;
         break;
       }
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
   if (warp < kConsumers / 32) {
     pdl_wait();  // the output / partial buffers may still be read by earlier kernels of the chain
     bool ok = !fail_s && nkb > 0;
-    if (ok) ok = mbar_wait_relaxed(smem_u32(&bar_done), 0, 64, a.spin_limit);
+    if (ok) ok = mbar_wait_relaxed(smem_u32(&bar_done), 0, 64, a.wait_limit_us);
     ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
     tc_fence_after();
     if (!ok && tid == 0 && nkb > 0) atomicCAS(&g_tc_status[0], 0, ((fail_s ? fail_s : 3) << 16) | (int)blockIdx.x);
@@ -456,7 +456,7 @@ int run_variant(const half* x, GemmArgs a, int splits, cudaStream_t st) {
 template <int MT>
 int run(const half* x, const GemmArgs& args, int splits, cudaStream_t st) {
   GemmArgs a = args;
-  a.spin_limit = g_spin_limit;
+  a.wait_limit_us = g_wait_limit_us;
   a.skip_kblock = g_skip_kblock;
   if (a.mtl == 2) {
     if constexpr (MT == 128) {
@@ -616,8 +616,8 @@ int* tc_status_words() {
   return g_status_host.words[dev];
 }
 
-void tc_test_hook(uint32_t* spin_limit, int32_t* skip_kblock) {
-  *spin_limit = g_spin_limit;
+void tc_test_hook(uint32_t* wait_limit_us, int32_t* skip_kblock) {
+  *wait_limit_us = g_wait_limit_us;
   *skip_kblock = g_skip_kblock;
 }
 
@@ -655,12 +655,12 @@ extern "C" int quic_w4a16_tensor_status(void) {
   return quic::tc_status_polled(nullptr);
 }
 
-// Test hook for the bounded waits of the tcgen05 GEMM: launches that follow probe at most
-// `spin_limit` times per wait (0 restores the default) and never request the packed weight
+// Test hook for the bounded waits of the tcgen05 GEMM: in launches that follow a wait gives up after
+// `wait_limit_us` microseconds (0 restores the default), and they never request the packed weight
 // tile of k block `skip_kblock` (128 k per block; -1: none), so the waits for it run out, the
 // CTA's roles leave their loops, the error word is set and the kernel returns with its tensor
 // memory released.  Nothing faults and nothing waits without a bound.
-extern "C" void quic_w4a16_tensor_test_hook(uint32_t spin_limit, int32_t skip_kblock) {
-  quic::g_spin_limit = spin_limit ? spin_limit : quic::kSpinLimit;
+extern "C" void quic_w4a16_tensor_test_hook(uint32_t wait_limit_us, int32_t skip_kblock) {
+  quic::g_wait_limit_us = wait_limit_us ? wait_limit_us : quic::kWaitLimitUs;
   quic::g_skip_kblock = skip_kblock;
 }

@@ -123,7 +123,7 @@ def test_batched_forward_logits_match_oracle(tiny_model, threshold):
 
 
 def test_a_gemm_wait_that_runs_out_is_reported_and_the_next_call_works(tiny_model):
-    """The bounded waits of the tcgen05 GEMM: with the probe limit lowered and one packed weight
+    """The bounded waits of the tcgen05 GEMM: with the limit lowered and one packed weight
     tile never requested (the library's test hook), the consumer warps' wait for that tile runs
     out, the MMA warp's and the epilogue's waits follow, every role leaves its loop, the CTA
     releases its tensor memory and returns; the status word names the wait.  Nothing faults.
@@ -171,9 +171,30 @@ def test_a_gemm_wait_that_runs_out_is_reported_and_the_next_call_works(tiny_mode
     assert lib.quic_w4a16_tensor_status() == 0
 
 
+def test_a_wait_that_runs_out_ends_after_its_limit(tiny_model):
+    """The limit is a time.  One launch with a weight tile that never comes: its roles' waits run out side by side, so the
+    kernel takes the limit of 20 ms and not three times that."""
+    from quic_cu_b200 import kernels as K
+
+    lib, weight = K.lib(), tiny_model[0].layers[0]["qkv"]
+    x = torch.randn(64, 896, device="cuda", dtype=torch.float16)
+    K.w4a16_linear(weight, x, use_tensor=1)
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    torch.cuda.synchronize()
+    lib.quic_w4a16_tensor_test_hook(20000, 0)
+    try:
+        start.record()
+        K.w4a16_linear(weight, x, use_tensor=1)
+        end.record()
+        assert lib.quic_w4a16_tensor_status() != 0
+        assert 20 <= start.elapsed_time(end) < 60
+    finally:
+        lib.quic_w4a16_tensor_test_hook(0, -1)
+
+
 def test_a_streamed_attention_wait_that_runs_out_is_reported_and_the_next_call_works(tiny_model):
     """The bounded waits of the streamed decode attention: under the library's test hook the first
-    tile of every row is never requested and the waits probe 20000 times at most; the consumer
+    tile of every row is never requested and the waits last 20 ms at most; the consumer
     warp's wait runs out, the producer's wait for that stage follows, the CTA reports and returns.
     decode() raises; with the hook cleared a fresh cache decodes what the oracle gives."""
     from quic_cu_b200 import kernels as K
