@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
       }
     }
   } else if (warp == 0 && elect_one()) {
+    pdl_wait();  // the activations cannot be here earlier, and a wait's limit is not for the kernel in front
     const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + L::kA);
     for (int it = 0; it < nkb; ++it) {
       const int stage = it % kDenseStages;

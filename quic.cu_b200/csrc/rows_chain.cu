@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int it = 0, s = 0, pass = 0, r = 0; it < n_st; ++it) {
         const int need = DENSE ? 1 : (2 * (it + 1) * ncols + kConsumers - 1) / kConsumers;  // rounds of weights up to this stage
         for (; r < need && ok; ++r) ok = mbar_wait(smem_u32(&bar_w[r]), 0, a.wait_limit_us);
+        if (it == 0) pdl_wait();  // the rows cannot be here earlier, and the limit is not for the kernel in front
         ok = ok && mbar_wait(smem_u32(C::norm ? &bar_ready[s] : &bar_x[s]), pass & 1, a.wait_limit_us);
         if (!ok) break;
         if (it == 0) tc_fence_after();

@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       const uint64_t b0 = umma_desc_sw128(base + kRawBytes), a0 = umma_desc_sw128(base + kRawBytes + L::kB);
+      pdl_wait();  // the rows cannot be here earlier, and a wait's limit is not for the kernel in front
       // One wait per k block (operand A written by the consumer warps and operand B landed by
       // TMA arrive on the same barrier) and a commit only where somebody waits for it: each
       // of these costs the issuing thread a round trip, and at these sizes the loop is bound
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
     for (int it = 0, stage = 0, pass = 0; it < nkb; ++it) {
       // "full" of this phase also means the MMAs of the stage's previous use are complete
       // (the TMA warp refilled it only after "empty"), so the A tile may be overwritten.
+      if (pass == 1 && stage == 0) pdl_wait();  // (a second use of a stage: behind MMAs over rows of the kernel in front)
       if (!mbar_wait(smem_u32(&bar_full[stage]), pass & 1, a.wait_limit_us)) {
         fail_s = 1;
         break;

@@ -95,3 +95,30 @@ def test_a_short_prefill_matches_the_operators_one_by_one(nets, weights, lens):
         worst = (norm(got - ref, dim=(2, 4)) / norm(ref, dim=(2, 4))).max().item()
         assert worst < 2 * (34 / 3) ** 0.5 * 2 ** -11, worst
     assert cache.pos[slots].tolist() == lens and cache.tok[slots].tolist() == first.tolist()
+
+
+def test_the_limit_of_a_wait_is_not_for_the_kernel_in_front(nets):
+    """The attention of 64 rows of 32000 tokens (1 GB a layer; no memory is faster than 8 TB/s, so 130 us and more) stands
+    before o_proj, whose CTAs are there from its start.  A limit of 60 us, enough for any wait of theirs once the attention has
+    ended, must not run out over it."""
+    from quic_cu_b200 import kernels as K
+
+    net, lib, rows, length = nets["w4"], K.lib(), 64, 32000
+    cache = net.new_cache(n_slots=rows, s_max=32064)
+    cache.kv.normal_(generator=torch.Generator(device="cuda").manual_seed(1))
+    tokens = torch.arange(rows, dtype=torch.int32, device="cuda")
+
+    def step():
+        cache.release_graphs()  # a graph holds the limit that it was captured with
+        cache.tok.copy_(tokens)
+        cache.pos.fill_(length)
+        cache.host_len[:] = [length] * rows
+        return net.decode(cache, list(range(rows)), 1)
+
+    want = step()
+    lib.quic_w4a16_tensor_test_hook(60, -1)
+    try:
+        assert step() == want
+    finally:
+        lib.quic_w4a16_tensor_test_hook(0, -1)
+    assert lib.quic_w4a16_tensor_status() == 0
