@@ -124,7 +124,9 @@ int quic_w4a16_tensor_status(void);
  * `wait_limit_us` microseconds at most (0: the default, two seconds) and never request
  * the packed weight tile of k block `skip_kblock` (128 k each; -1: none), so
  * the waits for it run out, every role of the CTA leaves its loop, the status
- * word is set and the kernel returns with its tensor memory released.  Call
+ * word is set and the kernel returns with its tensor memory released.  Below
+ * -1 nothing is left out, but every k block of a launch for up to 128 rows of
+ * a model comes -skip_kblock microseconds late.  Call
  * with (0, -1) to restore normal operation. */
 void quic_w4a16_tensor_test_hook(uint32_t wait_limit_us, int32_t skip_kblock);
 

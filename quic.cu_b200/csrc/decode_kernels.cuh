@@ -206,7 +206,7 @@ struct RowsArgs {
   const half* x;
   int32_t* status;
   uint32_t wait_limit_us;
-  int32_t skip_stage;
+  int32_t skip_stage;  // test hook: this stage never comes; below -1, all come late (-1: none)
 };
 void rows_next(RowsArgs* a, const quic_w4_t* w);  // nullptr: none
 int rows_qkv(const half* x, const RowsArgs& a, cudaStream_t st);

@@ -28,8 +28,10 @@
 // 844 / 911, 17 of 100..300 648 / 721, 48 of 64..200 696 / 768, 100 of 100..300 955 / 1080; un-quantised 17 rows 610 / 930,
 // 40 of 300..1500 761 / 1123, 100 934 / 1355.
 //
-// Every mbarrier wait is bounded: on a timeout the CTA records a code, takes part in the cluster's barriers, waits for
-// its own copies in flight, frees its tensor memory and returns.
+// Every mbarrier wait is bounded.  A role whose wait gives up says so to the CTA's others (fail_s) and goes on to the end; the CTA
+// records a code, takes part in the cluster's barriers, waits for its own copies and MMAs in flight, frees its tensor memory and
+// returns.  A wait for the accumulation may last as long as all of the MMA issuer's, and a CTA of a cluster sends its sums,
+// whatever they are, and waits for those of the others twice as long, so that no copy is on its way to or from it when it leaves.
 #include "tc_common.cuh"
 
 namespace quic {
@@ -111,13 +113,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   using C = Cfg<MODE, M, DENSE>;
   constexpr int kS = C::slots, kOwn = C::own, kR = C::rounds;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * kS + kR + 2];
+  __shared__ __align__(8) uint64_t bars[3 * kS + kR + 3];
   uint64_t* const bar_x = bars;               // a stage of rows landed
   uint64_t* const bar_ready = bar_x + kS;     // ... and is normalised
   uint64_t* const bar_empty = bar_ready + kS;  // ... and its MMAs are complete
   uint64_t* const bar_w = bar_empty + kS;     // a round of the CTA's weights is in shared memory (un-quantised: all of them)
-  uint64_t &bar_done = bar_w[kR], &bar_red = bar_w[kR + 1];
-  static_assert(3 * kS + kR + 2 <= 32, "a lane sets up a barrier");
+  uint64_t &bar_done = bar_w[kR], &bar_red = bar_w[kR + 1], &bar_drain = bar_w[kR + 2];
+  static_assert(3 * kS + kR + 3 <= 32, "a lane sets up a barrier");
+  constexpr uint32_t kIssuerWaits = C::n_stages + kR;
   __shared__ uint32_t tmem_s;
   __shared__ int fail_s;
   __shared__ float ssq_s[4][M];
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 
   if (warp == kWarpsC) {
-    if (lane < 3 * kS + kR + 2)
+    if (lane < 3 * kS + kR + 3)
       mbar_init(smem_u32(&bars[lane]), lane >= kS && lane < 2 * kS ? kWarpsC : lane >= 3 * kS && lane < 3 * kS + kR && !DENSE ? kWarpsC : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
@@ -210,6 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* const pow_s = reinterpret_cast<uint32_t*>(ln_s + C::k / 8);
   float* const rest_s = reinterpret_cast<float*>(pow_s + M);
 
+  bool issuer = false;
   if (warp == kWarpsC) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
@@ -229,6 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         const uint32_t full = smem_u32(&bar_x[s]);
+        if (a.skip_stage < -1) pause_us(-a.skip_stage);
         mbar_expect_tx(full, C::x_stage);
         if (issued != a.skip_stage) tma_load_3d(base + C::off_ring + s * C::x_stage, &tm_x, 0, m0, 2 * k_stage(issued), full);
         if (++s == kS) s = 0, ++pass;
@@ -247,7 +252,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kWarpsC + 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one()) {
+    issuer = elect_one();
+    if (issuer) {
       const uint32_t idesc = umma_idesc_f16(M, C::n);
       const uint64_t x0 = umma_desc_sw128(base + C::off_ring), w0 = umma_desc_sw128(base);
       bool ok = true;
@@ -410,6 +416,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (it + kAhead < C::n_stages) load_rows(it + kAhead);
         fence_proxy_async();
         __syncwarp();
+        if (a.skip_stage < -1) pause_us(-a.skip_stage);
         if (lane == 0 && it != a.skip_stage) mbar_arrive_one(smem_u32(&bar_ready[s]));
       }
     }
@@ -418,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   bool ok = true;
   if (warp < kWarpsC) {
-    ok = mbar_wait(smem_u32(&bar_done), 0, a.wait_limit_us);
+    ok = mbar_wait_unless(smem_u32(&bar_done), 0, &fail_s, a.wait_limit_us * (kIssuerWaits + 1));
     ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
     tc_fence_after();
     if (!ok) fail_s = 3;
@@ -540,7 +547,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       bulk_to_peer(peer_addr(base + C::off_red + rank * kPart, tid), base + C::off_ring + tid * kPart, kPart,
                    peer_addr(smem_u32(&bar_red), tid));
     if (warp < kWarpsC) {
-      if (!mbar_wait(smem_u32(&bar_red), 0, a.wait_limit_us)) {
+      if (!mbar_wait(smem_u32(&bar_red), 0, a.wait_limit_us * 2 * (kIssuerWaits + 1))) {
         ok = false;
         fail_s = 4;
       }
@@ -575,7 +582,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && fail_s != 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+  if (fail_s != 0) {
+    if (tid == 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+    mma_drain(issuer, smem_u32(&bar_drain));
+  }
   if (warp == kWarpsC + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(C::cols) : "memory");
 }
 

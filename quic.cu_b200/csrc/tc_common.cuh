@@ -45,6 +45,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return done;
 }
+// A wait for what other roles of the CTA bring about: it also ends when one of those has given up.
+__device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, const volatile int* given_up, uint32_t limit_us) {
+  bool done = mbar_try(bar, parity);
+  if (!done) {
+    const uint32_t t0 = clock_us();
+    do done = mbar_try(bar, parity);
+    while (!done && *given_up == 0 && clock_us() - t0 < limit_us);
+  }
+  return done;
+}
+// (test hook)
+__device__ __forceinline__ void pause_us(uint32_t us) {
+  const uint32_t t0 = clock_us();
+  while (clock_us() - t0 < us) __nanosleep(1000);
+}
 // The same wait for roles that are many warps wide and not on the critical path of the MMA
 // issue: sleeps between probes so the probes do not crowd the issuing thread's instructions
 // out of the shared-memory pipeline.
@@ -175,6 +190,20 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
+}
+// The way out of a CTA in which a wait gave up: nobody may have waited for its last MMAs, which read its shared memory and
+// write its tensor memory.  All threads, after the barrier that every role has reached; `issuer`: the thread that issued
+// the MMAs; `bar`: a barrier for one arrival, not in use.
+__device__ __forceinline__ void mma_drain(bool issuer, uint32_t bar) {
+  if (issuer) {
+    umma_commit(bar);
+    mbar_wait(bar, 0);
+    tc_fence_after();
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 }
 
 // Byte offset of 16-byte chunk c (0..7) of row r inside a swizzled tile.

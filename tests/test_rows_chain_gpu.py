@@ -122,3 +122,35 @@ def test_the_limit_of_a_wait_is_not_for_the_kernel_in_front(nets):
     finally:
         lib.quic_w4a16_tensor_test_hook(0, -1)
     assert lib.quic_w4a16_tensor_status() == 0
+
+
+@pytest.mark.parametrize("weights,rows", [("w4", 20), ("w4", 100), ("fp16", 20), ("fp16", 100)])
+def test_stages_that_come_late_and_too_late(nets, weights, rows):
+    """Every stage of the rows 2 ms late, with a limit of 3 ms a wait: the whole accumulation takes 14 ms, and nobody who waits
+    for all of it may give up before the issuer of the MMAs does.  With a limit of 1 ms the issuer gives up: decode() raises, the
+    CTAs leave in order, and the next decode() is right."""
+    from quic_cu_b200 import kernels as K
+
+    net, lib = nets[weights], K.lib()
+    gen = torch.Generator().manual_seed(rows)
+    prompts = [torch.randint(0, 2048, (int(n),), generator=gen) for n in torch.randint(4, 30, (rows,), generator=gen)]
+    slots = list(range(rows))
+
+    def step(limit, late):
+        cache = net.new_cache(n_slots=rows, s_max=64)
+        net.prefill(cache, slots, prompts)
+        torch.cuda.synchronize()
+        lib.quic_w4a16_tensor_test_hook(limit, late)
+        try:
+            return net.decode(cache, slots, 1), cache.kv
+        finally:
+            lib.quic_w4a16_tensor_test_hook(0, -1)
+
+    tokens, kv = step(0, -1)
+    late = step(3000, -2000)
+    assert late[0] == tokens and torch.equal(late[1], kv)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        step(1000, -2000)
+    again = step(0, -1)
+    assert again[0] == tokens and torch.equal(again[1], kv)
+    assert lib.quic_w4a16_tensor_status() == 0
