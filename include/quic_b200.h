@@ -120,14 +120,15 @@ int64_t quic_w4a16_workspace_bytes(int32_t m, int32_t n, int32_t k);
  * set.  No reference counterpart (Marlin's lock spins are unbounded,
  * kernels/cuda/marlin.cu:1467-1476). */
 int quic_w4a16_tensor_status(void);
-/* Test hook for those bounded waits: the GEMM launches that follow wait
- * `wait_limit_us` microseconds at most (0: the default, two seconds) and never request
- * the packed weight tile of k block `skip_kblock` (128 k each; -1: none), so
- * the waits for it run out, every role of the CTA leaves its loop, the status
- * word is set and the kernel returns with its tensor memory released.  Below
- * -1 nothing is left out, but every k block of a launch for up to 128 rows of
- * a model comes -skip_kblock microseconds late.  Call
- * with (0, -1) to restore normal operation. */
+/* Test hook for the bounded waits of the tcgen05 kernels (linears, lm_head,
+ * prefill attention, the decode step's rows chain): in launches that follow a
+ * wait lasts `wait_limit_us` microseconds at most (0: the default, two seconds)
+ * and the operand tile of k block (attention: key tile) `skip_kblock` never
+ * comes (-1: none), so the waits for it run out, every role of the CTA leaves
+ * its loop, the status word is set and the kernel returns with its MMAs and
+ * copies complete and its tensor memory released.  Below -1 nothing is left
+ * out, but every block comes -skip_kblock microseconds late.  Call with (0, -1)
+ * to restore normal operation. */
 void quic_w4a16_tensor_test_hook(uint32_t wait_limit_us, int32_t skip_kblock);
 
 /* Test hook for the streamed decode attention (more than 20 rows), for the launches and graph

@@ -26,7 +26,7 @@
 //
 // Roles: warps 0-3 softmax and epilogue, warp 4 TMA producer (two stages of K and V), warp 5 MMA issuer.
 // Every wait is bounded; a wait that runs out sets word 0 of the tensor path's error words
-// and the CTA leaves with its tensor memory released.
+// and the CTA leaves with its MMAs and copies complete and its tensor memory released.
 #include "tc_common.cuh"
 
 namespace quic {
@@ -49,6 +49,8 @@ struct PrefillTcArgs {
   half* out;               // [rows][896]
   int32_t rows, s_max, n_slots;
   float scale_log2;        // softmax scale x log2(e)
+  uint32_t wait_limit_us;
+  int32_t skip_tile;       // test hook: this key tile never comes; below -1, all come late (-1: none)
 };
 
 __device__ __forceinline__ uint32_t pack2(float x, float y) {
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
   // columns: S, O with P in S's place; or S of even and of odd tiles, O, P
   constexpr uint32_t kTmemCols = kAhead ? 256 : 128, kColS1 = kAhead ? 64 : 0, kColO = kAhead ? 128 : 64, kColP = kAhead ? 192 : 0;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bar_q, bar_full[2], bar_empty[2], bar_s[2], bar_p;
+  __shared__ __align__(8) uint64_t bar_q, bar_full[2], bar_empty[2], bar_s[2], bar_p, bar_drain;
   __shared__ uint32_t tmem_base_s;
   __shared__ int fail_s;
 
@@ -143,6 +145,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
       mbar_init(smem_u32(&bar_s[s]), 1);
     }
     mbar_init(smem_u32(&bar_p), kSoftmaxWarps);
+    mbar_init(smem_u32(&bar_drain), 1);
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
   pdl_launch_dependents();
   pdl_wait();  // queries and cache rows come from the kernels before this one
 
+  bool issuer = false;
   if (warp == kSoftmaxWarps) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
@@ -166,25 +170,27 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
       tma_load_2d(base + kSmemQ, &tm_q, 0, head * a.rows + start + r0, smem_u32(&bar_q));
       for (int i = 0; i < n_tiles; ++i) {
         const int st = i & 1;
-        if (i >= 2 && !mbar_wait(smem_u32(&bar_empty[st]), ((i >> 1) - 1) & 1)) {
+        if (i >= 2 && !mbar_wait(smem_u32(&bar_empty[st]), ((i >> 1) - 1) & 1, a.wait_limit_us)) {
           fail_s = 2;
           break;
         }
+        if (a.skip_tile < -1) pause_us(-a.skip_tile);
         const uint32_t full = smem_u32(&bar_full[st]);
         mbar_expect_tx(full, 2 * kTileBytes);
-        tma_load_2d(base + kSmemK + st * kTileBytes, &tm_k, 0, kv_row0 + i * kKeys, full);
+        if (i != a.skip_tile) tma_load_2d(base + kSmemK + st * kTileBytes, &tm_k, 0, kv_row0 + i * kKeys, full);
         tma_load_2d(base + kSmemV + st * kTileBytes, &tm_v, 0, kv_row0 + i * kKeys, full);
       }
     }
   } else if (warp == kSoftmaxWarps + 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one()) {
+    issuer = elect_one();
+    if (issuer) {
       const uint64_t q0 = umma_desc_sw128(base + kSmemQ), k0 = umma_desc_sw128(base + kSmemK), v0 = umma_desc_sw128(base + kSmemV);
       const uint32_t idesc = umma_idesc_f16(kKeys);         // M = 128, N = 64
       const uint32_t idesc_v = idesc | (1u << 16);           // B transposed: N (the head dims) contiguous
       auto scores = [&](int i) {
         const int st = i & 1;
-        if (!mbar_wait(smem_u32(&bar_full[st]), (i >> 1) & 1)) return false;
+        if (!mbar_wait(smem_u32(&bar_full[st]), (i >> 1) & 1, a.wait_limit_us)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -192,11 +198,11 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
         umma_commit(smem_u32(&bar_s[st]));
         return true;
       };
-      bool ok = mbar_wait(smem_u32(&bar_q), 0) && scores(0);
+      bool ok = mbar_wait(smem_u32(&bar_q), 0, a.wait_limit_us) && scores(0);
       for (int i = 0; ok && i < n_tiles; ++i) {
         const int st = i & 1;
         if (kAhead && i + 1 < n_tiles) ok = scores(i + 1);  // S(i - 1), the buffer's last, has been read: P(i - 1) came
-        if (!ok || !mbar_wait(smem_u32(&bar_p), i & 1)) {  // P(i) is in tensor memory, O rescaled where need be
+        if (!ok || !mbar_wait(smem_u32(&bar_p), i & 1, a.wait_limit_us)) {  // P(i) is in tensor memory, O rescaled where need be
           ok = false;
           break;
         }
@@ -207,7 +213,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
                       (i > 0 || k > 0) ? 1u : 0u);
         umma_commit(smem_u32(&bar_empty[st]));
         if (!kAhead && i + 1 < n_tiles)  // P(i) shares S's columns: its product has to be complete
-          ok = mbar_wait(smem_u32(&bar_empty[st]), (i >> 1) & 1) && scores(i + 1);
+          ok = mbar_wait(smem_u32(&bar_empty[st]), (i >> 1) & 1, a.wait_limit_us) && scores(i + 1);
       }
       if (!ok) fail_s = 3;
     }
@@ -219,10 +225,11 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
     const int last = min(pos, kv_len - 1);     // the row's last key
     float m_ref = -INFINITY, l_run = 0.f;
     bool ok = true;
+    const uint32_t limit = 4 * a.wait_limit_us;  // (the issuer waits up to three times between two tiles' scores)
     for (int i = 0; i < n_tiles; ++i) {
       const int t0 = i * kKeys;
       const uint32_t tmem_si = tmem_s + kColS1 * (i & 1) + lane_addr;
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_s[i & 1]), (i >> 1) & 1));
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_s[i & 1]), (i >> 1) & 1, limit));
       if (!ok) break;
       tc_fence_after();
       // a tile wholly below the diagonal of all 128 rows needs no mask (CTA-uniform)
@@ -246,7 +253,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
         for (int j = 0; j < 32; j += 2) mx[(j >> 1) & 3] = max3(mx[(j >> 1) & 3], part[j], part[j + 1]);
       }
       if (kAhead && i > 0) {  // P(i - 1) has been multiplied: P and O may be written
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[(i - 1) & 1]), ((i - 1) >> 1) & 1));
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[(i - 1) & 1]), ((i - 1) >> 1) & 1, limit));
         if (!ok) break;
         tc_fence_after();
       }
@@ -294,10 +301,10 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
       __syncwarp();
       if (lane == 0) mbar_arrive_cta(smem_u32(&bar_p));
     }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[(n_tiles - 1) & 1]), ((n_tiles - 1) >> 1) & 1));
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[(n_tiles - 1) & 1]), ((n_tiles - 1) >> 1) & 1, limit));
     tc_fence_after();
     ok = __all_sync(0xffffffffu, ok && !fail_s);
-    if (!ok && lane == 0) atomicCAS(status, 0, ((fail_s ? fail_s : 1) << 16) | 0x2000 | ((int)blockIdx.z & 0x1fff));
+    if (!ok && fail_s == 0) fail_s = 1;
     if (ok) {
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       half* op = a.out + (size_t)(start + r0 + row) * kHidden + head * kHeadDim;
@@ -322,6 +329,10 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
   __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (fail_s != 0) {
+    if (tid == 0) atomicCAS(status, 0, (fail_s << 16) | 0x2000 | ((int)blockIdx.z & 0x1fff));
+    drain_failed(issuer, smem_u32(&bar_drain));
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_s), "r"(kTmemCols) : "memory");
 }
@@ -359,6 +370,7 @@ int attn_prefill_tc_launch(const void* q, const void* kcache, const void* vcache
   a.rows = rows;
   a.s_max = s_max;
   a.n_slots = n_slots;
+  tc_test_hook(&a.wait_limit_us, &a.skip_tile);
   a.scale_log2 = (scale > 0.f ? scale : 0.125f) * 1.4426950408889634f;
   // Up to four CTAs an SM in all: too few to hide a tile's latency, so its scores run a tile ahead, in twice
   // the tensor memory (plain / ahead, us: 1 x 512 15.0 / 11.7, 1 x 2048 46.5 / 34.8, 4 x 1000 28.8 / 28.2,

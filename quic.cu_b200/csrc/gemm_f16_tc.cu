@@ -13,7 +13,7 @@
 //
 // Roles: warps 0-3 epilogue (thread 0 issues the MMAs), warp 4 the TMA producer.  Every wait
 // is bounded; a wait that runs out sets word 0 of the tensor path's error words and the CTA
-// leaves with its tensor memory released.
+// leaves with its MMAs and copies complete and its tensor memory released.
 #include "tc_common.cuh"
 
 namespace quic {
@@ -36,6 +36,8 @@ struct DenseArgs {
   float* part;       // split K: [splits][M][N] fp32 partial sums (then y and bias belong to the finish kernel)
   int m_total, n, k;
   int kb_per_split;  // 64-wide k blocks per CTA along grid.z
+  uint32_t wait_limit_us;
+  int skip_kblock;  // test hook: this k block never comes; below -1, all come late (-1: none)
 };
 
 template <int MT>
@@ -45,7 +47,7 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kDenseStages];
   __shared__ __align__(8) uint64_t bar_empty[kDenseStages];
-  __shared__ __align__(8) uint64_t bar_done;
+  __shared__ __align__(8) uint64_t bar_done, bar_drain;
   __shared__ uint32_t tmem_base_s;
   __shared__ int fail_s;
 
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     mbar_init(smem_u32(&bar_done), 1);
+    mbar_init(smem_u32(&bar_drain), 1);
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -83,6 +86,7 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
   const uint32_t idesc = umma_idesc_f16(MT);
   pdl_launch_dependents();
 
+  bool issuer = false;
   if (warp == 4) {
     if (lane == 0) {
       // The weight tiles of the first ring pass do not depend on the previous kernel: they are
@@ -92,30 +96,33 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
       for (int it = 0; it < first; ++it) {
         const uint32_t full = smem_u32(&bar_full[it]);
         mbar_expect_tx(full, L::kA + (uint32_t)MT * 128u);
-        tma_load_2d(base + it * L::kStage, &tm_w, (kb0 + it) * kBlockK, n0, full);
+        if (kb0 + it != a.skip_kblock) tma_load_2d(base + it * L::kStage, &tm_w, (kb0 + it) * kBlockK, n0, full);
       }
       pdl_wait();
-      for (int it = 0; it < first; ++it)
+      for (int it = 0; it < first; ++it) {
+        if (a.skip_kblock < -1) pause_us(-a.skip_kblock);
         tma_load_2d(base + it * L::kStage + L::kA, &tm_x, (kb0 + it) * kBlockK, m0, smem_u32(&bar_full[it]));
+      }
       for (int it = first; it < nkb; ++it) {
         const int stage = it % kDenseStages;
-        if (!mbar_wait(smem_u32(&bar_empty[stage]), ((it / kDenseStages) - 1) & 1)) {
+        if (!mbar_wait(smem_u32(&bar_empty[stage]), ((it / kDenseStages) - 1) & 1, a.wait_limit_us)) {
           fail_s = 2;
           break;
         }
+        if (a.skip_kblock < -1) pause_us(-a.skip_kblock);
         const uint32_t a_s = base + stage * L::kStage, b_s = a_s + L::kA;
         const uint32_t full = smem_u32(&bar_full[stage]);
         mbar_expect_tx(full, L::kA + (uint32_t)MT * 128u);
-        tma_load_2d(a_s, &tm_w, (kb0 + it) * kBlockK, n0, full);
+        if (kb0 + it != a.skip_kblock) tma_load_2d(a_s, &tm_w, (kb0 + it) * kBlockK, n0, full);
         tma_load_2d(b_s, &tm_x, (kb0 + it) * kBlockK, m0, full);
       }
     }
-  } else if (warp == 0 && elect_one()) {
+  } else if (warp == 0 && (issuer = elect_one())) {
     pdl_wait();  // the activations cannot be here earlier, and a wait's limit is not for the kernel in front
     const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + L::kA);
     for (int it = 0; it < nkb; ++it) {
       const int stage = it % kDenseStages;
-      if (!mbar_wait(smem_u32(&bar_full[stage]), (it / kDenseStages) & 1)) {
+      if (!mbar_wait(smem_u32(&bar_full[stage]), (it / kDenseStages) & 1, a.wait_limit_us)) {
         fail_s = 1;
         break;
       }
@@ -131,10 +138,11 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
 
   if (warp < 4) {
     pdl_wait();  // y may still be read by an earlier kernel of the chain
-    bool ok = mbar_wait_relaxed(smem_u32(&bar_done), 0, 32) && !fail_s;
+    // (the issuer has a wait for every k block)
+    bool ok = mbar_wait_relaxed(smem_u32(&bar_done), 0, 32, a.wait_limit_us * (uint32_t)min(nkb + 1, 1024), &fail_s);
     ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
     tc_fence_after();
-    if (!ok && tid == 0) atomicCAS(status, 0, ((fail_s ? fail_s : 3) << 16) | 0x4000 | ((int)blockIdx.x & 0x3fff));
+    if (!ok && fail_s == 0) fail_s = 3;
     const int col = n0 + warp * 32 + lane;  // TMEM lane = weight row = output column
     const float bias = a.bias != nullptr ? __half2float(a.bias[col]) : 0.f;
     if (ok) {
@@ -165,6 +173,10 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
   }
   tc_fence_before();
   __syncthreads();
+  if (fail_s != 0) {
+    if (tid == 0) atomicCAS(status, 0, (fail_s << 16) | 0x4000 | ((int)blockIdx.x & 0x3fff));
+    drain_failed(issuer, smem_u32(&bar_drain));
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kCols) : "memory");
 }
@@ -256,6 +268,7 @@ int gemm_f16_tc(const half* x, const half* w, const half* bias, half* y, int m, 
   a.kb_per_split = (nkb + splits - 1) / splits;
   splits = (nkb + a.kb_per_split - 1) / a.kb_per_split;
   a.part = splits > 1 ? ws : nullptr;
+  tc_test_hook(&a.wait_limit_us, &a.skip_kblock);
   int rc;
   switch (mt) {
     case 16: rc = run<16>(x, w, a, splits, st, pdl); break;

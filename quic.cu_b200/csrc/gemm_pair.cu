@@ -17,7 +17,7 @@
 // columns, so the epilogue of a tile runs under the next tile's MMAs.  Token rows are on
 // the M side: a thread of the epilogue owns a row and, with 128 gate and 128 up columns in a tile, both
 // factors of its SwiGLU outputs.  Waits are bounded by the clock: one that runs out sets word 0
-// of the tensor path's error words and the pair leaves with its tensor memory released.
+// of the tensor path's error words and the pair leaves with its MMAs and copies complete and its tensor memory released.
 #include "tc_common.cuh"
 
 namespace quic {
@@ -43,29 +43,10 @@ struct PairArgs {
   int splits;
   int* status;
   PairRope rope;
+  uint32_t wait_limit_us;
+  int32_t skip_kblock;  // test hook: this k block (of 64) of a tile never comes; below -1, all come late (-1: none)
 };
 
-// Waits at most a second or so for the phase with the given parity.
-__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity) {
-  uint64_t t0 = 0;
-  for (uint32_t i = 0;; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity), "r"(2000u)
-        : "memory");
-    if (done) return true;
-    if ((i & 255u) == 255u) {
-      uint64_t now;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-      if (t0 == 0) t0 = now;
-      if (now - t0 > 1000000000ull) return false;
-    }
-  }
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
@@ -140,6 +121,11 @@ __device__ __forceinline__ void pair_commit(uint32_t bar) {
       "h"((uint16_t)3)
       : "memory");
 }
+// a word at the same shared-memory address of the pair's second CTA
+__device__ __forceinline__ void tell_peer(uint32_t addr, int value) {
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 1;\n\tst.shared::cluster.u32 [ra], %1;\n\t}" ::"r"(addr), "r"(value)
+               : "memory");
+}
 __device__ __forceinline__ void arrive_leader(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_leader(bar)) : "memory");
 }
@@ -150,7 +136,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   using L = PairSmem<NT>;
   constexpr int kOut = kSwiglu ? NT / 2 : NT;  // output columns of a tile
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[kPairStages], bar_empty[kPairStages], bar_acc[2], bar_free[2];
+  __shared__ __align__(8) uint64_t bar_full[kPairStages], bar_empty[kPairStages], bar_acc[2], bar_free[2], bar_drain;
   __shared__ uint32_t tmem_base_s;
   __shared__ int fail_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -170,6 +156,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       mbar_init(smem_u32(&bar_acc[s]), 1);
       mbar_init(smem_u32(&bar_free[s]), 2 * kPairEpilogueWarps);
     }
+    mbar_init(smem_u32(&bar_drain), 1);
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -185,6 +172,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   pdl_launch_dependents();
   pdl_wait();
 
+  bool issuer = false;
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0, pass = 0;
@@ -194,15 +182,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         const int kb1 = kblocks * (split + 1) / a.splits;
         const int w0 = kSwiglu ? (int)rank * (a.n / 2) + nt * (NT / 2) : nt * NT + (int)rank * (NT / 2);
         for (int kb = kblocks * split / a.splits; kb < kb1; ++kb) {
-          if (pass > 0 && !pair_wait(smem_u32(&bar_empty[stage]), (pass - 1) & 1)) {
+          if (pass > 0 && !mbar_wait(smem_u32(&bar_empty[stage]), (pass - 1) & 1, a.wait_limit_us)) {
             fail_s = 2;
             ok = false;
-            for (int i = 0; i < 64; ++i) __nanosleep(1000);  // (copies in flight land within microseconds)
             break;
           }
+          if (a.skip_kblock < -1) pause_us(-a.skip_kblock);
           const uint32_t a_s = base + stage * L::kStage, full = smem_u32(&bar_full[stage]), lead = in_leader(full);
           if (rank == 0) mbar_expect_tx(full, 2 * L::kStage);
-          pair_load(a_s, &tm_x, kb * kBlockK, m0, lead);
+          if (kb != a.skip_kblock) pair_load(a_s, &tm_x, kb * kBlockK, m0, lead);
           pair_load(a_s + kPairA, &tm_w, kb * kBlockK, w0, lead);
           if (++stage == kPairStages) {
             stage = 0;
@@ -212,7 +200,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (rank == 0 && elect_one()) {
+    if (rank == 0 && (issuer = elect_one())) {
       const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + kPairA);
       // fp16 x fp16 -> fp32, both operands K-major, M = 256 over the pair, N = NT
       constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -220,7 +208,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       bool ok = true;
       for (int t = first; ok && t < tiles; t += pairs, ++j) {
         const int buf = j & 1;
-        if (j >= 2 && !pair_wait(smem_u32(&bar_free[buf]), ((j >> 1) - 1) & 1)) {
+        if (j >= 2 && !mbar_wait(smem_u32(&bar_free[buf]), ((j >> 1) - 1) & 1, a.wait_limit_us)) {
           fail_s = 4;
           break;
         }
@@ -228,7 +216,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         const uint32_t d = tmem_d + 256u * buf;
         const int split = t / flat, nkb = kblocks * (split + 1) / a.splits - kblocks * split / a.splits;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!pair_wait(smem_u32(&bar_full[stage]), pass & 1)) {
+          if (!mbar_wait(smem_u32(&bar_full[stage]), pass & 1, a.wait_limit_us)) {
             fail_s = 1;
             ok = false;
             break;
@@ -245,6 +233,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         }
         if (ok) pair_commit(smem_u32(&bar_acc[buf]));
       }
+      if (fail_s != 0) tell_peer(smem_u32(&fail_s), fail_s);  // (its epilogue waits for these MMAs too)
     }
   } else {
     const int quarter = warp & 3, group = (warp - 2) >> 2;  // TMEM lanes that this warp may read, 32-column share
@@ -259,7 +248,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       const int tok = row0 + lane;
       const bool live = kRope && tok < a.m_total;
       const int pos = live ? a.rope.positions[tok] : 0, slot = live ? a.rope.slots[tok] : -1;
-      if (!__all_sync(0xffffffffu, pair_wait(smem_u32(&bar_acc[buf]), (j >> 1) & 1))) {
+      // (the issuer has a wait for every k block)
+      const uint32_t limit = a.wait_limit_us * (uint32_t)min(kblocks + 2, 1024);
+      if (!__all_sync(0xffffffffu, mbar_wait_unless(smem_u32(&bar_acc[buf]), (j >> 1) & 1, &fail_s, limit))) {
         fail_s = 3;
         break;
       }
@@ -329,8 +320,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   }
   __syncwarp();
   tc_fence_before();
-  __syncthreads();
-  if (tid == 0 && fail_s != 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+  if (__syncthreads_or(fail_s)) {  // (the leader may set it at any time) the last MMAs and copies, as in drain_failed(); MMAs in flight that rank 0 has not waited for make it fail
+    if (tid == 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+    if (issuer) {
+      pair_commit(smem_u32(&bar_drain));
+      mbar_wait(smem_u32(&bar_drain), 0);
+      tc_fence_after();
+    }
+    if (tid == 0) pause_us(1000);
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+  }
   pair_sync();  // nobody leaves while the pair's copies, arrivals or MMAs use its shared memory
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_d) : "memory");
 }
@@ -445,7 +446,8 @@ int gemm_pair(const half* x, const half* w, const half* bias, half* y, int m, in
   QUIC_REQUIRE(gemm_pair_supported(m, n, k, swiglu), QUIC_E_SHAPE, "gemm_pair: unsupported shape");
   QUIC_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)part) % 16 == 0 && (uintptr_t)bias % 4 == 0, QUIC_E_ARG,
                "gemm_pair: tensors must be 16-byte aligned, the bias 4-byte");
-  PairArgs a = {bias, y, nullptr, m, n, k, 1, tc_status_words(), {}};
+  PairArgs a = {bias, y, nullptr, m, n, k, 1, tc_status_words()};
+  tc_test_hook(&a.wait_limit_us, &a.skip_kblock);
   if (splits != nullptr) *splits = 0;
   if (part != nullptr && gemm_pair_splits(m, n, k) > 1) {
     a.part = part;
@@ -466,6 +468,7 @@ int gemm_pair_qkv(const half* x, const half* w, const half* bias, int m, const P
   QUIC_REQUIRE(((uintptr_t)x | (uintptr_t)w) % 16 == 0 && (uintptr_t)bias % 4 == 0, QUIC_E_ARG,
                "gemm_pair: tensors must be 16-byte aligned, the bias 4-byte");
   PairArgs a = {bias, nullptr, nullptr, m, kQkvN, kHidden, 1, tc_status_words(), rope};
+  tc_test_hook(&a.wait_limit_us, &a.skip_kblock);
   QUIC_REQUIRE(a.status != nullptr, QUIC_E_CUDA, "gemm_pair: no address for the tensor path's error words");
   return run_pair<192, false, true>(x, w, a, st);
 }

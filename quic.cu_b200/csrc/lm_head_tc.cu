@@ -36,12 +36,13 @@ struct LmSmem {
 template <int MT>
 __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_constant__ CUtensorMap tm_e,
                                                                 const __grid_constant__ CUtensorMap tm_x,
-                                                                const LmHeadArgs a, int* status) {
+                                                                const LmHeadArgs a, int* status, uint32_t wait_limit_us,
+                                                                int skip_kblock) {
   constexpr int kLmStages = LmSmem<MT>::kStages;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kLmStages];
   __shared__ __align__(8) uint64_t bar_empty[kLmStages];
-  __shared__ __align__(8) uint64_t bar_done;
+  __shared__ __align__(8) uint64_t bar_done, bar_drain;
   __shared__ uint32_t tmem_base_s;
   __shared__ int fail_s;
   __shared__ int last_flag;
@@ -66,6 +67,7 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     mbar_init(smem_u32(&bar_done), 1);
+    mbar_init(smem_u32(&bar_drain), 1);
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -84,27 +86,29 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
   pdl_launch_dependents();
   pdl_wait();  // the normalised activations come from the previous kernel
 
+  bool issuer = false;
   if (warp == 4) {
     if (lane == 0) {
       for (int it = 0; it < nkb; ++it) {
         const int stage = it % kLmStages;
-        if (it >= kLmStages && !mbar_wait(smem_u32(&bar_empty[stage]), ((it / kLmStages) - 1) & 1)) {
+        if (it >= kLmStages && !mbar_wait(smem_u32(&bar_empty[stage]), ((it / kLmStages) - 1) & 1, wait_limit_us)) {
           fail_s = 2;
           break;
         }
+        if (skip_kblock < -1) pause_us(-skip_kblock);
         const uint32_t a_s = base + stage * L::kStage, b_s = a_s + L::kA;
         const uint32_t full = smem_u32(&bar_full[stage]);
         mbar_expect_tx(full, L::kA + (uint32_t)MT * 128u);
         const int kb = (it + rot) % nkb;
-        tma_load_2d(a_s, &tm_e, kb * kBlockK, n0, full);
+        if (it != skip_kblock) tma_load_2d(a_s, &tm_e, kb * kBlockK, n0, full);
         tma_load_2d(b_s, &tm_x, kb * kBlockK, 0, full);
       }
     }
-  } else if (warp == 0 && elect_one()) {
+  } else if (warp == 0 && (issuer = elect_one())) {
     const uint64_t a0 = umma_desc_sw128(base), b0 = umma_desc_sw128(base + L::kA);
     for (int it = 0; it < nkb; ++it) {
       const int stage = it % kLmStages;
-      if (!mbar_wait(smem_u32(&bar_full[stage]), (it / kLmStages) & 1)) {
+      if (!mbar_wait(smem_u32(&bar_full[stage]), (it / kLmStages) & 1, wait_limit_us)) {
         fail_s = 1;
         break;
       }
@@ -119,11 +123,11 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
   __syncwarp();
 
   if (warp < 4) {
-    // every epilogue thread waits for the accumulation itself (bounded)
-    bool ok = mbar_wait(smem_u32(&bar_done), 0) && !fail_s;
+    // every epilogue thread waits for the accumulation itself (bounded; the issuer has a wait for every k block)
+    bool ok = mbar_wait_unless(smem_u32(&bar_done), 0, &fail_s, wait_limit_us * (nkb + 1));
     ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
     tc_fence_after();
-    if (!ok && lane == 0 && warp == 0) atomicCAS(status, 0, ((fail_s ? fail_s : 3) << 16) | 0x8000 | (tile & 0x7fff));
+    if (!ok && fail_s == 0) fail_s = 3;
     const int row = n0 + warp * 32 + lane;
 #pragma unroll 1
     for (int c0 = 0; c0 < MT; c0 += 8) {
@@ -157,6 +161,10 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
   }
   tc_fence_before();
   __syncthreads();
+  if (fail_s != 0) {  // a bounded wait gave up: the tokens are invalid
+    if (tid == 0) atomicCAS(status, 0, (fail_s << 16) | 0x8000 | (tile & 0x7fff));
+    drain_failed(issuer, smem_u32(&bar_drain));
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kCols) : "memory");
 
@@ -214,10 +222,13 @@ int run(const LmHeadArgs& a, cudaStream_t st) {
   int* status = tc_status_words();  // word 1 is this kernel's
   QUIC_REQUIRE(status != nullptr, QUIC_E_CUDA, "lm_head: no address for the tensor path's error words");
   status += 1;
+  uint32_t wait_limit_us;
+  int32_t skip_kblock;
+  tc_test_hook(&wait_limit_us, &skip_kblock);
   const size_t smem = LmSmem<MT>::kTotal;
   QUIC_CUDA(allow_smem<lm_head_tc_kernel<MT>>(smem));
   QUIC_CUDA(launch(lm_head_tc_kernel<MT>, dim3(a.vocab / kTileN), dim3(kLmThreads), smem, st, true, tm_e, tm_x, a,
-                   status));
+                   status, wait_limit_us, skip_kblock));
   return QUIC_OK;
 }
 

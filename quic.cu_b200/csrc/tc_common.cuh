@@ -55,7 +55,6 @@ __device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, 
   }
   return done;
 }
-// (test hook)
 __device__ __forceinline__ void pause_us(uint32_t us) {
   const uint32_t t0 = clock_us();
   while (clock_us() - t0 < us) __nanosleep(1000);
@@ -63,15 +62,15 @@ __device__ __forceinline__ void pause_us(uint32_t us) {
 // The same wait for roles that are many warps wide and not on the critical path of the MMA
 // issue: sleeps between probes so the probes do not crowd the issuing thread's instructions
 // out of the shared-memory pipeline.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, uint32_t sleep_ns,
-                                                  uint32_t limit_us = kWaitLimitUs) {
+__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, uint32_t sleep_ns, uint32_t limit_us,
+                                                  const volatile int* given_up) {
   bool done = mbar_try(bar, parity);
   if (!done) {
     const uint32_t t0 = clock_us();
     do {
       __nanosleep(sleep_ns);
       done = mbar_try(bar, parity);
-    } while (!done && clock_us() - t0 < limit_us);
+    } while (!done && *given_up == 0 && clock_us() - t0 < limit_us);
   }
   return done;
 }
@@ -191,14 +190,16 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
-// The way out of a CTA in which a wait gave up: nobody may have waited for its last MMAs, which read its shared memory and
-// write its tensor memory.  All threads, after the barrier that every role has reached; `issuer`: the thread that issued
-// the MMAs; `bar`: a barrier for one arrival, not in use.
-__device__ __forceinline__ void mma_drain(bool issuer, uint32_t bar) {
+// The way out of a CTA in which a wait gave up: nobody may have waited for its last MMAs and copies, which use its shared memory
+// and its tensor memory.  All threads, after the barrier that every role has reached; `issuer`: the thread that issued
+// the MMAs; `bar`: a barrier for one arrival, not in use.  The MMAs are waited for; a copy, which waits for nothing, lands within
+// microseconds of its request and is given a millisecond.
+__device__ __forceinline__ void drain_failed(bool issuer, uint32_t bar) {
   if (issuer) {
     umma_commit(bar);
     mbar_wait(bar, 0);
     tc_fence_after();
+    pause_us(1000);
   }
   __syncwarp();
   tc_fence_before();

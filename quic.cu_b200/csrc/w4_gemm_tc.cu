@@ -20,7 +20,7 @@
 //      where the stage will be refilled, commits them to the stage's "empty" mbarrier.
 // Split-K CTAs write fp32 partials that the consumer kernel (or a small finish kernel) sums;
 // the gate|up form applies SwiGLU in its epilogue.  Every mbarrier wait is bounded: on a
-// timeout the kernel records an error code, still frees its tensor memory and returns.
+// timeout the CTA records an error code, waits for its MMAs and copies in flight, frees its tensor memory and returns.
 #include "tc_common.cuh"
 
 namespace quic {
@@ -45,7 +45,7 @@ struct GemmArgs {
   int kblocks_per_split;
   int mtl;     // batch-row tiles per CTA (2 from 129 rows up)
   uint32_t wait_limit_us;  // of a bounded wait
-  int skip_kblock;      // test hook: the weight tile of this k block is never requested (-1: none)
+  int skip_kblock;      // test hook: the weight tile of this k block is never requested; below -1, all come late (-1: none)
   // SwiGLU fused into the epilogue of the gate|up linear: the CTA's 128 weight rows are 64
   // gate rows and the 64 up rows of the same columns (two 64-row TMA boxes per stage), and y
   // is the activation [m_total, N / 2] = silu(gate) * up.
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
   __shared__ __align__(8) uint64_t bar_full[kMaxStages];    // packed weight tile landed (TMA bytes)
   __shared__ __align__(8) uint64_t bar_aready[kMaxStages];  // 16 consumer warps finished the A tile AND the x tile landed
   __shared__ __align__(8) uint64_t bar_empty[kMaxStages];   // MMAs that read the stage completed
-  __shared__ __align__(8) uint64_t bar_done;
+  __shared__ __align__(8) uint64_t bar_done, bar_drain;
   __shared__ uint32_t tmem_base_s;
   __shared__ int fail_s;
 
@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     mbar_init(smem_u32(&bar_done), 1);
+    mbar_init(smem_u32(&bar_drain), 1);
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
   // and requests the x tiles; the other roles wait before they touch global memory.
   pdl_launch_dependents();
 
+  bool issuer = false;
   if (warp == kConsumers / 32) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
@@ -178,6 +180,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
       };
       for (int it = 0; it < first; ++it) {
         if (kb0 + it == a.skip_kblock) continue;  // test hook: the consumers' wait for this tile runs out
+        if (a.skip_kblock < -1) pause_us(-a.skip_kblock);
         load_weights(base + it * L::kStage, kb0 + it, smem_u32(&bar_full[it]));
       }
       pdl_wait();
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
           fail_s = 2;
           break;
         }
+        if (a.skip_kblock < -1) pause_us(-a.skip_kblock);
         const uint32_t raw_s = base + stage * L::kStage, b_s = raw_s + kRawBytes;
         const uint32_t full = smem_u32(&bar_full[stage]), xfull = smem_u32(&bar_aready[stage]);
         if (kb0 + it != a.skip_kblock) load_weights(raw_s, kb0 + it, full);  // (test hook: see the first pass)
@@ -210,7 +214,8 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
     }
   } else if (warp == kConsumers / 32 + 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one()) {
+    issuer = elect_one();
+    if (issuer) {
       const uint64_t b0 = umma_desc_sw128(base + kRawBytes), a0 = umma_desc_sw128(base + kRawBytes + L::kB);
       pdl_wait();  // the rows cannot be here earlier, and a wait's limit is not for the kernel in front
       // One wait per k block (operand A written by the consumer warps and operand B landed by
@@ -292,10 +297,11 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
   if (warp < kConsumers / 32) {
     pdl_wait();  // the output / partial buffers may still be read by earlier kernels of the chain
     bool ok = !fail_s && nkb > 0;
-    if (ok) ok = mbar_wait_relaxed(smem_u32(&bar_done), 0, 64, a.wait_limit_us);
+    // (the issuer may have a wait to go for every stage)
+    if (ok) ok = mbar_wait_relaxed(smem_u32(&bar_done), 0, 64, a.wait_limit_us * (kStages + 1), &fail_s);
     ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
     tc_fence_after();
-    if (!ok && tid == 0 && nkb > 0) atomicCAS(&g_tc_status[0], 0, ((fail_s ? fail_s : 3) << 16) | (int)blockIdx.x);
+    if (!ok && nkb > 0 && fail_s == 0) fail_s = 3;
     constexpr int kOutCols = MT * MTL;       // accumulator columns = batch rows of the CTA
     constexpr int kWarpCols = kOutCols / 4;  // per warp of a lane quarter
     if (a.y != nullptr && gridDim.y == 1) {
@@ -393,6 +399,10 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
   }
   tc_fence_before();
   __syncthreads();
+  if (fail_s != 0) {
+    if (tid == 0) atomicCAS(&g_tc_status[0], 0, (fail_s << 16) | (int)blockIdx.x);
+    drain_failed(issuer, smem_u32(&bar_drain));
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kCols) : "memory");
 }

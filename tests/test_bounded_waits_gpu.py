@@ -1,0 +1,87 @@
+"""The bounded waits of the tcgen05 kernels, one operator at a time: operands that come late but within the limit change
+nothing, operands that come too late or never set the error word, the CTAs leave in order (MMAs and copies complete,
+tensor memory free), and the next call is right."""
+
+import pytest
+import torch
+
+from quic_cu_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def _linear(weight, m):
+    x = torch.randn(m, weight.size_k, device="cuda", generator=_gen(m)).half()
+    return lambda: K.w4a16_linear(weight, x)
+
+
+def _packed(n, k):
+    w = K.W4Weight(n, k, torch.device("cuda"))
+    w.qw.random_(-2 ** 31, 2 ** 31 - 1, generator=_gen(1))
+    w.zp.random_(0, 255, generator=_gen(2))
+    w.sc.copy_(torch.rand(w.sc.shape, device="cuda", generator=_gen(3)) * 0.02)
+    return w
+
+
+def _dense(n, k):
+    w = K.F16Weight(n, k, torch.device("cuda"))
+    w.w.copy_(torch.randn(n, k, device="cuda", generator=_gen(4)) * 0.05)
+    return w
+
+
+def _lm_head(rows):
+    x = torch.randn(rows, K.HIDDEN, device="cuda", generator=_gen(5)).half()
+    table = torch.randn(2048, K.HIDDEN, device="cuda", generator=_gen(6)).half()
+    return lambda: K.lm_head_argmax(x, table, want_logits=True)[1]
+
+
+def _attention(n_seq):
+    """130 rows a sequence behind 70 cached tokens; 45 sequences are more CTAs than the form with scores a tile ahead takes."""
+    rows, s_max = 130 * n_seq, 256
+    q = torch.randn(14, rows, 64, device="cuda", generator=_gen(7)).half()
+    k, v = (torch.randn(n_seq, 2, s_max, 64, device="cuda", generator=_gen(s)).half() for s in (8, 9))
+    table = torch.tensor([[130 * i for i in range(n_seq)], [130] * n_seq, list(range(n_seq)), [70] * n_seq], dtype=torch.int32,
+                         device="cuda")
+    return lambda: K.attn_prefill(q, k, v, table[0], table[1], table[2], 130, seq_off=table[3])
+
+
+CALLS = {
+    "w4a16, one wave": lambda: _linear(_packed(1152, 896), 64),
+    "w4a16, split K": lambda: _linear(_packed(896, 4864), 100),
+    "w4a16, two row tiles": lambda: _linear(_packed(9728, 896), 500),
+    "fp16": lambda: _linear(_dense(1152, 896), 64),
+    "fp16, split K": lambda: _linear(_dense(896, 4864), 20),
+    "pair": lambda: _linear(_dense(1152, 896), 700),
+    "pair, more tiles than pairs": lambda: _linear(_dense(9728, 896), 700),
+    "lm_head, 3 rows": lambda: _lm_head(3),
+    "lm_head, 128 rows": lambda: _lm_head(128),
+    "attention, ahead": lambda: _attention(1),
+    "attention": lambda: _attention(45),
+}
+
+
+# (limit, late): pauses of 0.6 ms a k block against limits of 1.5 and 0.3 ms; a first k block that never comes
+@pytest.mark.parametrize("name", list(CALLS))
+def test_late_operands(name):
+    call, lib = CALLS[name](), K.lib()
+
+    def run(limit, late):
+        lib.quic_w4a16_tensor_test_hook(limit, late)
+        try:
+            y = call().clone()
+        finally:
+            lib.quic_w4a16_tensor_test_hook(0, -1)
+        return y, lib.quic_w4a16_tensor_status()
+
+    want = call().clone()
+    assert lib.quic_w4a16_tensor_status() == 0
+    late, status = run(1500, -600)
+    assert status == 0 and torch.equal(late, want)
+    for limit, how in ((300, -600), (1500, 0)):
+        assert run(limit, how)[1] != 0
+        assert torch.equal(call(), want)
+        assert lib.quic_w4a16_tensor_status() == 0
