@@ -136,7 +136,7 @@ void quic_w4a16_tensor_test_hook(uint32_t wait_limit_us, int32_t skip_kblock);
  * kernel does when the step counter moved between request and wait.  2: never request the
  * first tile of a row and wait 20 ms at most, so that the bounded waits run out, the
  * kernel sets the error word read by quic_w4a16_tensor_status (code 5 or 6 in bits 16..,
- * bit 14 set) and returns.  0 restores the normal behaviour.  No reference counterpart. */
+ * bit 14 set) and returns.  3: both.  0 restores the normal behaviour.  No reference counterpart. */
 void quic_attn_stream_test_hook(int32_t mode);
 
 /* ------------------------------------------------------------------------

@@ -190,9 +190,10 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
   if (warp == kStreamWarps) {
     // ---------------- producer: one thread keeps the ring full ----------------
     if (lane == 0) {
-      int issued = pre;  // tiles requested so far
-      if (stale) {       // wait for the early copies to land, then fetch the same tiles again
-        for (int i = 0; i < pre; ++i) {
+      int issued = stale ? 0 : pre;  // tiles requested so far, but for early ones that are requested again
+      if (stale) {                   // wait for the early copies to land, then fetch the same tiles again
+        for (; issued < pre; ++issued) {
+          const int i = issued;
           const uint32_t full = smem_u32(&bar_full[i]), dst = base + i * kStageBytes;
           if (!mbar_wait(smem_u32(&bar_early[i]), 0, wait_limit_us)) {
             fail_s = 1;
@@ -219,6 +220,8 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
       // No copy may still be on its way into this CTA's shared memory when the CTA ends, whatever
       // became of its consumer: wait (with the usual bound) for the last copy into every stage.
       // In the normal course the consumers needed these phases anyway.
+      for (int i = 0; i < pre && stale; ++i)
+        if (!mbar_wait(smem_u32(&bar_early[i]), 0, wait_limit_us)) fail_s = 1;
       for (int i = issued > kStreamStages ? issued - kStreamStages : 0; i < issued; ++i) {
         const int s = i % kStreamStages;
         const bool early = i < pre && !stale;
@@ -298,7 +301,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
 
 // The cache planes must be the decode step's: [n_slots][2][s_max][64] fp16, 16-byte aligned.
 // a.s_cap bounds the tokens of a row; `status`: error word of the bounded waits.
-int g_stream_hook = 0;  // quic_attn_stream_test_hook: 1 repeat the early requests, 2 never request tile 0
+int g_stream_hook = 0;  // quic_attn_stream_test_hook: bit 0 repeat the early requests, bit 1 never request tile 0
 
 int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int n_slots, int s_max, int* status,
                        cudaStream_t stream, bool pdl) {
@@ -323,8 +326,8 @@ int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int 
   if (rc != QUIC_OK) return rc;
   QUIC_CUDA(allow_smem<attn_decode_stream_kernel>(kStreamSmem));
   QUIC_CUDA(launch(attn_decode_stream_kernel, dim3(kKvHeads, batch), dim3((kStreamWarps + 1) * 32), kStreamSmem, stream,
-                   pdl, tm_k, tm_v, a, fin, n_slots, s_max, status, g_stream_hook == 1 ? 1 : 0, g_stream_hook == 2 ? 1 : 0,
-                   g_stream_hook == 2 ? 20000u : kWaitLimitUs));
+                   pdl, tm_k, tm_v, a, fin, n_slots, s_max, status, g_stream_hook & 1, g_stream_hook >> 1,
+                   g_stream_hook & 2 ? 20000u : kWaitLimitUs));
   return QUIC_OK;
 }
 
@@ -334,5 +337,6 @@ int launch_attn_stream(const AttnArgs& a, const QkvFinish* fuse, int batch, int 
 // requests as made too early and repeats them, as it does when the step counter moved between the
 // request and the dependency wait.  2: the first tile of every row is never requested and the
 // waits last 20 ms at most, so the wait for that tile runs out, the other roles' waits
-// follow, the CTA sets the error word (code 5 or 6, bit 14) and returns; nothing faults.  0: normal.
-extern "C" void quic_attn_stream_test_hook(int32_t mode) { quic::g_stream_hook = (mode == 1 || mode == 2) ? mode : 0; }
+// follow, the CTA sets the error word (code 5 or 6, bit 14) and returns; nothing faults.  3: both, the wait for the early
+// copy of tile 0 runs out while those of the other tiles are on their way.  0: normal.
+extern "C" void quic_attn_stream_test_hook(int32_t mode) { quic::g_stream_hook = (mode >= 1 && mode <= 3) ? mode : 0; }

@@ -85,3 +85,26 @@ def test_late_operands(name):
         assert run(limit, how)[1] != 0
         assert torch.equal(call(), want)
         assert lib.quic_w4a16_tensor_status() == 0
+
+
+def test_an_early_tile_of_the_streamed_attention_that_never_lands(tiny_model):
+    """Tiles requested before the dependency wait that count as too early are requested again once the first copies have
+    landed.  Where that of the first tile never does, those of the others are on their way when the wait gives up."""
+    net, _, _, _ = tiny_model
+    lib, slots = K.lib(), list(range(24))
+    prompts = [torch.randint(0, 2048, (70 + 8 * i,), generator=torch.Generator().manual_seed(i)) for i in slots]
+
+    def decode():
+        cache = net.new_cache(n_slots=24, s_max=320)
+        net.prefill(cache, slots, prompts)
+        return net.decode(cache, slots, 2)
+
+    want = decode()
+    lib.quic_attn_stream_test_hook(3)
+    try:
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            decode()
+    finally:
+        lib.quic_attn_stream_test_hook(0)
+    assert decode() == want
+    assert lib.quic_w4a16_tensor_status() == 0
