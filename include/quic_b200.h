@@ -113,13 +113,20 @@ int quic_w4a16_linear(const void *x_f16, const quic_w4_t *w, void *y_f16,
                       void *stream);
 int64_t quic_w4a16_workspace_bytes(int32_t m, int32_t n, int32_t k);
 /* Error word of the tensor path: 0, or a non-zero code if a bounded wait inside
- * the tcgen05 kernel gave up since the last call (results are then invalid).
- * The word is taken (exchanged with zero on the device).  Synchronises the
- * device; quic_graph_run_host reads the same word together with the tokens,
- * without a synchronisation of its own, and returns QUIC_E_TIMEOUT when it is
- * set.  No reference counterpart (Marlin's lock spins are unbounded,
- * kernels/cuda/marlin.cu:1467-1476). */
+ * the tcgen05 kernels gave up since the last call (results are then invalid), in
+ * a call that reports here: stand-alone operators, quic_decode_step and
+ * quic_prefill.  The word is taken (exchanged with zero on the device).
+ * Synchronises the device.  No reference counterpart (Marlin's lock spins are
+ * unbounded, kernels/cuda/marlin.cu:1467-1476). */
 int quic_w4a16_tensor_status(void);
+/* Eight page-locked, zeroed int32 (NULL: none to be had) for the calls that report
+ * to words of their owner: two for quic_prefill_watch, two for
+ * quic_decode_graph_create_watch, one for quic_decode_persist_watch, written
+ * only when a wait gives up.  The host reads them whenever it has synchronised,
+ * and clears them.  Give them back when nothing that reports to them runs any
+ * more. */
+int32_t *quic_error_words_new(void);
+void quic_error_words_free(int32_t *words);
 /* Test hook for the bounded waits of the tcgen05 kernels (linears, lm_head,
  * prefill attention, the decode step's rows chain): in launches that follow a
  * wait lasts `wait_limit_us` microseconds at most (0: the default, two seconds)
@@ -135,7 +142,7 @@ void quic_w4a16_tensor_test_hook(uint32_t wait_limit_us, int32_t skip_kblock);
  * captures that follow.  1: repeat the tile requests made before the dependency wait, as the
  * kernel does when the step counter moved between request and wait.  2: never request the
  * first tile of a row and wait 20 ms at most, so that the bounded waits run out, the
- * kernel sets the error word read by quic_w4a16_tensor_status (code 5 or 6 in bits 16..,
+ * kernel sets an error word (code 5 or 6 in bits 16..,
  * bit 14 set) and returns.  3: both.  0 restores the normal behaviour.  No reference counterpart. */
 void quic_attn_stream_test_hook(int32_t mode);
 
@@ -379,6 +386,11 @@ typedef struct {
 } quic_prefill_t;
 int64_t quic_prefill_scratch_bytes(int32_t rows, int32_t n_seq, int32_t vocab);
 int quic_prefill(const quic_model_t *m, const quic_prefill_t *p, void *stream);
+/* The same, but its bounded waits report to two page-locked words of the caller
+ * (NULL: to quic_w4a16_tensor_status): when the call has run and one of them is
+ * not zero, what it wrote is invalid. */
+int quic_prefill_watch(const quic_model_t *m, const quic_prefill_t *p,
+                       int32_t *error_words, void *stream);
 
 /* Which form of the decode step a batch takes.  Batches of at least
  * quic_set_tensor_min_batch rows (default 16, range 2..17) run every linear on
@@ -408,13 +420,20 @@ int quic_decode_step(const quic_model_t *m, const quic_decode_t *d, void *stream
  * tokens, positions and the row->slot map are read from device memory. */
 int quic_decode_graph_create(const quic_model_t *m, const quic_decode_t *d,
                              int32_t steps, void *stream, void **graph_out);
+/* The same with page-locked error words of the caller, which it and
+ * quic_graph_run_host read (NULL: words of the graph's own, which
+ * quic_graph_run_host reads). */
+int quic_decode_graph_create_watch(const quic_model_t *m, const quic_decode_t *d,
+                                   int32_t steps, void *stream,
+                                   int32_t *error_words, void **graph_out);
 int quic_graph_launch(void *graph, void *stream);
 /* One host-driven call of a captured graph, the form the reference's token loop
  * has (src/engine.py:82-84 builds the next-token tensor on the host and copies
  * it to the device, src/engine.py:98-104 synchronises and reads the sampled ids
  * back with .tolist()): copies n_in int32 from host_in to dev_in (skipped when
  * n_in == 0), launches the graph, copies n_out int32 from dev_out to host_out
- * and waits for the stream.  Host buffers should be page-locked. */
+ * and waits for the stream.  QUIC_E_TIMEOUT if the graph's error words say that a
+ * bounded wait gave up (they are cleared).  Host buffers should be page-locked. */
 int quic_graph_run_host(void *graph, void *stream, const int32_t *host_in,
                         int32_t *dev_in, int32_t n_in, const int32_t *dev_out,
                         int32_t *host_out, int32_t n_out);
@@ -470,6 +489,11 @@ int quic_persist_pack(const quic_model_t *m, void *wstream_out, void *stream);
 int quic_decode_persist(const quic_model_t *m, const quic_decode_t *d,
                         const void *wstream, void *sync, int32_t steps,
                         void *stream);
+/* The same; a status that is not zero also goes to a page-locked word of the
+ * caller (NULL: none). */
+int quic_decode_persist_watch(const quic_model_t *m, const quic_decode_t *d,
+                              const void *wstream, void *sync, int32_t steps,
+                              void *stream, int32_t *host_status);
 int quic_decode_persist_status(void *sync, void *stream, int32_t *status_out);
 /* The host-driven form (compare quic_graph_run_host; src/engine.py:82-84,
  * 98-104): n_in int32 host -> device, the launch, n_out int32 and the status

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 2)
   flow_store(st, m_s[warp], l_s[warp], o_s[warp], lane);
   __syncthreads();
   if (fail_s != 0 && tid == 0)  // a bounded wait gave up: say so (the row's output is then invalid)
-    atomicCAS(status, 0, (7 << 16) | 0x4000 | ((int)blockIdx.z & 0x3fff));
+    tc_report(status, (7 << 16) | 0x4000 | ((int)blockIdx.z & 0x3fff));
   for (int idx = tid; idx < kGroupHeads * kHeadDim; idx += kFlowWarps * 32) {
     const int h = idx >> 6, d = idx & 63;
     float mx = -INFINITY, num = 0.f, den = 0.f;

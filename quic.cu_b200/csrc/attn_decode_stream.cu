@@ -271,7 +271,7 @@ __global__ void __launch_bounds__((kStreamWarps + 1) * 32, 1)
   if (warp < kStreamWarps) flow_store(st, m_s[warp], l_s[warp], o_s[warp], lane);
   __syncthreads();
   if (fail_s != 0) {  // a bounded wait gave up: say so, leave the row's output as it is
-    if (tid == 0) atomicCAS(status, 0, ((4 + fail_s) << 16) | 0x4000 | ((int)blockIdx.y & 0x3fff));
+    if (tid == 0) tc_report(status, ((4 + fail_s) << 16) | 0x4000 | ((int)blockIdx.y & 0x3fff));
     return;
   }
   // the warps' results -> the row's heads; thread -> (head, pair of dims), 224 of them

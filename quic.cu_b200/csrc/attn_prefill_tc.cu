@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kAttThreads, kAhead ? 2 : 4)
   tc_fence_before();
   __syncthreads();
   if (fail_s != 0) {
-    if (tid == 0) atomicCAS(status, 0, (fail_s << 16) | 0x2000 | ((int)blockIdx.z & 0x1fff));
+    if (tid == 0) tc_report(status, (fail_s << 16) | 0x2000 | ((int)blockIdx.z & 0x1fff));
     drain_failed(issuer, smem_u32(&bar_drain));
   }
   if (warp == 0)

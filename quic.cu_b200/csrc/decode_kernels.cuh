@@ -267,12 +267,17 @@ int w4a16_gemm_tc_swiglu(const half* x, const quic_w4_t& w, half* act, int m, cu
 bool lm_head_tc_supported(int batch, int vocab);
 int lm_head_tc_tiles(int vocab);
 int launch_lm_head_tc(const LmHeadArgs& a, cudaStream_t st);
-// Error words of the tcgen05 kernels ([0] GEMM, [1] lm_head; w4_gemm_tc.cu): device address,
-// an asynchronous copy to page-locked memory, and the value seen by that copy (taken, i.e.
-// exchanged with zero, when it is not 0).
+// Error words of the kernels with bounded waits ([0] linears and attention, [1] lm_head; w4_gemm_tc.cu).
 int* tc_status_words();
 void tc_test_hook(uint32_t* wait_limit_us, int32_t* skip_kblock);  // what quic_w4a16_tensor_test_hook last set
-int tc_status_poll_async(cudaStream_t st);
-int tc_status_polled(cudaStream_t st);
+// What this thread launches while the scope lasts reports to these page-locked words (nullptr: to the device's own).
+struct StatusScope {
+  explicit StatusScope(int32_t* host_words);
+  ~StatusScope();
+  StatusScope(const StatusScope&) = delete;
+  int* before;
+  bool ok = true;
+};
+int32_t error_words_take(int32_t* words);  // the first that is not zero; both are cleared
 
 }  // namespace quic

@@ -1610,6 +1610,13 @@ __device__ __forceinline__ void token_end(int step) {
   cbar();
 }
 
+// The status word goes to the host only where it says something: the host's word is zero before the launch, and one that nobody
+// waits for may be given back while the kernel runs.
+__device__ __forceinline__ void tell_host(const PersistArgs& a, const uint32_t* hdr) {
+  const int32_t status = (int32_t)ld_relaxed_u32(hdr + 1);
+  if (a.host_status != nullptr && status != 0) *a.host_status = status;
+}
+
 template <int MR, bool F16>
 __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constant__ PersistArgs a) {
   using L = SL<MR, F16>;
@@ -1624,7 +1631,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
   // after a wait that ran out the exchange area holds what it holds, until the status is read and the
   // area cleared by the host
   if (__syncthreads_or(tid == 0 && ld_relaxed_u32(hdr + 1) != 0u)) {
-    if (cta == 0 && tid == 0 && a.host_status != nullptr) *a.host_status = (int32_t)ld_relaxed_u32(hdr + 1);
+    if (cta == 0 && tid == 0) tell_host(a, hdr);
     return;
   }
   if (tid == 0) {
@@ -1724,7 +1731,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) {
       hdr[0] = sa.no0 + (uint32_t)(a.steps * a.n_layers);
-      if (a.host_status != nullptr) *a.host_status = (int32_t)ld_relaxed_u32(hdr + 1);
+      tell_host(a, hdr);
     }
     for (int i = threadIdx.x; i < a.n_out; i += kComp) a.host_out[i] = __ldcg(a.out_src + i);
   }
@@ -2084,7 +2091,15 @@ T* mapped(T* host) {
 
 extern "C" int quic_decode_persist(const quic_model_t* m, const quic_decode_t* d, const void* wstream, void* sync,
                                    int32_t steps, void* stream) {
-  return launch_persist(m, d, wstream, sync, steps, stream, HostIo());
+  return quic_decode_persist_watch(m, d, wstream, sync, steps, stream, nullptr);
+}
+
+extern "C" int quic_decode_persist_watch(const quic_model_t* m, const quic_decode_t* d, const void* wstream, void* sync,
+                                         int32_t steps, void* stream, int32_t* host_status) {
+  HostIo io;
+  io.status = mapped(host_status);
+  QUIC_REQUIRE(host_status == nullptr || io.status != nullptr, QUIC_E_ARG, "decode_persist: the status word is not page-locked");
+  return launch_persist(m, d, wstream, sync, steps, stream, io);
 }
 
 extern "C" int quic_decode_persist_status(void* sync, void* stream, int32_t* status_out) {
@@ -2128,6 +2143,7 @@ extern "C" int quic_decode_persist_run_host(const quic_model_t* m, const quic_de
     io.n_out = n_out;
   }
   io.status = status_dev;
+  *host_status = 0;
   const int rc = launch_persist(m, d, wstream, sync, steps, stream, io);
   if (rc != QUIC_OK) return rc;
   if (n_out > 0 && out_dev == nullptr)

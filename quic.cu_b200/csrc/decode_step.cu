@@ -655,7 +655,8 @@ int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cuda
 struct Graph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  bool tensor_kernels = false;  // the step holds kernels whose bounded waits report through error words
+  int32_t* words = nullptr;  // where its kernels' bounded waits report
+  bool own_words = false;
 };
 
 }  // namespace
@@ -706,8 +707,18 @@ extern "C" int quic_decode_step(const quic_model_t* m, const quic_decode_t* d, v
   return enqueue_step(m, d, (cudaStream_t)stream, true);
 }
 
-extern "C" int quic_decode_graph_create(const quic_model_t* m, const quic_decode_t* d,
-                                        int32_t steps, void* stream, void** graph_out) {
+extern "C" int quic_graph_destroy(void* graph) {
+  if (graph == nullptr) return QUIC_OK;
+  Graph* g = static_cast<Graph*>(graph);
+  if (g->exec) cudaGraphExecDestroy(g->exec);
+  if (g->graph) cudaGraphDestroy(g->graph);
+  if (g->own_words) quic_error_words_free(g->words);
+  delete g;
+  return QUIC_OK;
+}
+
+extern "C" int quic_decode_graph_create_watch(const quic_model_t* m, const quic_decode_t* d, int32_t steps, void* stream,
+                                              int32_t* error_words, void** graph_out) {
   int rc = check(m, d);
   if (rc != QUIC_OK) return rc;
   QUIC_REQUIRE(graph_out != nullptr && steps >= 1 && steps <= 4096, QUIC_E_ARG,
@@ -717,9 +728,16 @@ extern "C" int quic_decode_graph_create(const quic_model_t* m, const quic_decode
                "decode_graph_create: capture needs a non-default stream");
   Graph* g = new (std::nothrow) Graph();
   QUIC_REQUIRE(g != nullptr, QUIC_E_ARG, "decode_graph_create: out of host memory");
+  g->own_words = error_words == nullptr;
+  g->words = g->own_words ? quic_error_words_new() : error_words;
+  StatusScope scope(g->words);
+  if (g->words == nullptr || !scope.ok) {
+    quic_graph_destroy(g);
+    return fail(QUIC_E_CUDA, "decode_graph_create: no page-locked error words");
+  }
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) {
-    delete g;
+    quic_graph_destroy(g);
     return fail(QUIC_E_CUDA, cudaGetErrorString(e));
   }
   for (int s = 0; s < steps && rc == QUIC_OK; ++s) rc = enqueue_step(m, d, st, s == 0);
@@ -730,20 +748,17 @@ extern "C" int quic_decode_graph_create(const quic_model_t* m, const quic_decode
     if (e != cudaSuccess) rc = fail(QUIC_E_CUDA, cudaGetErrorString(e));
   }
   if (rc != QUIC_OK) {
-    if (g->graph) cudaGraphDestroy(g->graph);
-    delete g;
+    quic_graph_destroy(g);
     cudaGetLastError();
     return rc;
   }
-  const bool dense = m->layers[0].qkv.w16 != nullptr;
-  int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
-  if (ctx > d->s_max) ctx = d->s_max;
-  g->tensor_kernels = attention_form(d->batch, ctx) != kAttnCta ||
-                      (dense ? d->batch > kF16ChainMaxRows
-                             : (d->batch >= g_tensor_min_batch ||
-                                (d->batch >= g_mma_chain_min_batch && d->batch > 2 && lm_head_tc_supported(d->batch, m->vocab))));
   *graph_out = g;
   return QUIC_OK;
+}
+
+extern "C" int quic_decode_graph_create(const quic_model_t* m, const quic_decode_t* d,
+                                        int32_t steps, void* stream, void** graph_out) {
+  return quic_decode_graph_create_watch(m, d, steps, stream, nullptr, graph_out);
 }
 
 extern "C" int quic_graph_launch(void* graph, void* stream) {
@@ -767,29 +782,14 @@ extern "C" int quic_graph_run_host(void* graph, void* stream, const int32_t* hos
   QUIC_CUDA(cudaGraphLaunch(g->exec, st));
   if (n_out > 0)
     QUIC_CUDA(cudaMemcpyAsync(host_out, dev_out, sizeof(int32_t) * n_out, cudaMemcpyDeviceToHost, st));
-  // the error words of the kernels that wait on barriers ride along with the tokens (the GEMV and mma.sync
-  // chains hold none up to 4096 tokens: nothing to ask for)
-  if (g->tensor_kernels) {
-    const int rc = tc_status_poll_async(st);
-    if (rc != QUIC_OK) return rc;
-  }
   QUIC_CUDA(cudaStreamSynchronize(st));
-  const int word = g->tensor_kernels ? tc_status_polled(st) : 0;
+  const int32_t word = error_words_take(g->words);
   if (word != 0) {
-    static char msg[160];
+    char msg[160];
     snprintf(msg, sizeof(msg),
              "decode: a bounded wait of a tensor-core kernel gave up (status 0x%x); the tokens of this call are invalid",
-             word);
+             (unsigned)word);
     return fail(QUIC_E_TIMEOUT, msg);
   }
-  return QUIC_OK;
-}
-
-extern "C" int quic_graph_destroy(void* graph) {
-  if (graph == nullptr) return QUIC_OK;
-  Graph* g = static_cast<Graph*>(graph);
-  if (g->exec) cudaGraphExecDestroy(g->exec);
-  if (g->graph) cudaGraphDestroy(g->graph);
-  delete g;
   return QUIC_OK;
 }

@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kDenseThreads) gemm_f16_tc_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   if (fail_s != 0) {
-    if (tid == 0) atomicCAS(status, 0, (fail_s << 16) | 0x4000 | ((int)blockIdx.x & 0x3fff));
+    if (tid == 0) tc_report(status, (fail_s << 16) | 0x4000 | ((int)blockIdx.x & 0x3fff));
     drain_failed(issuer, smem_u32(&bar_drain));
   }
   if (warp == 0)

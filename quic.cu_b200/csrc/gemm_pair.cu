@@ -321,7 +321,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   __syncwarp();
   tc_fence_before();
   if (__syncthreads_or(fail_s)) {  // (the leader may set it at any time) the last MMAs and copies, as in drain_failed(); MMAs in flight that rank 0 has not waited for make it fail
-    if (tid == 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+    if (tid == 0) tc_report(a.status, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
     if (issuer) {
       pair_commit(smem_u32(&bar_drain));
       mbar_wait(smem_u32(&bar_drain), 0);

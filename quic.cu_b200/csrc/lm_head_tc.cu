@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kLmThreads) lm_head_tc_kernel(const __grid_con
   tc_fence_before();
   __syncthreads();
   if (fail_s != 0) {  // a bounded wait gave up: the tokens are invalid
-    if (tid == 0) atomicCAS(status, 0, (fail_s << 16) | 0x8000 | (tile & 0x7fff));
+    if (tid == 0) tc_report(status, (fail_s << 16) | 0x8000 | (tile & 0x7fff));
     drain_failed(issuer, smem_u32(&bar_drain));
   }
   if (warp == 0)

@@ -209,6 +209,10 @@ extern "C" int64_t quic_prefill_scratch_bytes(int32_t rows, int32_t n_seq, int32
 }
 
 extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void* stream) {
+  return quic_prefill_watch(m, p, nullptr, stream);
+}
+
+extern "C" int quic_prefill_watch(const quic_model_t* m, const quic_prefill_t* p, int32_t* error_words, void* stream) {
   QUIC_REQUIRE(m && p && m->layers && m->embed && m->final_norm && m->rope_cos && m->rope_sin, QUIC_E_ARG,
                "prefill: null model");
   QUIC_REQUIRE(p->ids && p->row_slot && p->row_pos && p->seq_start && p->seq_len && p->seq_slot && p->kv && p->tok &&
@@ -217,6 +221,8 @@ extern "C" int quic_prefill(const quic_model_t* m, const quic_prefill_t* p, void
   QUIC_REQUIRE(p->rows >= 1 && p->n_seq >= 1 && p->n_seq <= p->rows && p->n_seq <= 65535 && p->max_len >= 1 &&
                    p->max_len <= p->s_max && p->max_len <= m->max_pos && p->n_slots >= 1,
                QUIC_E_SHAPE, "prefill: bad row / sequence counts or a prompt longer than a KV slot");
+  const StatusScope scope(error_words);
+  QUIC_REQUIRE(scope.ok, QUIC_E_ARG, "prefill: the error words are not page-locked");
   cudaStream_t st = (cudaStream_t)stream;
   const int rows = p->rows;
   const PrefillArena ar = carve_prefill(rows, p->n_seq, m->vocab);

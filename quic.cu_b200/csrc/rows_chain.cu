@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   if (fail_s != 0) {
-    if (tid == 0) atomicCAS(a.status, 0, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+    if (tid == 0) tc_report(a.status, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
     drain_failed(issuer, smem_u32(&bar_drain));
   }
   if (warp == kWarpsC + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(C::cols) : "memory");

@@ -190,6 +190,11 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
+// Records that a wait gave up in an error word of the device or of page-locked host memory; an earlier record stays.
+__device__ __forceinline__ void tc_report(int* status, int code) {
+  volatile int* const word = status;
+  if (*word == 0) *word = code;
+}
 // The way out of a CTA in which a wait gave up: nobody may have waited for its last MMAs and copies, which use its shared memory
 // and its tensor memory.  All threads, after the barrier that every role has reached; `issuer`: the thread that issued
 // the MMAs; `bar`: a barrier for one arrival, not in use.  The MMAs are waited for; a copy, which waits for nothing, lands within

@@ -21,6 +21,9 @@
 // Split-K CTAs write fp32 partials that the consumer kernel (or a small finish kernel) sums;
 // the gate|up form applies SwiGLU in its epilogue.  Every mbarrier wait is bounded: on a
 // timeout the CTA records an error code, waits for its MMAs and copies in flight, frees its tensor memory and returns.
+#include <mutex>
+#include <vector>
+
 #include "tc_common.cuh"
 
 namespace quic {
@@ -28,9 +31,10 @@ namespace {
 
 constexpr int kHeadInts = 4096;  // reserved at the head of the split-K workspace
 
-// Error words of the tensor path: [0] the GEMM, [1] the tensor lm_head.  0 = ok; otherwise
-// (code << 16) | block of the first bounded wait that gave up.
+// Error words of the tensor path for calls that bring none of their own: [0] linears and attention, [1] the tensor
+// lm_head.  0 = ok; otherwise (code << 16) | block of a bounded wait that gave up.
 __device__ int g_tc_status[2];
+__device__ int g_tc_taken[2];
 
 // What a test may change for the launches that follow (quic_w4a16_tensor_test_hook): the limit
 // of the bounded waits and one k block whose packed weight tile the producer never requests.
@@ -42,6 +46,7 @@ struct GemmArgs {
   half* y;         // [m_total, N]    (splits == 1)
   float* part;     // [splits, m_total, N] fp32 (splits > 1)
   int m_total;
+  int* status;
   int kblocks_per_split;
   int mtl;     // batch-row tiles per CTA (2 from 129 rows up)
   uint32_t wait_limit_us;  // of a bounded wait
@@ -400,7 +405,7 @@ __global__ void __launch_bounds__(kGemmThreads) w4a16_gemm_tc_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   if (fail_s != 0) {
-    if (tid == 0) atomicCAS(&g_tc_status[0], 0, (fail_s << 16) | (int)blockIdx.x);
+    if (tid == 0) tc_report(a.status, (fail_s << 16) | (int)blockIdx.x);
     drain_failed(issuer, smem_u32(&bar_drain));
   }
   if (warp == 0)
@@ -468,6 +473,8 @@ int run_variant(const half* x, GemmArgs a, int splits, cudaStream_t st) {
 template <int MT>
 int run(const half* x, const GemmArgs& args, int splits, cudaStream_t st) {
   GemmArgs a = args;
+  a.status = tc_status_words();
+  QUIC_REQUIRE(a.status != nullptr, QUIC_E_CUDA, "w4a16_linear: no address for the tensor path's error words");
   a.wait_limit_us = g_wait_limit_us;
   a.skip_kblock = g_skip_kblock;
   if (a.mtl == 2) {
@@ -606,65 +613,91 @@ int w4a16_gemm_tc_swiglu(const half* x, const quic_w4_t& w, half* act, int m, cu
 
 namespace quic {
 namespace {
-__global__ void tc_status_take_kernel(int* out) {
-  out[0] = atomicExch(&g_tc_status[0], 0);
-  out[1] = atomicExch(&g_tc_status[1], 0);
+__global__ void tc_status_take_kernel() {
+  g_tc_taken[0] = atomicExch(&g_tc_status[0], 0);
+  g_tc_taken[1] = atomicExch(&g_tc_status[1], 0);
 }
-struct StatusHost {
-  int* words[16] = {};   // device address of g_tc_status per device
-  int* pinned = nullptr;  // two page-locked ints the status travels through
+int* g_status_address[16] = {};  // of g_tc_status, per device
+thread_local int* t_status_words = nullptr;
+
+// Page-locked error words, 128 times eight at a time.  Pages stay for the process; words that were given back are used again.
+constexpr int kWordsEach = 8, kWordsPage = 128;
+struct WordPool {
+  std::mutex mu;
+  std::vector<int32_t*> free;
 };
-StatusHost g_status_host;
+WordPool& word_pool() {
+  static WordPool* pool = new WordPool();  // (objects that give words back may outlive static destruction)
+  return *pool;
+}
 }  // namespace
 
-// Device address of the error words (index 1 is the tensor lm_head's).  Looks the symbol up on
-// first use per device: call it once outside any stream capture.
+// Device address of the error words of what this thread launches (index 1 is the tensor lm_head's): those of the call
+// (StatusScope), else the device's own.  Looks the symbol up on first use per device: call it once outside any stream capture.
 int* tc_status_words() {
+  if (t_status_words != nullptr) return t_status_words;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return nullptr;
-  if (g_status_host.words[dev] == nullptr)
-    if (cudaGetSymbolAddress(reinterpret_cast<void**>(&g_status_host.words[dev]), g_tc_status) != cudaSuccess)
+  if (g_status_address[dev] == nullptr)
+    if (cudaGetSymbolAddress(reinterpret_cast<void**>(&g_status_address[dev]), g_tc_status) != cudaSuccess)
       return nullptr;
-  return g_status_host.words[dev];
+  return g_status_address[dev];
+}
+StatusScope::StatusScope(int32_t* host_words) : before(t_status_words) {
+  void* p = nullptr;
+  if (host_words != nullptr) ok = cudaHostGetDevicePointer(&p, host_words, 0) == cudaSuccess;
+  if (!ok) (void)cudaGetLastError();
+  t_status_words = static_cast<int*>(p);
+}
+StatusScope::~StatusScope() { t_status_words = before; }
+
+int32_t error_words_take(int32_t* words) {
+  volatile int32_t* const w = words;
+  const int32_t v = w[0] != 0 ? w[0] : w[1];
+  if (v != 0) w[0] = w[1] = 0;
+  return v;
 }
 
 void tc_test_hook(uint32_t* wait_limit_us, int32_t* skip_kblock) {
   *wait_limit_us = g_wait_limit_us;
   *skip_kblock = g_skip_kblock;
 }
-
-// Enqueues a copy of the error words to page-locked host memory on `st`; tc_status_polled()
-// reads them once the stream has been synchronised.  Costs no synchronisation of its own.
-int tc_status_poll_async(cudaStream_t st) {
-  int* words = tc_status_words();
-  if (words == nullptr) return QUIC_OK;
-  if (g_status_host.pinned == nullptr)
-    QUIC_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&g_status_host.pinned), 2 * sizeof(int), cudaHostAllocDefault));
-  QUIC_CUDA(cudaMemcpyAsync(g_status_host.pinned, words, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  return QUIC_OK;
-}
-// After the stream of tc_status_poll_async is idle: 0, or the first non-zero word, which is then
-// taken (exchanged with zero on the device, so a word set meanwhile is not lost).
-int tc_status_polled(cudaStream_t st) {
-  if (g_status_host.pinned == nullptr) return 0;
-  const int v = g_status_host.pinned[0] ? g_status_host.pinned[0] : g_status_host.pinned[1];
-  if (v == 0) return 0;
-  tc_status_take_kernel<<<1, 1, 0, st>>>(g_status_host.pinned);  // page-locked memory is device-accessible (UVA)
-  cudaStreamSynchronize(st);
-  return v;
-}
 }  // namespace quic
 
-// Error word of the tensor path: 0, or (code << 16 | block) of the first bounded wait that gave
+extern "C" int32_t* quic_error_words_new(void) {
+  quic::WordPool& pool = quic::word_pool();
+  std::lock_guard<std::mutex> hold(pool.mu);
+  if (pool.free.empty()) {
+    int32_t* page = nullptr;
+    const unsigned flags = cudaHostAllocPortable | cudaHostAllocMapped;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&page), quic::kWordsPage * quic::kWordsEach * sizeof(int32_t), flags) != cudaSuccess) {
+      quic::set_error(cudaGetErrorString(cudaGetLastError()));
+      return nullptr;
+    }
+    for (int i = 0; i < quic::kWordsPage; ++i) pool.free.push_back(page + i * quic::kWordsEach);
+  }
+  int32_t* const words = pool.free.back();
+  pool.free.pop_back();
+  for (int i = 0; i < quic::kWordsEach; ++i) words[i] = 0;
+  return words;
+}
+extern "C" void quic_error_words_free(int32_t* words) {
+  if (words == nullptr) return;
+  quic::WordPool& pool = quic::word_pool();
+  std::lock_guard<std::mutex> hold(pool.mu);
+  pool.free.push_back(words);
+}
+
+// Error word of the calls that brought no words of their own: 0, or (code << 16 | block) of a bounded wait that gave
 // up since the last call (code 1: a weight tile never landed, 2: a ring stage never drained,
 // 3: operands or the accumulation never completed; bit 15 marks the tensor lm_head).  The word
 // is exchanged with zero on the device.  Synchronises the device.
 extern "C" int quic_w4a16_tensor_status(void) {
-  if (quic::tc_status_words() == nullptr) return -1;
+  int taken[2];
   if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-  if (quic::tc_status_poll_async(nullptr) != QUIC_OK) return -1;
-  if (cudaStreamSynchronize(nullptr) != cudaSuccess) return -1;
-  return quic::tc_status_polled(nullptr);
+  quic::tc_status_take_kernel<<<1, 1>>>();
+  if (cudaMemcpyFromSymbol(taken, quic::g_tc_taken, sizeof(taken)) != cudaSuccess) return -1;
+  return taken[0] != 0 ? taken[0] : taken[1];
 }
 
 // Test hook for the bounded waits of the tcgen05 GEMM: in launches that follow a wait gives up after

@@ -191,6 +191,8 @@ class Engine:
         if stream is not None:
             stream.synchronize()  # the slots are complete before any later decode launch
         first = first.tolist() if hasattr(first, "tolist") else list(first)
+        if hasattr(self.cache, "raise_errors"):
+            self.cache.raise_errors()  # (the prefill has run: its first tokens are here)
         complete, self.prefilling = [], []
         for seq, token, end in zip(sequences, first, done):
             if end >= seq.prompt_tokens.numel():

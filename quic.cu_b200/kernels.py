@@ -130,6 +130,8 @@ SIGNATURES = {
     "quic_w4a16_linear": (C.c_int, [_P, C.POINTER(W4), _P, _I32, _I32, _P, _P]),
     "quic_w4a16_workspace_bytes": (_I64, [_I32, _I32, _I32]),
     "quic_w4a16_tensor_status": (C.c_int, []),
+    "quic_error_words_new": (_P, []),
+    "quic_error_words_free": (None, [_P]),
     "quic_w4a16_tensor_test_hook": (None, [C.c_uint32, _I32]),
     "quic_attn_stream_test_hook": (None, [_I32]),
     "quic_rmsnorm": (C.c_int, [_P, _P, _P, _F, _P, _P, _I32, _P]),
@@ -160,7 +162,9 @@ SIGNATURES = {
     "quic_decode_step": (C.c_int, [C.POINTER(Model), C.POINTER(Decode), _P]),
     "quic_prefill_scratch_bytes": (_I64, [_I32, _I32, _I32]),
     "quic_prefill": (C.c_int, [C.POINTER(Model), C.POINTER(Prefill), _P]),
+    "quic_prefill_watch": (C.c_int, [C.POINTER(Model), C.POINTER(Prefill), _P, _P]),
     "quic_decode_graph_create": (C.c_int, [C.POINTER(Model), C.POINTER(Decode), _I32, _P, C.POINTER(_P)]),
+    "quic_decode_graph_create_watch": (C.c_int, [C.POINTER(Model), C.POINTER(Decode), _I32, _P, _P, C.POINTER(_P)]),
     "quic_graph_launch": (C.c_int, [_P, _P]),
     "quic_graph_run_host": (C.c_int, [_P, _P, _P, _P, C.c_int32, _P, _P, C.c_int32]),
     "quic_graph_destroy": (C.c_int, [_P]),
@@ -172,6 +176,7 @@ SIGNATURES = {
     "quic_persist_pick_splits": (_I32, [_I32, _I32]),
     "quic_persist_pack": (C.c_int, [C.POINTER(Model), _P, _P]),
     "quic_decode_persist": (C.c_int, [C.POINTER(Model), C.POINTER(Decode), _P, _P, _I32, _P]),
+    "quic_decode_persist_watch": (C.c_int, [C.POINTER(Model), C.POINTER(Decode), _P, _P, _I32, _P, _P]),
     "quic_decode_persist_status": (C.c_int, [_P, _P, C.POINTER(_I32)]),
     "quic_decode_persist_run_host": (C.c_int, [C.POINTER(Model), C.POINTER(Decode), _P, _P, _I32, _P, _P, _P, _I32,
                                                _P, _P, _I32, _P]),

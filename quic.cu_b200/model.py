@@ -72,6 +72,9 @@ class SlotCache:
         self._plans: dict[tuple, _DecodePlan] = {}  # decode(): per (rows, steps) launch plan
         self._rows_loaded: dict[int, torch.Tensor] = {}  # row->slot map now on the device, per batch size
         self.host_steps = 0                        # host mirror of step_counter
+        self._error_words = 0                      # address of page-locked words, where bounded waits that gave up report:
+        self._step_error = self._prefill_error = C.c_int64(0)  # two words each of captured steps and of prefills, as one number
+        self._persist_error = C.c_int32(0)                     # ... and that of the persistent kernel under decode_async()
 
     def check_slots(self, slots, count: int, what: str) -> None:
         """Every kernel indexes the KV planes and the per-slot state by slot: a slot outside
@@ -105,6 +108,30 @@ class SlotCache:
             self._scratch[key] = t
         return t
 
+    def error_words(self) -> int:
+        """Address of this cache's error words: captured steps +0, prefills +8, the persistent kernel +16."""
+        if not self._error_words:
+            at = K.lib().quic_error_words_new()
+            if not at:
+                raise RuntimeError(K.lib().quic_last_error().decode("utf-8", "replace"))
+            self._step_error, self._prefill_error = C.c_int64.from_address(at), C.c_int64.from_address(at + 8)
+            self._persist_error = C.c_int32.from_address(at + 16)
+            self._error_words = at
+        return self._error_words
+
+    def raise_errors(self) -> None:
+        """Raises if a bounded wait gave up in a prefill or step of this cache, as far as they have run: a caller who
+        has synchronised hears of all of them.  Reads page-locked memory and costs no synchronisation."""
+        for what, word in (("a prefill", self._prefill_error), ("a step", self._step_error), ("a step", self._persist_error)):
+            if word.value:
+                status = word.value & 0xffffffff or word.value >> 32
+                word.value = 0
+                if word is self._persist_error:  # (its exchange area is as the wait left it)
+                    K.check(K.lib().quic_decode_persist_status(K.ptr(self._persist_sync), K.stream_ptr(), C.byref(C.c_int32())),
+                            "decode_persist_status")
+                raise RuntimeError(f"quic_b200: a bounded wait of a kernel gave up (status 0x{status & 0xffffffff:x}) in {what} "
+                                   "of this cache: its results and the rows' cache entries are invalid")
+
     def persist_sync(self) -> torch.Tensor:
         """Exchange area of the persistent decode kernel (zeroed once)."""
         t = self.__dict__.get("_persist_sync")
@@ -134,6 +161,9 @@ class SlotCache:
     def __del__(self):
         try:
             self.release_graphs()
+            if self._error_words:
+                K.lib().quic_error_words_free(self._error_words)
+                self._error_words = 0
         except Exception:
             pass
 
@@ -352,6 +382,7 @@ class QUICForCausalLM:
             # a long-lived engine with ragged batches meets ever new (rows, context bound, steps):
             # start over rather than keep thousands of graphs and their scratch arenas
             torch.cuda.synchronize(self.device)
+            cache.raise_errors()
             cache.release_graphs()
         d, rows = self._decode_struct(cache, batch, ctx, logits)
         if g is None:
@@ -360,8 +391,8 @@ class QUICForCausalLM:
                 # ahead of a prefill that runs beside them on another stream
                 self._capture_stream = torch.cuda.Stream(device=self.device, priority=-1)
             out = C.c_void_p()
-            K.check(K.lib().quic_decode_graph_create(C.byref(self._c_model), C.byref(d), steps,
-                                                     self._capture_stream.cuda_stream, C.byref(out)),
+            K.check(K.lib().quic_decode_graph_create_watch(C.byref(self._c_model), C.byref(d), steps,
+                                                           self._capture_stream.cuda_stream, cache.error_words(), C.byref(out)),
                     "decode_graph_create")
             g = out.value
             cache._graphs[key] = g
@@ -436,7 +467,8 @@ class QUICForCausalLM:
 
     def decode_async(self, cache: SlotCache, slots: list[int], steps: int,
                      logits: torch.Tensor | None = None) -> int:
-        """Enqueues ``steps`` greedy decode steps for the rows ``slots`` (no host sync).
+        """Enqueues ``steps`` greedy decode steps for the rows ``slots`` (no host sync; ``SlotCache.raise_errors`` says
+        after one whether they are valid).
         Returns the ring index of the first generated token row in ``cache.out_tokens``."""
         g, first = self._prepare_decode(cache, slots, steps, logits)
         self._launch(cache, g, steps)
@@ -444,8 +476,9 @@ class QUICForCausalLM:
 
     def _launch(self, cache: SlotCache, handle, steps: int) -> None:
         if isinstance(handle, K.Decode):
-            K.check(K.lib().quic_decode_persist(C.byref(self._c_model), C.byref(handle), K.ptr(self.persist_stream()),
-                                                K.ptr(cache.persist_sync()), steps, K.stream_ptr()), "decode_persist")
+            K.check(K.lib().quic_decode_persist_watch(C.byref(self._c_model), C.byref(handle), K.ptr(self.persist_stream()),
+                                                      K.ptr(cache.persist_sync()), steps, K.stream_ptr(),
+                                                      cache.error_words() + 16), "decode_persist")
         else:
             K.check(K.lib().quic_graph_launch(handle, K.stream_ptr()), "graph_launch")
 
@@ -455,6 +488,7 @@ class QUICForCausalLM:
         out = C.c_int32(0)
         K.check(K.lib().quic_decode_persist_status(K.ptr(cache.persist_sync()), K.stream_ptr(), C.byref(out)),
                 "decode_persist_status")
+        cache._persist_error.value = 0
         return int(out.value)
 
     def decode(self, cache: SlotCache, slots: list[int], steps: int,
@@ -513,6 +547,8 @@ class QUICForCausalLM:
                                              plan.out + offset, plan.host + offset, count)
         if rc != 0:
             K.check(rc, "decode run_host")
+        if cache._prefill_error.value:  # (the rows' prompts may not have been waited for before)
+            cache.raise_errors()
         if steps == 1 and len(slots) == 1:
             return [[int(plan.host_np[first, slots[0]])]]
         rows = [(first + j) % ring for j in range(steps)] if wraps else slice(first, first + steps)
@@ -606,7 +642,8 @@ class QUICForCausalLM:
                       base + 12 * rows + 8 * n_seq, rows, n_seq, max(lens), K.ptr(cache.kv), cache.n_slots,
                       cache.s_max, K.ptr(cache.tok), K.ptr(cache.pos), K.ptr(first), K.ptr(logits), K.ptr(scratch),
                       base + 12 * rows + 12 * n_seq if any(offs) else None)
-        K.check(K.lib().quic_prefill(C.byref(self._c_model), C.byref(p), K.stream_ptr()), "prefill")
+        K.check(K.lib().quic_prefill_watch(C.byref(self._c_model), C.byref(p), cache.error_words() + 8, K.stream_ptr()),
+                "prefill")
         for s_, n, o in zip(slots, lens, offs):
             cache.host_len[s_] = o + n
         return first, logits
@@ -631,6 +668,7 @@ class QUICForCausalLM:
         if len(cache.batch_slots) != batch:
             raise ValueError(f"cache holds {len(cache.batch_slots)} rows, input has {batch}")
         cache.check_slots(cache.batch_slots, batch, "forward")
+        cache.raise_errors()  # of the call before, as far as it has run
         past_len = cache.get_seq_length()
         kv_len = past_len + seq_len
         input_ids = input_ids.to(self.device)

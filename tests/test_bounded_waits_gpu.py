@@ -108,3 +108,73 @@ def test_an_early_tile_of_the_streamed_attention_that_never_lands(tiny_model):
         lib.quic_attn_stream_test_hook(0)
     assert decode() == want
     assert lib.quic_w4a16_tensor_status() == 0
+
+
+def _prompts(count, length):
+    return [torch.randint(0, 2048, (length,), generator=torch.Generator().manual_seed(i)) for i in range(count)]
+
+
+class _Hook:
+    """Operands that never come, for what is launched or captured meanwhile."""
+
+    def __enter__(self):
+        K.lib().quic_w4a16_tensor_test_hook(2000, 0)
+
+    def __exit__(self, *_):
+        K.lib().quic_w4a16_tensor_test_hook(0, -1)
+
+
+@pytest.mark.parametrize("length", [40, 200])
+def test_a_prefill_that_gave_up_is_heard_of_by_its_own_cache(tiny_model, length):
+    """Both chains of a short prefill.  The error is raised where its results are first waited for: by raise_errors() after a
+    synchronisation, by the next decode() or forward() of the same cache; not by a decode() of another."""
+    net, slots = tiny_model[0], [0, 1]
+    good, bad = (net.new_cache(n_slots=2, s_max=256) for _ in range(2))
+    net.prefill(good, slots, _prompts(2, length))
+    for hears in ("decode", "forward", "raise_errors"):
+        with _Hook():
+            net.prefill(bad, slots, _prompts(2, length))
+        net.decode(good, slots, 2)
+        torch.cuda.synchronize()
+        good.raise_errors()
+        bad.batch_slots = slots
+        with pytest.raises(RuntimeError, match="bounded wait.*in a prefill"):
+            net.decode(bad, slots, 2) if hears == "decode" else bad.raise_errors() if hears == "raise_errors" else net(
+                torch.zeros(2, 1, dtype=torch.long), past_key_values=bad)
+        bad.raise_errors()  # (heard of once)
+    first, _ = net.prefill(bad, slots, _prompts(2, length))
+    again, _ = net.prefill(good, slots, _prompts(2, length))
+    assert torch.equal(first, again) and net.decode(bad, slots, 3) == net.decode(good, slots, 3)
+    assert K.lib().quic_w4a16_tensor_status() == 0
+
+
+def test_a_forward_step_that_gave_up_is_heard_of_by_the_next(tiny_model):
+    """forward() does not wait for its step: the next one raises, or raise_errors() after a synchronisation."""
+    net, rows = tiny_model[0], 20
+    ids = torch.stack(_prompts(rows, 30))
+    good, bad = net(ids).past_key_values, net(ids).past_key_values
+    token = torch.zeros(rows, 1, dtype=torch.long)
+    for hears in ("forward", "raise_errors"):
+        bad.release_graphs()
+        with _Hook():
+            net(token, past_key_values=bad)
+        torch.cuda.synchronize()
+        net.decode(good, good.batch_slots, 1)
+        with pytest.raises(RuntimeError, match="bounded wait.*in a step"):
+            net(token, past_key_values=bad) if hears == "forward" else bad.raise_errors()
+    assert K.lib().quic_w4a16_tensor_status() == 0
+
+
+def test_the_engine_hears_of_a_prefill_that_gave_up(tiny_model):
+    from types import SimpleNamespace
+
+    from quic_cu_b200.config import EngineConfig
+    from quic_cu_b200.engine import Engine
+
+    net = tiny_model[0]
+    engine = Engine(config=EngineConfig(batching="continuous", max_context=256, decode_burst=4), max_batch_size=4,
+                    model_module=SimpleNamespace(load=lambda **options: (net, None)))
+    engine.add_request_ids(_prompts(1, 60)[0], max_tokens=4)
+    with _Hook(), pytest.raises(RuntimeError, match="bounded wait.*in a prefill"):
+        engine.run()
+    assert K.lib().quic_w4a16_tensor_status() == 0
