@@ -181,6 +181,12 @@ def _ctx_bucket(n: int, batch: int = 1) -> int:
     return b
 
 
+def _persist_bound(n: int, batch: int) -> int:
+    """The bound that _persist_pays is asked about: multiples of 128 up to 4096, since its lines lie between 2048 and 4096
+    tokens too (two packed rows of 2100 are ahead on the persistent kernel, and no less so in a cache of 8192)."""
+    return (n + 127) // 128 * 128 if 2048 < n <= 4096 else _ctx_bucket(n, batch)
+
+
 class _DecodePlan:
     """What decode() keeps between calls for the same rows (see there)."""
 
@@ -451,7 +457,8 @@ class QUICForCausalLM:
         if longest + steps > cache.s_max or longest + steps > self.max_pos:
             raise RuntimeError("decode: context would exceed the KV slot length")
         ctx = min(_ctx_bucket(longest + steps, len(slots)), cache.s_max)
-        if (logits is None or steps == 1) and self.persist_ok(len(slots), ctx):  # (it keeps one step's logits)
+        near = min(_persist_bound(longest + steps, len(slots)), cache.s_max)
+        if (logits is None or steps == 1) and self.persist_ok(len(slots), near):  # (it keeps one step's logits)
             g, rows = self._decode_struct(cache, len(slots), ctx, logits, persist=True)
         else:
             g, rows = self._graph(cache, len(slots), ctx, steps, logits)
@@ -523,7 +530,8 @@ class QUICForCausalLM:
             handle, first = self._prepare_decode(cache, slots, steps, None)
             longest = max(host_len[s] for s in slots)  # already advanced by `steps`
             plan = _DecodePlan()
-            plan.bound = min(_ctx_bucket(longest, len(slots)), cache.s_max, self.max_pos)
+            bound = _persist_bound if isinstance(handle, K.Decode) else _ctx_bucket
+            plan.bound = min(bound(longest, len(slots)), cache.s_max, self.max_pos)
             plan.rows = cache.rows_tensor(slots)
             plan.tok = cache.tok.data_ptr() + 4 * slots[0]
             plan.out, plan.host, plan.host_np = cache.out_tokens.data_ptr(), cache.host_out().data_ptr(), cache.host_out().numpy()
