@@ -160,6 +160,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     fail_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();
+  // An allocation of the pair is made by both CTAs, and each takes part in the other's.  So both are known to run before either
+  // allocates, and neither leaves before both have given back: the next CTA on its SM, of another kernel and stream, may
+  // allocate by itself at once.  (Without, a pair beside decode steps on another stream stood still for good: the first CTA's
+  // allocation had returned, the second's never did.)
+  pair_sync();
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base_s)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -334,6 +340,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   }
   pair_sync();  // nobody leaves while the pair's copies, arrivals or MMAs use its shared memory
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_d) : "memory");
+  __syncwarp();
+  pair_sync();
 }
 
 template <int NT, bool kSwiglu, bool kRope = false>

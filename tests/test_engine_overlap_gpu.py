@@ -69,3 +69,38 @@ def test_steps_of_many_rows_beside_prefills_of_every_form(net, shortest, longest
     assert torch.equal(other.cache.kv, kv)
     assert serve(engine(False)) == tokens
     assert K.lib().quic_w4a16_tensor_status() == 0
+
+
+def test_prefills_on_sm_pairs_beside_decode_steps_keep_their_bits(net):
+    """Prefills of 770..1250 rows, eight launches on CTA pairs each, on one stream beside bursts of 62 rows on another of high
+    priority: one-CTA and two-CTA allocations of tensor memory take turns on every SM.  Every prefill leaves the bits that it
+    leaves alone."""
+    gen = torch.Generator().manual_seed(11)
+    lens = [(406, 773), (770,), (500, 300, 450), (1200,), (900, 33)]
+    prompts = [[torch.randint(0, 2048, (n,), generator=gen) for n in group] for group in lens]
+    rows = list(range(62))
+    cache = net.new_cache(n_slots=65, s_max=1280)
+    net.prefill(cache, rows, [torch.randint(0, 2048, (20 + i,), generator=gen) for i in rows])
+    want = []
+    for group in prompts:
+        first, logits = net.prefill(cache, [62, 63, 64][:len(group)], group)
+        want.append((first.clone(), logits.clone()))
+    tok, pos, length = cache.tok.clone(), cache.pos.clone(), list(cache.host_len)
+    alone = net.decode(cache, rows, 16)
+    main, side = torch.cuda.Stream(priority=-1), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for i in range(150):
+        with torch.cuda.stream(main):
+            cache.tok[:62].copy_(tok[:62])
+            cache.pos[:62].copy_(pos[:62])
+        cache.host_len[:62] = length[:62]
+        got = []
+        with torch.cuda.stream(side):
+            for group in prompts:
+                got.append(net.prefill(cache, [62, 63, 64][:len(group)], group))
+        with torch.cuda.stream(main):
+            assert net.decode(cache, rows, 16) == alone
+        side.synchronize()
+        cache.raise_errors()
+        for (first, logits), (first_alone, logits_alone) in zip(got, want):
+            assert torch.equal(first, first_alone) and torch.equal(logits, logits_alone)
