@@ -365,7 +365,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if ((tid & 7) == 0) {
           const int r = (tid >> 3) + i * (kConsumers / 8);
-          const float rs = rsqrtf(sum * (1.0f / kHidden) + a.eps), pw = __uint_as_float(__float_as_uint(rs) & 0x7f800000u);
+          // (at most 2^15, what fp16 holds: eps below 2^-32 lets rows of zeros and of its smallest values go beyond)
+          const float rs = rsqrtf(sum * (1.0f / kHidden) + a.eps), pw = fminf(__uint_as_float(__float_as_uint(rs) & 0x7f800000u), 32768.f);
           const half2 h = __float2half2_rn(pw);
           pow_s[r] = *reinterpret_cast<const uint32_t*>(&h);
           rest_s[r] = rs / pw;
@@ -389,8 +390,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     if constexpr (C::norm) {
       // ---------------- the rows' norm ----------------
-      // fp16(x * 2^e * w): 2^e * x is exact, and the rest of 1 / rms, 1 <= r < 2, is a factor of the row's sums in the
-      // epilogue.  One rounding, as fp16(x / rms * w) has, for two multiplies of pairs.
+      // fp16(x * 2^e * w), and the rest of 1 / rms, 1 <= r < 2, is a factor of the row's sums in the epilogue.  2^e * x is
+      // exact, so there is one rounding, as fp16(x / rms * w) has, for two multiplies of pairs.  (What lies below 2^-14 of
+      // the row's root mean square is rounded to fp16's subnormals first: up to 2^-25 (|w| + 1) r off, against the
+      // 2^-12 |w| of a value as large as the mean.)
       half2 pw[kRows];
 #pragma unroll
       for (int i = 0; i < kRows; ++i) pw[i] = u32_as_half2(pow_s[r0 + i * kRow]);

@@ -75,6 +75,28 @@ def test_rows_of_very_small_and_large_norm(nets):
         net.embed.copy_(embed)
 
 
+@pytest.mark.parametrize("weights", ["w4", "fp16"])
+def test_a_row_of_zeros_under_a_small_eps(nets, weights):
+    """eps 1e-12: 1 / rms of a row of zeros is 1e6, and of a row of fp16's smallest values 7.8e5, more than fp16 holds.  The
+    chain of a short prefill against the per-operator one, whose factor is in 32 bits."""
+    net = nets[weights]
+    embed, eps = net.embed.clone(), net.eps
+    try:
+        net.eps = net._c_model.eps = 1e-12
+        net.embed[0], net.embed[1] = 0, 2.0 ** -24
+        cache, other = (net.new_cache(n_slots=20, s_max=64) for _ in range(2))
+        prompts = [torch.tensor([i]) for i in range(20)]
+        net.prefill(cache, list(range(20)), prompts)
+        net.prefill(other, list(range(20)), prompts, all_logits=True)
+        got, want = cache.kv[0, :, :, :, 0].float(), other.kv[0, :, :, :, 0].float()
+        assert torch.isfinite(want).all()
+        worst = (norm(got - want, dim=(2, 3)) / norm(want, dim=(2, 3))).max().item()
+        assert worst < 2 * 3 ** 0.5 * 2 ** -12, worst  # three roundings on either side
+    finally:
+        net.embed.copy_(embed)
+        net.eps = net._c_model.eps = eps
+
+
 @pytest.mark.parametrize("weights,lens", [("w4", [2]), ("w4", [64]), ("w4", [40, 25]), ("w4", [128]), ("w4", [1] * 20), ("fp16", [3]),
                                           ("fp16", [65]), ("fp16", [129]), ("fp16", [200, 120])])
 def test_a_short_prefill_matches_the_operators_one_by_one(nets, weights, lens):
