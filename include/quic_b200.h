@@ -405,6 +405,10 @@ int quic_prefill_watch(const quic_model_t *m, const quic_prefill_t *p,
  * (Marlin picks its tile shapes per call, kernels/cuda/marlin.cu:3795-3805). */
 void quic_set_tensor_min_batch(int32_t batch);
 void quic_set_mma_chain_min_batch(int32_t batch);
+/* Attention kernel of a decode step of `batch` rows with a context bound of `ctx` tokens: CTAs of 512 tokens, merged in
+ * clusters; one CTA per (row, KV head); every row cut into equal ranges, a cluster each. */
+enum { QUIC_ATTN_CTA = 0, QUIC_ATTN_STREAM = 1, QUIC_ATTN_FLOW = 2 };
+int32_t quic_decode_attention_form(int32_t batch, int32_t ctx);
 /* Split count that sizes the decode step's scratch for `batch` rows whose contexts are
  * at most `ctx` tokens (pass the result as attn_splits and to the scratch size). */
 int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx);

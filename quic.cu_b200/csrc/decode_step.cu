@@ -143,7 +143,7 @@ constexpr int kRowsChainMaxRows = 128;
 //           CTA's walk.  Instead of cta: 16 x 3000 857 -> 814, 20 x 3500 1048 -> 841; instead of stream, from three ranges and 1536 tokens:
 //           24 x 2000 871 -> 812, 24 x 5000 1234 -> 1005, 37 x 3000 1010 -> 974 (24 x 900 would be 709 -> 734); and
 //           instead of splits merged in global memory, beyond 4096 tokens: 1 x 4200 462 -> 424, 5 x 7000 1140 -> 742, 15 x 8000 1624 -> 1008.
-enum AttnForm { kAttnCta, kAttnStream, kAttnFlow };
+enum AttnForm { kAttnCta = QUIC_ATTN_CTA, kAttnStream = QUIC_ATTN_STREAM, kAttnFlow = QUIC_ATTN_FLOW };
 constexpr int kCtaAttnMaxRows = 20, kStreamAnyCtxRows = 48, kFlowMinCtx = 1536;
 AttnForm attention_form(int batch, int ctx) {
   const int parts = attn_cta_splits(ctx);
@@ -152,9 +152,12 @@ AttnForm attention_form(int batch, int ctx) {
   return batch < kStreamAnyCtxRows && ctx > kFlowMinCtx && attn_flow_splits(batch, ctx) >= 3 ? kAttnFlow : kAttnStream;
 }
 
+static_assert(kRowsChainMaxRows + 1 >= kStreamAnyCtxRows, "steps that leave the QKV linear to the attention take the form that finishes it");
+
 // a: queries, cache, rows, positions, scale, output.  `fuse` (form stream only): the kernel finishes the QKV linear itself.
 int launch_attention(AttnArgs a, const quic_decode_t* d, int ctx, cudaStream_t st, const QkvFinish* fuse = nullptr) {
   const AttnForm form = attention_form(d->batch, ctx);
+  QUIC_REQUIRE(fuse == nullptr || form == kAttnStream, QUIC_E_ARG, "decode_step: only the streaming attention finishes the QKV linear");
   a.prefetch = d->step_counter != nullptr ? 1 : 0;
   if (form == kAttnCta) {
     a.splits = attn_cta_splits(ctx);
@@ -380,7 +383,7 @@ int enqueue_step_rows16(const quic_model_t* m, const quic_decode_t* d, cudaStrea
 // More than kRowsChainMaxRows rows: every linear is the tcgen05 GEMM, norms are
 // separate small kernels (at these sizes each kernel does microseconds of real work, so
 // the launch chain is no longer what bounds the step).
-// `fuse`: the attention kernel finishes the QKV linear itself (only where attention_streams()).
+// `fuse`: the attention kernel finishes the QKV linear itself (the streaming form, which every step of these takes).
 int enqueue_attention(const quic_decode_t* d, int ctx, half* qbuf, half* kc, half* vc, half* attn_out, cudaStream_t st,
                       const QkvFinish* fuse = nullptr);
 
@@ -473,7 +476,7 @@ int enqueue_attention(const quic_decode_t* d, int ctx, half* qbuf, half* kc, hal
 
 LmHeadArgs lm_head_args(const quic_model_t* m, const quic_decode_t* d, const Arena& ar);
 
-// 17..128 rows, un-quantised from 3: five launches a layer (rows_chain.cu).
+// 16..128 rows, un-quantised from 3: five launches a layer (rows_chain.cu).
 int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
   const int splits = pick_splits(d);
@@ -670,6 +673,10 @@ extern "C" void quic_set_tensor_min_batch(int32_t batch) {
 
 extern "C" void quic_set_mma_chain_min_batch(int32_t batch) {
   g_mma_chain_min_batch = batch < 2 ? 2 : (batch > kMmaChainMaxRows + 1 ? kMmaChainMaxRows + 1 : batch);
+}
+
+extern "C" int32_t quic_decode_attention_form(int32_t batch, int32_t ctx) {
+  return attention_form(batch < 1 ? 1 : batch, ctx < 1 ? 1 : ctx);
 }
 
 extern "C" int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx) {

@@ -156,6 +156,7 @@ SIGNATURES = {
     "quic_set_tensor_min_batch": (None, [_I32]),
     "quic_set_prefill_tensor_attention": (None, [C.c_int]),
     "quic_set_mma_chain_min_batch": (None, [_I32]),
+    "quic_decode_attention_form": (_I32, [_I32, _I32]),
     "quic_decode_pick_splits": (_I32, [_I32, _I32]),
     "quic_decode_scratch_bytes": (_I64, [_I32, _I32, _I32]),
     "quic_decode_launch_count": (_I32, [C.POINTER(Model), C.POINTER(Decode)]),
@@ -246,6 +247,7 @@ def _thread_scratch(key: tuple[str, int, int], need: int, least: int, head: int)
     return t
 
 
+ATTN_CTA, ATTN_STREAM, ATTN_FLOW = 0, 1, 2  # quic_decode_attention_form
 _HALF = torch.float16
 
 

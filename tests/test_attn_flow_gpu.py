@@ -73,14 +73,17 @@ def test_queries_at_an_odd_address_are_refused_where_they_are_read_in_pairs(rows
 
 @pytest.mark.parametrize("rows,longest", [(1, 4200), (2, 4161), (3, 4500), (9, 4097), (16, 3300), (17, 4200), (20, 3500), (21, 1990), (40, 2100)])
 def test_decode_steps_over_long_rows_match_a_prefill_of_the_same_tokens(tiny_model, rows, longest):
-    """The streaming attention inside a decode step (rows beyond 4096 tokens, more CTAs of 512 tokens than SMs, 21 rows and
-    more from three ranges on): what the step appends in the second layer went through its attention.  A prefill of
+    """The attention over ranges of a cluster inside a decode step (rows beyond 4096 tokens, more CTAs of 512 tokens than
+    SMs, 21 rows and more from three ranges on): what the step appends in the second layer went through its attention.  A prefill of
     prompt + token leaves the same there, up to the roundings to fp16 (34 of 2^-11 / sqrt(3), see test_rows_chain_gpu.py)."""
     from quic_cu_b200 import model as qmodel
 
     _, _, state, config = tiny_model
     state = {k: v * 0.25 if k.endswith("weight_scale") else v for k, v in state.items()}
     net = qmodel.from_state_dict(state, config)
+    net.use_persist = False
+    bound = min(qmodel._ctx_bucket(longest + 1, rows), 4608)
+    assert kernels.lib().quic_decode_attention_form(rows, bound) == kernels.ATTN_FLOW
     gen = torch.Generator().manual_seed(rows)
     lens = torch.randint(1, longest, (rows,), generator=gen).tolist()
     lens[0] = longest

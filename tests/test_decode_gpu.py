@@ -222,9 +222,8 @@ def test_batched_rows_are_independent(tiny_model):
 
 @pytest.mark.parametrize("prompt_len,steps", [(1100, 5), (2043, 9)])
 def test_single_row_decode_beyond_1024_tokens(tiny_model, prompt_len, steps):
-    """One row at 1025..2048 tokens of context runs the single-warp attention kernel with 17..32
-    splits, which the o_proj kernel merges in two passes of loads; the second case also crosses
-    2048 tokens, where the throughput kernel takes over."""
+    """One row at 1025..2048 tokens of context: the attention is a cluster of three or four CTAs of 512 tokens for each KV
+    head; the second case crosses 2048 tokens, where it becomes one of five."""
     net, ref, _, _ = tiny_model
     prompt = torch.randint(0, 2048, (prompt_len,), generator=torch.Generator().manual_seed(prompt_len)).tolist()
     ref_tokens, ref_logits = ref.greedy(prompt, steps)
@@ -248,9 +247,8 @@ def test_single_row_decode_beyond_1024_tokens(tiny_model, prompt_len, steps):
 
 
 def test_single_row_long_context_matches_the_batched_step(tiny_model):
-    """Beyond 2048 tokens one row runs the throughput attention kernel with up to 64 splits that
-    the o_proj kernel merges in passes of 16; four rows run the tensor-core step, whose splits
-    the last CTA merges.  Same prompt, same fed tokens: the logits of the two must agree."""
+    """One row of 4300 tokens runs the GEMV chain, four rows the mma.sync chain; the attention of either cuts a row into
+    ranges of a cluster.  Same prompt, same fed tokens: the logits of the two must agree."""
     net, _, _, _ = tiny_model
     gen = torch.Generator().manual_seed(77)
     prompt = torch.randint(0, 2048, (4300,), generator=gen)
@@ -280,10 +278,10 @@ def test_single_row_long_context_matches_the_batched_step(tiny_model):
 
 
 @pytest.mark.parametrize("repeat_early_requests", [False, True])
-def test_many_ragged_rows_streamed_attention_matches_the_small_batch_chain(tiny_model, repeat_early_requests):
-    """24 rows of 5..1900 tokens in one tensor-core step: from 21 rows on, up to 2048 tokens of
-    context, a CTA per (row, KV head) streams the row's cache through an eight-stage ring (rows
-    beyond 512 tokens wrap it, the longest four times) and four warps keep running softmaxes.
+def test_many_ragged_rows_streamed_attention_matches_the_small_batch_chain(tiny_model, monkeypatch,
+                                                                                       repeat_early_requests):
+    """24 rows of 1..1530 tokens in one step: up to 1536 tokens of context a CTA per (row, KV head) streams the row's cache
+    through a twelve-stage ring (rows beyond 768 tokens wrap it) and four warps keep running softmaxes.
     The same rows as two batches of 12 run the mma.sync chain with the cluster attention; fed the
     same tokens, the logits of the two must agree.  Second form: the kernel repeats the tile requests
     it made before the dependency wait (its path for a step counter that moved meanwhile)."""
@@ -291,14 +289,16 @@ def test_many_ragged_rows_streamed_attention_matches_the_small_batch_chain(tiny_
 
     net, _, _, _ = tiny_model
     gen = torch.Generator().manual_seed(79)
-    lens = [5, 63, 64, 65, 127, 128, 129, 300, 511, 512, 513, 700, 1023, 1024, 1025, 1300, 1536, 1700, 1900, 1, 2,
-            450, 900, 33]
+    lens = [5, 63, 64, 65, 127, 128, 129, 300, 511, 512, 513, 700, 767, 768, 769, 832, 1023, 1024, 1025, 1530, 1, 2, 450, 1300]
     prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
     steps = 3
+    form = K.lib().quic_decode_attention_form
+    assert (form(24, 1536), form(12, 1536)) == (K.ATTN_STREAM, K.ATTN_CTA)
 
-    halves = net.new_cache(n_slots=24, s_max=2048)
+    halves = net.new_cache(n_slots=24, s_max=1536)
     firsts, _ = net.prefill(halves, list(range(24)), prompts)
     fed, chain = [firsts.view(24, 1).clone()], []
+    monkeypatch.setattr(net, "use_persist", False)
     for _ in range(steps):
         rows = []
         for lo in (0, 12):
@@ -307,7 +307,7 @@ def test_many_ragged_rows_streamed_attention_matches_the_small_batch_chain(tiny_
         chain.append(torch.cat(rows))
         fed.append(chain[-1].argmax(dim=-1, keepdim=True))
 
-    whole = net.new_cache(n_slots=24, s_max=2048)
+    whole = net.new_cache(n_slots=24, s_max=1536)
     firsts24, _ = net.prefill(whole, list(range(24)), prompts)
     assert firsts24.tolist() == firsts.tolist()
     whole.batch_slots = list(range(24))
@@ -320,41 +320,40 @@ def test_many_ragged_rows_streamed_attention_matches_the_small_batch_chain(tiny_
         torch.cuda.synchronize()
     finally:
         K.lib().quic_attn_stream_test_hook(0)
+    whole.raise_errors()
     assert K.lib().quic_w4a16_tensor_status() == 0
 
 
-def test_many_rows_beyond_2048_tokens_streamed_attention_matches_the_split_kernel(tiny_model):
-    """22 rows, one of 4300 tokens: the streamed attention walks 68 tiles of that row through its
-    twelve-stage ring.  The same rows as two batches of 11 run the mma.sync chain, whose attention
-    beyond 4096 tokens is the split kernel; fed the same tokens, the logits must agree."""
+@pytest.mark.parametrize("rows", [22, 48])
+def test_many_rows_beyond_2048_tokens_match_the_operators_one_by_one(tiny_model, rows):
+    """One of the rows has 4300 tokens.  22 rows: every row is cut into ranges of a cluster; 48: one CTA walks the 68 tiles of
+    that row through its twelve-stage ring.  The logits of two steps against those of a per-operator prefill of the
+    same tokens."""
+    from quic_cu_b200 import kernels as K
+
     net, _, _, _ = tiny_model
+    assert K.lib().quic_decode_attention_form(rows, 4608) == (K.ATTN_FLOW if rows == 22 else K.ATTN_STREAM)
     gen = torch.Generator().manual_seed(80)
-    lens = [4300, 2049, 2048, 3000] + [17 * (i + 1) for i in range(18)]
+    lens = [4300, 2049, 2048, 3000] + [17 * (i + 1) for i in range(rows - 4)]
     prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in lens]
-    halves = net.new_cache(n_slots=22, s_max=4608)
-    firsts, _ = net.prefill(halves, list(range(22)), prompts)
-    fed, chain = [firsts.view(22, 1).clone()], []
+    slots = list(range(rows))
+    cache, other = (net.new_cache(n_slots=rows, s_max=4608) for _ in range(2))
+    first, _ = net.prefill(cache, slots, prompts)
+    cache.batch_slots, fed, steps = slots, [first.view(rows, 1).clone()], []
     for _ in range(2):
-        rows = []
-        for lo in (0, 11):
-            halves.batch_slots = list(range(lo, lo + 11))
-            rows.append(net(fed[-1][lo:lo + 11], past_key_values=halves).logits[:, 0].clone())
-        chain.append(torch.cat(rows))
-        fed.append(chain[-1].argmax(dim=-1, keepdim=True))
-    whole = net.new_cache(n_slots=22, s_max=4608)
-    firsts22, _ = net.prefill(whole, list(range(22)), prompts)
-    assert firsts22.tolist() == firsts.tolist()
-    whole.batch_slots = list(range(22))
+        steps.append(net(fed[-1], past_key_values=cache).logits[:, 0].clone())
+        fed.append(steps[-1].argmax(dim=-1, keepdim=True))
+    both = torch.cat(fed[:2], 1).cpu()
+    _, logits = net.prefill(other, slots, [torch.cat([p, both[i]]) for i, p in enumerate(prompts)], all_logits=True)
+    end = torch.tensor([n + 2 for n in lens]).cumsum(0)
     for i in range(2):
-        logits = net(fed[i], past_key_values=whole).logits[:, 0]
-        ok, err = _close(logits, chain[i])
+        ok, err = _close(steps[i], logits.view(-1, 2048)[end - 2 + i])
         assert ok, (i, err)
 
 
 def test_three_ragged_rows_long_context_match_the_batched_step(tiny_model):
-    """Three rows of 4300 / 40 / 2500 tokens on the GEMV chain (3-row kernels, throughput
-    attention kernel, splits without tokens for the short rows, o_proj merging 64 splits)
-    against the same rows inside a 4-row tensor-core step, fed the same tokens."""
+    """Three rows of 4300 / 40 / 2500 tokens (attention over ranges of a cluster, most of them without tokens for the short
+    row) against the same rows inside a step of four, fed the same tokens."""
     net, _, _, _ = tiny_model
     gen = torch.Generator().manual_seed(78)
     prompts = [torch.randint(0, 2048, (n,), generator=gen) for n in (4300, 40, 2500, 900)]

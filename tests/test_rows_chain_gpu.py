@@ -1,5 +1,5 @@
-"""The decode step of 17..128 rows (un-quantised from 3): one launch per linear with norm, RoPE + KV
-append, residual or SwiGLU inside, `down` over clusters of eight CTAs."""
+"""The decode step of 16..128 rows (un-quantised from 3): one launch per linear with norm, RoPE + KV
+append, residual or SwiGLU inside, `down` over clusters of eight CTAs; and the step of more rows, a GEMM per linear."""
 
 import pytest
 import torch
@@ -23,9 +23,10 @@ def nets(tiny_model):
             "fp16": qmodel.from_state_dict(synthetic_dense_checkpoint(n_layers=2, vocab=2048, seed=99), config)}
 
 
-@pytest.mark.parametrize("weights,rows", [("w4", n) for n in (17, 63, 64, 65, 127, 128)] + [("fp16", n) for n in (3, 16, 64, 65, 128)])
-def test_appended_keys_and_values_match_a_prefill_of_the_same_tokens(nets, weights, rows):
-    """Edges of the row tiles (64, 128) and of what the path takes.  A step appends K and V of the token it feeds
+@pytest.mark.parametrize("weights,rows", [("w4", n) for n in (16, 17, 63, 64, 65, 127, 128, 129, 201)] +
+                         [("fp16", n) for n in (3, 16, 64, 65, 128, 129, 201)])
+def test_appended_keys_and_values_match_a_prefill_of_the_same_tokens(nets, monkeypatch, weights, rows):
+    """Edges of the row tiles (64, 128) and of what the path takes (beyond: GEMMs, the attention finishes the QKV linear).  A step appends K and V of the token it feeds
     in every layer; a prefill of prompt + token, other kernels, has to leave the same there.  On the way to K and V of
     the second layer lie 17 roundings to fp16 (two norms and the third, four linears with their sums, bias, rotation,
     probabilities, activation), each 2^-11 / sqrt(3) in the root mean square, on either side; the worst of up to
@@ -33,6 +34,7 @@ def test_appended_keys_and_values_match_a_prefill_of_the_same_tokens(nets, weigh
     from quic_cu_b200 import kernels as K
 
     net = nets[weights]
+    monkeypatch.setattr(net, "use_persist", False)
     gen = torch.Generator().manual_seed(rows)
     lens = torch.randint(8, 90, (rows,), generator=gen).tolist()
     lens[0] = 300  # (more rows in the prefills than any of the forms under test takes)
@@ -40,6 +42,8 @@ def test_appended_keys_and_values_match_a_prefill_of_the_same_tokens(nets, weigh
     slots = torch.randperm(rows + 2, generator=gen)[:rows].tolist()  # rows need not sit in slot order, nor fill the cache
     cache, other = (net.new_cache(n_slots=rows + 2, s_max=320) for _ in range(2))
     first, _ = net.prefill(cache, slots, prompts)
+    per_layer = 5 if rows <= 128 else 7 if weights == "w4" else 8
+    assert net.launches_per_step(cache, rows, 320) == per_layer * net.n_layers + 3
     idle = [s for s in range(rows + 2) if s not in slots]
     before = cache.kv[:, :, idle].clone()
     net.decode(cache, slots, 1)
@@ -54,25 +58,47 @@ def test_appended_keys_and_values_match_a_prefill_of_the_same_tokens(nets, weigh
 
 def test_rows_of_very_small_and_large_norm(nets):
     """The rows' factors are a power of two, applied before the product, and a rest of 1 to 2, after it: rows far from 1 in
-    size must come out as a norm in 32 bits gives them."""
+    size must come out as a norm in 32 bits gives them, that of the per-operator prefill.  In the decode step and in a
+    short prefill."""
     net = nets["w4"]
     embed = net.embed.clone()
     try:
         scale = torch.tensor([2.0 ** -14, 2.0 ** -7, 1.0, 37.0, 1500.0], device="cuda", dtype=torch.float32)
         net.embed[:40] = (embed[:40].float().sign() * scale.repeat(8).view(40, 1) *
                           (0.5 + torch.rand(40, 896, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)))).half()
-        ids = torch.arange(40).view(40, 1)
-        cache, other = (net.new_cache(n_slots=40, s_max=64) for _ in range(2))
-        for c in (cache, other):
-            net.prefill(c, list(range(40)), [torch.tensor([5])] * 40)
-        cache.tok.copy_(ids.view(-1))
-        net.decode(cache, list(range(40)), 1)
-        net.prefill(other, list(range(40)), list(ids), offsets=[1] * 40)
-        got, want = cache.kv[0, :, :, :, 1].float(), other.kv[0, :, :, :, 1].float()
-        worst = (norm(got - want, dim=(2, 3)) / norm(want, dim=(2, 3))).max().item()
-        assert worst < 2 * 3 ** 0.5 * 2 ** -12, worst  # three roundings on either side
+        ids, slots = torch.arange(40).view(40, 1), list(range(40))
+        step, short, other = (net.new_cache(n_slots=40, s_max=64) for _ in range(3))
+        for c in (step, short, other):
+            net.prefill(c, slots, [torch.tensor([5])] * 40)
+        step.tok.copy_(ids.view(-1))
+        net.decode(step, slots, 1)
+        net.prefill(short, slots, list(ids), offsets=[1] * 40)
+        net.prefill(other, slots, list(ids), offsets=[1] * 40, all_logits=True)
+        want = other.kv[0, :, :, :, 1].float()
+        for c in (step, short):
+            got = c.kv[0, :, :, :, 1].float()
+            worst = (norm(got - want, dim=(2, 3)) / norm(want, dim=(2, 3))).max().item()
+            assert worst < 2 * 3 ** 0.5 * 2 ** -12, worst  # three roundings on either side
     finally:
         net.embed.copy_(embed)
+
+
+def test_a_row_with_an_infinity(nets):
+    """Its keys and values are NaN, as the per-operator prefill leaves them; the other rows keep their bits."""
+    net, prompts, slots = nets["w4"], [torch.tensor([i]) for i in range(20)], list(range(20))
+    clean, spoilt, other = (net.new_cache(n_slots=20, s_max=64) for _ in range(3))
+    net.prefill(clean, slots, prompts)
+    before = net.embed[7, 100].clone()
+    try:
+        net.embed[7, 100] = float("inf")
+        net.prefill(spoilt, slots, prompts)
+        net.prefill(other, slots, prompts, all_logits=True)
+    finally:
+        net.embed[7, 100] = before
+    for c in (spoilt, other):
+        assert torch.isnan(c.kv[:, :, 7, :, 0]).all()
+    others = [i for i in slots if i != 7]
+    assert torch.equal(spoilt.kv[:, :, others], clean.kv[:, :, others])
 
 
 @pytest.mark.parametrize("weights", ["w4", "fp16"])
@@ -176,3 +202,19 @@ def test_stages_that_come_late_and_too_late(nets, weights, rows):
     again = step(0, -1)
     assert again[0] == tokens and torch.equal(again[1], kv)
     assert lib.quic_w4a16_tensor_status() == 0
+
+
+@pytest.mark.parametrize("weights,length", [("w4", 300), ("fp16", 400)])
+def test_chunks_on_the_chain_agree_with_a_whole_prompt_on_the_gemms(nets, weights, length):
+    """Chunks of 100 tokens run the chain, the whole prompt the GEMMs: other sums, so not the same bits, but the same up to the
+    roundings (as above)."""
+    net = nets[weights]
+    prompt = torch.randint(0, 2048, (length,), generator=torch.Generator().manual_seed(length))
+    whole, cache = (net.new_cache(n_slots=1, s_max=448) for _ in range(2))
+    _, want = net.prefill(whole, [0], [prompt])
+    for at in range(0, length, 100):
+        _, got = net.prefill(cache, [0], [prompt[at:at + 100]], offsets=[at])
+    assert (norm(got.float() - want.float()) / norm(want.float())).item() < 2 * (40 / 3) ** 0.5 * 2 ** -11
+    a, b = cache.kv[:, :, 0, :, :length].float(), whole.kv[:, :, 0, :, :length].float()
+    worst = (norm(a - b, dim=(2, 4)) / norm(b, dim=(2, 4))).max().item()
+    assert worst < 2 * (34 / 3) ** 0.5 * 2 ** -11, worst
