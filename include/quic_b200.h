@@ -409,8 +409,8 @@ void quic_set_mma_chain_min_batch(int32_t batch);
  * clusters; one CTA per (row, KV head); every row cut into equal ranges, a cluster each. */
 enum { QUIC_ATTN_CTA = 0, QUIC_ATTN_STREAM = 1, QUIC_ATTN_FLOW = 2 };
 int32_t quic_decode_attention_form(int32_t batch, int32_t ctx);
-/* Split count that sizes the decode step's scratch for `batch` rows whose contexts are
- * at most `ctx` tokens (pass the result as attn_splits and to the scratch size). */
+/* Ranges of `ctx` tokens that a merge in global memory would use.  No decode step has one any more: the scratch is a
+ * matter of the batch, whatever the splits given here (at least 1) and in quic_decode_t. */
 int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx);
 int64_t quic_decode_scratch_bytes(int32_t batch, int32_t vocab, int32_t attn_splits);
 /* Number of kernels one quic_decode_step launches. */

@@ -17,8 +17,7 @@ namespace {
 inline int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
 
 struct Arena {
-  int64_t lm_counter, attn, xres, qbuf, attn_out, act, partial, best_val, best_idx, total;
-  // batched step (batch > kMaxM) only
+  int64_t lm_counter, xres, qbuf, attn_out, act, partial, best_val, best_idx, total;
   int64_t xn, qkv, gu, act16, tcws;
 };
 
@@ -39,24 +38,27 @@ int64_t tc_workspace_bytes(int batch) {
   return w;
 }
 
-// The regions that must start zeroed (arrival counters) come first.
-Arena carve(int batch, int vocab, int splits) {
+// Rows that the chain of rows_chain.cu serves (from g_tensor_min_batch, un-quantised from kF16ChainMaxRows + 1 rows):
+// one tile of 128 on the M side of its MMAs.
+constexpr int kRowsChainMaxRows = 128;
+
+// What the forms that a batch can take ask for.  The regions that must start zeroed (arrival counters) come first.
+Arena carve(int batch, int vocab) {
   Arena a;
   int64_t off = 0;
   a.lm_counter = off;  // arrival counter, then the lm_head's per-row maxima (up to 128 rows)
   off += 256 + 128 * 8;
-  a.attn = off;
-  off += align256(quic_attn_scratch_bytes(batch, splits));
   a.xres = off;
   off += align256((int64_t)2 * batch * kHidden * 2);
   a.qbuf = off;
   off += align256((int64_t)batch * kHidden * 2);
   a.attn_out = off;
   off += align256((int64_t)batch * kHidden * 2);
-  a.act = off;
-  off += align256((int64_t)4 * batch * kInter * 4);
+  const bool few = batch <= kMmaChainMaxRows, gemms = batch > kRowsChainMaxRows;
+  a.act = off;  // partial sums of gate|up, or sums of squares: of the mma.sync chain, of the rows chain
+  off += align256((int64_t)batch * (few ? 4 * kInter * 4 : 2 * kRowsSsq * 4));
   a.partial = off;
-  off += align256((int64_t)kDownSplits * batch * kHidden * 4);
+  if (few) off += align256((int64_t)kDownSplits * batch * kHidden * 4);
   int grid = lm_head_grid(vocab);
   if (lm_head_tc_supported(batch, vocab) && lm_head_tc_tiles(vocab) > grid) grid = lm_head_tc_tiles(vocab);
   a.best_val = off;
@@ -64,27 +66,22 @@ Arena carve(int batch, int vocab, int splits) {
   a.best_idx = off;
   off += align256((int64_t)batch * grid * 4);
   a.xn = a.qkv = a.gu = a.act16 = a.tcws = off;
-  if (batch >= 2) {  // the tensor-core step may be selected from batch 2 upwards
+  if (batch >= 2) {  // the mma.sync and rows chains may be selected from batch 2 upwards
     a.xn = off;
     off += align256((int64_t)batch * kHidden * 2);
+    a.act16 = off;
+    off += align256((int64_t)batch * kInter * 2);
+  }
+  if (gemms) {
     a.qkv = off;
     off += align256((int64_t)batch * kQkvN * 2);
     a.gu = off;
     off += align256((int64_t)batch * 2 * kInter * 2);
-    a.act16 = off;
-    off += align256((int64_t)batch * kInter * 2);
     a.tcws = off;
     off += align256(16384 + tc_workspace_bytes(batch));
   }
   a.total = off;
   return a;
-}
-
-int pick_splits(const quic_decode_t* d) {
-  if (d->attn_splits > 0) return d->attn_splits;
-  int ctx = d->ctx_hint > 0 ? d->ctx_hint : d->s_max;
-  if (ctx > d->s_max) ctx = d->s_max;
-  return quic_decode_pick_splits(d->batch, ctx);
 }
 
 int check(const quic_model_t* m, const quic_decode_t* d) {
@@ -130,10 +127,6 @@ int enqueue_step_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t
 int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head);
 
 int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head);
-
-// Rows that the chain of rows_chain.cu serves (from g_tensor_min_batch, un-quantised from kF16ChainMaxRows + 1 rows):
-// one tile of 128 on the M side of its MMAs.
-constexpr int kRowsChainMaxRows = 128;
 
 // Which attention kernel a step takes.
 //   cta     CTAs of 512 tokens, their tiles requested before the dependency wait, clusters beyond: up to 20 rows while the CTAs have
@@ -182,8 +175,7 @@ int enqueue_step(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st,
     return B <= kF16ChainMaxRows ? enqueue_step_f16(m, d, st, chain_head) : enqueue_step_batched_f16(m, d, st, chain_head);
   if (B >= g_tensor_min_batch) return enqueue_step_batched(m, d, st, chain_head);
   if (B >= g_mma_chain_min_batch) return enqueue_step_rows16(m, d, st, chain_head);
-  const int splits = pick_splits(d);
-  const Arena ar = carve(B, m->vocab, splits);
+  const Arena ar = carve(B, m->vocab);
   char* base = static_cast<char*>(d->scratch);
   half* xres[2] = {reinterpret_cast<half*>(base + ar.xres),
                    reinterpret_cast<half*>(base + ar.xres) + (size_t)B * kHidden};
@@ -299,8 +291,7 @@ int enqueue_step(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st,
 // the M side; each kernel writes a finished fp16 tensor (decode_layers_mma.cu).
 int enqueue_step_rows16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
-  const int splits = pick_splits(d);
-  const Arena ar = carve(B, m->vocab, splits);
+  const Arena ar = carve(B, m->vocab);
   char* base = static_cast<char*>(d->scratch);
   half* xa = reinterpret_cast<half*>(base + ar.xres);  // residual stream entering a layer
   half* xb = xa + (size_t)B * kHidden;                  // after the attention block
@@ -389,8 +380,7 @@ int enqueue_attention(const quic_decode_t* d, int ctx, half* qbuf, half* kc, hal
 
 int enqueue_step_batched(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
-  const int splits = pick_splits(d);
-  const Arena ar = carve(B, m->vocab, splits);
+  const Arena ar = carve(B, m->vocab);
   char* base = static_cast<char*>(d->scratch);
   half* h = reinterpret_cast<half*>(base + ar.xres);        // residual stream
   half* qbuf = reinterpret_cast<half*>(base + ar.qbuf);
@@ -479,8 +469,7 @@ LmHeadArgs lm_head_args(const quic_model_t* m, const quic_decode_t* d, const Are
 // 16..128 rows, un-quantised from 3: five launches a layer (rows_chain.cu).
 int enqueue_step_rows(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
-  const int splits = pick_splits(d);
-  const Arena ar = carve(B, m->vocab, splits);
+  const Arena ar = carve(B, m->vocab);
   char* base = static_cast<char*>(d->scratch);
   half* h = reinterpret_cast<half*>(base + ar.xres);  // residual stream
   half* qbuf = reinterpret_cast<half*>(base + ar.qbuf);
@@ -571,8 +560,7 @@ LmHeadArgs lm_head_args(const quic_model_t* m, const quic_decode_t* d, const Are
 // lm_head with the final norm fused.
 int enqueue_step_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
-  const int splits = pick_splits(d);
-  const Arena ar = carve(B, m->vocab, splits);
+  const Arena ar = carve(B, m->vocab);
   char* base = static_cast<char*>(d->scratch);
   half* xa = reinterpret_cast<half*>(base + ar.xres);  // residual stream entering a layer
   half* xb = xa + (size_t)B * kHidden;                  // after the attention block
@@ -611,8 +599,7 @@ int enqueue_step_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t
 // and SwiGLU are the small kernels of the batched W4A16 step.
 int enqueue_step_batched_f16(const quic_model_t* m, const quic_decode_t* d, cudaStream_t st, bool chain_head) {
   const int B = d->batch;
-  const int splits = pick_splits(d);
-  const Arena ar = carve(B, m->vocab, splits);
+  const Arena ar = carve(B, m->vocab);
   char* base = static_cast<char*>(d->scratch);
   half* h = reinterpret_cast<half*>(base + ar.xres);
   half* qbuf = reinterpret_cast<half*>(base + ar.qbuf);
@@ -682,7 +669,7 @@ extern "C" int32_t quic_decode_attention_form(int32_t batch, int32_t ctx) {
 extern "C" int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx) {
   if (batch < 1) batch = 1;
   if (ctx < 1) ctx = 1;
-  // (no step's attention merges splits in global memory any more; the number only sizes the scratch, and callers pass it on)
+  // (no step's attention merges splits in global memory any more: the number is for callers that ask for it)
   if (ctx <= 2048) return (ctx + 63) / 64;
   const int by_len = (ctx + 127) / 128, most = batch >= g_tensor_min_batch ? 1184 / (batch * kKvHeads) : 64;
   const int s = by_len < most ? by_len : most;
@@ -691,7 +678,7 @@ extern "C" int32_t quic_decode_pick_splits(int32_t batch, int32_t ctx) {
 
 extern "C" int64_t quic_decode_scratch_bytes(int32_t batch, int32_t vocab, int32_t attn_splits) {
   if (batch < 1 || vocab < 2 || attn_splits < 1) return 0;
-  return carve(batch, vocab, attn_splits).total;
+  return carve(batch, vocab).total;
 }
 
 extern "C" int32_t quic_decode_launch_count(const quic_model_t* m, const quic_decode_t* d) {

@@ -66,7 +66,7 @@ class SlotCache:
         self.batch_slots: list[int] = []  # slots of the batch rows, for the forward() API
         self._rows: dict[tuple, torch.Tensor] = {}      # row->slot maps by slot tuple (evictable)
         self._row_bufs: dict[int, torch.Tensor] = {}    # per batch size: the buffer captured graphs read
-        self._scratch: dict[tuple, torch.Tensor] = {}
+        self._scratch: dict[int, torch.Tensor] = {}     # decode scratch arena per batch size
         self._graphs: dict[tuple, int] = {}
         self.max_graphs = 512                      # captured graphs kept; beyond that all are dropped and rebuilt
         self._plans: dict[tuple, _DecodePlan] = {}  # decode(): per (rows, steps) launch plan
@@ -99,13 +99,12 @@ class SlotCache:
             self._rows[key] = t
         return t
 
-    def scratch(self, batch: int, splits: int) -> torch.Tensor:
-        key = (batch, splits)
-        t = self._scratch.get(key)
+    def scratch(self, batch: int) -> torch.Tensor:
+        t = self._scratch.get(batch)
         if t is None:
-            need = K.lib().quic_decode_scratch_bytes(batch, self.vocab, splits)
+            need = K.lib().quic_decode_scratch_bytes(batch, self.vocab, 1)
             t = torch.zeros(need, dtype=torch.uint8, device=self.device)
-            self._scratch[key] = t
+            self._scratch[batch] = t
         return t
 
     def error_words(self) -> int:
@@ -371,14 +370,13 @@ class QUICForCausalLM:
                          K.ptr(rows), batch, K.ptr(cache.out_tokens), cache.ring, K.ptr(cache.step_counter),
                          K.ptr(logits), None, 0, ctx)
             return d, rows
-        splits = K.lib().quic_decode_pick_splits(batch, ctx)
         # captured graphs keep this buffer's address: it lives as long as the cache
         rows = cache._row_bufs.get(batch)
         if rows is None:
             rows = cache._row_bufs[batch] = torch.zeros(batch, dtype=torch.int32, device=self.device)
         d = K.Decode(K.ptr(cache.kv), cache.n_slots, cache.s_max, K.ptr(cache.tok), K.ptr(cache.pos),
                      K.ptr(rows), batch, K.ptr(cache.out_tokens), cache.ring, K.ptr(cache.step_counter),
-                     K.ptr(logits), K.ptr(cache.scratch(batch, splits)), splits, ctx)
+                     K.ptr(logits), K.ptr(cache.scratch(batch)), 0, ctx)
         return d, rows
 
     def _graph(self, cache: SlotCache, batch: int, ctx: int, steps: int, logits: torch.Tensor | None):

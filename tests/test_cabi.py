@@ -36,6 +36,10 @@ def test_host_only_queries():
     assert lib.quic_attn_pick_splits(4096, 32768) == 1
     assert lib.quic_attn_scratch_bytes(4, 8) > 4 * 14 * 8 * 64 * 4
     assert lib.quic_decode_scratch_bytes(1, 151936, 4) > 0
+    # what the forms of a batch ask for, whatever the context
+    sizes = [lib.quic_decode_scratch_bytes(b, 151936, 1) for b in (1, 2, 16, 17, 64, 128)]
+    assert sizes == [lib.quic_decode_scratch_bytes(b, 151936, 64) for b in (1, 2, 16, 17, 64, 128)]
+    assert all(lib.quic_decode_scratch_bytes(b, 151936, 1) < b * 40000 + 4096 for b in (17, 64, 128))
     assert lib.quic_w4a16_workspace_bytes(1, 896, 4864) >= 896 * 4
     # fused prefill arena: grows with the rows, holds at least the gate|up activations
     small, big = lib.quic_prefill_scratch_bytes(128, 1, 151936), lib.quic_prefill_scratch_bytes(4096, 8, 151936)
