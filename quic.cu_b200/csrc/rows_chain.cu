@@ -25,8 +25,8 @@
 //     it adds them in the order of K.
 //
 // us per step, this / the GEMM step with norms and split-K sums between (7 or 8 launches a layer): 64 rows of 200..1500 tokens
-// 844 / 911, 17 of 100..300 648 / 721, 48 of 64..200 696 / 768, 100 of 100..300 955 / 1080; un-quantised 17 rows 610 / 930,
-// 40 of 300..1500 761 / 1123, 100 934 / 1355.
+// 834..850 / 911, 17 of 100..300 648..662 / 721, 48 of 64..200 696..710 / 768, 100 of 100..300 955 / 1080; un-quantised 17 rows
+// 610..616 / 930, 40 of 300..1500 761..766 / 1123, 100 935 / 1355.
 //
 // Every mbarrier wait is bounded.  A role whose wait gives up says so to the CTA's others (fail_s) and goes on to the end; the CTA
 // records a code, takes part in the cluster's barriers, waits for its own copies and MMAs in flight, frees its tensor memory and
@@ -585,11 +585,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
-  if (fail_s != 0) {
-    if (tid == 0) tc_report(a.status, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
-    drain_failed(issuer, smem_u32(&bar_drain));
+  if (warp == kWarpsC + 1) {  // (the issuer's warp: the CTA's memory stays until it has left, whenever the others do)
+    if (fail_s != 0) {
+      if (lane == 0) tc_report(a.status, (fail_s << 16) | 0x2000 | (int)(blockIdx.x & 0x1fff));
+      drain_failed_warp(issuer, smem_u32(&bar_drain));
+    }
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(C::cols) : "memory");
   }
-  if (warp == kWarpsC + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(C::cols) : "memory");
 }
 
 // x[b] = embed[token of row b] and the row's sum of squares.

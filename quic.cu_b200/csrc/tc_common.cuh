@@ -199,7 +199,7 @@ __device__ __forceinline__ void tc_report(int* status, int code) {
 // and its tensor memory.  All threads, after the barrier that every role has reached; `issuer`: the thread that issued
 // the MMAs; `bar`: a barrier for one arrival, not in use.  The MMAs are waited for; a copy, which waits for nothing, lands within
 // microseconds of its request and is given a millisecond.
-__device__ __forceinline__ void drain_failed(bool issuer, uint32_t bar) {
+__device__ __forceinline__ void drain_failed_warp(bool issuer, uint32_t bar) {  // (where one warp issues and frees)
   if (issuer) {
     umma_commit(bar);
     mbar_wait(bar, 0);
@@ -208,6 +208,9 @@ __device__ __forceinline__ void drain_failed(bool issuer, uint32_t bar) {
   }
   __syncwarp();
   tc_fence_before();
+}
+__device__ __forceinline__ void drain_failed(bool issuer, uint32_t bar) {
+  drain_failed_warp(issuer, bar);
   __syncthreads();
   tc_fence_after();
 }
