@@ -52,6 +52,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ void pair_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pair_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void pair_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -145,6 +147,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   const int ntiles = a.n / NT, flat = ntiles * ((a.m_total + 255) / 256), tiles = flat * a.splits, kblocks = a.k / kBlockK;
   const int first = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
+  pair_arrive();
   if (tid == 0) {
     tma_prefetch_desc(&tm_x);
     tma_prefetch_desc(&tm_w);
@@ -165,7 +168,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   // allocates, and neither leaves before both have given back: the next CTA on its SM, of another kernel and stream, may
   // allocate by itself at once.  (Without, a pair beside decode steps on another stream stood still for good: the first CTA's
   // allocation had returned, the second's never did.)
-  pair_sync();
+  pair_wait();
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base_s)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
