@@ -225,7 +225,8 @@ int launch_attn_flow(const AttnArgs& a, int batch, int* status, cudaStream_t str
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   // Only where two CTAs share an SM anyway: the CTAs of the next call find room beside those of this one, and where each
-  // was to have an SM to itself some then share one (16 x 8192 16.4 -> 14.9 us a call, 9 x 8252 11.2 -> 11.8).
+  // was to have an SM to itself some then share one (16 x 8192 16.4 -> 14.9 us a call, 9 x 8252 11.2 -> 11.8).  What it hides is
+  // the set-up, and only behind a kernel that triggers early, one of this library's: those times are of calls in a row.
   cfg.numAttrs = pdl_enabled() && (n_slots > 0 || kKvHeads * batch * a.splits > 148) ? 2 : 1;
   QUIC_CUDA(cudaLaunchKernelEx(&cfg, attn_decode_flow_kernel, tm_k, tm_v, a, status));
   return QUIC_OK;

@@ -17,8 +17,8 @@
 // tiles that hold only tokens of earlier steps (up to the ring's depth): those rows are complete
 // once the step counter shows the current step.  The counter is read (acquire) before the
 // requests and again after the wait; if it moved, the previous step was still finishing when
-// the tiles were requested, and they are requested again (a second phase of the same stages'
-// barriers, which their consumers then wait for).  The tile of the row that the preceding
+// the tiles were requested, and they are requested again (early requests have barriers of their
+// own; the repeated ones complete on those of all other tiles, which their consumers then wait for).  The tile of the row that the preceding
 // kernel appends is never requested early.
 //
 // With `fin.part` (or `fin.qkv`, a finished fp16 output) set the CTA first finishes the fused QKV linear for its row and KV head, which a

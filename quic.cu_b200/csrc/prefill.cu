@@ -14,8 +14,9 @@ namespace {
 // 1 x 200 1768 -> 1747, 1 x 500 2426 -> 2041, 2 x 1024 5826 -> 3196.
 constexpr int kPairRows = 768, kDensePairRows = 192;
 // Rows up to which a layer runs on the chain of rows_chain.cu: one tile of 128 rows of packed weights (us, GEMMs / chain: 2 rows
-// 816 / 772, 40 948 / 802, 87 1146 / 958, 128 1168 / 1041, 129 1402 / 1419, 256 1432 / 1573), which it unpacks again for every
-// tile; un-quantised ones it reads again (40 1142 / 739, 128 1550 / 1047, 256 1687 / 1461, 300 1927 / 1728, 384 1903 / 1902).
+// 746 / 708, 40 867 / 747, 87 1069 / 913, 128 1116 / 1004, 129 1347 / 1370, 256 1358 / 1508), which it unpacks again for every
+// tile; un-quantised ones it reads again (40 1079 / 696, 128 1424 / 979, 256 1685 / 1413, 300 1913 / 1678; the line was drawn at
+// 1903 / 1902 for 384 rows, which are 1909 / 1786 now).
 constexpr int kRowsChain = 128, kDenseRowsChain = 320;
 constexpr int64_t kLayerWeights = (int64_t)(kQkvN + kHidden + 2 * kInter) * kHidden + (int64_t)kHidden * kInter;
 
