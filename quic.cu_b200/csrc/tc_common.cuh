@@ -28,6 +28,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
+// A probe that may sleep for 20 us: fewer of them beside the CTA's other roles (prefill of 16 x 2048 tokens 30.35 -> 30.13 ms).
+__device__ __forceinline__ bool mbar_try_long(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity), "r"(20000u)
+      : "memory");
+  return done != 0;
+}
 // Time in units of 1.024 us.
 __device__ __forceinline__ uint32_t clock_us() {
   uint64_t t;
@@ -35,12 +47,13 @@ __device__ __forceinline__ uint32_t clock_us() {
   return (uint32_t)(t >> 10);
 }
 // Bounded wait for the phase with the given parity; false after `limit_us`.  A probe sleeps until the phase is complete
-// or 4 us are over, so the clock is read only by a wait that is late already.  (A limit in probes, 2^22, was 16.6 s.)
+// or some us are over; the clock is read by a wait whose first probe has failed.  (A limit in probes is none: 2^22 of them were
+// 16.6 s where nothing came, and with a limit of probes of 4 us each the tests of late stages failed.)
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit_us = kWaitLimitUs) {
   bool done = mbar_try(bar, parity);
   if (!done) {
     const uint32_t t0 = clock_us();
-    do done = mbar_try(bar, parity);
+    do done = mbar_try_long(bar, parity);
     while (!done && clock_us() - t0 < limit_us);
   }
   return done;
@@ -50,7 +63,7 @@ __device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, 
   bool done = mbar_try(bar, parity);
   if (!done) {
     const uint32_t t0 = clock_us();
-    do done = mbar_try(bar, parity);
+    do done = mbar_try_long(bar, parity);
     while (!done && *given_up == 0 && clock_us() - t0 < limit_us);
   }
   return done;
